@@ -145,15 +145,26 @@ struct AdjPlan {
   }
 };
 
+// Launch size class of the tuner: the power of two below the number of work items (32-instance
+// tiles, times directions in the derivative sweeps). One class for everything up to 16 tiles per
+// SM kept the variant that a first call of 4 tiles chose for launches of 2000: the cart-pole step
+// at 65536 instances ran the cooperative sweep a 100-instance call had picked, 129 us against 69.
+constexpr int kSizeClasses = 32;
+int size_class(long long items) {
+  int c = 0;
+  while (c + 1 < kSizeClasses && (items >> (c + 1)) > 0) ++c;
+  return c;
+}
+
 struct Tape {
   int device = 0;
   int n_instr = 0, n_in = 0, n_out = 0, sz_w = 0, n_partials = 0, n_chunks = 0;
   int ref_sz_w = 0;  // the work-vector length the tape came with (sz_w: after scheduling)
   int residence = 0;  // work vector: 0 auto (shared memory when it fits, value sweeps tuned),
                       // 1 global memory, 2 shared memory whenever it fits
-  // per PrimalKind and launch size class (0: at most 16 tiles per SM): 0 shared, 1 global,
-  // 2 cooperative level sweep (autotuned)
-  std::atomic<int> primal_tuned[5][2];
+  // per PrimalKind and launch size class (size_class of the tiles): 0 shared, 1 global,
+  // 2 and up cooperative level sweep (autotuned)
+  std::atomic<int> primal_tuned[5][kSizeClasses];
   // level schedule of the cooperative value/record sweeps, built on first use
   int lv_state = 0;  // 0 not built, 1 built, -1 unavailable
   u64* d_lcode = nullptr;
@@ -185,13 +196,15 @@ struct Tape {
   int primal_block = 128, primal_grid_cap = 1;
   std::mutex shape_mtx;
   // derivative-sweep variant per kind (seeded/identity tangent, adjoint) and launch size class
-  // (0: at most 16 tiles per SM); tangent kinds may keep the cooperative sweep (TV_COUNT)
-  std::atomic<int> tuned[3][2];
+  // (size_class of tiles x directions); tangent kinds may keep the cooperative sweep (TV_COUNT)
+  std::atomic<int> tuned[3][kSizeClasses];
   // one thread tunes a tape at a time; others meanwhile run the untuned defaults
   std::mutex tune_mtx;
   Tape() {
-    for (auto& k : primal_tuned) k[0] = k[1] = -1;
-    for (auto& k : tuned) k[0] = k[1] = -1;
+    for (auto& k : primal_tuned)
+      for (auto& c : k) c = -1;
+    for (auto& k : tuned)
+      for (auto& c : k) c = -1;
   }
   std::vector<double> h_consts;  // constant pool (host copy, for inlining into callers)
   std::vector<u64> h_code;                            // padded instruction stream
@@ -1156,17 +1169,26 @@ const AdjPlan* adj_plan(Tape& t, int dw, int ch, const std::vector<char>& seeded
   return t.adj_plans.back().get();
 }
 
-// Runs `fn` (launches on stream s) once between two events and waits for it.
+// Device time of `fn` (launches on stream s): one run to load the kernel and warm the caches,
+// then the fastest of three timed ones (of one when it takes over half a millisecond; a run
+// that takes 50 us when warm takes several times that when its kernel is loaded first). With
+// `warm` false, one timed run only.
 template <class F>
-int time_once(cudaStream_t s, F fn, float* ms) {
+int time_runs(cudaStream_t s, F fn, float* ms, bool warm = true) {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   cudaError_t e = cudaEventCreate(&e0);
   if (e == cudaSuccess) e = cudaEventCreate(&e1);
-  if (e == cudaSuccess) e = cudaEventRecord(e0, s);
-  if (e == cudaSuccess) e = fn();
-  if (e == cudaSuccess) e = cudaEventRecord(e1, s);
-  if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-  if (e == cudaSuccess) e = cudaEventElapsedTime(ms, e0, e1);
+  if (warm && e == cudaSuccess) e = fn();
+  for (int r = 0; r < (warm ? 3 : 1) && e == cudaSuccess; ++r) {
+    float t = 0;
+    e = cudaEventRecord(e0, s);
+    if (e == cudaSuccess) e = fn();
+    if (e == cudaSuccess) e = cudaEventRecord(e1, s);
+    if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+    if (e == cudaSuccess) e = cudaEventElapsedTime(&t, e0, e1);
+    *ms = r == 0 ? t : std::min(*ms, t);
+    if (*ms > 0.5f) break;
+  }
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
   return e == cudaSuccess ? 0 : cuda_fail(e, "autotune timing");
@@ -1234,7 +1256,18 @@ bool ensure_levels(Tape& t, bool reverse = false) {
 }
 
 void reset_primal_tuning(Tape& t) {
-  for (auto& k : t.primal_tuned) k[0] = k[1] = -1;
+  for (auto& k : t.primal_tuned)
+    for (auto& c : k) c = -1;
+}
+
+// The kept choice of class c, or of the nearest tuned class (calls that cannot tune: under
+// capture, or while another thread tunes the tape); -1: none.
+int kept_choice(const std::atomic<int> (&row)[kSizeClasses], int c) {
+  for (int d = 0; d < kSizeClasses; ++d) {
+    if (c - d >= 0 && row[c - d] >= 0) return row[c - d];
+    if (c + d < kSizeClasses && row[c + d] >= 0) return row[c + d];
+  }
+  return -1;
 }
 
 int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStream_t s) {
@@ -1305,10 +1338,11 @@ int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStrea
   };
   const bool coop_kind = kind == PK_EVAL || kind == PK_RECORD || sp_kind;
   const bool rev = kind == PK_SP_REVERSE;
-  const int cls = (m + 31) / 32 <= 16ll * sm_count() ? 0 : 1;
+  const int cls = size_class((m + 31) / 32);
+  const bool few = (m + 31) / 32 <= 16ll * sm_count();
   // the cooperative sweep is a candidate for launches of few tiles (or when forced); the
   // sparsity sweeps' version needs its schedule's work vector in shared memory
-  const bool want_coop = coop_kind && (cls == 0 || t.residence == 3);
+  const bool want_coop = coop_kind && (few || t.residence == 3);
   bool can_coop = want_coop && (capturing(s) ? (rev ? t.rlv_state : t.lv_state) > 0
                                              : ensure_levels(t, rev));
   if (can_coop && sp_kind)
@@ -1317,20 +1351,20 @@ int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStrea
                                          ? 2 : coop_threads_for((m + 31) / 32) == 512 ? 1 : 0);
   if (t.residence == 3 && coop_kind && can_coop) return run(coop_default, true);
   if (t.residence == 1 || !fits_smem(t.sz_w)) {
-    if (!(coop_kind && can_coop && cls == 0 && t.residence != 1)) return run(M_GLOBAL, true);
+    if (!(coop_kind && can_coop && few && t.residence != 1)) return run(M_GLOBAL, true);
   } else if (t.residence == 2) {
     return run(M_SHARED, true);
   }
   int cand[5], nc = 0;
   if (fits_smem(t.sz_w)) cand[nc++] = M_SHARED;
   cand[nc++] = M_GLOBAL;
-  if (coop_kind && can_coop && (cls == 0 || t.residence == 3))
+  if (coop_kind && can_coop && (few || t.residence == 3))
     for (int c = M_COOP; c <= M_COOP_LAST; ++c) cand[nc++] = c;
   std::atomic<int>& choice = t.primal_tuned[kind][cls];
   // sp_reverse consumes its seeds and cannot be timed twice: it follows sp_forward's choice
   if (rev && choice < 0 && t.primal_tuned[PK_SP_FORWARD][cls] >= 0)
     choice = t.primal_tuned[PK_SP_FORWARD][cls].load();
-  // residence is tuned like the derivative variants: every candidate timed once on the first
+  // residence is tuned like the derivative variants: every candidate timed on the first
   // call of each kind and size class (every sweep here but sp_reverse, which consumes its
   // seeds, can run twice with the same results)
   std::unique_lock<std::mutex> tune_lock(t.tune_mtx, std::defer_lock);
@@ -1339,7 +1373,7 @@ int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStrea
     float ms[5] = {0, 0, 0, 0, 0};
     for (int c = 0; c < nc; ++c) {
       int rc = 0;
-      if (int trc = time_once(s, [&] { rc = run(cand[c], false); return cudaSuccess; }, &ms[c]))
+      if (int trc = time_runs(s, [&] { rc = run(cand[c], false); return cudaSuccess; }, &ms[c]))
         return trc;
       if (rc) return rc;
     }
@@ -1349,7 +1383,7 @@ int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStrea
     choice = cand[best];
     return 0;  // every run produced the same (complete) results
   }
-  const int chosen = choice;
+  const int chosen = kept_choice(t.primal_tuned[kind], cls);
   if (chosen >= 0 && (chosen < M_COOP || can_coop) && (chosen != M_SHARED || fits_smem(t.sz_w)))
     return run(chosen, true);
   return run(cand[0], true);
@@ -1465,11 +1499,12 @@ int run_deriv(Tape& t, SweepArgs a, long long m, const DerivReq& rq, cudaStream_
     return launch_tangent_queued(a, grid, grid < work_of(v), v, s);
   };
   const long long work = tiles * ndir;
-  const int cls = tiles <= 16ll * sms ? 0 : 1;
+  const int cls = size_class(work);
+  const bool few = tiles <= 16ll * sms;
   // the cooperative tangent sweep: a candidate for launches of few tiles whose level schedule
   // (tangents + activity bytes) fits shared memory
   const bool coop_ok =
-      cls == 0 &&
+      few &&
       (capturing(s) ? (adjoint ? t.rlv_state : t.lv_state) > 0 : ensure_levels(t, adjoint)) &&
       smem_tangent_coop(adjoint ? t.rlv_sz_w : t.lv_sz_w, false) <=
           static_cast<size_t>(max_smem_optin());
@@ -1561,11 +1596,12 @@ int run_deriv(Tape& t, SweepArgs a, long long m, const DerivReq& rq, cudaStream_
   std::atomic<int>& kept = t.tuned[kind][cls];
   int variant = kept;
   if (variant >= 0 && !usable(variant)) variant = -1;
-  if (variant < 0) {
+  bool tuned_here = variant >= 0;
+  if (!tuned_here) {
     // tune outside capture: on waves that fill the GPU at least twice at 8 warps per SM, and
     // on every small launch, where the cooperative sweep is a candidate too
     std::unique_lock<std::mutex> tune_lock(t.tune_mtx, std::defer_lock);
-    if (g_autotune && !capturing(s) && (work >= 2ll * sms * 8 || cls == 0) &&
+    if (g_autotune && !capturing(s) && (work >= 2ll * sms * 8 || few) &&
         tune_lock.try_lock()) {
       float best = 0;
       for (int c = 0; c <= n_variants + (adjoint ? 0 : 1); ++c) {
@@ -1573,7 +1609,7 @@ int run_deriv(Tape& t, SweepArgs a, long long m, const DerivReq& rq, cudaStream_
         const int v = c < n_variants ? c : (c == n_variants ? kCoop : kWin);
         if (!usable(v)) continue;
         float ms = 0;
-        if (int rc = time_once(s, [&] { return run_v(v); }, &ms)) return plan_err ? plan_err : rc;
+        if (int rc = time_runs(s, [&] { return run_v(v); }, &ms)) return plan_err ? plan_err : rc;
         if (variant < 0 || ms < best) {
           best = ms;
           variant = v;
@@ -1582,9 +1618,14 @@ int run_deriv(Tape& t, SweepArgs a, long long m, const DerivReq& rq, cudaStream_
       kept = variant;
       return 0;  // every variant's run produced this wave's (identical) results
     }
-    variant = 0;  // the first variant of each list: fastest on the tapes measured
-    while (variant < n_variants && !fits(variant)) ++variant;
-    if (variant == n_variants)
+    // the nearest class's choice, else the first variant of each list: fastest on the tapes
+    // measured
+    variant = kept_choice(t.tuned[kind], cls);
+    if (variant < 0 || !usable(variant)) {
+      variant = 0;
+      while (variant < n_variants && !fits(variant)) ++variant;
+    }
+    if (variant == n_variants && !usable(variant))
       return fail(CASADI_GB300_ERR_UNSUPPORTED, "no derivative-sweep variant fits");
   }
   cudaError_t e = timed(adjoint ? F_ADJOINT : F_TANGENT, s, [&] { return run_v(variant); });
@@ -2514,7 +2555,7 @@ int casadi_gb300_tuned_variant(int id, int kind, int* variant) {
   Tape* t = get_tape(id);
   if (!t) return fail(CASADI_GB300_ERR_ID, "no tape with id %d", id);
   if (kind < 0 || kind > 2 || !variant) return fail(CASADI_GB300_ERR_ARG, "bad arguments");
-  *variant = t->tuned[kind][1] >= 0 ? t->tuned[kind][1] : t->tuned[kind][0];
+  *variant = kept_choice(t->tuned[kind], kSizeClasses - 1);  // the largest launches' choice
   return 0;
 }
 
@@ -2532,7 +2573,7 @@ int casadi_gb300_set_variant(int id, int kind, int variant) {
   if (!t) return fail(CASADI_GB300_ERR_ID, "no tape with id %d", id);
   if (kind < 0 || kind > 2 || variant < -1 || variant > (kind == 2 ? AV_COUNT : TV_COUNT + 1))
     return fail(CASADI_GB300_ERR_ARG, "bad arguments");
-  t->tuned[kind][0] = t->tuned[kind][1] = variant;
+  for (auto& c : t->tuned[kind]) c = variant;
   return 0;
 }
 

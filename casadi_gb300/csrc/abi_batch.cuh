@@ -404,10 +404,10 @@ int casadi_gb300_batch_run(int batch, void* scratch, size_t scratch_bytes, int u
           continue;
         }
         int rc = 0;
-        if (int trc = time_once(b->stream, [&] {
+        if (int trc = time_runs(b->stream, [&] {
               rc = batch_enqueue(*b, scratch, b->stream, gw == 1);
               return cudaSuccess;
-            }, &ms[gw]))
+            }, &ms[gw], false))
           return trc;
         if (rc) return rc;
       }

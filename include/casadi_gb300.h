@@ -394,13 +394,15 @@ CASADI_GB300_API int casadi_gb300_map_jacobian_reverse(int id, int mem, int64_t 
                            int nadj, const double* const* aseed, double* const* asens);
 
 /* Autotuning of the derivative sweeps (on by default): the first call of each kind
- * (0 seeded forward, 1 Jacobian, 2 adjoint) and launch size (at most 16 tiles per SM, or more)
- * on a tape runs each kernel variant once on that wave (large launches: those that fill the
- * GPU several times; small launches also try the cooperative level sweep), keeps the fastest
- * for the tape and synchronizes the stream once; it is skipped while the stream is being
- * captured into a CUDA graph.
+ * (0 seeded forward, 1 Jacobian, 2 adjoint) and launch size (powers of two of the work items:
+ * 32-instance tiles times directions) on a tape times each kernel variant warm on that wave
+ * (large launches: those that fill the GPU several times; small launches also try the
+ * cooperative level sweep), keeps the fastest for the tape and synchronizes the stream; it is
+ * skipped while the stream is being captured into a CUDA graph, where the choice of the nearest
+ * tuned size runs.
  * Variants differ only in speed: every variant does the same arithmetic in the same order.
- * casadi_gb300_tuned_variant reports the kept variant (-1: not tuned yet). No counterpart in
+ * casadi_gb300_tuned_variant reports the kept variant of the largest tuned size (-1: not tuned
+ * yet). No counterpart in
  * the reference, whose Map has one code path per parallelization (casadi/core/map.cpp:39-51). */
 CASADI_GB300_API int casadi_gb300_autotune(int enable);
 CASADI_GB300_API int casadi_gb300_tuned_variant(int id, int kind, int* variant);
