@@ -168,6 +168,9 @@ struct Tape {
   // level schedule of the cooperative value/record sweeps, built on first use
   int lv_state = 0;  // 0 not built, 1 built, -1 unavailable
   u64* d_lcode = nullptr;
+  // the value entries of the level schedule, one stream per warp of a 4 << k warp team
+  uint4* d_team[kTeamSizes] = {};
+  int2* d_team_at[kTeamSizes] = {};  // per warp: first entry, blocks
   int* d_lbegin = nullptr;
   int* d_lpidx = nullptr;
   int n_levels = 0, lv_sz_w = 0;
@@ -188,6 +191,8 @@ struct Tape {
   std::vector<int2> absent_in;
   std::vector<int> pofs;    // partials recorded before instruction k*kPofsGran
   u64* d_code = nullptr;
+  uint4* d_ventries = nullptr;  // value entries of the scheduled order
+  int n_vblocks = 0;
   int* d_pofs = nullptr;
   double* d_consts = nullptr;
   int2* d_absent = nullptr;
@@ -227,6 +232,11 @@ struct Tape {
     adj_plans.clear();
     seg.clear();
     cudaFree(d_code);
+    cudaFree(d_ventries);
+    for (int k = 0; k < kTeamSizes; ++k) {
+      cudaFree(d_team[k]);
+      cudaFree(d_team_at[k]);
+    }
     cudaFree(d_pofs);
     cudaFree(d_consts);
     cudaFree(d_absent);
@@ -246,6 +256,8 @@ struct Tape {
   TapeView view() const {
     TapeView v;
     v.code = d_code;
+    v.ventries = d_ventries;
+    v.n_vblocks = n_vblocks;
     v.pofs = d_pofs;
     v.consts = d_consts;
     v.absent_in = d_absent;
@@ -378,7 +390,8 @@ int sm_count() {
   return n;
 }
 
-// Pick the CTA shapes that keep the most threads resident given the shared-memory footprint.
+// Pick the CTA shape of the sparsity sweeps that keeps the most threads resident given the
+// shared-memory footprint.
 void choose_shapes(Tape& t) {
   const int max_smem = max_smem_optin();
   const int sms = sm_count();
@@ -386,7 +399,7 @@ void choose_shapes(Tape& t) {
   for (int bs : {256, 128, 64, 32}) {
     const size_t sm = smem_primal(t.sz_w, bs);
     if (sm > static_cast<size_t>(max_smem)) continue;
-    const int occ = occupancy_primal(bs, sm);
+    const int occ = occupancy_sp(bs, sm);
     if (occ * bs > best_threads) {
       best_threads = occ * bs;
       t.primal_block = bs;
@@ -499,6 +512,15 @@ SweepArgs base_args(const Tape& t, long long n, long long i_begin) {
   a.n_in = t.n_in;
   a.n_out = t.n_out;
   return a;
+}
+
+constexpr int kMaxGrid = 1 << 30;
+
+// Pads an entry stream to whole blocks (at least one); returns their number.
+int pad_block(std::vector<uint4>& v, size_t first = 0) {
+  const size_t n = std::max<size_t>(1, (v.size() - first + kEntBlock - 1) / kEntBlock);
+  v.resize(first + n * kEntBlock, make_uint4(0, 0, 0, D_NOP));
+  return static_cast<int>(n);
 }
 
 int grid_for(long long tiles, int cap) {
@@ -1203,23 +1225,71 @@ enum PrimalKind { PK_EVAL = 0, PK_RECORD, PK_SP_FORWARD, PK_SP_REVERSE, PK_ACTIV
 // Level schedule of the cooperative sweeps (host scheduling + upload, once per tape). Returns
 // whether it is available; never called while the stream is being captured.
 constexpr int kLevelWidth = 64;      // instructions per level
-// CTA size of the cooperative value/record/sparsity sweeps: 256, 512 or 1024 threads (tuned);
-// without tuning, enough warps per tile that the tiles of the launch fill the GPU
+
+// Entry streams of a `warps`-warp team over the level schedule; at: per warp the first entry and
+// the blocks. The costs (latencies in dependent FP64 operations of about 150 cycles, dispatch
+// and work-vector accesses included) balance the warps: a sincos takes 820 cycles, a recorded
+// division 700, a first read of an input a trip to L2 or HBM.
+void team_entries(const Levels& lv, int warps, const std::vector<double>& consts,
+                  std::vector<uint4>& entries, std::vector<int2>& at) {
+  float cost[64];
+  for (float& c : cost) c = 1.0f;
+  cost[D_CONST] = 0.5f;
+  cost[D_INPUT] = cost[D_DIV] = cost[D_LOG] = cost[D_TANH] = cost[D_SQRT] = 4.0f;
+  cost[D_SIN] = cost[D_COS] = 5.0f;
+  cost[D_EXP] = 3.5f;
+  cost[D_INV] = 2.0f;
+  for (unsigned op : {D_POW, D_CONSTPOW, D_TAN, D_ASIN, D_ACOS, D_ATAN, D_ERF, D_SINH, D_COSH,
+                      D_ASINH, D_ACOSH, D_ATANH, D_ATAN2, D_ERFINV, D_LOG1P, D_EXPM1, D_HYPOT,
+                      D_FMOD, D_REMAINDER})
+    cost[op] = 10.0f;
+  for (const std::vector<int>& warp : team_streams(lv, warps, cost)) {
+    const size_t first = entries.size();
+    bool open = false;  // the last entry carries no meeting yet
+    for (int k : warp) {
+      if (k == kTeamBarrier) {
+        if (!open) entries.push_back(make_uint4(0, 0, 0, D_NOP));
+        entries.back().w |= kTeamMeet;
+        open = false;
+        continue;
+      }
+      uint4 e = value_entry_of(lv.code[k], consts.data());
+      e.w |= (static_cast<unsigned>(lv.pidx[k]) & kTeamPidxMask) << kTeamPidxShift;
+      entries.push_back(e);
+      open = true;
+    }
+    at.push_back(make_int2(static_cast<int>(first), pad_block(entries, first)));
+  }
+}
+
+// The team streams of a.block / 32 warps into a launch's arguments.
+void set_team(SweepArgs& a, const Tape& t) {
+  int k = 0;
+  while (k + 1 < kTeamSizes && (128 << k) < a.block) ++k;
+  a.dstream = t.d_team[k];
+  a.dchunks = t.d_team_at[k];
+}
+
+// CTA size of the cooperative value/record/sparsity sweeps: 128, 256, 512 or 1024 threads
+// (tuned); without tuning, enough warps per tile that the tiles of the launch fill the GPU
 int coop_threads_for(long long tiles) {
   const long long want = static_cast<long long>(sm_count()) * 32 / std::max(1ll, tiles);
-  return want >= 32 ? 1024 : (want >= 16 ? 512 : 256);
+  return want >= 32 ? 1024 : (want >= 16 ? 512 : (want >= 8 ? 256 : 128));
 }
 bool ensure_levels(Tape& t, bool reverse = false) {
   std::lock_guard<std::mutex> lk(t.shape_mtx);
   int& state = reverse ? t.rlv_state : t.lv_state;
   if (state != 0) return state > 0;
   state = -1;
+  if (static_cast<unsigned>(t.n_partials) > kTeamPidxMask) return false;  // not addressed
   Levels lv;
   std::string err;
   const int cap = t.sz_w <= 400 ? 400 : t.sz_w + kLevelWidth;
   const int nl = level_schedule(t.h_code, kLevelWidth, cap, lv, err, reverse);
   if (nl <= 0 || lv.code.empty()) return false;
   u64* code = nullptr;
+  uint4* team[kTeamSizes] = {};
+  int2* team_at[kTeamSizes] = {};
   int *begin = nullptr, *pidx = nullptr;
   bool ok = cudaMalloc(&code, lv.code.size() * sizeof(u64)) == cudaSuccess &&
             cudaMalloc(&begin, lv.begin.size() * sizeof(int)) == cudaSuccess &&
@@ -1231,8 +1301,18 @@ bool ensure_levels(Tape& t, bool reverse = false) {
                   cudaMemcpyHostToDevice) == cudaSuccess &&
        cudaMemcpy(pidx, lv.pidx.data(), lv.pidx.size() * sizeof(int), cudaMemcpyHostToDevice) ==
            cudaSuccess;
+  for (int k = 0; k < kTeamSizes && ok && !reverse; ++k) {
+    std::vector<uint4> entries;
+    std::vector<int2> at;
+    team_entries(lv, 4 << k, t.h_consts, entries, at);
+    ok = upload(&team[k], entries) == cudaSuccess && upload(&team_at[k], at) == cudaSuccess;
+  }
   if (!ok) {
     cudaFree(code);
+    for (int k = 0; k < kTeamSizes; ++k) {
+      cudaFree(team[k]);
+      cudaFree(team_at[k]);
+    }
     cudaFree(begin);
     cudaFree(pidx);
     cudaGetLastError();
@@ -1246,6 +1326,10 @@ bool ensure_levels(Tape& t, bool reverse = false) {
     t.rlv_sz_w = lv.sz_w;
   } else {
     t.d_lcode = code;
+    for (int k = 0; k < kTeamSizes; ++k) {
+      t.d_team[k] = team[k];
+      t.d_team_at[k] = team_at[k];
+    }
     t.d_lbegin = begin;
     t.d_lpidx = pidx;
     t.n_levels = nl;
@@ -1274,9 +1358,9 @@ int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStrea
   static const int fam[] = {F_EVAL, F_RECORD, F_SP_FORWARD, F_SP_REVERSE, F_ACTIVITY};
   static const char* what[] = {"eval launch", "record sweep launch", "sp_forward launch",
                                "sp_reverse launch", "activity launch"};
-  // modes: shared, global, cooperative with 256, 512 or 1024 threads per CTA
-  enum { M_SHARED = 0, M_GLOBAL = 1, M_COOP = 2, M_COOP_LAST = 4 };
-  auto coop_threads = [](int mode) { return 256 << (mode - M_COOP); };
+  // modes: shared, global, cooperative with 128, 256, 512 or 1024 threads per CTA
+  enum { M_SHARED = 0, M_GLOBAL = 1, M_COOP = 2, M_COOP_LAST = M_COOP + kTeamSizes - 1 };
+  auto coop_threads = [](int mode) { return 128 << (mode - M_COOP); };
   const bool sp_kind = kind == PK_SP_FORWARD || kind == PK_SP_REVERSE;
   auto go = [&](int grid) {
     switch (kind) {
@@ -1300,23 +1384,29 @@ int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStrea
     } else if (mode >= M_COOP) {
       a.block = coop_threads(mode);
       a.t = t.view();
-      const size_t sm = smem_coop(t.lv_sz_w);
-      global = sm > static_cast<size_t>(max_smem_optin());
+      set_team(a, t);
+      global = smem_team(t.lv_sz_w, a.block, false) > static_cast<size_t>(max_smem_optin());
+      const size_t sm = smem_team(t.lv_sz_w, a.block, global);
       const int occ = std::max(1, occupancy_coop(a.block, sm, global));
       grid = grid_for((m + 31) / 32, occ * sm_count());
       a.wglob = nullptr;
       if (global)
         if (int rc = gw_prepare(t, a, &grid, static_cast<size_t>(t.lv_sz_w) * 32 * 8, s)) return rc;
     } else if (global) {
-      a.block = kGwBlock;
+      // value and record sweeps run one-warp CTAs, the sparsity sweeps kGwBlock threads
+      const bool value = kind == PK_EVAL || kind == PK_RECORD;
+      a.block = value ? 32 : kGwBlock;
       const int occ =
-          std::max(1, kind >= PK_SP_FORWARD ? occupancy_gw_sp()
-                                            : occupancy_gw_primal(kind == PK_RECORD));
-      grid = grid_for((m + kGwBlock - 1) / kGwBlock, occ * sm_count());
+          std::max(1, value ? occupancy_gw_value(kind == PK_RECORD) : occupancy_gw_sp());
+      grid = grid_for((m + a.block - 1) / a.block, occ * sm_count());
       const size_t elem = 8;  // a double or a bvec_t per slot and instance
       if (int rc = gw_prepare(t, a, &grid,
-                              static_cast<size_t>(std::max(1, t.sz_w)) * kGwBlock * elem, s))
+                              static_cast<size_t>(std::max(1, t.sz_w)) * a.block * elem, s))
         return rc;
+    } else if (kind == PK_EVAL || kind == PK_RECORD) {
+      a.block = 32;
+      a.wglob = nullptr;
+      grid = grid_for((m + 31) / 32, kMaxGrid);  // a CTA per tile
     } else {
       a.block = t.primal_block;
       a.wglob = nullptr;
@@ -1347,15 +1437,15 @@ int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStrea
                                              : ensure_levels(t, rev));
   if (can_coop && sp_kind)
     can_coop = smem_coop(rev ? t.rlv_sz_w : t.lv_sz_w) <= static_cast<size_t>(max_smem_optin());
-  const int coop_default = M_COOP + (coop_threads_for((m + 31) / 32) == 1024
-                                         ? 2 : coop_threads_for((m + 31) / 32) == 512 ? 1 : 0);
+  int coop_default = M_COOP;
+  while (coop_threads(coop_default) < coop_threads_for((m + 31) / 32)) ++coop_default;
   if (t.residence == 3 && coop_kind && can_coop) return run(coop_default, true);
   if (t.residence == 1 || !fits_smem(t.sz_w)) {
     if (!(coop_kind && can_coop && few && t.residence != 1)) return run(M_GLOBAL, true);
   } else if (t.residence == 2) {
     return run(M_SHARED, true);
   }
-  int cand[5], nc = 0;
+  int cand[2 + kTeamSizes], nc = 0;
   if (fits_smem(t.sz_w)) cand[nc++] = M_SHARED;
   cand[nc++] = M_GLOBAL;
   if (coop_kind && can_coop && (few || t.residence == 3))
@@ -1370,7 +1460,7 @@ int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStrea
   std::unique_lock<std::mutex> tune_lock(t.tune_mtx, std::defer_lock);
   if (choice < 0 && nc > 1 && g_autotune && kind != PK_SP_REVERSE && !capturing(s) &&
       tune_lock.try_lock()) {
-    float ms[5] = {0, 0, 0, 0, 0};
+    float ms[2 + kTeamSizes] = {};
     for (int c = 0; c < nc; ++c) {
       int rc = 0;
       if (int trc = time_runs(s, [&] { rc = run(cand[c], false); return cudaSuccess; }, &ms[c]))
@@ -1792,18 +1882,16 @@ int encode_tape(const casadi_gb300_atomic* alg, int n_instr, int n_in, const int
   return 0;
 }
 
-// Sine/cosine pairs. The record sweeps compute sin and cos of the operand together for either
-// op (one is the value, the other its partial), so a SIN or COS whose operand is the value the
-// previous SIN/COS read -- no instruction rewrote that slot in between -- takes that result
-// again: bit 63 of its word, which every decoder ignores; the first of such a pair gets bit 62
-// (clear on unary ops otherwise), so the value sweeps compute it as one sincos where they would
-// call sin and cos. Orders that differ (level schedules, segment tapes) are re-encoded without
-// either bit. The 20-step rollout's 80 SIN/COS pairs each save one sincos.
+// Sine/cosine pairs. The value and record sweeps compute sin and cos of the operand together for
+// either op, so a SIN or COS whose operand is the value the previous SIN/COS read -- no
+// instruction rewrote that slot in between -- takes that result again: bit 63 of its word, which
+// every decoder ignores. Orders that differ (level schedules, segment tapes) are re-encoded
+// without it. The 20-step rollout's 80 SIN/COS pairs each save one sincos.
 void mark_sincos_pairs(std::vector<u64>& code) {
   unsigned slots = 1;
   for (u64 w : code) slots = std::max(slots, std::max(dec_a(w), std::max(dec_b(w), dec_c(w))) + 1);
   std::vector<long long> ver(slots, -1);  // slot -> instruction that last wrote it
-  long long cache_slot = -1, cache_ver = -1, cache_at = -1;
+  long long cache_slot = -1, cache_ver = -1;
   for (size_t k = 0; k < code.size(); ++k) {
     const u64 w = code[k];
     const unsigned op = dec_op(w);
@@ -1811,11 +1899,9 @@ void mark_sincos_pairs(std::vector<u64>& code) {
       const unsigned b = dec_b(w);
       if (static_cast<long long>(b) == cache_slot && ver[b] == cache_ver) {
         code[k] = w | kSincosReuse;
-        code[cache_at] |= kSincosFirst;  // the value sweeps compute the pair there
       } else {
         cache_slot = b;
         cache_ver = ver[b];
-        cache_at = static_cast<long long>(k);
       }
     }
     if (op != D_OUTPUT && op != D_NOP) ver[dec_a(w)] = static_cast<long long>(k);
@@ -1919,6 +2005,11 @@ int make_tape(const casadi_gb300_atomic* alg, int n_instr, int n_in, const int* 
   if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
   if ((e = cudaMalloc(&t->d_code, code.size() * sizeof(u64))) != cudaSuccess)
     return cuda_fail(e, "cudaMalloc(code)");
+  std::vector<uint4> ventries;
+  for (int k = 0; k < n_instr; ++k) ventries.push_back(value_entry_of(code[k], consts.data()));
+  t->n_vblocks = pad_block(ventries);
+  if ((e = upload(&t->d_ventries, ventries)) != cudaSuccess)
+    return cuda_fail(e, "upload value entries");
   if ((e = cudaMalloc(&t->d_consts, consts.size() * sizeof(double))) != cudaSuccess)
     return cuda_fail(e, "cudaMalloc(consts)");
   if ((e = cudaMalloc(&t->d_absent, std::max<size_t>(1, t->absent_in.size()) * sizeof(int2))) !=

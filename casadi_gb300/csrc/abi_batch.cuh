@@ -107,7 +107,6 @@ int batch_prepare(BatchHost& b) {
     BatchItem bi;
     std::memset(&bi, 0, sizeof(bi));
     bi.t = t->view();
-    bi.n_code = t->n_chunks * kChunk;
     bi.ndir = it.ndir;
     bi.n = it.n;
     bi.forward = it.forward ? 1 : 0;
@@ -154,7 +153,8 @@ int batch_prepare(BatchHost& b) {
       // few tiles: the record sweep runs cooperatively (several warps per tile) before the
       // persistent launch instead of as one-warp record units
       const bool pre = tiles <= 4ll * sm_count() && ensure_levels(*t) &&
-                       smem_coop(t->lv_sz_w) <= static_cast<size_t>(max_smem_optin());
+                       smem_team(t->lv_sz_w, coop_threads_for((it.n + 31) / 32), false) <=
+                           static_cast<size_t>(max_smem_optin());
       if (pre) {
         b.pre.push_back({static_cast<int>(k), n_flags, tiles, tp});
         bi.t = t->view();
@@ -200,14 +200,14 @@ int batch_prepare(BatchHost& b) {
   if (!b.d_counter && (e = cudaMalloc(&b.d_counter, 2 * sizeof(unsigned))) != cudaSuccess)
     return cuda_fail(e, "cudaMalloc(counter)");
   b.n_units = static_cast<int>(ulist.size());
-  b.smem = static_cast<size_t>(b.szw) * 256;
+  b.smem = smem_value(b.szw);
   const int occ = b.smem <= static_cast<size_t>(max_smem_optin())
                       ? std::max(1, occupancy_batch(b.smem, b.n_flags > 0, false))
                       : 1;
   b.grid = std::max(1, std::min(sm_count() * occ, std::max(1, b.n_units)));
   // global-memory work vectors: residency capped by registers (and at 8 CTAs per SM, which
   // bounds the per-CTA partial scratch the caller provides)
-  const int occ_gw = std::max(1, std::min(8, occupancy_batch(0, b.n_flags > 0, true)));
+  const int occ_gw = std::max(1, std::min(8, occupancy_batch(kEntRingBytes, b.n_flags > 0, true)));
   b.grid_gw = std::max(1, std::min(sm_count() * occ_gw, std::max(1, b.n_units)));
   cudaFree(b.d_gw);
   b.d_gw = nullptr;
@@ -233,7 +233,8 @@ int batch_enqueue(BatchHost& b, void* scratch, cudaStream_t s, bool gw) {
     for (int j = 0; j < t->n_out; ++j) a.out[j] = it.io[kMaxIo + j];
     a.partials = pr.partials;
     a.block = coop_threads_for(pr.tiles);
-    const size_t sm = smem_coop(t->lv_sz_w);
+    set_team(a, *t);
+    const size_t sm = smem_team(t->lv_sz_w, a.block, false);
     const int occ = std::max(1, occupancy_coop(a.block, sm, false));
     const int grid = static_cast<int>(std::min<long long>(pr.tiles, 1ll * occ * sm_count()));
     if ((e = launch_coop(a, true, grid, s)) != cudaSuccess) return cuda_fail(e, "batch record");

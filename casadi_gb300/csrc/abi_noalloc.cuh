@@ -87,15 +87,9 @@ int casadi_gb300_reverse_noalloc(int id, int64_t n, int64_t ld, int nadj,
   if (nadj < 0 || nadj > 65535) return fail(CASADI_GB300_ERR_ARG, "bad direction count %d", nadj);
   if (n == 0) return 0;
   // both sweeps keep the work vector in shared memory (the global-memory form would need
-  // device buffers of its own): find the record sweep's block size and the adjoint's shape
-  int block = 0;
-  for (int bs : {t->primal_block, 128, 64, 32})
-    if (bs >= 32 && smem_primal(t->sz_w, bs) <= static_cast<size_t>(max_smem_optin())) {
-      block = bs;
-      break;
-    }
+  // device buffers of its own): find the adjoint's shape
   const DirShape ds = noalloc_shape(*t, std::max(nadj, 1));
-  if (block == 0 || (nadj > 0 && ds.dw == 0))
+  if (!fits_smem(t->sz_w) || (nadj > 0 && ds.dw == 0))
     return fail(CASADI_GB300_ERR_UNSUPPORTED,
                 "allocation-free adjoint: the tape's work vector (%d slots, %zu bytes per "
                 "32-instance tile) does not fit in shared memory, where this entry point keeps "
@@ -119,10 +113,8 @@ int casadi_gb300_reverse_noalloc(int id, int64_t n, int64_t ld, int nadj,
   a.ndir = nadj;
   fill_io(a.in, t->n_in, vptrs(arg), t->nnz_in, ld, false);
   fill_io(a.out, t->n_out, vptrs(res), t->nnz_out, ld, false);
-  a.block = block;
-  const int rgrid = grid_for((n + a.block - 1) / a.block,
-                             sm_count() * std::max(1, occupancy_primal(
-                                                          block, smem_primal(t->sz_w, block))));
+  a.block = 32;
+  const int rgrid = grid_for((n + 31) / 32, kMaxGrid);
   cudaError_t e = timed(F_RECORD, s, [&] { return launch_record(a, rgrid, s); });
   if (e != cudaSuccess) return cuda_fail(e, "record sweep launch");
   if (nadj == 0) return 0;

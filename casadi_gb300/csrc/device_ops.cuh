@@ -4,14 +4,18 @@
 // macro :1302-1355); partial derivatives follow BinaryOperation<OP>::der with the same
 // operation order (calculus.hpp:598-1018, dispatch :1388-1439). Every arithmetic step is an
 // explicitly rounded intrinsic (__dadd_rn, __dmul_rn, ...): nothing is contracted into an
-// FMA, so +,-,*,/,sqrt tapes reproduce the CPU reference bit for bit. Transcendentals call
-// CUDA's own double-precision functions.
+// FMA, so +,-,*,/,sqrt tapes reproduce the CPU reference bit for bit. Division, square root,
+// sin, cos, exp, log and tanh run in integer arithmetic (fixed_math.cuh); the arguments those
+// routines leave out, and the other transcendentals, call CUDA's double-precision functions.
 //
-// NEG, FABS, SIGN and COPYSIGN act on the sign bit with integer instructions: bit-identical
-// to the FP64 forms and they keep the FP64 pipe (the scarce unit on GB300) free.
+// NEG, FABS, SIGN and COPYSIGN act on the sign bit and comparisons on the bit patterns with
+// integer instructions: bit-identical to the FP64 forms and they keep the FP64 pipe (the scarce
+// unit on GB300) free.
 #pragma once
 #include <cstdint>
 #include <math_constants.h>
+
+#include "fixed_math.cuh"
 
 namespace cgb {
 
@@ -46,11 +50,8 @@ __host__ __device__ __forceinline__ unsigned dec_c(u64 w) { return (unsigned)(w 
 __host__ __device__ __forceinline__ unsigned dec_pmask(u64 w) { return (unsigned)(w >> 60) & 3u; }
 __host__ __device__ __forceinline__ bool dec_binary(u64 w) { return (w >> 62) & 1u; }
 // Bit 63: a SIN or COS whose sin/cos pair the previous SIN/COS of the same operand value
-// computed (the sweeps take it again); bit 62 on a SIN or COS (unary ops leave it clear): the
-// first of such a pair, which the value sweeps then compute as one sincos (see
-// mark_sincos_pairs).
+// computed (the sweeps take it again; see mark_sincos_pairs).
 constexpr u64 kSincosReuse = 1ull << 63;
-constexpr u64 kSincosFirst = 1ull << 62;
 
 // Partials an instruction records for the AD sweeps: bit 0 = d0, bit 1 = d1.
 // Ops whose partials are constants (ADD, SUB, NEG, TWICE, ASSIGN, comparisons, ...) record
@@ -190,17 +191,74 @@ __device__ __forceinline__ double d_copysign(double x, double y) {
   long long sy = __double_as_longlong(y) & (long long)kSignBit;
   return __longlong_as_double(bx | sy);
 }
+// Order of the non-NaN doubles on an integer key: -0 and +0 share 0.
+__device__ __forceinline__ long long d_key(double x) {
+  const long long b = __double_as_longlong(x);
+  return b < 0 ? (long long)(kSignBit - (unsigned long long)b) : b;
+}
+// x < y and x <= y as FP64 comparisons decide them (false with a NaN operand)
+__device__ __forceinline__ bool d_lt(double x, double y) {
+  return d_key(x) < d_key(y) && !d_isnan(x) && !d_isnan(y);
+}
+__device__ __forceinline__ bool d_le(double x, double y) {
+  return d_key(x) <= d_key(y) && !d_isnan(x) && !d_isnan(y);
+}
+__device__ __forceinline__ bool d_eq(double x, double y) {
+  return d_key(x) == d_key(y) && !d_isnan(x) && !d_isnan(y);
+}
 // fmin/fmax: NaN operand yields the other; ties (+0/-0 included) yield the first operand,
 // as the x86-64 reference build resolves std::fmin/fmax.
 __device__ __forceinline__ double d_fmin(double x, double y) {
   if (d_isnan(x)) return y;
   if (d_isnan(y)) return x;
-  return y < x ? y : x;
+  return d_key(y) < d_key(x) ? y : x;
 }
 __device__ __forceinline__ double d_fmax(double x, double y) {
   if (d_isnan(x)) return y;
   if (d_isnan(y)) return x;
-  return y > x ? y : x;
+  return d_key(y) > d_key(x) ? y : x;
+}
+
+// CUDA's functions for the arguments the integer routines leave out, out of line: rarely
+// reached, and one copy serves every use in a kernel.
+static __device__ __noinline__ double slow_div(double x, double y) { return __ddiv_rn(x, y); }
+static __device__ __noinline__ double slow_sqrt(double x) { return __dsqrt_rn(x); }
+static __device__ __noinline__ double slow_sin(double x) { return sin(x); }
+static __device__ __noinline__ double slow_cos(double x) { return cos(x); }
+static __device__ __noinline__ double slow_exp(double x) { return exp(x); }
+static __device__ __noinline__ double slow_log(double x) { return log(x); }
+static __device__ __noinline__ double slow_tanh(double x) { return tanh(x); }
+
+// x / y for a divisor prepared once (y: the same value)
+__device__ __forceinline__ double d_div(double x, double y, const FxDivisor& d) {
+  double q;
+  return fx_div(x, d, &q) ? q : slow_div(x, y);
+}
+__device__ __forceinline__ double d_div(double x, double y) {
+  return d_div(x, y, fx_divisor(y));
+}
+__device__ __forceinline__ double d_rcp(double y) { return d_div(1.0, y); }
+__device__ __forceinline__ double d_sqrt(double x) {
+  double r;
+  return fx_sqrt(x, &r) ? r : slow_sqrt(x);
+}
+__device__ __forceinline__ void d_sincos(double x, double* s, double* c) {
+  if (!fx_sincos(x, s, c)) {
+    *s = slow_sin(x);
+    *c = slow_cos(x);
+  }
+}
+__device__ __forceinline__ double d_exp(double x) {
+  double r;
+  return fx_exp(x, &r) ? r : slow_exp(x);
+}
+__device__ __forceinline__ double d_log(double x) {
+  double r;
+  return fx_log(x, &r) ? r : slow_log(x);
+}
+__device__ __forceinline__ double d_tanh(double x) {
+  double r;
+  return fx_tanh(x, &r) ? r : slow_tanh(x);
 }
 
 // The reference's erfinv (calculus.hpp:297-328; glibc provides none): rational start value,
@@ -244,27 +302,30 @@ __device__ __forceinline__ double dev_fun(unsigned op, double x, double y) {
     case D_ADD: return __dadd_rn(x, y);
     case D_SUB: return __dsub_rn(x, y);
     case D_MUL: return __dmul_rn(x, y);
-    case D_DIV: return __ddiv_rn(x, y);
+    case D_DIV: return d_div(x, y);
     case D_NEG: return d_neg(x);
-    case D_EXP: return exp(x);
-    case D_LOG: return log(x);
+    case D_EXP: return d_exp(x);
+    case D_LOG: return d_log(x);
     case D_POW: case D_CONSTPOW: return pow(x, y);
-    case D_SQRT: return __dsqrt_rn(x);
+    case D_SQRT: return d_sqrt(x);
     case D_SQ: return __dmul_rn(x, x);
     case D_TWICE: return d_twice(x);  // == 2.*x exactly
-    case D_SIN: return sin(x);
-    case D_COS: return cos(x);
+    case D_SIN: case D_COS: {
+      double s, c;
+      d_sincos(x, &s, &c);
+      return op == D_SIN ? s : c;
+    }
     case D_TAN: return tan(x);
     case D_ASIN: return asin(x);
     case D_ACOS: return acos(x);
     case D_ATAN: return atan(x);
-    case D_LT: return x < y ? 1.0 : 0.0;
-    case D_LE: return x <= y ? 1.0 : 0.0;
-    case D_EQ: return x == y ? 1.0 : 0.0;
-    case D_NE: return x != y ? 1.0 : 0.0;
-    case D_NOT: return x == 0.0 ? 1.0 : 0.0;
-    case D_AND: return (x != 0.0 && y != 0.0) ? 1.0 : 0.0;
-    case D_OR: return (x != 0.0 || y != 0.0) ? 1.0 : 0.0;
+    case D_LT: return d_lt(x, y) ? 1.0 : 0.0;
+    case D_LE: return d_le(x, y) ? 1.0 : 0.0;
+    case D_EQ: return d_eq(x, y) ? 1.0 : 0.0;
+    case D_NE: return d_eq(x, y) ? 0.0 : 1.0;
+    case D_NOT: return d_iszero(x) ? 1.0 : 0.0;
+    case D_AND: return (!d_iszero(x) && !d_iszero(y)) ? 1.0 : 0.0;
+    case D_OR: return (!d_iszero(x) || !d_iszero(y)) ? 1.0 : 0.0;
     case D_FLOOR: return floor(x);
     case D_CEIL: return ceil(x);
     case D_FMOD: return fmod(x, y);
@@ -272,14 +333,14 @@ __device__ __forceinline__ double dev_fun(unsigned op, double x, double y) {
     case D_FABS: return d_fabs(x);
     case D_SIGN: return d_sign(x);
     case D_COPYSIGN: return d_copysign(x, y);
-    case D_IF_ELSE_ZERO: return x == 0.0 ? 0.0 : y;
+    case D_IF_ELSE_ZERO: return d_iszero(x) ? 0.0 : y;
     case D_ERF: return erf(x);
     case D_FMIN: return d_fmin(x, y);
     case D_FMAX: return d_fmax(x, y);
-    case D_INV: return __drcp_rn(x);
+    case D_INV: return d_rcp(x);
     case D_SINH: return sinh(x);
     case D_COSH: return cosh(x);
-    case D_TANH: return tanh(x);
+    case D_TANH: return d_tanh(x);
     case D_ASINH: return asinh(x);
     case D_ACOSH: return acosh(x);
     case D_ATANH: return atanh(x);
@@ -301,18 +362,24 @@ __device__ __forceinline__ double dev_fun_der(unsigned op, double x, double y, d
   double f;
   switch (op) {
     case D_MUL: f = __dmul_rn(x, y); d0 = y; d1 = x; return f;
-    case D_DIV:
-      f = __ddiv_rn(x, y); d0 = __drcp_rn(y); d1 = __ddiv_rn(d_neg(f), y); return f;
-    case D_EXP: f = exp(x); d0 = f; return f;
-    case D_LOG: f = log(x); d0 = __drcp_rn(x); return f;
+    case D_DIV: {
+      const FxDivisor d = fx_divisor(y);
+      f = d_div(x, y, d); d0 = d_div(1.0, y, d); d1 = d_div(d_neg(f), y, d); return f;
+    }
+    case D_EXP: f = d_exp(x); d0 = f; return f;
+    case D_LOG: f = d_log(x); d0 = d_rcp(x); return f;
     case D_POW:
       f = pow(x, y); d0 = __dmul_rn(y, pow(x, __dsub_rn(y, 1.0))); d1 = __dmul_rn(log(x), f);
       return f;
     case D_CONSTPOW: f = pow(x, y); d0 = __dmul_rn(y, pow(x, __dsub_rn(y, 1.0))); return f;
-    case D_SQRT: f = __dsqrt_rn(x); d0 = __drcp_rn(__dadd_rn(f, f)); return f;
+    case D_SQRT: f = d_sqrt(x); d0 = d_rcp(d_twice(f)); return f;
     case D_SQ: f = __dmul_rn(x, x); d0 = d_twice(x); return f;
-    case D_SIN: { double s, c; sincos(x, &s, &c); d0 = c; return s; }
-    case D_COS: { double s, c; sincos(x, &s, &c); d0 = d_neg(s); return c; }
+    case D_SIN: case D_COS: {
+      double s, c;
+      d_sincos(x, &s, &c);
+      d0 = op == D_SIN ? c : d_neg(s);
+      return op == D_SIN ? s : c;
+    }
     case D_TAN: { f = tan(x); double c = cos(x); d0 = __drcp_rn(__dmul_rn(c, c)); return f; }
     case D_ASIN:
       f = asin(x); d0 = __drcp_rn(__dsqrt_rn(__dsub_rn(1.0, __dmul_rn(x, x)))); return f;
@@ -323,24 +390,24 @@ __device__ __forceinline__ double dev_fun_der(unsigned op, double x, double y, d
     case D_REMAINDER: f = remainder(x, y); d1 = __ddiv_rn(__dsub_rn(f, x), y); return f;
     case D_FABS: f = d_fabs(x); d0 = d_sign(x); return f;
     case D_COPYSIGN: f = d_copysign(x, y); d0 = d_copysign(1.0, y); return f;
-    case D_IF_ELSE_ZERO: f = x == 0.0 ? 0.0 : y; d1 = x; return f;
+    case D_IF_ELSE_ZERO: f = d_iszero(x) ? 0.0 : y; d1 = x; return f;
     case D_ERF:
       f = erf(x);
       d0 = __dmul_rn(__ddiv_rn(2.0, __dsqrt_rn(CUDART_PI)), exp(d_neg(__dmul_rn(x, x))));
       return f;
     case D_FMIN: case D_FMAX: {
       f = op == D_FMIN ? d_fmin(x, y) : d_fmax(x, y);
-      bool le = x <= y, ge = y <= x;
+      bool le = d_le(x, y), ge = d_le(y, x);
       bool a = op == D_FMIN ? le : ge, b = op == D_FMIN ? ge : le;
       if (a && b) { d0 = 0.5; d1 = 0.5; }
       else if (a || b) { d0 = a ? 1.0 : 0.0; d1 = b ? 1.0 : 0.0; }
       else { d0 = CUDART_NAN; d1 = CUDART_NAN; }  // 0/0 in the reference formula
       return f;
     }
-    case D_INV: f = __drcp_rn(x); d0 = d_neg(__dmul_rn(f, f)); return f;
+    case D_INV: f = d_rcp(x); d0 = d_neg(__dmul_rn(f, f)); return f;
     case D_SINH: f = sinh(x); d0 = cosh(x); return f;
     case D_COSH: f = cosh(x); d0 = sinh(x); return f;
-    case D_TANH: f = tanh(x); d0 = __dsub_rn(1.0, __dmul_rn(f, f)); return f;
+    case D_TANH: f = d_tanh(x); d0 = __dsub_rn(1.0, __dmul_rn(f, f)); return f;
     case D_ASINH:
       f = asinh(x); d0 = __drcp_rn(__dsqrt_rn(__dadd_rn(1.0, __dmul_rn(x, x)))); return f;
     case D_ACOSH:
@@ -365,29 +432,18 @@ __device__ __forceinline__ double dev_fun_der(unsigned op, double x, double y, d
   }
 }
 
-// dev_fun_der with the record sweeps' sin/cos pair (s, c): a SIN or COS computes the pair and
-// keeps it, or, marked kSincosReuse, takes the kept pair of the same operand value; the bits
-// are dev_fun_der's either way.
-__device__ __forceinline__ double dev_fun_der_pair(unsigned op, double x, double y, double& d0,
-                                                   double& d1, u64 ins, double& s, double& c) {
-  if (op == D_SIN || op == D_COS) {
-    if (!(ins & kSincosReuse)) sincos(x, &s, &c);
-    d0 = op == D_SIN ? c : d_neg(s);
-    return op == D_SIN ? s : c;
-  }
-  return dev_fun_der(op, x, y, d0, d1);
-}
-
-// dev_fun with the value sweeps' sin/cos pair: the first of a marked pair computes both as one
-// sincos and keeps them, the second takes the kept one; unpaired SIN/COS call sin or cos. Same
-// bits as dev_fun (sincos gives sin's and cos's results).
-__device__ __forceinline__ double dev_fun_pair(unsigned op, double x, double y, u64 ins,
-                                               double& s, double& c) {
-  if ((op == D_SIN || op == D_COS) && (ins & (kSincosReuse | kSincosFirst))) {
-    if (!(ins & kSincosReuse)) sincos(x, &s, &c);
-    return op == D_SIN ? s : c;
-  }
+// The operations without a case of their own in the value walk, out of line.
+struct FunDer {
+  double f, d0, d1;
+};
+static __device__ __noinline__ double rare_fun(unsigned op, double x, double y) {
   return dev_fun(op, x, y);
+}
+static __device__ __noinline__ FunDer rare_fun_der(unsigned op, double x, double y) {
+  FunDer r;
+  r.d0 = r.d1 = 0.0;
+  r.f = dev_fun_der(op, x, y, r.d0, r.d1);
+  return r;
 }
 #endif  // __CUDACC__
 

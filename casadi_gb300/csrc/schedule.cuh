@@ -43,4 +43,13 @@ struct Levels {
 int level_schedule(const std::vector<u64>& in, int width, int slot_cap, Levels& out,
                    std::string& err, bool ordered_users = false);
 
+// The levels as one instruction stream per warp of a `warps`-warp team: per warp, indices into
+// lv.code in execution order, kTeamBarrier where the whole team meets. A warp runs its own
+// instructions in order, so the team meets before a level only where an instruction would read
+// a slot another warp wrote since the last meeting, or write one another warp wrote or read,
+// or where meeting spreads the level's work enough better (costs in dependent FP64 operations,
+// `cost[op]`).
+constexpr int kTeamBarrier = -1;
+std::vector<std::vector<int>> team_streams(const Levels& lv, int warps, const float (&cost)[64]);
+
 }  // namespace cgb

@@ -1,10 +1,10 @@
 // Tape-sweep kernels for sm_103a.
 //
-// The value and sparsity sweeps interpret the instruction stream, staged chunk by chunk
-// (kChunk 8-byte words) from global memory into a two-slot shared-memory ring with TMA bulk
-// copies (cp.async.bulk ... mbarrier::complete_tx) while the previous chunk is being
-// interpreted; the warp-level derivative sweeps walk host-compiled keyed entry streams over the
-// recorded partials (see "Derivative sweeps, warp-independent" below). Every thread of a CTA
+// The sparsity sweeps interpret the instruction stream, staged chunk by chunk (kChunk 8-byte
+// words) from global memory into a two-slot shared-memory ring with TMA bulk copies
+// (cp.async.bulk ... mbarrier::complete_tx) while the previous chunk is being interpreted; the
+// warp-level value and derivative sweeps walk host-compiled keyed entry streams (sweeps_value.cuh
+// and "Derivative sweeps, warp-independent" below). Every thread of a CTA
 // runs the same instruction on a different instance (or instance/direction pair), so the
 // dispatch is warp-uniform and never diverges.
 // The work vector lives in shared memory in slot-major order, w[slot*BS + thread]:
@@ -14,8 +14,8 @@
 // layout of CasADi's Map (casadi/core/map.cpp:150-153) without a separate transpose pass.
 //
 // Kernels:
-//   k_primal<BS,false>  forward value sweep           SXFunction::eval (sx_function.cpp:110-124)
-//   k_primal<BS,true>   values + recorded partials    (first half of the AD sweeps)
+//   k_value<false>      forward value sweep           SXFunction::eval (sx_function.cpp:110-124)
+//   k_value<true>       values + recorded partials    (first half of the AD sweeps)
 //   k_tangent<G,MB,IPT,K>  forward-mode directions    ad_forward, numeric
 //                                                     (sx_function.cpp:1318-1364)
 //   k_adjoint<G,MB,IPT>    adjoint directions         ad_reverse, numeric
@@ -147,79 +147,11 @@ __device__ __forceinline__ long long io_off(const IoDesc& d, long long dir, long
   return dir * d.dir_stride + nz * d.nz_stride + inst * d.inst_stride;
 }
 
-// ---------------------------------------------------------------------------------------------
-// Forward value sweep (RECORD=false) and value + partials sweep (RECORD=true).
-// One thread per instance; BS instances per tile; persistent over tiles.
-// ---------------------------------------------------------------------------------------------
-// GW: the work vector lives in global memory (a per-CTA block of a.wglob, L1/L2-cached)
-// instead of shared memory, for tapes whose work vector does not fit or is worth trading for
-// residency.
-// The last sin/cos pair of a value or record sweep (dev_fun_pair, dev_fun_der_pair).
-struct PairState {
-  double s = 0.0, c = 0.0;
-};
-
-template <int BS, bool RECORD, bool GW = false>
-__global__ void __launch_bounds__(BS) k_primal(const __grid_constant__ SweepArgs a) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  u64* ring = reinterpret_cast<u64*>(smem);
-  u64* bars = ring + 2 * kChunk;
-  double* w = GW ? reinterpret_cast<double*>(a.wglob + blockIdx.x * a.wglob_stride)
-                 : reinterpret_cast<double*>(smem + kHeaderBytes);
-  const int tid = threadIdx.x;
-  if (tid == 0) stage_init(bars);
-  __syncthreads();
-  unsigned seq = 0;
-  const long long ntiles = (a.n + BS - 1) / BS;
-  for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const long long il = tile * BS + tid;
-    const bool active = il < a.n;
-    const long long ig = a.i_begin + il;
-    long long pidx = 0;
-    PairState pair;
-    const bool ok = sweep_forward(a.t, ring, bars, seq, [&](u64 ins) {
-      const unsigned op = dec_op(ins), A = dec_a(ins), B = dec_b(ins), C = dec_c(ins);
-      switch (op) {
-        case D_NOP:
-          break;
-        case D_CONST:
-          w[A * BS + tid] = __ldg(a.t.consts + B);
-          break;
-        case D_INPUT: {
-          const IoDesc& d = a.in[B];
-          double v = 0.0;
-          if (active && d.ptr) v = __ldg(static_cast<const double*>(d.ptr) + io_off(d, 0, C, ig));
-          w[A * BS + tid] = v;
-        } break;
-        case D_OUTPUT: {
-          const IoDesc& d = a.out[A];
-          if (active && d.ptr) static_cast<double*>(d.ptr)[io_off(d, 0, C, ig)] = w[B * BS + tid];
-        } break;
-        default: {
-          const double x = w[B * BS + tid], y = w[C * BS + tid];
-          if constexpr (RECORD) {
-            const unsigned m = partial_mask(op);
-            double d0 = 0.0, d1 = 0.0;
-            const double f = dev_fun_der_pair(op, x, y, d0, d1, ins, pair.s, pair.c);
-            if (m & 1u) {
-              if (active) a.partials[((il >> 5) * a.t.n_partials + pidx) * 32 + (il & 31)] = d0;
-              ++pidx;
-            }
-            if (m & 2u) {
-              if (active) a.partials[((il >> 5) * a.t.n_partials + pidx) * 32 + (il & 31)] = d1;
-              ++pidx;
-            }
-            w[A * BS + tid] = f;
-          } else {
-            w[A * BS + tid] = dev_fun_pair(op, x, y, ins, pair.s, pair.c);
-          }
-        }
-      }
-    });
-    if (!ok) return;
-  }
+__device__ __forceinline__ double& wreg(unsigned char* base, unsigned off) {
+  return *reinterpret_cast<double*>(base + off);
 }
 
+#include "sweeps_value.cuh"
 #include "sweeps_coop.cuh"
 
 // ---------------------------------------------------------------------------------------------
@@ -412,10 +344,6 @@ __global__ void __launch_bounds__(32 * DW) k_adjoint_tape(const __grid_constant_
 // operations and work-vector accesses that entry needs. Shared memory holds only the work
 // vector, w[slot][lane], so as many warps fit as the work vector allows.
 // ---------------------------------------------------------------------------------------------
-
-__device__ __forceinline__ double& wreg(unsigned char* base, unsigned off) {
-  return *reinterpret_cast<double*>(base + off);
-}
 
 // Meta word of the windowed tangent sweep's entries (k_tangent_win): bits 0-4 flags (1/2
 // operand b/c carries a derivative), 5-8 kind, 9-10 recorded-partial mask, 11-31 index of the
@@ -947,6 +875,9 @@ __global__ void __launch_bounds__(BS) k_sp_reverse(const __grid_constant__ Sweep
 size_t smem_primal(int sz_w, int block) {
   return kHeaderBytes + static_cast<size_t>(sz_w > 0 ? sz_w : 1) * block * 8;
 }
+size_t smem_value(int sz_w) {
+  return kEntRingBytes + static_cast<size_t>(sz_w > 0 ? sz_w : 1) * 256;
+}
 size_t smem_lean(int sz_w, int dir_warps, int chunk) {
   (void)chunk;
   return static_cast<size_t>(sz_w > 0 ? sz_w : 1) * 32 * dir_warps * 8;
@@ -997,17 +928,19 @@ static cudaError_t launch_k(K kernel, dim3 grid, int block, size_t smem, const S
     default: return cudaErrorInvalidValue;                                              \
   }
 
-// With a.wglob set the global-work-vector instance runs (block kGwBlock, ring header only).
+// With a.wglob set the global-work-vector instance runs.
+template <bool RECORD>
+static cudaError_t launch_value(const SweepArgs& a, int grid, cudaStream_t s) {
+  if (a.wglob) return launch_k(k_value<RECORD, true>, grid, 32, kEntRingBytes, a, s);
+  return launch_k(k_value<RECORD, false>, grid, 32, smem_value(a.t.sz_w), a, s);
+}
+
 cudaError_t launch_eval(const SweepArgs& a, int grid, cudaStream_t s) {
-  if (a.wglob) return launch_k(k_primal<kGwBlock, false, true>, grid, kGwBlock, kHeaderBytes, a, s);
-  const size_t smem = smem_primal(a.t.sz_w, a.block);
-  CGB_DISPATCH_BS(k_primal, , false)
+  return launch_value<false>(a, grid, s);
 }
 
 cudaError_t launch_record(const SweepArgs& a, int grid, cudaStream_t s) {
-  if (a.wglob) return launch_k(k_primal<kGwBlock, true, true>, grid, kGwBlock, kHeaderBytes, a, s);
-  const size_t smem = smem_primal(a.t.sz_w, a.block);
-  CGB_DISPATCH_BS(k_primal, , true)
+  return launch_value<true>(a, grid, s);
 }
 
 cudaError_t launch_sp_forward(const SweepArgs& a, int grid, cudaStream_t s) {
@@ -1023,14 +956,18 @@ cudaError_t launch_activity(const SweepArgs& a, int grid, cudaStream_t s) {
   CGB_DISPATCH_BS(k_sp_forward, , false, true)
 }
 
+size_t smem_team(int lv_sz_w, int threads, bool global) {
+  return static_cast<size_t>(threads / 32) * kEntRingBytes + (global ? 0 : smem_coop(lv_sz_w));
+}
+
 size_t smem_coop(int lv_sz_w) { return static_cast<size_t>(lv_sz_w > 0 ? lv_sz_w : 1) * 32 * 8; }
 
 cudaError_t launch_coop(const SweepArgs& a, bool record, int grid, cudaStream_t s) {
   if (a.block < 32 || a.block > kCoopMaxThreads || a.block % 32) return cudaErrorInvalidValue;
+  const size_t smem = smem_team(a.t.lv_sz_w, a.block, a.wglob != nullptr);
   if (a.wglob)
-    return record ? launch_k(k_coop<true, true>, grid, a.block, 0, a, s)
-                  : launch_k(k_coop<false, true>, grid, a.block, 0, a, s);
-  const size_t smem = smem_coop(a.t.lv_sz_w);
+    return record ? launch_k(k_coop<true, true>, grid, a.block, smem, a, s)
+                  : launch_k(k_coop<false, true>, grid, a.block, smem, a, s);
   return record ? launch_k(k_coop<true, false>, grid, a.block, smem, a, s)
                 : launch_k(k_coop<false, false>, grid, a.block, smem, a, s);
 }
@@ -1074,7 +1011,7 @@ int occupancy_adjoint_coop(size_t smem) {
 }
 
 int occupancy_coop(int threads, size_t smem, bool global) {
-  return global ? occ_of_k(k_coop<true, true>, threads, 0)
+  return global ? occ_of_k(k_coop<true, true>, threads, smem)
                 : occ_of_k(k_coop<true, false>, threads, smem);
 }
 
@@ -1084,9 +1021,9 @@ cudaError_t launch_sp_reverse(const SweepArgs& a, int grid, cudaStream_t s) {
   CGB_DISPATCH_BS(k_sp_reverse)
 }
 
-int occupancy_gw_primal(bool record) {
-  return record ? occ_of_k(k_primal<kGwBlock, true, true>, kGwBlock, kHeaderBytes)
-                : occ_of_k(k_primal<kGwBlock, false, true>, kGwBlock, kHeaderBytes);
+int occupancy_gw_value(bool record) {
+  return record ? occ_of_k(k_value<true, true>, 32, kEntRingBytes)
+                : occ_of_k(k_value<false, true>, 32, kEntRingBytes);
 }
 int occupancy_gw_sp() { return occ_of_k(k_sp_reverse<kGwBlock, true>, kGwBlock, kHeaderBytes); }
 
@@ -1245,9 +1182,9 @@ cudaError_t launch_batch(const BatchArgs& b, int grid, size_t smem, bool split, 
   if (smem > static_cast<size_t>(max_smem_optin())) return cudaErrorInvalidValue;
   if (gw) {
     if (split)
-      k_batch<true, true><<<grid, 32, 0, s>>>(b);
+      k_batch<true, true><<<grid, 32, kEntRingBytes, s>>>(b);
     else
-      k_batch<false, true><<<grid, 32, 0, s>>>(b);
+      k_batch<false, true><<<grid, 32, kEntRingBytes, s>>>(b);
   } else if (split) {
     k_batch<true, false><<<grid, 32, smem, s>>>(b);
   } else {
@@ -1256,28 +1193,14 @@ cudaError_t launch_batch(const BatchArgs& b, int grid, size_t smem, bool split, 
   return cudaGetLastError();
 }
 
-int occupancy_primal(int block, size_t smem) {
-  int n = 0;
-  cudaError_t e = cudaErrorInvalidValue;
+int occupancy_sp(int block, size_t smem) {
   switch (block) {
-    case 32:
-      cudaFuncSetAttribute(k_primal<32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_primal<32, true>, 32, smem);
-      break;
-    case 64:
-      cudaFuncSetAttribute(k_primal<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_primal<64, true>, 64, smem);
-      break;
-    case 128:
-      cudaFuncSetAttribute(k_primal<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_primal<128, true>, 128, smem);
-      break;
-    case 256:
-      cudaFuncSetAttribute(k_primal<256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_primal<256, true>, 256, smem);
-      break;
+    case 32: return std::max(1, occ_of_k(k_sp_forward<32>, 32, smem));
+    case 64: return std::max(1, occ_of_k(k_sp_forward<64>, 64, smem));
+    case 128: return std::max(1, occ_of_k(k_sp_forward<128>, 128, smem));
+    case 256: return std::max(1, occ_of_k(k_sp_forward<256>, 256, smem));
+    default: return 1;
   }
-  return (e == cudaSuccess && n > 0) ? n : 1;
 }
 
 template <class K>
@@ -1292,7 +1215,9 @@ static int occ_of(K kernel, int block, size_t smem) {
 }
 
 int occupancy_batch(size_t smem, bool split, bool gw) {
-  if (gw) return split ? occ_of(k_batch<true, true>, 32, 0) : occ_of(k_batch<false, true>, 32, 0);
+  if (gw)
+    return split ? occ_of(k_batch<true, true>, 32, kEntRingBytes)
+                 : occ_of(k_batch<false, true>, 32, kEntRingBytes);
   int n = 0;
   if (split) {
     if (cudaFuncSetAttribute(k_batch<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -123,6 +123,40 @@ enum AdjKey : unsigned {
 static_assert(AK_COUNT <= 64, "adjoint keys fit 6 bits");
 #undef CGB_KEY_ENUM
 
+// Value entries (k_value, k_batch, k_coop): 16 bytes per instruction.
+//   x  byte offset of the result slot in the work vector (OUTPUT: output index)
+//   y, z  byte offsets of the operand slots (CONST: the constant's low and high word; INPUT:
+//      input index and nonzero; OUTPUT: slot offset and nonzero)
+//   w  bits 0-5 the key: the opcode, or VK_SIN_REUSE / VK_COS_REUSE for a SIN or COS that takes
+//      the previous pair; bits 6-7 its recorded-partial mask; in the streams of a cooperative
+//      sweep's warps also its first recorded partial (bits 8-30) and whether the team meets
+//      after it (bit 31)
+constexpr int kEntBlock = 16;  // entries staged at a time
+constexpr int kEntRingBytes = 2 * kEntBlock * 16;
+constexpr unsigned kTeamPidxShift = 8, kTeamPidxMask = (1u << 23) - 1, kTeamMeet = 1u << 31;
+constexpr int kTeamSizes = 4;  // teams of 4, 8, 16 and 32 warps
+enum ValueKey : unsigned { VK_SIN_REUSE = 54, VK_COS_REUSE = 55 };
+inline uint4 value_entry_of(u64 ins, const double* consts) {
+  const unsigned op = dec_op(ins);
+  uint4 e = make_uint4(dec_a(ins) * 256u, dec_b(ins) * 256u, dec_c(ins) * 256u,
+                       op | (partial_mask(op) << 6));
+  if (op == D_CONST) {
+    u64 b;
+    memcpy(&b, consts + dec_b(ins), 8);
+    e.y = static_cast<unsigned>(b);
+    e.z = static_cast<unsigned>(b >> 32);
+  } else if (op == D_INPUT) {
+    e.y = dec_b(ins);
+    e.z = dec_c(ins);
+  } else if (op == D_OUTPUT) {
+    e.x = dec_a(ins);
+    e.z = dec_c(ins);
+  } else if ((op == D_SIN || op == D_COS) && (ins & kSincosReuse)) {
+    e.w = (op == D_SIN ? VK_SIN_REUSE : VK_COS_REUSE) | (partial_mask(op) << 6);
+  }
+  return e;
+}
+
 // One input/output block: element (direction d, nonzero k, instance i) lives at
 // ptr[d*dir_stride + k*nz_stride + i*inst_stride].
 struct IoDesc {
@@ -138,6 +172,8 @@ struct TapeView {
   const int* pofs;          // pofs[k]: partials recorded before instruction k*kPofsGran
   const double* consts;     // constant pool
   const int2* absent_in;    // (input, nonzero) pairs the tape never reads
+  const uint4* ventries;    // value entries of the scheduled order
+  int n_vblocks;            // their blocks of kEntBlock (NOP padding)
   int n_chunks;
   int n_absent_in;
   int sz_w;
@@ -209,7 +245,6 @@ struct SweepArgs {
 // One item of a persistent batch: a tape over its own instance range.
 struct BatchItem {
   TapeView t;
-  int n_code;
   int ndir;                 // 0: value sweep only; >0: value + derivative directions
   int forward;              // directions are tangent (1, identity-seeded) or adjoint (0)
   long long n;              // instances
@@ -241,7 +276,7 @@ struct BatchArgs {
 };
 
 constexpr int kGwBlock = 128;   // threads per CTA of the global-work-vector value sweeps
-int occupancy_gw_primal(bool record);  // CTAs per SM of the global-work-vector value/record sweep
+int occupancy_gw_value(bool record);  // CTAs per SM of the global-work-vector value/record sweep
 int occupancy_gw_sp();           // ... of the sparsity sweeps
 int occupancy_gw_dir(bool adjoint);  // ... of the derivative sweeps (one warp per CTA)
 cudaError_t launch_gather(long long n, long long ld, int count, const long long* src_row,
@@ -255,7 +290,8 @@ constexpr int kErrWaitTimeout = 1;   // a bounded wait on a staged chunk ran out
 constexpr int kErrBadOpcode = 2;     // an instruction with an unknown opcode was met
 
 // Shared memory a launch needs (bytes).
-size_t smem_primal(int sz_w, int block);
+size_t smem_primal(int sz_w, int block);  // sparsity and activity sweeps: ring + work vectors
+size_t smem_value(int sz_w);              // value and record sweeps: one tile's work vector
 size_t smem_dir(int sz_w, int dir_warps, int chunk);   // plan-free adjoint (8-byte stream)
 size_t smem_lean(int sz_w, int dir_warps, int chunk);  // lean tangent / adjoint
 int max_smem_optin();
@@ -305,7 +341,9 @@ cudaError_t launch_wait_probe(const unsigned* flag, unsigned* err, cudaStream_t 
 // most kCoopMaxThreads) share one 32-instance tile and run its level schedule; the work vector
 // in shared memory (lv_sz_w x 32 doubles), or in a.wglob blocks when set.
 constexpr int kCoopMaxThreads = 1024;
+// a.dstream, a.dchunks: the streams of a.block / 32 warps
 cudaError_t launch_coop(const SweepArgs& a, bool record, int grid, cudaStream_t s);
+size_t smem_team(int lv_sz_w, int threads, bool global);
 // Cooperative sparsity sweeps (forward: the value sweep's levels; reverse: the reverse
 // schedule's levels, last first); shared memory smem_coop of the schedule's work vector.
 cudaError_t launch_coop_sp(const SweepArgs& a, bool reverse, int grid, cudaStream_t s);
@@ -328,7 +366,7 @@ size_t smem_coop(int lv_sz_w);
 int occupancy_coop(int threads, size_t smem, bool global);
 
 // Resident CTAs per SM for a given kernel family and shared-memory footprint.
-int occupancy_primal(int block, size_t smem);
+int occupancy_sp(int block, size_t smem);
 int occupancy_dir(int variant, bool adjoint, size_t smem);  // warp-independent sweeps
 int occupancy_dense(int dir_warps, size_t smem);   // plan-free adjoint
 

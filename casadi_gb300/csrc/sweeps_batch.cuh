@@ -13,55 +13,6 @@
 // direction, then grabs the next unit. Tapes of any length and
 // instance count share the GPU in one launch instead of one underfilled launch per tape.
 // ---------------------------------------------------------------------------------------------
-// Warp-level value sweep of one tile; instruction words are read straight from the tape
-// (uniform across the warp, cached) with the next word prefetched. RECORD writes partials to
-// pt (lane-offset, tile-local [partial][lane]).
-template <bool RECORD>
-__device__ __forceinline__ void primal_walk(const TapeView& t, int n_code, double* pt,
-                                            unsigned char* wb, const IoDesc* in,
-                                            const IoDesc* out, bool active, long long ig) {
-  const u64* code = t.code;
-  int pidx = 0;
-  PairState pair;  // the last sin/cos pair
-  u64 nxt = __ldg(code);
-#pragma unroll 1
-  for (int k = 0; k < n_code; ++k) {
-    const u64 ins = nxt;
-    if (k + 1 < n_code) nxt = __ldg(code + k + 1);
-    const unsigned op = dec_op(ins), A = dec_a(ins), B = dec_b(ins), C = dec_c(ins);
-    switch (op) {
-      case D_NOP:
-        break;
-      case D_CONST:
-        wreg(wb, A * 256u) = __ldg(t.consts + B);
-        break;
-      case D_INPUT: {
-        const IoDesc& d = in[B];
-        double v = 0.0;
-        if (active && d.ptr) v = __ldg(static_cast<const double*>(d.ptr) + io_off(d, 0, C, ig));
-        wreg(wb, A * 256u) = v;
-      } break;
-      case D_OUTPUT: {
-        const IoDesc& d = out[A];
-        if (active && d.ptr) static_cast<double*>(d.ptr)[io_off(d, 0, C, ig)] = wreg(wb, B * 256u);
-      } break;
-      default: {
-        const double x = wreg(wb, B * 256u), y = wreg(wb, C * 256u);
-        if constexpr (RECORD) {
-          const unsigned m = dec_pmask(ins);
-          double d0 = 0.0, d1 = 0.0;
-          const double f = dev_fun_der_pair(op, x, y, d0, d1, ins, pair.s, pair.c);
-          if (m & 1u) pt[32 * pidx++] = d0;
-          if (m & 2u) pt[32 * pidx++] = d1;
-          wreg(wb, A * 256u) = f;
-        } else {
-          wreg(wb, A * 256u) = dev_fun_pair(op, x, y, ins, pair.s, pair.c);
-        }
-      }
-    }
-  }
-}
-
 // Bounded wait (lane 0, then shared with the warp) for a split item's tile flag. Every record
 // unit precedes every direction unit in the list, so the unit that sets the flag was taken by
 // a CTA that is already running and waits on nothing: the wait ends unless that CTA faults.
@@ -101,7 +52,9 @@ template <bool kSplit, bool GW>
 __global__ void __launch_bounds__(32, 16) k_batch(const __grid_constant__ BatchArgs b) {
   extern __shared__ __align__(128) unsigned char smem[];
   const int lane = threadIdx.x;
-  unsigned char* wb = (GW ? b.wglob + blockIdx.x * b.wglob_stride : smem) + lane * 8;
+  uint4* ring = reinterpret_cast<uint4*>(smem);
+  unsigned char* wb =
+      (GW ? b.wglob + blockIdx.x * b.wglob_stride : smem + kEntRingBytes) + lane * 8;
   double* const pcta = b.scratch + static_cast<size_t>(blockIdx.x) * b.scratch_stride + lane;
   for (;;) {
     unsigned u = 0;
@@ -121,10 +74,11 @@ __global__ void __launch_bounds__(32, 16) k_batch(const __grid_constant__ BatchA
     if (!kSplit || unit.z < 0) {
       // record (or value) unit
       if (it.ndir == 0) {
-        primal_walk<false>(it.t, it.n_code, pt, wb, io, io + kMaxIo, active, il);
+        value_walk<false>(it.t.ventries, it.t.n_vblocks, ring, nullptr, wb, io, io + kMaxIo, active,
+                          il);
         continue;
       }
-      primal_walk<true>(it.t, it.n_code, pt, wb, io, io + kMaxIo, active, il);
+      value_walk<true>(it.t.ventries, it.t.n_vblocks, ring, pt, wb, io, io + kMaxIo, active, il);
       if (kSplit && it.tile_partials) {
         // split item: publish the tile's partials; its directions are separate units
         __threadfence();

@@ -7,68 +7,40 @@
 // ---------------------------------------------------------------------------------------------
 // Cooperative value / record sweep for launches with few instances.
 //
-// One 32-instance tile per CTA (lane = instance) and several warps per CTA: the host's level
-// schedule groups the tape into levels of independent instructions; the warps of the CTA split
-// each level between them and meet at a barrier before the next, so a tile's sweep advances
-// by a whole level of independent instructions per step instead of one instruction. Each
-// instruction is the same operation on the same operand values as in the sequential sweep
-// (identical bits), and writes its partials at its index of the sequential order.
+// One 32-instance tile per CTA (lane = instance) and several warps per CTA. The host's level
+// schedule groups the tape into levels of independent instructions and lays each level out over
+// the warps of the team, balanced by the operations' latencies, as one entry stream per warp
+// (team_streams): the warps meet at a barrier only where one needs a slot another one wrote, so
+// chains of dependent instructions run on one warp without meeting. Each instruction is the same
+// operation on the same operand values as in the sequential sweep (identical bits), and writes
+// its partials at its index of the sequential order. Against a barrier after every level and
+// entries decoded from global memory: record of the 10000-node random graph at 16384 instances
+// 3.72 -> 1.27 ms, of the MPC constraint and gradient tapes at 4096 scenarios 6.1 -> 2.1 ms.
 // ---------------------------------------------------------------------------------------------
 template <bool RECORD, bool GW>
 __global__ void __launch_bounds__(kCoopMaxThreads) k_coop(const __grid_constant__ SweepArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
-  double* w = GW ? reinterpret_cast<double*>(a.wglob + blockIdx.x * a.wglob_stride)
-                 : reinterpret_cast<double*>(smem);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  uint4* ring = reinterpret_cast<uint4*>(smem) + warp * (2 * kEntBlock);
+  unsigned char* wb = (GW ? a.wglob + blockIdx.x * a.wglob_stride : smem + nw * kEntRingBytes) +
+                      lane * 8;
   const long long ntiles = (a.n + 31) / 32;
-  const int nl = a.t.n_levels;
+  const int2 se = __ldg(a.dchunks + warp);  // (first entry, blocks) of this warp's stream
+  const uint4* st = a.dstream + se.x;
   for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const long long il = tile * 32 + lane;
     const bool active = il < a.n;
     const long long ig = a.i_begin + il;
     double* pt = RECORD ? a.partials + static_cast<size_t>(tile) * a.t.n_partials * 32 + lane
                         : nullptr;
-    int end = __ldg(a.t.lbegin);
-    for (int l = 0; l < nl; ++l) {
-      const int beg = end;
-      end = __ldg(a.t.lbegin + l + 1);
-      for (int i = beg + warp; i < end; i += nw) {
-        const u64 ins = __ldg(a.t.lcode + i);
-        const unsigned op = dec_op(ins), A = dec_a(ins), B = dec_b(ins), C = dec_c(ins);
-        switch (op) {
-          case D_CONST:
-            w[A * 32 + lane] = __ldg(a.t.consts + B);
-            break;
-          case D_INPUT: {
-            const IoDesc& d = a.in[B];
-            double v = 0.0;
-            if (active && d.ptr) v = __ldg(static_cast<const double*>(d.ptr) + io_off(d, 0, C, ig));
-            w[A * 32 + lane] = v;
-          } break;
-          case D_OUTPUT: {
-            const IoDesc& d = a.out[A];
-            if (active && d.ptr) static_cast<double*>(d.ptr)[io_off(d, 0, C, ig)] = w[B * 32 + lane];
-          } break;
-          default: {
-            const double x = w[B * 32 + lane], y = w[C * 32 + lane];
-            if (RECORD) {
-              const unsigned m = partial_mask(op);
-              double d0 = 0.0, d1 = 0.0;
-              const double f = dev_fun_der(op, x, y, d0, d1);
-              if (m && active) {
-                const size_t p = static_cast<size_t>(__ldg(a.t.lpidx + i));
-                if (m & 1u) pt[p * 32] = d0;
-                if (m & 2u) pt[(p + (m & 1u)) * 32] = d1;
-              }
-              w[A * 32 + lane] = f;
-            } else {
-              w[A * 32 + lane] = dev_fun(op, x, y);
-            }
-          }
-        }
-      }
-      __syncthreads();
-    }
+    PairState pair;
+    staged_walk(st, se.y, ring, [&](const uint4& e) {
+      double* p = RECORD ? pt + static_cast<size_t>((e.w >> kTeamPidxShift) & kTeamPidxMask) * 32
+                         : nullptr;
+      value_entry<RECORD>(e, wb, p, a.in, a.out, active, ig, pair);
+      if (e.w & kTeamMeet) __syncthreads();
+    });
+    __syncthreads();  // the next tile's entries write the slots this one reads
   }
 }
 

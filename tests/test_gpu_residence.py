@@ -126,3 +126,26 @@ def test_cooperative_sweeps_on_wide_tapes(gpu_lib, n):
             want = O.eval(F.tape, sub, m)
             for g, w, b in zip(out[3][0], want, value_bounds(F.tape, sub, m)):
                 assert_close(g[:, :m], w, "values", bound=b)
+
+
+@pytest.mark.parametrize("tiles", [1000, 500, 250, 3])
+def test_every_team_size_gives_the_sequential_bits(gpu_lib, tiles):
+    """The cooperative value and record sweeps with teams of 4, 8, 16 and 32 warps (chosen by the
+    tiles of the launch when the residence is forced): long chains, wide levels and every op kind
+    give the sequential sweep's values and adjoints bit for bit, with a ragged last tile."""
+    n = 32 * tiles - 5
+    rng = np.random.default_rng(tiles)
+    for F, args in ((W.cartpole_rollout(6), W.cartpole_inputs(n, steps=6, seed=2)),
+                    (W.random_dag(n_in=20, n_nodes=700, n_out=5, seed=4, window=90, bounded=True),
+                     W.dag_inputs(n, n_in=20, seed=4))):
+        dargs = _dev(args)
+        seeds = _dev([rng.standard_normal((1, k, n)) for k in F.tape.nnz_out])
+        got = []
+        for mode in (2, 3):
+            t = R.CudaTape(F)
+            t.set_residence(mode)
+            t.set_variant(2, 0)
+            got.append(_host(t.eval(dargs)) + sum((_host(x) for x in t.reverse(dargs, seeds)), []))
+            t.sync()
+        for a, b in zip(*got):
+            assert_bitexact(a, b, "team, %d tiles" % tiles)
