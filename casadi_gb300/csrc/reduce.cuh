@@ -3,8 +3,7 @@
 // A block of `rows` rows, row r holding the values of one output nonzero (of one direction)
 // for n instances at src + r*ld. Sums are either
 //   kOrderInstance  in instance order from +0: ((0 + x0) + x1) + ... -- MapSum's own order
-//                   (casadi_clear, then casadi_add per instance), identical bits; a chain of
-//                   n dependent adds per row
+//                   (casadi_clear, then casadi_add per instance), identical bits
 //   kOrderTree      a fixed blocked tree: per level, 256-instance blocks; lane l of a warp
 //                   adds x[b*256 + m*32 + l] for m = 0..7 in order starting from +0, then a
 //                   butterfly over lanes (xor 16, 8, 4, 2, 1); the block sums form the next
@@ -29,10 +28,8 @@ size_t reduce_scratch_bytes(long long rows, long long n, int order);
 // dst[r] (= or +=, see `accumulate`) the sum of row r. `scratch` as reduce_scratch_bytes.
 cudaError_t reduce_sum(long long rows, long long n, const double* src, long long ld, double* dst,
                        int order, double* scratch, cudaStream_t s);
-// Several blocks of rows summed in instance order (kOrderInstance) by one launch, one thread
-// per row: the rows' chains of n dependent adds run concurrently instead of one block after
-// the other (each add waits for the previous one, ~85 cycles on GB300's FP64 pipe, so a chain
-// costs ~40 ns per instance whatever else runs beside it). Same bits as reduce_sum.
+// Several blocks of rows summed in instance order (kOrderInstance) by one launch, one CTA per
+// row. Same bits as reduce_sum.
 struct SumRows {
   const double* src;  // rows of n values, row r at src + r*ld
   long long ld;

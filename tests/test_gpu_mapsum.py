@@ -231,3 +231,41 @@ def test_edges_zero_instances_signed_zero_and_errors(gpu_lib):
     with pytest.raises(CasadiGpuError):
         CudaMapSum(f, n, [False], [True, True], order=2)(dev(args))
     F.tape.sync()
+
+
+def _summands(kind, n, rng):
+    if kind == "positive":
+        return rng.uniform(0.0, 3.0, n)
+    if kind == "walk":
+        return rng.standard_normal(n)
+    if kind == "ties":  # multiples of half an ulp of the running sum, a few steps apart
+        x = rng.integers(-3, 4, n) * 2.0 ** rng.integers(-54, -50, n).astype(float)
+        x[0] = 1.0
+        return x
+    if kind == "scales":
+        return rng.standard_normal(n) * 2.0 ** rng.integers(-60, 60, n).astype(float)
+    if kind == "tiny":
+        return rng.integers(-5, 6, n) * 5e-324
+    x = rng.standard_normal(n)  # "specials"
+    x[rng.integers(0, n, 1 + n // 700)] = 0.0
+    x[rng.integers(0, n, 1)] = -0.0
+    if n > 4000:
+        x[3 * n // 4] = np.inf if n % 2 else np.nan
+    return x
+
+
+@pytest.mark.parametrize("kind", ["positive", "walk", "ties", "scales", "tiny", "specials"])
+@pytest.mark.parametrize("n", [1, 31, 512, 4095, 4097, 40001])
+def test_instance_order_sum_is_the_sequential_sum(gpu_lib, kind, n):
+    """The instance-order sum (a scan of rounded steps inside a binade, FP64 additions where the
+    sum leaves it) against the additions one after the other: the same bits, for sums that stay
+    in a binade, cross many, stay near zero, tie at every step or meet infinities and NaN."""
+    rng = np.random.default_rng(n)
+    x = S.sym("x", 3)
+    f = S.Function("I", [x], [[x[0], x[1], -x[2]]])
+    rows = np.stack([_summands(kind, n, rng) for _ in range(3)])
+    got = host(CudaMapSum(f, n, reduce_out=[True]).eval(dev([rows])))[0]
+    with np.errstate(all="ignore"):
+        want = np.cumsum(np.concatenate([np.zeros((3, 1)), rows * [[1], [1], [-1]]], 1), 1)[:, -1]
+    both_nan = np.isnan(got) & np.isnan(want)
+    assert (both_nan | (got.view(np.uint64) == want.view(np.uint64))).all(), (got, want)
