@@ -401,17 +401,17 @@ __device__ __forceinline__ void issue_partials(const uint4 (&E)[G], const double
 }
 
 // Tangent of form F from the operand tangents a, b and the partials p, q.
-template <int F>
-__device__ __forceinline__ double tf_eval(double p, double q, double a, double b) {
-  if constexpr (F == TF_PY) return __dmul_rn(p, a);
-  else if constexpr (F == TF_QZ) return __dmul_rn(q, b);
-  else if constexpr (F == TF_PYQZ) return __fma_rn(p, a, __dmul_rn(q, b));
+template <int F, class Units>
+__device__ __forceinline__ double tf_eval(const Units& u, double p, double q, double a, double b) {
+  if constexpr (F == TF_PY) return u_mul(u, p, a);
+  else if constexpr (F == TF_QZ) return u_mul(u, q, b);
+  else if constexpr (F == TF_PYQZ) return __fma_rn(p, a, u_mul(u, q, b));
   else if constexpr (F == TF_Y) return a;
   else if constexpr (F == TF_Z) return b;
-  else if constexpr (F == TF_YQZ) return __dadd_rn(a, __dmul_rn(q, b));
-  else if constexpr (F == TF_YZ) return __dadd_rn(a, b);
+  else if constexpr (F == TF_YQZ) return u_add(u, a, u_mul(u, q, b));
+  else if constexpr (F == TF_YZ) return u_add(u, a, b);
   else if constexpr (F == TF_NZ) return d_neg(b);
-  else if constexpr (F == TF_YMZ) return __dsub_rn(a, b);
+  else if constexpr (F == TF_YMZ) return u_sub(u, a, b);
   else if constexpr (F == TF_NY) return d_neg(a);
   else if constexpr (F == TF_2Y) return d_twice(a);
   else return d_iszero(q) ? 0.0 : b;  // TF_IFZ
@@ -419,17 +419,18 @@ __device__ __forceinline__ double tf_eval(double p, double q, double a, double b
 
 // Tangent of one direction of a mixed union-stream entry: instruction kind rk, flags fk
 // (1/2: operand b/c carries a derivative), partials p (1 when d0 is not recorded) and q.
-__device__ __forceinline__ double tan_mixed(unsigned rk, unsigned fk, double p, double q,
-                                            double a, double b) {
+template <class Units>
+__device__ __forceinline__ double tan_mixed(const Units& u, unsigned rk, unsigned fk, double p,
+                                            double q, double a, double b) {
   switch ((rk << 2) | fk) {
-    case (LK_GEN << 2) | 1u: return __dmul_rn(p, a);
-    case (LK_GEN << 2) | 2u: return __dmul_rn(q, b);
-    case (LK_GEN << 2) | 3u: return __fma_rn(p, a, __dmul_rn(q, b));
+    case (LK_GEN << 2) | 1u: return u_mul(u, p, a);
+    case (LK_GEN << 2) | 2u: return u_mul(u, q, b);
+    case (LK_GEN << 2) | 3u: return __fma_rn(p, a, u_mul(u, q, b));
     case (LK_ADD << 2) | 1u: case (LK_SUB << 2) | 1u: case (LK_ASSIGN << 2) | 1u: return a;
     case (LK_ADD << 2) | 2u: return b;
-    case (LK_ADD << 2) | 3u: return __dadd_rn(a, b);
+    case (LK_ADD << 2) | 3u: return u_add(u, a, b);
     case (LK_SUB << 2) | 2u: return d_neg(b);
-    case (LK_SUB << 2) | 3u: return __dsub_rn(a, b);
+    case (LK_SUB << 2) | 3u: return u_sub(u, a, b);
     case (LK_NEG << 2) | 1u: return d_neg(a);
     case (LK_TWICE << 2) | 1u: return d_twice(a);
     case (LK_IFZ << 2) | 2u: return d_iszero(q) ? 0.0 : b;
@@ -442,8 +443,8 @@ constexpr unsigned kTanXMask = (1u << 19) - 1;
 
 // One group of tangent entries (IPT tiles, K directions dir0..): their keys in E, their
 // partials in P/Q.
-template <int G, int IPT, int K>
-__device__ __forceinline__ void tan_group(const uint4 (&E)[G], const double (&P)[G][IPT],
+template <int G, int IPT, int K, class Units>
+__device__ __forceinline__ void tan_group(const Units& u, const uint4 (&E)[G], const double (&P)[G][IPT],
                                           const double (&Q)[G][IPT], unsigned char* wb,
                                           const IoDesc* seed, const IoDesc* sens, bool identity,
                                           const bool (&active)[IPT], int dir0, int ndir,
@@ -482,7 +483,7 @@ __device__ __forceinline__ void tan_group(const uint4 (&E)[G], const double (&P)
     CGB_JK {                                                             \
       const double av = tf_uses_y(F) ? CGB_W(cur.y, j, k) : 0.0;         \
       const double bv = tf_uses_z(F) ? CGB_W(cur.z, j, k) : 0.0;         \
-      r[j][k] = tf_eval<F>(P[i][j], Q[i][j], av, bv);                    \
+      r[j][k] = tf_eval<F>(u, P[i][j], Q[i][j], av, bv);                    \
     }                                                                    \
     break;
       CGB_TK_ARITH(CGB_TK_CASE)
@@ -526,7 +527,7 @@ __device__ __forceinline__ void tan_group(const uint4 (&E)[G], const double (&P)
           for (int j = 0; j < IPT; ++j) {
             const double a = (fk & 1u) ? CGB_W(cur.y, j, k) : 0.0;
             const double b = (fk & 2u) ? CGB_W(cur.z, j, k) : 0.0;
-            CGB_W(xo, j, k) = tan_mixed(rk, fk, (pm & 1u) ? P[i][j] : 1.0,
+            CGB_W(xo, j, k) = tan_mixed(u, rk, fk, (pm & 1u) ? P[i][j] : 1.0,
                                         (pm & 2u) ? Q[i][j] : 0.0, a, b);
           }
         }
@@ -544,8 +545,8 @@ __device__ __forceinline__ void tan_group(const uint4 (&E)[G], const double (&P)
 // One tangent sweep by one warp over its keyed stream st (body of ngr groups of G, ngr even):
 // IPT tiles (tile j's partials at pt + j*tstride), K directions dir0.. (the union stream of
 // the K directions).
-template <bool kNC, int G, int IPT, int K>
-__device__ __forceinline__ void tangent_walk(const uint4* st, int ngr, const double* pt,
+template <bool kNC, int G, int IPT, int K, class Units>
+__device__ __forceinline__ void tangent_walk(const Units& u, const uint4* st, int ngr, const double* pt,
                                              size_t tstride, const bool (&tok)[IPT],
                                              unsigned char* wb, const IoDesc* seed,
                                              const IoDesc* sens, bool identity,
@@ -564,10 +565,10 @@ __device__ __forceinline__ void tangent_walk(const uint4* st, int ngr, const dou
   for (int g = 0; g < ngr; g += 2) {
     load_grp<G>(st, g + 2, Eb);
     issue_partials<kNC, G, IPT>(Ea, pt, tstride, tok, Pb, Qb);
-    tan_group<G, IPT, K>(Ea, Pa, Qa, wb, seed, sens, identity, active, dir0, ndir, ig);
+    tan_group<G, IPT, K>(u, Ea, Pa, Qa, wb, seed, sens, identity, active, dir0, ndir, ig);
     load_grp<G>(st, g + 3, Ea);
     issue_partials<kNC, G, IPT>(Eb, pt, tstride, tok, Pa, Qa);
-    tan_group<G, IPT, K>(Eb, Pb, Qb, wb, seed, sens, identity, active, dir0, ndir, ig);
+    tan_group<G, IPT, K>(u, Eb, Pb, Qb, wb, seed, sens, identity, active, dir0, ndir, ig);
   }
 }
 
@@ -582,6 +583,7 @@ __device__ __forceinline__ void tangent_walk(const uint4* st, int ngr, const dou
 template <int G, int MB, int IPT, int K, bool GW = false>
 __global__ void __launch_bounds__(32, MB) k_tangent(const __grid_constant__ SweepArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
+  const FmaUnits u = fma_units();
   const int lane = threadIdx.x & 31;
   unsigned char* wb = (GW ? a.wglob + blockIdx.x * a.wglob_stride : smem) + lane * 8;
   const long long ntiles = (a.n + 31) / 32;
@@ -619,7 +621,7 @@ __global__ void __launch_bounds__(32, MB) k_tangent(const __grid_constant__ Swee
     const uint4* st = a.dstream + se.x;
     const int ngr = se.y / G;
     const double* pt = a.partials + static_cast<size_t>(tg * IPT) * tstride + lane;
-    tangent_walk<true, G, IPT, K>(st, ngr, pt, tstride, tok, wb, a.seed, a.sens,
+    tangent_walk<true, G, IPT, K>(u, st, ngr, pt, tstride, tok, wb, a.seed, a.sens,
                                   a.identity_seed != 0, active, dir0, a.ndir, ig);
     work = next;
   }
@@ -631,25 +633,25 @@ __global__ void __launch_bounds__(32, MB) k_tangent(const __grid_constant__ Swee
 
 // Adjoint contribution of form F into a slot holding w, from the entry's adjoint s and the
 // operand's partial m.
-template <int F>
-__device__ __forceinline__ double cf_eval(double w, double m, double s) {
-  if constexpr (F == CF_RF) return __dmul_rn(m, s);
+template <int F, class Units>
+__device__ __forceinline__ double cf_eval(const Units& u, double w, double m, double s) {
+  if constexpr (F == CF_RF) return u_mul(u, m, s);
   else if constexpr (F == CF_RA) return __fma_rn(m, s, w);
   else if constexpr (F == CF_UF) return s;
-  else if constexpr (F == CF_UA) return __dadd_rn(w, s);
+  else if constexpr (F == CF_UA) return u_add(u, w, s);
   else if constexpr (F == CF_MF) return d_neg(s);
-  else if constexpr (F == CF_MA) return __dsub_rn(w, s);
+  else if constexpr (F == CF_MA) return u_sub(u, w, s);
   else if constexpr (F == CF_TF) return d_twice(s);
-  else if constexpr (F == CF_TA) return __dadd_rn(w, d_twice(s));
+  else if constexpr (F == CF_TA) return u_add(u, w, d_twice(s));
   else if constexpr (F == CF_IF) return d_iszero(m) ? 0.0 : s;
-  else return __dadd_rn(w, d_iszero(m) ? 0.0 : s);  // CF_IA
+  else return u_add(u, w, d_iszero(m) ? 0.0 : s);  // CF_IA
 }
 
 // One group of adjoint entries (IPT tiles, direction dir): keys in E, partials in P/Q. Every
 // slot's first contribution (in sweep order) is assigned, so a slot is never read before it
 // is written and the adjoint read by an entry needs no reset afterwards.
-template <int G, int IPT>
-__device__ __forceinline__ void adj_group(const uint4 (&E)[G], const double (&P)[G][IPT],
+template <int G, int IPT, class Units>
+__device__ __forceinline__ void adj_group(const Units& u, const uint4 (&E)[G], const double (&P)[G][IPT],
                                           const double (&Q)[G][IPT], unsigned char* wb,
                                           const IoDesc* seed, const IoDesc* sens,
                                           const bool (&active)[IPT], long long dir,
@@ -665,7 +667,7 @@ __device__ __forceinline__ void adj_group(const uint4 (&E)[G], const double (&P)
           const double sd = active[j]
               ? __ldg(static_cast<const double*>(d.ptr) + io_off(d, dir, cur.z, ig[j])) : 0.0;
           double& w = wj<IPT>(wb, cur.y, j);
-          w = ent_key(cur.w) == AK_OUT_SET ? sd : __dadd_rn(w, sd);
+          w = ent_key(cur.w) == AK_OUT_SET ? sd : u_add(u, w, sd);
         }
       } break;
       case AK_IN: {
@@ -681,11 +683,11 @@ __device__ __forceinline__ void adj_group(const uint4 (&E)[G], const double (&P)
       const double sd = wj<IPT>(wb, cur.x, j);                       \
       if constexpr (BF != CF_N) {                                    \
         double& w1 = wj<IPT>(wb, cur.y, j);                          \
-        w1 = cf_eval<BF>(cf_reads(BF) ? w1 : 0.0, P[i][j], sd);      \
+        w1 = cf_eval<BF>(u, cf_reads(BF) ? w1 : 0.0, P[i][j], sd);      \
       }                                                              \
       if constexpr (CF != CF_N) {                                    \
         double& w2 = wj<IPT>(wb, cur.z, j);                          \
-        w2 = cf_eval<CF>(cf_reads(CF) ? w2 : 0.0, Q[i][j], sd);      \
+        w2 = cf_eval<CF>(u, cf_reads(CF) ? w2 : 0.0, Q[i][j], sd);      \
       }                                                              \
     }                                                                \
     break;
@@ -700,8 +702,8 @@ __device__ __forceinline__ void adj_group(const uint4 (&E)[G], const double (&P)
 // One adjoint sweep of IPT 32-instance tiles by one warp: keyed stream st (body of ngr groups,
 // ngr even, last instruction first), recorded partials at pt (lane-offset, first tile; tile j
 // at pt + j*tstride), work vector at wb (lane-offset, w[slot][j][lane]).
-template <bool kNC, int G, int IPT>
-__device__ __forceinline__ void adjoint_walk(const uint4* st, int ngr, const double* pt,
+template <bool kNC, int G, int IPT, class Units>
+__device__ __forceinline__ void adjoint_walk(const Units& u, const uint4* st, int ngr, const double* pt,
                                              size_t tstride, const bool (&tok)[IPT],
                                              unsigned char* wb, const IoDesc* seed,
                                              const IoDesc* sens, const bool (&active)[IPT],
@@ -719,10 +721,10 @@ __device__ __forceinline__ void adjoint_walk(const uint4* st, int ngr, const dou
   for (int g = 0; g < ngr; g += 2) {
     load_grp<G>(st, g + 2, Eb);
     issue_partials<kNC, G, IPT>(Ea, pt, tstride, tok, Pb, Qb);
-    adj_group<G, IPT>(Ea, Pa, Qa, wb, seed, sens, active, dir, ig);
+    adj_group<G, IPT>(u, Ea, Pa, Qa, wb, seed, sens, active, dir, ig);
     load_grp<G>(st, g + 3, Ea);
     issue_partials<kNC, G, IPT>(Eb, pt, tstride, tok, Pa, Qa);
-    adj_group<G, IPT>(Eb, Pb, Qb, wb, seed, sens, active, dir, ig);
+    adj_group<G, IPT>(u, Eb, Pb, Qb, wb, seed, sens, active, dir, ig);
   }
 }
 
@@ -731,6 +733,7 @@ __device__ __forceinline__ void adjoint_walk(const uint4* st, int ngr, const dou
 template <int G, int MB, int IPT, bool GW = false>
 __global__ void __launch_bounds__(32, MB) k_adjoint(const __grid_constant__ SweepArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
+  const FmaUnits u = fma_units();
   const int lane = threadIdx.x & 31;
   unsigned char* wb = (GW ? a.wglob + blockIdx.x * a.wglob_stride : smem) + lane * 8;
   const long long ntiles = (a.n + 31) / 32;
@@ -762,7 +765,7 @@ __global__ void __launch_bounds__(32, MB) k_adjoint(const __grid_constant__ Swee
       }
     }
     const double* pt = a.partials + static_cast<size_t>(tg * IPT) * tstride + lane;
-    adjoint_walk<true, G, IPT>(st, ngr, pt, tstride, tok, wb, a.seed, a.sens, active, dir, ig);
+    adjoint_walk<true, G, IPT>(u, st, ngr, pt, tstride, tok, wb, a.seed, a.sens, active, dir, ig);
   }
 }
 #undef CGB_J

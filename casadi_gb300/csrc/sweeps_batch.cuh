@@ -51,6 +51,7 @@ cudaError_t launch_wait_probe(const unsigned* flag, unsigned* err, cudaStream_t 
 template <bool kSplit, bool GW>
 __global__ void __launch_bounds__(32, 16) k_batch(const __grid_constant__ BatchArgs b) {
   extern __shared__ __align__(128) unsigned char smem[];
+  const PlainUnits fu;
   const int lane = threadIdx.x;
   uint4* ring = reinterpret_cast<uint4*>(smem);
   unsigned char* wb =
@@ -74,11 +75,11 @@ __global__ void __launch_bounds__(32, 16) k_batch(const __grid_constant__ BatchA
     if (!kSplit || unit.z < 0) {
       // record (or value) unit
       if (it.ndir == 0) {
-        value_walk<false>(it.t.ventries, it.t.n_vblocks, ring, nullptr, wb, io, io + kMaxIo, active,
+        value_walk<false>(fu, it.t.ventries, it.t.n_vblocks, ring, nullptr, wb, io, io + kMaxIo, active,
                           il);
         continue;
       }
-      value_walk<true>(it.t.ventries, it.t.n_vblocks, ring, pt, wb, io, io + kMaxIo, active, il);
+      value_walk<true>(fu, it.t.ventries, it.t.n_vblocks, ring, pt, wb, io, io + kMaxIo, active, il);
       if (kSplit && it.tile_partials) {
         // split item: publish the tile's partials; its directions are separate units
         __threadfence();
@@ -99,7 +100,7 @@ __global__ void __launch_bounds__(32, 16) k_batch(const __grid_constant__ BatchA
     for (int dir = d0; dir < d1; ++dir) {
       if (it.forward) {
         const int2 se = __ldg(it.tan_chunks + dir);
-        tangent_walk<false, kBatchTanGroup, 1, 1>(it.tan_stream + se.x, se.y / kBatchTanGroup,
+        tangent_walk<false, kBatchTanGroup, 1, 1>(fu, it.tan_stream + se.x, se.y / kBatchTanGroup,
                                                   pt, 0, tok1, wb, io + 2 * kMaxIo,
                                                   io + 3 * kMaxIo, true, act1, dir, it.ndir, ig1);
         continue;
@@ -112,7 +113,7 @@ __global__ void __launch_bounds__(32, 16) k_batch(const __grid_constant__ BatchA
           if (d.ptr) static_cast<double*>(d.ptr)[io_off(d, dir, jk.y, il)] = 0.0;
         }
       }
-      adjoint_walk<false, kBatchAdjGroup, 1>(it.adj_stream, it.adj_ngr, pt, 0, tok1, wb,
+      adjoint_walk<false, kBatchAdjGroup, 1>(fu, it.adj_stream, it.adj_ngr, pt, 0, tok1, wb,
                                              io + 2 * kMaxIo, io + 3 * kMaxIo, act1, dir, ig1);
     }
   }

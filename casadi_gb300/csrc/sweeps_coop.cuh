@@ -20,6 +20,7 @@
 template <bool RECORD, bool GW>
 __global__ void __launch_bounds__(kCoopMaxThreads) k_coop(const __grid_constant__ SweepArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
+  const PlainUnits u;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   uint4* ring = reinterpret_cast<uint4*>(smem) + warp * (2 * kEntBlock);
   unsigned char* wb = (GW ? a.wglob + blockIdx.x * a.wglob_stride : smem + nw * kEntRingBytes) +
@@ -37,7 +38,7 @@ __global__ void __launch_bounds__(kCoopMaxThreads) k_coop(const __grid_constant_
     staged_walk(st, se.y, ring, [&](const uint4& e) {
       double* p = RECORD ? pt + static_cast<size_t>((e.w >> kTeamPidxShift) & kTeamPidxMask) * 32
                          : nullptr;
-      value_entry<RECORD>(e, wb, p, a.in, a.out, active, ig, pair);
+      value_entry<RECORD>(u, e, wb, p, a.in, a.out, active, ig, pair);
       if (e.w & kTeamMeet) __syncthreads();
     });
     __syncthreads();  // the next tile's entries write the slots this one reads
@@ -131,6 +132,7 @@ __device__ __forceinline__ bool is_arith(unsigned op) {
 template <int Q, bool GW>
 __global__ void __launch_bounds__(kCoopTanThreads)
     k_tangent_coop(const __grid_constant__ SweepArgs a) {
+  const FmaUnits u = fma_units();
   extern __shared__ __align__(128) unsigned char smem[];
   const int lv = a.t.lv_sz_w;
   double* wd = GW ? reinterpret_cast<double*>(a.wglob + blockIdx.x * a.wglob_stride)
@@ -223,10 +225,10 @@ __global__ void __launch_bounds__(kCoopTanThreads)
           double r;
           switch (op) {
             case D_ADD:
-              r = f == 3u ? __dadd_rn(xb[q], xc[q]) : (f == 1u ? xb[q] : xc[q]);
+              r = f == 3u ? u_add(u, xb[q], xc[q]) : (f == 1u ? xb[q] : xc[q]);
               break;
             case D_SUB:
-              r = f == 3u ? __dsub_rn(xb[q], xc[q]) : (f == 1u ? xb[q] : d_neg(xc[q]));
+              r = f == 3u ? u_sub(u, xb[q], xc[q]) : (f == 1u ? xb[q] : d_neg(xc[q]));
               break;
             case D_NEG:
               r = d_neg(xb[q]);
@@ -241,8 +243,8 @@ __global__ void __launch_bounds__(kCoopTanThreads)
               r = d_iszero(p1[q]) ? 0.0 : xc[q];
               break;
             default:
-              r = f == 3u ? __fma_rn(p0[q], xb[q], __dmul_rn(p1[q], xc[q]))
-                          : (f == 1u ? __dmul_rn(p0[q], xb[q]) : __dmul_rn(p1[q], xc[q]));
+              r = f == 3u ? __fma_rn(p0[q], xb[q], u_mul(u, p1[q], xc[q]))
+                          : (f == 1u ? u_mul(u, p0[q], xb[q]) : u_mul(u, p1[q], xc[q]));
           }
           wd[A * 32 + lane] = r;
           if (lane == 0) act[A] = 1;
@@ -262,6 +264,7 @@ __global__ void __launch_bounds__(kCoopTanThreads)
 template <int Q>
 __global__ void __launch_bounds__(kCoopTanThreads)
     k_adjoint_coop(const __grid_constant__ SweepArgs a) {
+  const FmaUnits u = fma_units();
   extern __shared__ __align__(128) unsigned char smem[];
   const int lv = a.t.rlv_sz_w;
   double* wd = reinterpret_cast<double*>(smem);
@@ -348,7 +351,7 @@ __global__ void __launch_bounds__(kCoopTanThreads)
           const unsigned f = fl[q];
           if (!f) continue;
           if (op == D_OUTPUT) {
-            wd[B * 32 + lane] = (f & 8u) ? sd[q] : __dadd_rn(ob[q], sd[q]);
+            wd[B * 32 + lane] = (f & 8u) ? sd[q] : u_add(u, ob[q], sd[q]);
             if (lane == 0) act[B] = 1;
             continue;
           }
@@ -366,16 +369,16 @@ __global__ void __launch_bounds__(kCoopTanThreads)
             const bool first = f & 8u;
             switch (op) {
               case D_ADD: case D_SUB: case D_ASSIGN:
-                nb = first ? s : __dadd_rn(ob[q], s);
+                nb = first ? s : u_add(u, ob[q], s);
                 break;
               case D_NEG:
-                nb = first ? d_neg(s) : __dsub_rn(ob[q], s);
+                nb = first ? d_neg(s) : u_sub(u, ob[q], s);
                 break;
               case D_TWICE:
-                nb = first ? d_twice(s) : __dadd_rn(ob[q], d_twice(s));
+                nb = first ? d_twice(s) : u_add(u, ob[q], d_twice(s));
                 break;
               default:
-                nb = first ? __dmul_rn(p0[q], s) : __fma_rn(p0[q], s, ob[q]);
+                nb = first ? u_mul(u, p0[q], s) : __fma_rn(p0[q], s, ob[q]);
             }
             wd[B * 32 + lane] = nb;
             if (lane == 0) act[B] = 1;
@@ -386,17 +389,17 @@ __global__ void __launch_bounds__(kCoopTanThreads)
             double nc;
             switch (op) {
               case D_ADD:
-                nc = first ? s : __dadd_rn(old, s);
+                nc = first ? s : u_add(u, old, s);
                 break;
               case D_SUB:
-                nc = first ? d_neg(s) : __dsub_rn(old, s);
+                nc = first ? d_neg(s) : u_sub(u, old, s);
                 break;
               case D_IF_ELSE_ZERO:
                 nc = first ? (d_iszero(p1[q]) ? 0.0 : s)
-                           : (d_iszero(p1[q]) ? __dadd_rn(old, 0.0) : __dadd_rn(old, s));
+                           : (d_iszero(p1[q]) ? u_add(u, old, 0.0) : u_add(u, old, s));
                 break;
               default:
-                nc = first ? __dmul_rn(p1[q], s) : __fma_rn(p1[q], s, old);
+                nc = first ? u_mul(u, p1[q], s) : __fma_rn(p1[q], s, old);
             }
             wd[C * 32 + lane] = nc;
             if (lane == 0) act[C] = 1;

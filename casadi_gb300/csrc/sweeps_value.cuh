@@ -18,8 +18,8 @@ struct PairState {
 
 // One entry. pt: where the instruction's first recorded partial of this lane goes (RECORD);
 // advanced past the partials recorded (rows of 32 lanes).
-template <bool RECORD>
-__device__ __forceinline__ void value_entry(const uint4& e, unsigned char* wb, double*& pt,
+template <bool RECORD, class Units>
+__device__ __forceinline__ void value_entry(const Units& u, const uint4& e, unsigned char* wb, double*& pt,
                                             const IoDesc* in, const IoDesc* out, bool active,
                                             long long ig, PairState& pair) {
 #define CGB_X wreg(wb, e.y)
@@ -45,13 +45,13 @@ __device__ __forceinline__ void value_entry(const uint4& e, unsigned char* wb, d
       return;
     }
     case D_ASSIGN: f = CGB_X; break;
-    case D_ADD: f = __dadd_rn(CGB_X, CGB_Y); break;
-    case D_SUB: f = __dsub_rn(CGB_X, CGB_Y); break;
+    case D_ADD: f = u_add(u, CGB_X, CGB_Y); break;
+    case D_SUB: f = u_sub(u, CGB_X, CGB_Y); break;
     case D_MUL: {
       const double x = CGB_X, y = CGB_Y;
       CGB_REC(y)
       CGB_REC(x)
-      f = __dmul_rn(x, y);
+      f = u_mul(u, x, y);
     } break;
     case D_DIV: {
       const double x = CGB_X, y = CGB_Y;
@@ -64,7 +64,7 @@ __device__ __forceinline__ void value_entry(const uint4& e, unsigned char* wb, d
     case D_SQ: {
       const double x = CGB_X;
       CGB_REC(d_twice(x))
-      f = __dmul_rn(x, x);
+      f = u_mul(u, x, x);
     } break;
     case D_TWICE: f = d_twice(CGB_X); break;
     case D_SIN:
@@ -84,8 +84,8 @@ __device__ __forceinline__ void value_entry(const uint4& e, unsigned char* wb, d
       CGB_REC(d_rcp(x))
     } break;
     case D_SQRT: f = d_sqrt(CGB_X); CGB_REC(d_rcp(d_twice(f))) break;
-    case D_INV: f = d_rcp(CGB_X); CGB_REC(d_neg(__dmul_rn(f, f))) break;
-    case D_TANH: f = d_tanh(CGB_X); CGB_REC(__dsub_rn(1.0, __dmul_rn(f, f))) break;
+    case D_INV: f = d_rcp(CGB_X); CGB_REC(d_neg(u_mul(u, f, f))) break;
+    case D_TANH: f = d_tanh(CGB_X); CGB_REC(u_sub(u, 1.0, u_mul(u, f, f))) break;
     case D_FABS: {
       const double x = CGB_X;
       f = d_fabs(x);
@@ -152,12 +152,12 @@ __device__ __forceinline__ void staged_walk(const uint4* st, int nblocks, uint4*
 
 // The nblocks entry blocks of one tile by one warp.
 template <bool RECORD>
-__device__ __forceinline__ void value_walk(const uint4* st, int nblocks, uint4* ring, double* pt,
+__device__ __forceinline__ void value_walk(const PlainUnits& u, const uint4* st, int nblocks, uint4* ring, double* pt,
                                            unsigned char* wb, const IoDesc* in,
                                            const IoDesc* out, bool active, long long ig) {
   PairState pair;
   staged_walk(st, nblocks, ring, [&](const uint4& e) {
-    value_entry<RECORD>(e, wb, pt, in, out, active, ig, pair);
+    value_entry<RECORD>(u, e, wb, pt, in, out, active, ig, pair);
   });
 }
 
@@ -172,6 +172,7 @@ __device__ __forceinline__ void value_walk(const uint4* st, int nblocks, uint4* 
 template <bool RECORD, bool GW>
 __global__ void __launch_bounds__(32, 28) k_value(const __grid_constant__ SweepArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
+  const PlainUnits u;
   const int lane = threadIdx.x;
   uint4* ring = reinterpret_cast<uint4*>(smem);
   unsigned char* wb =
@@ -181,7 +182,7 @@ __global__ void __launch_bounds__(32, 28) k_value(const __grid_constant__ SweepA
     const long long il = tile * 32 + lane;
     double* pt = RECORD ? a.partials + static_cast<size_t>(tile) * a.t.n_partials * 32 + lane
                         : nullptr;
-    value_walk<RECORD>(a.t.ventries, a.t.n_vblocks, ring, pt, wb, a.in, a.out, il < a.n,
+    value_walk<RECORD>(u, a.t.ventries, a.t.n_vblocks, ring, pt, wb, a.in, a.out, il < a.n,
                        a.i_begin + il);
   }
 }

@@ -71,7 +71,7 @@ __device__ __forceinline__ bool mbar_wait(u64* bar, unsigned parity, volatile in
 // the direction wrote (operand forwarding carries across windows). Only the partials and
 // operands an entry uses are read. (Loading the next entry's partials and operands before the
 // current one computes made the sweep slower on the rollout, 29.9 -> 41.0 ms.)
-__device__ __forceinline__ void win_walk(const uint4* ents, int cnt, const double* pw,
+__device__ __forceinline__ void win_walk(const FmaUnits& u, const uint4* ents, int cnt, const double* pw,
                                          unsigned p0, unsigned char* wb, double& last,
                                          const SweepArgs& a, int dir, bool active,
                                          long long ig) {
@@ -104,21 +104,21 @@ __device__ __forceinline__ void win_walk(const uint4* ents, int cnt, const doubl
         }
         break;
       case (LK_GEN << 2) | 1u:
-        r = __dmul_rn((m & 1u) ? pw[r0 * 32] : 1.0, CGB_WOP(cur.y));
+        r = u_mul(u, (m & 1u) ? pw[r0 * 32] : 1.0, CGB_WOP(cur.y));
         break;
       case (LK_GEN << 2) | 2u:
-        r = __dmul_rn((m & 2u) ? pw[r1 * 32] : 0.0, CGB_WOP(cur.z));
+        r = u_mul(u, (m & 2u) ? pw[r1 * 32] : 0.0, CGB_WOP(cur.z));
         break;
       case (LK_GEN << 2) | 3u:
         r = __fma_rn((m & 1u) ? pw[r0 * 32] : 1.0, CGB_WOP(cur.y),
-                     __dmul_rn((m & 2u) ? pw[r1 * 32] : 0.0, CGB_WOP(cur.z)));
+                     u_mul(u, (m & 2u) ? pw[r1 * 32] : 0.0, CGB_WOP(cur.z)));
         break;
       case (LK_ADD << 2) | 1u: r = CGB_WOP(cur.y); break;
       case (LK_ADD << 2) | 2u: r = CGB_WOP(cur.z); break;
-      case (LK_ADD << 2) | 3u: r = __dadd_rn(CGB_WOP(cur.y), CGB_WOP(cur.z)); break;
+      case (LK_ADD << 2) | 3u: r = u_add(u, CGB_WOP(cur.y), CGB_WOP(cur.z)); break;
       case (LK_SUB << 2) | 1u: r = CGB_WOP(cur.y); break;
       case (LK_SUB << 2) | 2u: r = d_neg(CGB_WOP(cur.z)); break;
-      case (LK_SUB << 2) | 3u: r = __dsub_rn(CGB_WOP(cur.y), CGB_WOP(cur.z)); break;
+      case (LK_SUB << 2) | 3u: r = u_sub(u, CGB_WOP(cur.y), CGB_WOP(cur.z)); break;
       case (LK_NEG << 2) | 1u: r = d_neg(CGB_WOP(cur.y)); break;
       case (LK_TWICE << 2) | 1u: r = d_twice(CGB_WOP(cur.y)); break;
       case (LK_ASSIGN << 2) | 1u: r = CGB_WOP(cur.y); break;
@@ -136,6 +136,7 @@ __device__ __forceinline__ void win_walk(const uint4* ents, int cnt, const doubl
 
 __global__ void __launch_bounds__(kWinMaxThreads, 1)
     k_tangent_win(const __grid_constant__ SweepArgs a) {
+  const FmaUnits u = fma_units();
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ int abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(kWinMaxThreads, 1)
           reinterpret_cast<const unsigned*>(st + static_cast<size_t>(a.win_rows) * 256);
       if (dir_ok) {
         const unsigned e0 = hdr[2 + sj], e1 = hdr[3 + sj];
-        win_walk(reinterpret_cast<const uint4*>(hdr + hw) + e0, static_cast<int>(e1 - e0),
+        win_walk(u, reinterpret_cast<const uint4*>(hdr + hw) + e0, static_cast<int>(e1 - e0),
                  reinterpret_cast<const double*>(st) + lane, hdr[0], wb, last, a, dir, active,
                  ig);
       }
