@@ -15,6 +15,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/casadi_gb300.h"
@@ -211,6 +212,11 @@ struct Tape {
     for (auto& k : tuned)
       for (auto& c : k) c = -1;
   }
+  // per instruction of h_code: which operands are constants (1 b, 2 c; an output's source: 1),
+  // and the constant partial of the other operand (index into pconsts, -1: none)
+  std::vector<unsigned char> const_ops;
+  std::vector<int> const_part;
+  double* d_pconsts = nullptr;
   std::vector<double> h_consts;  // constant pool (host copy, for inlining into callers)
   std::vector<u64> h_code;                            // padded instruction stream
   std::vector<std::unique_ptr<TanPlan>> tan_plans;
@@ -239,6 +245,7 @@ struct Tape {
     }
     cudaFree(d_pofs);
     cudaFree(d_consts);
+    cudaFree(d_pconsts);
     cudaFree(d_absent);
     cudaFree(d_err);
     cudaFree(d_lcode);
@@ -260,6 +267,7 @@ struct Tape {
     v.n_vblocks = n_vblocks;
     v.pofs = d_pofs;
     v.consts = d_consts;
+    v.pconsts = d_pconsts;
     v.absent_in = d_absent;
     v.n_chunks = n_chunks;
     v.n_absent_in = static_cast<int>(absent_in.size());
@@ -620,8 +628,12 @@ struct KEnt {
 
 // The partial loads of an entry: P (its d0) and/or Q (its d1) of an instruction with
 // recorded-partial mask pm whose first recorded partial is pk.
-unsigned pinfo_of(bool lp, bool lq, unsigned pm, int pk) {
+// cp >= 0: the one partial loaded is the tape's constant partial cp.
+unsigned pinfo_of(bool lp, bool lq, unsigned pm, int pk, int cp) {
   if (!lp && !lq) return 0;
+  if (cp >= 0 && lp != lq)
+    return (lp ? kPiP : kPiQ) |
+           ((kPiConst | static_cast<unsigned>(cp)) << (kPiIndexShift - kPiShift));
   return (lp ? kPiP : 0u) | (lq ? kPiQ : 0u) | ((pm & 1u) ? kPiQNext : 0u) |
          (static_cast<unsigned>(pk) << (kPiIndexShift - kPiShift));
 }
@@ -653,11 +665,12 @@ constexpr int kGroupSizeOf[kNumGroupSizes] = {1, 2, 4, 8};
 struct TanRaw {
   unsigned x = 0, y = 0, z = 0;
   unsigned op = 0, kind = 0, f = 0, pm = 0;
-  int pk = 0;
+  unsigned cops = 0;  // constant operands
+  int pk = 0, cp = -1;
   bool mixed = false;
 };
 
-TanRaw tan_raw(u64 w, unsigned flags, int pk) {
+TanRaw tan_raw(u64 w, unsigned flags, int pk, unsigned cops, int cp) {
   const unsigned op = dec_op(w), A = dec_a(w), B = dec_b(w), C = dec_c(w);
   TanRaw e;
   if (op == D_INPUT) {
@@ -672,6 +685,8 @@ TanRaw tan_raw(u64 w, unsigned flags, int pk) {
   e.f = flags & 3u;
   e.pm = dec_pmask(w);
   e.pk = pk;
+  e.cops = cops;
+  e.cp = cp;
   return e;
 }
 
@@ -711,8 +726,9 @@ bool tan_keyed(const TanRaw& e, KEnt* k) {
   k->x = e.x, k->y = e.y, k->z = e.z;
   k->pinfo = 0;
   if (e.mixed) {
-    k->key = TK_MIXED + e.pm;
-    k->pinfo = pinfo_of(e.pm & 1u, e.pm & 2u, e.pm, e.pk);
+    const unsigned m = e.pm & ~e.cops;  // a constant operand is active in no direction
+    k->key = TK_MIXED + m;
+    k->pinfo = pinfo_of(m & 1u, m & 2u, e.pm, e.pk, e.cp);
     return true;
   }
   if (e.kind == LK_OUTPUT) {
@@ -726,7 +742,7 @@ bool tan_keyed(const TanRaw& e, KEnt* k) {
   const int form = tan_form(e);
   if (form < 0) return false;
   k->key = tan_key_of(form);
-  k->pinfo = pinfo_of(tf_uses_p(form), tf_uses_q(form), e.pm, e.pk);
+  k->pinfo = pinfo_of(tf_uses_p(form), tf_uses_q(form), e.pm, e.pk, e.cp);
   return k->key != ~0u;
 }
 
@@ -764,6 +780,50 @@ unsigned adj_key_of(int bf, int cf) {
   CGB_AK_ARITH(CGB_FIND)
 #undef CGB_FIND
   return ~0u;
+}
+
+// The constant operands of every instruction, and the values of the partials that they make
+// constant: the factor of a product, the reciprocal of a divisor (rounded as the record sweep
+// rounds it). Over half the products of the rollout have a constant factor.
+void find_const_operands(Tape& t) {
+  const size_t n = t.h_code.size();
+  t.const_ops.assign(n, 0);
+  t.const_part.assign(n, -1);
+  std::vector<char> isc(std::max(1, t.sz_w), 0);
+  for (size_t k = 0; k < n; ++k) {
+    const u64 w = t.h_code[k];
+    const unsigned op = dec_op(w);
+    if (op == D_NOP) continue;
+    if (op == D_OUTPUT) {
+      t.const_ops[k] = isc[dec_b(w)] ? 1 : 0;
+      continue;
+    }
+    if (op != D_CONST && op != D_INPUT)
+      t.const_ops[k] = static_cast<unsigned char>((isc[dec_b(w)] ? 1 : 0) |
+                                                  (is_binary(op) && isc[dec_c(w)] ? 2 : 0));
+    isc[dec_a(w)] = op == D_CONST;
+  }
+}
+std::vector<double> const_partials(Tape& t) {
+  std::vector<double> vals;
+  std::unordered_map<u64, int> at;  // by bits
+  std::vector<double> slot(std::max(1, t.sz_w), 0.0);
+  for (size_t k = 0; k < t.h_code.size(); ++k) {
+    const u64 w = t.h_code[k];
+    const unsigned op = dec_op(w), cops = t.const_ops[k];
+    if (op == D_CONST) slot[dec_a(w)] = t.h_consts[dec_b(w)];
+    double v;
+    if (op == D_MUL && (cops == 1 || cops == 2)) v = slot[cops == 1 ? dec_b(w) : dec_c(w)];
+    else if (op == D_DIV && cops == 2) v = 1.0 / slot[dec_c(w)];
+    else continue;
+    if (vals.size() >= kPiIndexMask) break;
+    u64 b;
+    std::memcpy(&b, &v, 8);
+    const auto hit = at.emplace(b, static_cast<int>(vals.size()));
+    if (hit.second) vals.push_back(v);
+    t.const_part[k] = hit.first->second;
+  }
+  return vals;
 }
 
 std::vector<int> partial_starts(const Tape& t) {
@@ -901,9 +961,9 @@ const TanPlan* tan_plan(Tape& t, int ndir, int dw, int ch, bool identity,
       bool uniform = true;
       for (int d = 1; d < kv; ++d) uniform = uniform && ((gb >> (2 * d)) & 3u) == f0;
       if (uniform) {
-        raw.push_back(tan_raw(w, f0, pk[k]));
+        raw.push_back(tan_raw(w, f0, pk[k], t.const_ops[k], t.const_part[k]));
       } else {
-        TanRaw e = tan_raw(w, 0, pk[k]);
+        TanRaw e = tan_raw(w, 0, pk[k], t.const_ops[k], t.const_part[k]);
         e.x |= (lean_kind(op) << 19) | ((gb & 0xffu) << 24);
         e.mixed = true;
         raw.push_back(e);
@@ -1110,8 +1170,9 @@ const AdjPlan* adj_plan(Tape& t, int dw, int ch, const std::vector<char>& seeded
     const unsigned op = dec_op(w), A = dec_a(w), B = dec_b(w), C = dec_c(w);
     unsigned f = 0;
     if (op == D_NOP) continue;
+    const unsigned cops = t.const_ops[kk];  // no contribution goes to a constant
     if (op == D_OUTPUT) {
-      if (seeded[A]) {
+      if (seeded[A] && !cops) {
         f = 32u | (act[B] ? 0u : 8u);
         act[B] = 1;
       }
@@ -1130,11 +1191,11 @@ const AdjPlan* adj_plan(Tape& t, int dw, int ch, const std::vector<char>& seeded
     } else if (act[A]) {
       f = 1;
       act[A] = 0;
-      if (carries_d0(op)) {
+      if (carries_d0(op) && !(cops & 1u)) {
         f |= 2u | (act[B] ? 0u : 8u);
         act[B] = 1;
       }
-      if (carries_d1(op)) {
+      if (carries_d1(op) && !(cops & 2u)) {
         f |= 4u | (act[C] ? 0u : 16u);
         act[C] = 1;
       }
@@ -1162,16 +1223,22 @@ const AdjPlan* adj_plan(Tape& t, int dw, int ch, const std::vector<char>& seeded
       continue;
     } else {
       const unsigned kind = lean_kind(op), pm = dec_pmask(w);
-      const int bf = adj_bform(op, kind, pm, f), cf = adj_cform(kind, pm, f);
+      int bf = adj_bform(op, kind, pm, f), cf = adj_cform(kind, pm, f);
       if (bf == CF_N && cf == CF_N) continue;
       e.x = A * 256u, e.y = B * 256u, e.z = C * 256u;
+      if (bf == CF_N && (cf == CF_UF || cf == CF_UA || cf == CF_MF || cf == CF_MA)) {
+        // c + y, c - y with a constant c: the one contribution takes the first operand's form
+        std::swap(bf, cf);
+        std::swap(e.y, e.z);
+      }
       e.key = (bf < 0 || cf < 0) ? ~0u : adj_key_of(bf, cf);
       if (e.key == ~0u) {
         *err = fail(CASADI_GB300_ERR_UNSUPPORTED, "adjoint entry of op %u has no form", op);
         return nullptr;
       }
       e.pinfo = pinfo_of(bf == CF_RF || bf == CF_RA,
-                         cf == CF_RF || cf == CF_RA || cf == CF_IF || cf == CF_IA, pm, pk[kk]);
+                         cf == CF_RF || cf == CF_RA || cf == CF_IF || cf == CF_IA, pm, pk[kk],
+                         t.const_part[kk]);
     }
     ents.push_back(e);
   }
@@ -1230,8 +1297,8 @@ constexpr int kLevelWidth = 64;      // instructions per level
 // the blocks. The costs (latencies in dependent FP64 operations of about 150 cycles, dispatch
 // and work-vector accesses included) balance the warps: a sincos takes 820 cycles, a recorded
 // division 700, a first read of an input a trip to L2 or HBM.
-void team_entries(const Levels& lv, int warps, const std::vector<double>& consts,
-                  std::vector<uint4>& entries, std::vector<int2>& at) {
+void team_entries(const Tape& t, const Levels& lv, int warps, std::vector<uint4>& entries,
+                  std::vector<int2>& at) {
   float cost[64];
   for (float& c : cost) c = 1.0f;
   cost[D_CONST] = 0.5f;
@@ -1253,7 +1320,7 @@ void team_entries(const Levels& lv, int warps, const std::vector<double>& consts
         open = false;
         continue;
       }
-      uint4 e = value_entry_of(lv.code[k], consts.data());
+      uint4 e = value_entry_of(lv.code[k], t.h_consts.data(), t.const_ops[lv.src[k]]);
       e.w |= (static_cast<unsigned>(lv.pidx[k]) & kTeamPidxMask) << kTeamPidxShift;
       entries.push_back(e);
       open = true;
@@ -1304,7 +1371,7 @@ bool ensure_levels(Tape& t, bool reverse = false) {
   for (int k = 0; k < kTeamSizes && ok && !reverse; ++k) {
     std::vector<uint4> entries;
     std::vector<int2> at;
-    team_entries(lv, 4 << k, t.h_consts, entries, at);
+    team_entries(t, lv, 4 << k, entries, at);
     ok = upload(&team[k], entries) == cudaSuccess && upload(&team_at[k], at) == cudaSuccess;
   }
   if (!ok) {
@@ -2006,7 +2073,12 @@ int make_tape(const casadi_gb300_atomic* alg, int n_instr, int n_in, const int* 
   if ((e = cudaMalloc(&t->d_code, code.size() * sizeof(u64))) != cudaSuccess)
     return cuda_fail(e, "cudaMalloc(code)");
   std::vector<uint4> ventries;
-  for (int k = 0; k < n_instr; ++k) ventries.push_back(value_entry_of(code[k], consts.data()));
+  find_const_operands(*t);
+  std::vector<double> pconsts = const_partials(*t);
+  if ((e = upload(&t->d_pconsts, pconsts)) != cudaSuccess)
+    return cuda_fail(e, "upload constant partials");
+  for (int k = 0; k < n_instr; ++k)
+    ventries.push_back(value_entry_of(code[k], consts.data(), t->const_ops[k]));
   t->n_vblocks = pad_block(ventries);
   if ((e = upload(&t->d_ventries, ventries)) != cudaSuccess)
     return cuda_fail(e, "upload value entries");

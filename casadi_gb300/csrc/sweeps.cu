@@ -378,24 +378,27 @@ __device__ __forceinline__ void load_grp(const uint4* st, int gi, uint4 (&E)[G])
 }
 
 // The partials group E describes (those of the next group) for IPT tiles, tile j's block at
-// pt + j*tstride; tiles past the wave's end are not read. Registers of partials not loaded
+// pt + j*tstride, constant ones at pc; tiles past the wave's end are not read. Registers of partials not loaded
 // keep stale values that the entries' cases do not read.
 template <bool kNC, int G, int IPT>
 __device__ __forceinline__ void issue_partials(const uint4 (&E)[G], const double* pt,
-                                               size_t tstride, const bool (&tok)[IPT],
+                                               const double* pc, size_t tstride, const bool (&tok)[IPT],
                                                double (&P)[G][IPT], double (&Q)[G][IPT]) {
 #pragma unroll
   for (int i = 0; i < G; ++i) {
     const unsigned w = E[i].w;
-    const double* pp = pt + static_cast<size_t>(w >> kPiIndexShift) * 32;
+    const bool isc = static_cast<int>(w) < 0;  // kPiConst: the same value for every instance
+    const unsigned idx = (w >> kPiIndexShift) & kPiIndexMask;
+    const double* pp = isc ? pc + idx : pt + static_cast<size_t>(idx) * 32;
+    const size_t ts = isc ? 0 : tstride;
     // Q's row: P's, or the next one (32 doubles on) when kPiQNext is set; the shift moves that
     // bit (bit 8 of w) onto the value 32 (bit 5)
     static_assert(kPiQNext << kPiShift == (32u << 3), "kPiQNext sits at bit 8 of the key word");
     const double* pq = pp + ((w >> 3) & 32u);
 #pragma unroll
     for (int j = 0; j < IPT; ++j) {
-      if ((w & (kPiP << kPiShift)) && tok[j]) P[i][j] = ld_partial<kNC>(pp + j * tstride);
-      if ((w & (kPiQ << kPiShift)) && tok[j]) Q[i][j] = ld_partial<kNC>(pq + j * tstride);
+      if ((w & (kPiP << kPiShift)) && tok[j]) P[i][j] = ld_partial<kNC>(pp + j * ts);
+      if ((w & (kPiQ << kPiShift)) && tok[j]) Q[i][j] = ld_partial<kNC>(pq + j * ts);
     }
   }
 }
@@ -547,6 +550,7 @@ __device__ __forceinline__ void tan_group(const Units& u, const uint4 (&E)[G], c
 // the K directions).
 template <bool kNC, int G, int IPT, int K, class Units>
 __device__ __forceinline__ void tangent_walk(const Units& u, const uint4* st, int ngr, const double* pt,
+                                             const double* pc,
                                              size_t tstride, const bool (&tok)[IPT],
                                              unsigned char* wb, const IoDesc* seed,
                                              const IoDesc* sens, bool identity,
@@ -559,15 +563,15 @@ __device__ __forceinline__ void tangent_walk(const Units& u, const uint4* st, in
 #pragma unroll
     for (int j = 0; j < IPT; ++j) Pa[i][j] = Qa[i][j] = Pb[i][j] = Qb[i][j] = 0.0;
   load_grp<G>(st, 0, Eb);  // the header: the first group's partials
-  issue_partials<kNC, G, IPT>(Eb, pt, tstride, tok, Pa, Qa);
+  issue_partials<kNC, G, IPT>(Eb, pt, pc, tstride, tok, Pa, Qa);
   load_grp<G>(st, 1, Ea);
 #pragma unroll 1
   for (int g = 0; g < ngr; g += 2) {
     load_grp<G>(st, g + 2, Eb);
-    issue_partials<kNC, G, IPT>(Ea, pt, tstride, tok, Pb, Qb);
+    issue_partials<kNC, G, IPT>(Ea, pt, pc, tstride, tok, Pb, Qb);
     tan_group<G, IPT, K>(u, Ea, Pa, Qa, wb, seed, sens, identity, active, dir0, ndir, ig);
     load_grp<G>(st, g + 3, Ea);
-    issue_partials<kNC, G, IPT>(Eb, pt, tstride, tok, Pa, Qa);
+    issue_partials<kNC, G, IPT>(Eb, pt, pc, tstride, tok, Pa, Qa);
     tan_group<G, IPT, K>(u, Eb, Pb, Qb, wb, seed, sens, identity, active, dir0, ndir, ig);
   }
 }
@@ -621,7 +625,7 @@ __global__ void __launch_bounds__(32, MB) k_tangent(const __grid_constant__ Swee
     const uint4* st = a.dstream + se.x;
     const int ngr = se.y / G;
     const double* pt = a.partials + static_cast<size_t>(tg * IPT) * tstride + lane;
-    tangent_walk<true, G, IPT, K>(u, st, ngr, pt, tstride, tok, wb, a.seed, a.sens,
+    tangent_walk<true, G, IPT, K>(u, st, ngr, pt, a.t.pconsts, tstride, tok, wb, a.seed, a.sens,
                                   a.identity_seed != 0, active, dir0, a.ndir, ig);
     work = next;
   }
@@ -704,6 +708,7 @@ __device__ __forceinline__ void adj_group(const Units& u, const uint4 (&E)[G], c
 // at pt + j*tstride), work vector at wb (lane-offset, w[slot][j][lane]).
 template <bool kNC, int G, int IPT, class Units>
 __device__ __forceinline__ void adjoint_walk(const Units& u, const uint4* st, int ngr, const double* pt,
+                                             const double* pc,
                                              size_t tstride, const bool (&tok)[IPT],
                                              unsigned char* wb, const IoDesc* seed,
                                              const IoDesc* sens, const bool (&active)[IPT],
@@ -715,15 +720,15 @@ __device__ __forceinline__ void adjoint_walk(const Units& u, const uint4* st, in
 #pragma unroll
     for (int j = 0; j < IPT; ++j) Pa[i][j] = Qa[i][j] = Pb[i][j] = Qb[i][j] = 0.0;
   load_grp<G>(st, 0, Eb);  // the header: the first group's partials
-  issue_partials<kNC, G, IPT>(Eb, pt, tstride, tok, Pa, Qa);
+  issue_partials<kNC, G, IPT>(Eb, pt, pc, tstride, tok, Pa, Qa);
   load_grp<G>(st, 1, Ea);
 #pragma unroll 1
   for (int g = 0; g < ngr; g += 2) {
     load_grp<G>(st, g + 2, Eb);
-    issue_partials<kNC, G, IPT>(Ea, pt, tstride, tok, Pb, Qb);
+    issue_partials<kNC, G, IPT>(Ea, pt, pc, tstride, tok, Pb, Qb);
     adj_group<G, IPT>(u, Ea, Pa, Qa, wb, seed, sens, active, dir, ig);
     load_grp<G>(st, g + 3, Ea);
-    issue_partials<kNC, G, IPT>(Eb, pt, tstride, tok, Pa, Qa);
+    issue_partials<kNC, G, IPT>(Eb, pt, pc, tstride, tok, Pa, Qa);
     adj_group<G, IPT>(u, Eb, Pb, Qb, wb, seed, sens, active, dir, ig);
   }
 }
@@ -765,7 +770,7 @@ __global__ void __launch_bounds__(32, MB) k_adjoint(const __grid_constant__ Swee
       }
     }
     const double* pt = a.partials + static_cast<size_t>(tg * IPT) * tstride + lane;
-    adjoint_walk<true, G, IPT>(u, st, ngr, pt, tstride, tok, wb, a.seed, a.sens, active, dir, ig);
+    adjoint_walk<true, G, IPT>(u, st, ngr, pt, a.t.pconsts, tstride, tok, wb, a.seed, a.sens, active, dir, ig);
   }
 }
 #undef CGB_J

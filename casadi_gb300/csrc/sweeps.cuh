@@ -45,7 +45,12 @@ __host__ __device__ constexpr int group_slot(int g) { return g >= 8 ? 3 : g >= 4
 __host__ __device__ constexpr unsigned ent_key(unsigned w) { return w & 63u; }
 constexpr unsigned kPiP = 1u, kPiQ = 2u, kPiQNext = 4u;  // partial-info bits (w >> 6)
 constexpr unsigned kPiShift = 6, kPiIndexShift = 9;
-static_assert(kMaxPartials <= (1u << (32 - kPiIndexShift)), "partial indices fit the key word");
+// bit 22 of the index: not a recorded partial but entry `index` of the tape's constant partials
+// (TapeView::pconsts; the factor of a product with a constant, the reciprocal of a constant
+// divisor), which takes no trip to the partials in HBM
+constexpr unsigned kPiConst = 1u << 22, kPiIndexMask = kPiConst - 1;
+static_assert(kMaxPartials <= kPiConst, "partial indices fit the key word");
+static_assert(kPiConst << kPiIndexShift == 1u << 31, "kPiConst is the key word's top bit");
 
 // Tangent forms: the tangent of one arithmetic entry from operand tangents a (y) and b (z) and
 // the recorded partials p (d0) and q (d1).
@@ -128,7 +133,8 @@ static_assert(AK_COUNT <= 64, "adjoint keys fit 6 bits");
 //   y, z  byte offsets of the operand slots (CONST: the constant's low and high word; INPUT:
 //      input index and nonzero; OUTPUT: slot offset and nonzero)
 //   w  bits 0-5 the key: the opcode, or VK_SIN_REUSE / VK_COS_REUSE for a SIN or COS that takes
-//      the previous pair; bits 6-7 its recorded-partial mask; in the streams of a cooperative
+//      the previous pair; bits 6-7 which of its recorded partials are stored (their places in the
+//      order stay: the partials of constant operands are never read); in the streams of a cooperative
 //      sweep's warps also its first recorded partial (bits 8-30) and whether the team meets
 //      after it (bit 31)
 constexpr int kEntBlock = 16;  // entries staged at a time
@@ -136,10 +142,11 @@ constexpr int kEntRingBytes = 2 * kEntBlock * 16;
 constexpr unsigned kTeamPidxShift = 8, kTeamPidxMask = (1u << 23) - 1, kTeamMeet = 1u << 31;
 constexpr int kTeamSizes = 4;  // teams of 4, 8, 16 and 32 warps
 enum ValueKey : unsigned { VK_SIN_REUSE = 54, VK_COS_REUSE = 55 };
-inline uint4 value_entry_of(u64 ins, const double* consts) {
-  const unsigned op = dec_op(ins);
+// const_ops: the operands that are constants (1 b, 2 c): their partials are not stored.
+inline uint4 value_entry_of(u64 ins, const double* consts, unsigned const_ops) {
+  const unsigned op = dec_op(ins), keep = (partial_mask(op) & ~const_ops) << 6;
   uint4 e = make_uint4(dec_a(ins) * 256u, dec_b(ins) * 256u, dec_c(ins) * 256u,
-                       op | (partial_mask(op) << 6));
+                       op | keep);
   if (op == D_CONST) {
     u64 b;
     memcpy(&b, consts + dec_b(ins), 8);
@@ -152,7 +159,7 @@ inline uint4 value_entry_of(u64 ins, const double* consts) {
     e.x = dec_a(ins);
     e.z = dec_c(ins);
   } else if ((op == D_SIN || op == D_COS) && (ins & kSincosReuse)) {
-    e.w = (op == D_SIN ? VK_SIN_REUSE : VK_COS_REUSE) | (partial_mask(op) << 6);
+    e.w = (op == D_SIN ? VK_SIN_REUSE : VK_COS_REUSE) | keep;
   }
   return e;
 }
@@ -171,6 +178,7 @@ struct TapeView {
   const u64* code;          // kChunk-padded instruction stream (NOP padding)
   const int* pofs;          // pofs[k]: partials recorded before instruction k*kPofsGran
   const double* consts;     // constant pool
+  const double* pconsts;    // constant partials (kPiConst)
   const int2* absent_in;    // (input, nonzero) pairs the tape never reads
   const uint4* ventries;    // value entries of the scheduled order
   int n_vblocks;            // their blocks of kEntBlock (NOP padding)

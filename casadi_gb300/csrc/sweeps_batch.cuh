@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(32, 16) k_batch(const __grid_constant__ BatchA
       if (it.forward) {
         const int2 se = __ldg(it.tan_chunks + dir);
         tangent_walk<false, kBatchTanGroup, 1, 1>(fu, it.tan_stream + se.x, se.y / kBatchTanGroup,
-                                                  pt, 0, tok1, wb, io + 2 * kMaxIo,
+                                                  pt, it.t.pconsts, 0, tok1, wb, io + 2 * kMaxIo,
                                                   io + 3 * kMaxIo, true, act1, dir, it.ndir, ig1);
         continue;
       }
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(32, 16) k_batch(const __grid_constant__ BatchA
           if (d.ptr) static_cast<double*>(d.ptr)[io_off(d, dir, jk.y, il)] = 0.0;
         }
       }
-      adjoint_walk<false, kBatchAdjGroup, 1>(fu, it.adj_stream, it.adj_ngr, pt, 0, tok1, wb,
+      adjoint_walk<false, kBatchAdjGroup, 1>(fu, it.adj_stream, it.adj_ngr, pt, it.t.pconsts, 0, tok1, wb,
                                              io + 2 * kMaxIo, io + 3 * kMaxIo, act1, dir, ig1);
     }
   }

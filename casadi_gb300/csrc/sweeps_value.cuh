@@ -24,11 +24,13 @@ __device__ __forceinline__ void value_entry(const Units& u, const uint4& e, unsi
                                             long long ig, PairState& pair) {
 #define CGB_X wreg(wb, e.y)
 #define CGB_Y wreg(wb, e.z)
-#define CGB_REC(d)                  \
-  if (RECORD) {                     \
-    const double dv = (d);          \
-    if (active) *pt = dv;           \
-    pt += 32;                       \
+#define CGB_REC(bit, d)                     \
+  if (RECORD) {                             \
+    if (e.w & (bit)) {                      \
+      const double dv = (d);                \
+      if (active) *pt = dv;                 \
+    }                                       \
+    pt += 32;                               \
   }
   double f;
   switch (e.w & 63u) {
@@ -49,21 +51,21 @@ __device__ __forceinline__ void value_entry(const Units& u, const uint4& e, unsi
     case D_SUB: f = u_sub(u, CGB_X, CGB_Y); break;
     case D_MUL: {
       const double x = CGB_X, y = CGB_Y;
-      CGB_REC(y)
-      CGB_REC(x)
+      CGB_REC(64u, y)
+      CGB_REC(128u, x)
       f = u_mul(u, x, y);
     } break;
     case D_DIV: {
       const double x = CGB_X, y = CGB_Y;
       const FxDivisor d = fx_divisor(y);
       f = d_div(x, y, d);
-      CGB_REC(d_div(1.0, y, d))
-      CGB_REC(d_div(d_neg(f), y, d))
+      CGB_REC(64u, d_div(1.0, y, d))
+      CGB_REC(128u, d_div(d_neg(f), y, d))
     } break;
     case D_NEG: f = d_neg(CGB_X); break;
     case D_SQ: {
       const double x = CGB_X;
-      CGB_REC(d_twice(x))
+      CGB_REC(64u, d_twice(x))
       f = u_mul(u, x, x);
     } break;
     case D_TWICE: f = d_twice(CGB_X); break;
@@ -75,21 +77,21 @@ __device__ __forceinline__ void value_entry(const Units& u, const uint4& e, unsi
       if (k == D_SIN || k == D_COS) d_sincos(CGB_X, &pair.s, &pair.c);
       const bool sine = k == D_SIN || k == VK_SIN_REUSE;
       f = sine ? pair.s : pair.c;
-      CGB_REC(sine ? pair.c : d_neg(pair.s))
+      CGB_REC(64u, sine ? pair.c : d_neg(pair.s))
     } break;
-    case D_EXP: f = d_exp(CGB_X); CGB_REC(f) break;
+    case D_EXP: f = d_exp(CGB_X); CGB_REC(64u, f) break;
     case D_LOG: {
       const double x = CGB_X;
       f = d_log(x);
-      CGB_REC(d_rcp(x))
+      CGB_REC(64u, d_rcp(x))
     } break;
-    case D_SQRT: f = d_sqrt(CGB_X); CGB_REC(d_rcp(d_twice(f))) break;
-    case D_INV: f = d_rcp(CGB_X); CGB_REC(d_neg(u_mul(u, f, f))) break;
-    case D_TANH: f = d_tanh(CGB_X); CGB_REC(u_sub(u, 1.0, u_mul(u, f, f))) break;
+    case D_SQRT: f = d_sqrt(CGB_X); CGB_REC(64u, d_rcp(d_twice(f))) break;
+    case D_INV: f = d_rcp(CGB_X); CGB_REC(64u, d_neg(u_mul(u, f, f))) break;
+    case D_TANH: f = d_tanh(CGB_X); CGB_REC(64u, u_sub(u, 1.0, u_mul(u, f, f))) break;
     case D_FABS: {
       const double x = CGB_X;
       f = d_fabs(x);
-      CGB_REC(d_sign(x))
+      CGB_REC(64u, d_sign(x))
     } break;
     default: {
       // the other operations, out of line: one copy serves every kernel
@@ -97,8 +99,9 @@ __device__ __forceinline__ void value_entry(const Units& u, const uint4& e, unsi
       if constexpr (RECORD) {
         const FunDer r = rare_fun_der(e.w & 63u, x, y);
         f = r.f;
-        if (e.w & 64u) CGB_REC(r.d0)
-        if (e.w & 128u) CGB_REC(r.d1)
+        const unsigned m = partial_mask(e.w & 63u);
+        if (m & 1u) CGB_REC(64u, r.d0)
+        if (m & 2u) CGB_REC(128u, r.d1)
       } else {
         f = rare_fun(e.w & 63u, x, y);
       }
