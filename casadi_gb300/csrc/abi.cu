@@ -137,7 +137,16 @@ struct AdjPlan {
   int2 h_chunks[kNumGroupSizes] = {};
   int2* d_zero = nullptr;
   int n_zero = 0;
+  // the cooperative sweep: one keyed stream per warp of a 4 << k warp team over the reverse level
+  // schedule, laid out for groups of kTeamAdjGroup
+  int team_state = 0;  // 0 not built, 1 built, -1 unavailable
+  uint4* d_team[kTeamAdjSizes] = {};
+  int2* d_team_at[kTeamAdjSizes] = {};
   ~AdjPlan() {
+    for (int k = 0; k < kTeamAdjSizes; ++k) {
+      cudaFree(d_team[k]);
+      cudaFree(d_team_at[k]);
+    }
     for (int g = 0; g < kNumGroupSizes; ++g) {
       cudaFree(d_stream[g]);
       cudaFree(d_chunks[g]);
@@ -179,8 +188,8 @@ struct Tape {
   int rlv_state = 0;
   u64* d_rcode = nullptr;
   int* d_rbegin = nullptr;
-  int* d_rpidx = nullptr;
   int n_rlevels = 0, rlv_sz_w = 0;
+  std::unique_ptr<Levels> h_rlv;  // for the adjoint plans' teams
   // global work vector: per-CTA blocks, grown on demand; uses on different streams are
   // ordered by gw_event
   std::mutex gw_mtx;
@@ -253,7 +262,6 @@ struct Tape {
     cudaFree(d_lpidx);
     cudaFree(d_rcode);
     cudaFree(d_rbegin);
-    cudaFree(d_rpidx);
     if (gw_event) cudaEventSynchronize(gw_event);
     cudaFree(d_gw);
     if (gw_event) cudaEventDestroy(gw_event);
@@ -281,7 +289,6 @@ struct Tape {
     v.lv_sz_w = lv_sz_w;
     v.rcode = d_rcode;
     v.rbegin = d_rbegin;
-    v.rpidx = d_rpidx;
     v.n_rlevels = n_rlevels;
     v.rlv_sz_w = rlv_sz_w;
     return v;
@@ -1149,28 +1156,23 @@ const WinPlan* win_plan(Tape& t, int ndir, bool identity, const std::vector<char
   return t.win_plans.back().get();
 }
 
-// Structural activity of the adjoint sweep (direction-independent), last instruction first.
-// Flags: 1 adjoint of the result is nonzero, 2/4 operand b/c receives a contribution,
-// 8/16 that contribution is the first to b/c, 32 a seeded output. Entries without work are
-// left out of the stream; inputs whose adjoint is structurally zero go to the zero list.
-const AdjPlan* adj_plan(Tape& t, int dw, int ch, const std::vector<char>& seeded, int* err) {
-  std::lock_guard<std::mutex> lk(t.shape_mtx);
-  for (auto& p : t.adj_plans)
-    if (p->ch == ch && p->dw == dw && p->seeded == seeded) return p.get();
-  auto p = std::make_unique<AdjPlan>();
-  p->ch = ch;
-  p->dw = dw;
-  p->seeded = seeded;
-  const size_t nc = t.h_code.size();
+// Keyed adjoint entries of `code` walked from its last instruction to its first, one per
+// instruction (AK_NOP: no work): `slots` the length of its work vector, src its instructions'
+// indices in t.h_code (null: the same), pk their first recorded partials. With `zero`, the inputs
+// whose sensitivity is a structural zero are appended to it.
+bool adj_entries(const Tape& t, const std::vector<u64>& code, const int* src,
+                 const std::vector<int>& pk, int slots, const std::vector<char>& seeded,
+                 std::vector<KEnt>* ents, std::vector<int2>* zero, int* err) {
+  const size_t nc = code.size();
   std::vector<unsigned char> bits(nc, 0);
-  std::vector<char> act(std::max(1, t.sz_w), 0);
-  std::vector<int2> zero(t.absent_in);
+  std::vector<char> act(std::max(1, slots), 0);
   for (size_t kk = nc; kk-- > 0;) {
-    const u64 w = t.h_code[kk];
+    const u64 w = code[kk];
     const unsigned op = dec_op(w), A = dec_a(w), B = dec_b(w), C = dec_c(w);
     unsigned f = 0;
     if (op == D_NOP) continue;
-    const unsigned cops = t.const_ops[kk];  // no contribution goes to a constant
+    // no contribution goes to a constant
+    const unsigned cops = t.const_ops[src ? src[kk] : static_cast<int>(kk)];
     if (op == D_OUTPUT) {
       if (seeded[A] && !cops) {
         f = 32u | (act[B] ? 0u : 8u);
@@ -1181,7 +1183,7 @@ const AdjPlan* adj_plan(Tape& t, int dw, int ch, const std::vector<char>& seeded
         f = 1;
         act[A] = 0;
       } else {
-        zero.push_back(make_int2(static_cast<int>(B), static_cast<int>(C)));
+        if (zero) zero->push_back(make_int2(static_cast<int>(B), static_cast<int>(C)));
       }
     } else if (op == D_CONST) {
       if (act[A]) {
@@ -1202,15 +1204,13 @@ const AdjPlan* adj_plan(Tape& t, int dw, int ch, const std::vector<char>& seeded
     }
     bits[kk] = static_cast<unsigned char>(f);
   }
-  // keyed entries in sweep order (last instruction first). Constants and arithmetic entries
-  // that pass nothing on are left out: every slot's first contribution is assigned, so no
-  // adjoint needs resetting after it is read.
-  const std::vector<int> pk = partial_starts(t);
-  std::vector<KEnt> ents;
+  // Constants and arithmetic entries that pass nothing on are left out: every slot's first
+  // contribution is assigned, so no adjoint needs resetting after it is read.
+  ents->assign(nc, KEnt());
   for (size_t kk = nc; kk-- > 0;) {
     const unsigned f = bits[kk];
     if (!f) continue;
-    const u64 w = t.h_code[kk];
+    const u64 w = code[kk];
     const unsigned op = dec_op(w), A = dec_a(w), B = dec_b(w), C = dec_c(w);
     KEnt e;
     if (op == D_OUTPUT) {
@@ -1234,14 +1234,35 @@ const AdjPlan* adj_plan(Tape& t, int dw, int ch, const std::vector<char>& seeded
       e.key = (bf < 0 || cf < 0) ? ~0u : adj_key_of(bf, cf);
       if (e.key == ~0u) {
         *err = fail(CASADI_GB300_ERR_UNSUPPORTED, "adjoint entry of op %u has no form", op);
-        return nullptr;
+        return false;
       }
       e.pinfo = pinfo_of(bf == CF_RF || bf == CF_RA,
                          cf == CF_RF || cf == CF_RA || cf == CF_IF || cf == CF_IA, pm, pk[kk],
-                         t.const_part[kk]);
+                         t.const_part[src ? src[kk] : static_cast<int>(kk)]);
     }
-    ents.push_back(e);
+    (*ents)[kk] = e;
   }
+  return true;
+}
+
+// Structural activity of the adjoint sweep (direction-independent), last instruction first.
+// Flags: 1 adjoint of the result is nonzero, 2/4 operand b/c receives a contribution,
+// 8/16 that contribution is the first to b/c, 32 a seeded output. Entries without work are
+// left out of the stream; inputs whose adjoint is structurally zero go to the zero list.
+AdjPlan* adj_plan(Tape& t, int dw, int ch, const std::vector<char>& seeded, int* err) {
+  std::lock_guard<std::mutex> lk(t.shape_mtx);
+  for (auto& p : t.adj_plans)
+    if (p->ch == ch && p->dw == dw && p->seeded == seeded) return p.get();
+  auto p = std::make_unique<AdjPlan>();
+  p->ch = ch;
+  p->dw = dw;
+  p->seeded = seeded;
+  std::vector<int2> zero(t.absent_in);
+  std::vector<KEnt> all_ents, ents;
+  if (!adj_entries(t, t.h_code, nullptr, partial_starts(t), t.sz_w, seeded, &all_ents, &zero, err))
+    return nullptr;
+  for (size_t kk = all_ents.size(); kk-- > 0;)
+    if (all_ents[kk].key != AK_NOP) ents.push_back(all_ents[kk]);
   p->n_zero = static_cast<int>(zero.size());
   cudaError_t e = cudaSuccess;
   for (int gs = 0; gs < kNumGroupSizes && e == cudaSuccess; ++gs) {
@@ -1256,6 +1277,71 @@ const AdjPlan* adj_plan(Tape& t, int dw, int ch, const std::vector<char>& seeded
   }
   t.adj_plans.push_back(std::move(p));
   return t.adj_plans.back().get();
+}
+
+// The adjoint plan's streams for teams of 4, 8 and 16 warps (once per plan; the reverse level
+// schedule is built). False when they could not be made.
+bool adj_team(Tape& t, AdjPlan& p) {
+  std::lock_guard<std::mutex> lk(t.shape_mtx);
+  if (p.team_state != 0) return p.team_state > 0;
+  p.team_state = -1;
+  const Levels& lv = *t.h_rlv;
+  std::vector<KEnt> ents;
+  int err = 0;
+  if (!adj_entries(t, lv.code, lv.src.data(), lv.pidx, lv.sz_w, p.seeded, &ents, nullptr, &err))
+    return false;
+  // the levels last first, entries without work dropped
+  std::vector<TeamItem> items;
+  std::vector<int> begin{0}, at;
+  for (int l = static_cast<int>(lv.begin.size()) - 2; l >= 0; --l) {
+    for (int k = lv.begin[l]; k < lv.begin[l + 1]; ++k) {
+      const KEnt& e = ents[k];
+      if (e.key == AK_NOP) continue;
+      const u64 w = lv.code[k];
+      const int A = static_cast<int>(dec_a(w)), B = static_cast<int>(dec_b(w)),
+                C = static_cast<int>(dec_c(w));
+      TeamItem it;
+      if (e.key == AK_OUT_SET || e.key == AK_OUT_ADD) {
+        if (e.key == AK_OUT_ADD) it.rd[0] = B;
+        it.wr[0] = B;
+        it.cost = 3.0f;  // reads a seed from global memory
+      } else if (e.key == AK_IN) {
+        it.rd[0] = A;
+      } else {
+        it.rd[0] = A;
+        it.rd[1] = it.wr[0] = B;
+        if (is_binary(dec_op(w))) it.rd[2] = it.wr[1] = C;
+      }
+      items.push_back(it);
+      at.push_back(k);
+    }
+    begin.push_back(static_cast<int>(items.size()));
+  }
+  for (int k = 0; k < kTeamAdjSizes; ++k) {
+    std::vector<uint4> all;
+    std::vector<int2> where;
+    for (const std::vector<int>& warp : team_streams(items, begin, lv.sz_w, 4 << k)) {
+      std::vector<KEnt> seq;
+      bool open = false;  // the last entry carries no meeting yet
+      for (int q : warp) {
+        if (q != kTeamBarrier) {
+          seq.push_back(ents[at[q]]);
+          open = true;
+          continue;
+        }
+        if (!open) seq.push_back(KEnt());
+        seq.back().key |= kTeamKeyMeet;
+        open = false;
+      }
+      where.push_back(lay_out(all, seq, kTeamAdjGroup));
+    }
+    if (upload(&p.d_team[k], all) != cudaSuccess || upload(&p.d_team_at[k], where) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+  }
+  p.team_state = 1;
+  return true;
 }
 
 // Device time of `fn` (launches on stream s): one run to load the kernel and warm the caches,
@@ -1310,7 +1396,17 @@ void team_entries(const Tape& t, const Levels& lv, int warps, std::vector<uint4>
                       D_ASINH, D_ACOSH, D_ATANH, D_ATAN2, D_ERFINV, D_LOG1P, D_EXPM1, D_HYPOT,
                       D_FMOD, D_REMAINDER})
     cost[op] = 10.0f;
-  for (const std::vector<int>& warp : team_streams(lv, warps, cost)) {
+  std::vector<TeamItem> items(lv.code.size());
+  for (size_t k = 0; k < items.size(); ++k) {
+    const u64 w = lv.code[k];
+    const unsigned op = dec_op(w);
+    items[k].cost = cost[op];
+    if (op == D_OUTPUT || (op != D_CONST && op != D_INPUT)) items[k].rd[0] = static_cast<int>(dec_b(w));
+    if (op != D_OUTPUT && op != D_CONST && op != D_INPUT)
+      items[k].rd[1] = static_cast<int>(dec_c(w));
+    if (op != D_OUTPUT) items[k].wr[0] = static_cast<int>(dec_a(w));
+  }
+  for (const std::vector<int>& warp : team_streams(items, lv.begin, lv.sz_w, warps)) {
     const size_t first = entries.size();
     bool open = false;  // the last entry carries no meeting yet
     for (int k : warp) {
@@ -1388,9 +1484,10 @@ bool ensure_levels(Tape& t, bool reverse = false) {
   if (reverse) {
     t.d_rcode = code;
     t.d_rbegin = begin;
-    t.d_rpidx = pidx;
+    cudaFree(pidx);
+    t.h_rlv = std::make_unique<Levels>(std::move(lv));
     t.n_rlevels = nl;
-    t.rlv_sz_w = lv.sz_w;
+    t.rlv_sz_w = t.h_rlv->sz_w;
   } else {
     t.d_lcode = code;
     for (int k = 0; k < kTeamSizes; ++k) {
@@ -1584,7 +1681,7 @@ int run_deriv(Tape& t, SweepArgs a, long long m, const DerivReq& rq, cudaStream_
   const int kind = adjoint ? 2 : (identity ? 1 : 0);
   const int sms = sm_count();
   int err = 0;
-  const AdjPlan* ap = nullptr;
+  AdjPlan* ap = nullptr;
   std::vector<char> seeded_in(t.n_in);
   for (int j = 0; j < t.n_in; ++j) seeded_in[j] = rq.seed && rq.seed[j].ptr != nullptr;
   // tangents: outputs whose sensitivities are requested (the others' instructions are pruned)
@@ -1663,19 +1760,22 @@ int run_deriv(Tape& t, SweepArgs a, long long m, const DerivReq& rq, cudaStream_
   const bool coop_ok =
       few &&
       (capturing(s) ? (adjoint ? t.rlv_state : t.lv_state) > 0 : ensure_levels(t, adjoint)) &&
-      smem_tangent_coop(adjoint ? t.rlv_sz_w : t.lv_sz_w, false) <=
-          static_cast<size_t>(max_smem_optin());
+      (adjoint ? smem_coop(t.rlv_sz_w) : smem_tangent_coop(t.lv_sz_w, false)) <=
+          static_cast<size_t>(max_smem_optin()) &&
+      (!adjoint || (capturing(s) ? ap->team_state > 0 : adj_team(t, *ap)));
   const int kCoop = adjoint ? AV_COUNT : TV_COUNT;
-  auto launch_coop_adj = [&]() -> cudaError_t {
+  // adjoint variants kCoop + k: the cooperative sweep by teams of 4 << k warps
+  auto launch_coop_adj = [&](int k) -> cudaError_t {
     SweepArgs c = a;
     c.t = t.view();
-    c.block = kCoopTanThreads;
+    c.block = 128 << k;
     c.wglob = nullptr;
-    const int occ =
-        std::max(1, occupancy_adjoint_coop(smem_tangent_coop(t.rlv_sz_w, false)));
+    c.dstream = ap->d_team[k];
+    c.dchunks = ap->d_team_at[k];
+    const int occ = std::max(1, occupancy_adjoint_team(c.block, smem_coop(t.rlv_sz_w)));
     const int grid = static_cast<int>(std::max<long long>(
         1, std::min<long long>(work, static_cast<long long>(sms) * occ)));
-    return launch_adjoint_coop(c, grid, s);
+    return launch_adjoint_team(c, grid, s);
   };
   auto launch_coop_tan = [&]() -> cudaError_t {
     static const std::vector<int> kNoMap;
@@ -1743,12 +1843,14 @@ int run_deriv(Tape& t, SweepArgs a, long long m, const DerivReq& rq, cudaStream_
   };
   const int n_variants = adjoint ? AV_COUNT : TV_COUNT;
   auto usable = [&](int v) {
-    if (v == kWin) return !adjoint && win() && win()->usable;
-    return v == kCoop ? coop_ok : (v >= 0 && v < n_variants && fits(v));
+    if (!adjoint && v == kWin) return win() && win()->usable;
+    if (v >= kCoop && v < kCoop + (adjoint ? kTeamAdjSizes : 1)) return coop_ok;
+    return v >= 0 && v < n_variants && fits(v);
   };
   auto run_v = [&](int v) {
+    if (adjoint) return v >= kCoop ? launch_coop_adj(v - kCoop) : launch(v);
     if (v == kWin) return launch_win();
-    return v == kCoop ? (adjoint ? launch_coop_adj() : launch_coop_tan()) : launch(v);
+    return v == kCoop ? launch_coop_tan() : launch(v);
   };
   std::atomic<int>& kept = t.tuned[kind][cls];
   int variant = kept;
@@ -1761,9 +1863,9 @@ int run_deriv(Tape& t, SweepArgs a, long long m, const DerivReq& rq, cudaStream_
     if (g_autotune && !capturing(s) && (work >= 2ll * sms * 8 || few) &&
         tune_lock.try_lock()) {
       float best = 0;
-      for (int c = 0; c <= n_variants + (adjoint ? 0 : 1); ++c) {
-        // the variants of the kind, then the cooperative sweep, then (tangents) the windowed
-        const int v = c < n_variants ? c : (c == n_variants ? kCoop : kWin);
+      // the variants of the kind, then the cooperative sweep (adjoint: by team size), then
+      // (tangents) the windowed
+      for (int v = 0; v < n_variants + (adjoint ? kTeamAdjSizes : 2); ++v) {
         if (!usable(v)) continue;
         float ms = 0;
         if (int rc = time_runs(s, [&] { return run_v(v); }, &ms)) return plan_err ? plan_err : rc;
@@ -2718,7 +2820,9 @@ int casadi_gb300_tuned_variant(int id, int kind, int* variant) {
   Tape* t = get_tape(id);
   if (!t) return fail(CASADI_GB300_ERR_ID, "no tape with id %d", id);
   if (kind < 0 || kind > 2 || !variant) return fail(CASADI_GB300_ERR_ARG, "bad arguments");
-  *variant = kept_choice(t->tuned[kind], kSizeClasses - 1);  // the largest launches' choice
+  // the largest launches' choice (the cooperative adjoint is one variant, whatever its team)
+  *variant = std::min(kept_choice(t->tuned[kind], kSizeClasses - 1),
+                      kind == 2 ? AV_COUNT : TV_COUNT + 1);
   return 0;
 }
 

@@ -376,77 +376,69 @@ int level_schedule(const std::vector<u64>& in, int width, int slot_cap, Levels& 
   return static_cast<int>(out.begin.size()) - 1;
 }
 
-std::vector<std::vector<int>> team_streams(const Levels& lv, int warps, const float (&cost)[64]) {
+std::vector<std::vector<int>> team_streams(const std::vector<TeamItem>& items,
+                                           const std::vector<int>& begin, int n_slots,
+                                           int warps) {
   constexpr float kBarrierCost = 0.5f;
   std::vector<std::vector<int>> out(warps);
   struct Slot {
     int epoch = -1, writer = -1;
     unsigned readers = 0;  // warps
   };
-  std::vector<Slot> slots(std::max(1, lv.sz_w));
+  std::vector<Slot> slots(std::max(1, n_slots));
   std::vector<float> load(warps, 0.0f), trial(warps), level(warps);
   int epoch = 0;
-  // the warp an instruction has to run on without a meeting: -1 any, -2 none
-  auto owner_of = [&](u64 w) {
+  // the warp an item has to run on without a meeting: -1 any, -2 none
+  auto owner_of = [&](const TeamItem& it) {
     int own = -1;
     auto need = [&](int v) { own = own == -1 || own == v ? v : -2; };
-    const unsigned op = dec_op(w);
-    auto reads = [&](unsigned s) {
-      if (slots[s].epoch == epoch && slots[s].writer >= 0 && own != -2) need(slots[s].writer);
-    };
-    if (op == D_OUTPUT) {
-      reads(dec_b(w));
-    } else if (op != D_CONST && op != D_INPUT) {
-      reads(dec_b(w));
-      reads(dec_c(w));
-    }
-    if (op != D_OUTPUT) {
-      const Slot& d = slots[dec_a(w)];
-      if (d.epoch == epoch) {
-        if (d.writer >= 0 && own != -2) need(d.writer);
-        for (int v = 0; v < warps && own != -2; ++v)
-          if ((d.readers >> v) & 1u) need(v);
-      }
+    for (int s : it.rd)
+      if (s >= 0 && slots[s].epoch == epoch && slots[s].writer >= 0) need(slots[s].writer);
+    for (int s : it.wr) {
+      if (s < 0 || slots[s].epoch != epoch) continue;
+      if (slots[s].writer >= 0) need(slots[s].writer);
+      for (int v = 0; v < warps; ++v)
+        if ((slots[s].readers >> v) & 1u) need(v);
     }
     return own;
   };
-  auto touch = [&](unsigned s) -> Slot& {
+  auto touch = [&](int s) -> Slot& {
     Slot& x = slots[s];
     if (x.epoch != epoch) x = Slot{epoch, -1, 0u};
     return x;
   };
+  auto lightest = [&](const std::vector<float>& v) {
+    return static_cast<int>(std::min_element(v.begin(), v.end()) - v.begin());
+  };
   std::vector<int> order, place;
-  for (size_t l = 0; l + 1 < lv.begin.size(); ++l) {
-    const int b = lv.begin[l], e = lv.begin[l + 1];
+  for (size_t l = 0; l + 1 < begin.size(); ++l) {
+    const int b = begin[l], e = begin[l + 1];
+    if (b == e) continue;
     order.resize(e - b);
     for (int k = b; k < e; ++k) order[k - b] = k;
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
-      return cost[dec_op(lv.code[x])] > cost[dec_op(lv.code[y])];
-    });
-    auto lightest = [&](const std::vector<float>& v) {
-      return static_cast<int>(std::min_element(v.begin(), v.end()) - v.begin());
-    };
+    std::stable_sort(order.begin(), order.end(),
+                     [&](int x, int y) { return items[x].cost > items[y].cost; });
     // meeting first: the level spread over idle warps
     std::fill(level.begin(), level.end(), 0.0f);
-    for (int k : order) level[lightest(level)] += cost[dec_op(lv.code[k])];
+    for (int k : order) level[lightest(level)] += items[k].cost;
     const float met = *std::max_element(load.begin(), load.end()) + kBarrierCost +
                       *std::max_element(level.begin(), level.end());
-    // not meeting: forced instructions first, the others to the least loaded warps
+    // not meeting: forced items first, the others to the least loaded warps
     trial = load;
     place.assign(e - b, -1);
     bool ok = true;
     for (int k : order) {
-      const int own = owner_of(lv.code[k]);
+      const int own = owner_of(items[k]);
       if (own == -2) ok = false;
       if (own >= 0) {
         place[k - b] = own;
-        trial[own] += cost[dec_op(lv.code[k])];
+        trial[own] += items[k].cost;
       }
     }
     for (int k : order)
       if (place[k - b] < 0) {
         place[k - b] = lightest(trial);
-        trial[place[k - b]] += cost[dec_op(lv.code[k])];
+        trial[place[k - b]] += items[k].cost;
       }
     if (!ok || *std::max_element(trial.begin(), trial.end()) > met) {
       for (auto& w : out) w.push_back(kTeamBarrier);
@@ -455,26 +447,17 @@ std::vector<std::vector<int>> team_streams(const Levels& lv, int warps, const fl
       trial = load;
       for (int k : order) {
         place[k - b] = lightest(trial);
-        trial[place[k - b]] += cost[dec_op(lv.code[k])];
+        trial[place[k - b]] += items[k].cost;
       }
     }
     load = trial;
-    // a warp runs its instructions of a level in any order; reads are marked before writes
-    // (no instruction of a level touches a slot another one writes)
     for (int k : order) {
-      const u64 w = lv.code[k];
-      const unsigned op = dec_op(w);
       const int v = place[k - b];
       out[v].push_back(k);
-      if (op == D_OUTPUT) {
-        touch(dec_b(w)).readers |= 1u << v;
-      } else {
-        if (op != D_CONST && op != D_INPUT) {
-          touch(dec_b(w)).readers |= 1u << v;
-          touch(dec_c(w)).readers |= 1u << v;
-        }
-        touch(dec_a(w)).writer = v;
-      }
+      for (int s : items[k].rd)
+        if (s >= 0) touch(s).readers |= 1u << v;
+      for (int s : items[k].wr)
+        if (s >= 0) touch(s).writer = v;
     }
   }
   return out;

@@ -43,13 +43,19 @@ struct Levels {
 int level_schedule(const std::vector<u64>& in, int width, int slot_cap, Levels& out,
                    std::string& err, bool ordered_users = false);
 
-// The levels as one instruction stream per warp of a `warps`-warp team: per warp, indices into
-// lv.code in execution order, kTeamBarrier where the whole team meets. A warp runs its own
-// instructions in order, so the team meets before a level only where an instruction would read
-// a slot another warp wrote since the last meeting, or write one another warp wrote or read,
-// or where meeting spreads the level's work enough better (costs in dependent FP64 operations,
-// `cost[op]`).
+// Work items of a level schedule as one stream per warp of a `warps`-warp team: per warp, item
+// indices in execution order, kTeamBarrier where the whole team meets. A warp runs its own items in
+// order, so the team meets before a level only where an item would read a slot another warp wrote
+// since the last meeting, or write one another warp wrote or read, or where meeting spreads the
+// level's work enough better (costs in dependent FP64 operations). Level l holds items
+// [begin[l], begin[l+1]); within a level no item touches a slot another one writes.
 constexpr int kTeamBarrier = -1;
-std::vector<std::vector<int>> team_streams(const Levels& lv, int warps, const float (&cost)[64]);
+struct TeamItem {
+  int rd[3] = {-1, -1, -1};  // slots read
+  int wr[2] = {-1, -1};      // slots written
+  float cost = 1.0f;
+};
+std::vector<std::vector<int>> team_streams(const std::vector<TeamItem>& items,
+                                           const std::vector<int>& begin, int slots, int warps);
 
 }  // namespace cgb

