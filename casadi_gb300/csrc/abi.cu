@@ -1557,20 +1557,23 @@ int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStrea
       if (global)
         if (int rc = gw_prepare(t, a, &grid, static_cast<size_t>(t.lv_sz_w) * 32 * 8, s)) return rc;
     } else if (global) {
-      // value and record sweeps run one-warp CTAs, the sparsity sweeps kGwBlock threads
+      // a work-vector block per thread: several warps per CTA in every kind
       const bool value = kind == PK_EVAL || kind == PK_RECORD;
-      a.block = value ? 32 : kGwBlock;
-      const int occ =
-          std::max(1, value ? occupancy_gw_value(kind == PK_RECORD) : occupancy_gw_sp());
-      grid = grid_for((m + a.block - 1) / a.block, occ * sm_count());
+      const WarpShape sh = value ? shape_value(kind == PK_RECORD, t.sz_w, true,
+                                             (m + 31) / 32, sm_count())
+                                 : WarpShape{std::max(1, occupancy_gw_sp()), kGwBlock};
+      a.block = sh.block;
+      grid = grid_for((m + a.block - 1) / a.block, sh.ctas * sm_count());
       const size_t elem = 8;  // a double or a bvec_t per slot and instance
       if (int rc = gw_prepare(t, a, &grid,
                               static_cast<size_t>(std::max(1, t.sz_w)) * a.block * elem, s))
         return rc;
+      if (value) a.wglob_stride = static_cast<long long>(std::max(1, t.sz_w)) * 256;  // per warp
     } else if (kind == PK_EVAL || kind == PK_RECORD) {
-      a.block = 32;
+      a.block =
+          shape_value(kind == PK_RECORD, t.sz_w, false, (m + 31) / 32, sm_count()).block;
       a.wglob = nullptr;
-      grid = grid_for((m + 31) / 32, kMaxGrid);  // a CTA per tile
+      grid = grid_for((m + a.block - 1) / a.block, kMaxGrid);  // a warp per tile
     } else {
       a.block = t.primal_block;
       a.wglob = nullptr;

@@ -287,7 +287,13 @@ struct BatchArgs {
 };
 
 constexpr int kGwBlock = 128;   // threads per CTA of the global-work-vector value sweeps
-int occupancy_gw_value(bool record);  // CTAs per SM of the global-work-vector value/record sweep
+constexpr int kDirWarps = 4;     // most warps per CTA of the sweeps of independent warps
+struct WarpShape {
+  int ctas;    // resident CTAs per SM
+  int block;   // threads per CTA
+};
+// Shape of a value/record launch of `warps` tiles
+WarpShape shape_value(bool record, int sz_w, bool global, long long warps, int sms);
 int occupancy_gw_sp();           // ... of the sparsity sweeps
 int occupancy_gw_dir(bool adjoint);  // ... of the derivative sweeps (one warp per CTA)
 cudaError_t launch_gather(long long n, long long ld, int count, const long long* src_row,

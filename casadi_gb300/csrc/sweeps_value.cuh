@@ -164,24 +164,30 @@ __device__ __forceinline__ void value_walk(const PlainUnits& u, const uint4* st,
   });
 }
 
-// Value (RECORD false) and record sweeps: one warp per CTA, tiles strided over the grid. GW: the
-// work vector lives in global memory (per-CTA blocks of a.wglob) instead of shared memory.
+// Value (RECORD false) and record sweeps: the warps of a CTA are independent, tiles strided over
+// them; a CTA has several warps so that the shared memory it reserves for itself is paid once (28
+// instead of 26 resident warps on the 28-slot rollout: 131072 instances are 4096 tiles, which 28
+// warps on 152 SMs hold at once and 26 do not). GW: the work vector lives in global memory
+// (per-warp blocks of a.wglob) instead of shared memory.
 //
 // Bound by the FP64 pipe's additions and products and, in the record sweep, by the partials'
 // HBM writes. The 20-step cart-pole rollout (3057 instructions, 3400 partials) at 262144
-// instances: record 5.02 -> 2.19 ms (7.1 GB of partials, 3.3 TB/s) against the sweep that decoded
+// instances: record 5.02 -> 1.98 ms (5.3 GB of partials, 2.7 TB/s) against the sweep that decoded
 // 8-byte words with CUDA's functions inline: 177 thousand instead of 422 thousand executed
 // instructions per tile, a third of the FP64 ones.
 template <bool RECORD, bool GW>
-__global__ void __launch_bounds__(32, 28) k_value(const __grid_constant__ SweepArgs a) {
+__global__ void __launch_bounds__(32 * kDirWarps, 28 / kDirWarps) k_value(const __grid_constant__ SweepArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   const PlainUnits u;
-  const int lane = threadIdx.x;
-  uint4* ring = reinterpret_cast<uint4*>(smem);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const long long wid = static_cast<long long>(blockIdx.x) * nw + warp;
+  const long long nwarps = static_cast<long long>(gridDim.x) * nw;
+  const size_t wsmem = kEntRingBytes + (GW ? 0 : static_cast<size_t>(a.t.sz_w) * 256);
+  uint4* ring = reinterpret_cast<uint4*>(smem + warp * wsmem);
   unsigned char* wb =
-      (GW ? a.wglob + blockIdx.x * a.wglob_stride : smem + kEntRingBytes) + lane * 8;
+      (GW ? a.wglob + wid * a.wglob_stride : smem + warp * wsmem + kEntRingBytes) + lane * 8;
   const long long ntiles = (a.n + 31) / 32;
-  for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+  for (long long tile = wid; tile < ntiles; tile += nwarps) {
     const long long il = tile * 32 + lane;
     double* pt = RECORD ? a.partials + static_cast<size_t>(tile) * a.t.n_partials * 32 + lane
                         : nullptr;
