@@ -96,14 +96,21 @@ struct TanPlan {
   uint4* d_stream[kNumGroupSizes] = {};
   int2* d_chunks[kNumGroupSizes] = {};  // per direction group: (first entry, body entries)
   std::vector<int2> h_chunks[kNumGroupSizes];
-  int* d_dirmap = nullptr;    // identity mode with a dirmap: its device copy
   int* d_order = nullptr;     // groups in work order, longest stream first (null: natural)
+  // the cooperative sweep (dw 1): per direction, one keyed stream per warp of a 4 << k warp team
+  // over the level schedule, laid out for groups of kTeamGroup
+  int team_state[kTeamDirSizes] = {};  // 0 not built, 1 built, -1 unavailable
+  uint4* d_team[kTeamDirSizes] = {};
+  int2* d_team_at[kTeamDirSizes] = {};  // [direction][warp]
   ~TanPlan() {
+    for (int k = 0; k < kTeamDirSizes; ++k) {
+      cudaFree(d_team[k]);
+      cudaFree(d_team_at[k]);
+    }
     for (int g = 0; g < kNumGroupSizes; ++g) {
       cudaFree(d_stream[g]);
       cudaFree(d_chunks[g]);
     }
-    cudaFree(d_dirmap);
     cudaFree(d_order);
   }
 };
@@ -138,12 +145,12 @@ struct AdjPlan {
   int2* d_zero = nullptr;
   int n_zero = 0;
   // the cooperative sweep: one keyed stream per warp of a 4 << k warp team over the reverse level
-  // schedule, laid out for groups of kTeamAdjGroup
+  // schedule, laid out for groups of kTeamGroup
   int team_state = 0;  // 0 not built, 1 built, -1 unavailable
-  uint4* d_team[kTeamAdjSizes] = {};
-  int2* d_team_at[kTeamAdjSizes] = {};
+  uint4* d_team[kTeamDirSizes] = {};
+  int2* d_team_at[kTeamDirSizes] = {};
   ~AdjPlan() {
-    for (int k = 0; k < kTeamAdjSizes; ++k) {
+    for (int k = 0; k < kTeamDirSizes; ++k) {
       cudaFree(d_team[k]);
       cudaFree(d_team_at[k]);
     }
@@ -182,7 +189,6 @@ struct Tape {
   uint4* d_team[kTeamSizes] = {};
   int2* d_team_at[kTeamSizes] = {};  // per warp: first entry, blocks
   int* d_lbegin = nullptr;
-  int* d_lpidx = nullptr;
   int n_levels = 0, lv_sz_w = 0;
   // the reverse sweep's level schedule (users of each value in order), built on first use
   int rlv_state = 0;
@@ -190,6 +196,10 @@ struct Tape {
   int* d_rbegin = nullptr;
   int n_rlevels = 0, rlv_sz_w = 0;
   std::unique_ptr<Levels> h_rlv;  // for the adjoint plans' teams
+  // level schedule of the cooperative tangent sweep: fewer live slots than the record sweep's (its
+  // work vector decides how many teams an SM holds), host only, built on first use
+  int tlv_state = 0;
+  std::unique_ptr<Levels> h_tlv;
   // global work vector: per-CTA blocks, grown on demand; uses on different streams are
   // ordered by gw_event
   std::mutex gw_mtx;
@@ -259,7 +269,6 @@ struct Tape {
     cudaFree(d_err);
     cudaFree(d_lcode);
     cudaFree(d_lbegin);
-    cudaFree(d_lpidx);
     cudaFree(d_rcode);
     cudaFree(d_rbegin);
     if (gw_event) cudaEventSynchronize(gw_event);
@@ -284,7 +293,6 @@ struct Tape {
     v.err = d_err;
     v.lcode = d_lcode;
     v.lbegin = d_lbegin;
-    v.lpidx = d_lpidx;
     v.n_levels = n_levels;
     v.lv_sz_w = lv_sz_w;
     v.rcode = d_rcode;
@@ -923,7 +931,7 @@ std::vector<unsigned short> tan_activity(const Tape& t, int ndir, int dw, bool i
 }
 
 // Each direction group gets a compacted entry stream of the instructions with work for it.
-const TanPlan* tan_plan(Tape& t, int ndir, int dw, int ch, bool identity,
+TanPlan* tan_plan(Tape& t, int ndir, int dw, int ch, bool identity,
                         const std::vector<char>& seeded, const std::vector<int>& dirmap,
                         const std::vector<char>& wanted, int* err) {
   std::lock_guard<std::mutex> lk(t.shape_mtx);
@@ -999,8 +1007,7 @@ const TanPlan* tan_plan(Tape& t, int ndir, int dw, int ch, bool identity,
     if ((e = upload(&p->d_stream[gs], all[gs])) == cudaSuccess)
       e = upload(&p->d_chunks[gs], p->h_chunks[gs]);
   if (e != cudaSuccess ||
-      (!natural && (e = upload(&p->d_order, order)) != cudaSuccess) ||
-      (identity && !dirmap.empty() && (e = upload(&p->d_dirmap, dirmap)) != cudaSuccess)) {
+      (!natural && (e = upload(&p->d_order, order)) != cudaSuccess)) {
     *err = cuda_fail(e, "upload tangent plan");
     return nullptr;
   }
@@ -1279,6 +1286,97 @@ AdjPlan* adj_plan(Tape& t, int dw, int ch, const std::vector<char>& seeded, int*
   return t.adj_plans.back().get();
 }
 
+// Appends a team's keyed streams to `all`, one per warp, and their places to `where`; item q of
+// the levels is entry ents[at[q]].
+void lay_out_team(std::vector<uint4>& all, std::vector<int2>& where,
+                  const std::vector<TeamItem>& items, const std::vector<int>& begin, int slots,
+                  int warps, const std::vector<KEnt>& ents, const std::vector<int>& at) {
+  for (const std::vector<int>& warp : team_streams(items, begin, slots, warps)) {
+    std::vector<KEnt> seq;
+    bool open = false;  // the last entry carries no meeting yet
+    for (int q : warp) {
+      if (q != kTeamBarrier) {
+        seq.push_back(ents[at[q]]);
+        open = true;
+        continue;
+      }
+      if (!open) seq.push_back(KEnt());
+      seq.back().key |= kTeamKeyMeet;
+      open = false;
+    }
+    where.push_back(lay_out(all, seq, kTeamGroup));
+  }
+}
+
+// The level schedule of the cooperative tangent sweep: up to 64 slots more than the sequential order
+// keeps live. The MPC constraints' 34156 instructions: 128 slots in 1382 levels, seven teams of 4
+// warps per SM (the record sweep's schedule: 341 slots in 548 levels, two).
+bool ensure_tangent_levels(Tape& t) {
+  std::lock_guard<std::mutex> lk(t.shape_mtx);
+  if (t.tlv_state != 0) return t.tlv_state > 0;
+  t.tlv_state = -1;
+  auto lv = std::make_unique<Levels>();
+  std::string err;
+  if (level_schedule(t.h_code, 64, std::max(t.sz_w + 64, 128), *lv, err) <= 0 || lv->code.empty())
+    return false;
+  t.h_tlv = std::move(lv);
+  t.tlv_state = 1;
+  return true;
+}
+
+// The tangent plan's streams for teams of 4 << k warps (once per plan and size; the level schedule
+// is built). False when they could not be made.
+bool tan_team(Tape& t, TanPlan& p, int k) {
+  std::lock_guard<std::mutex> lk(t.shape_mtx);
+  if (p.team_state[k] != 0) return p.team_state[k] > 0;
+  p.team_state[k] = -1;
+  if (p.dw != 1) return false;
+  const Levels& lv = *t.h_tlv;
+  const size_t nc = t.h_code.size(), n = lv.code.size();
+  const std::vector<unsigned short> bits =
+      tan_activity(t, p.ndir, 1, p.identity, p.seeded, p.dirmap, p.wanted);
+  std::vector<uint4> all;
+  std::vector<int2> where;
+  std::vector<KEnt> ents(n);
+  for (int d = 0; d < p.ndir; ++d) {
+    if (!p.identity && d > 0) {  // general seeds: one set of streams serves every direction
+      where.insert(where.end(), where.begin(), where.begin() + (4 << k));
+      continue;
+    }
+    std::vector<TeamItem> items;
+    std::vector<int> begin{0}, at;
+    for (size_t l = 0; l + 1 < lv.begin.size(); ++l) {
+      for (int i = lv.begin[l]; i < lv.begin[l + 1]; ++i) {
+        const u64 w = lv.code[i];
+        const int src = lv.src[i];
+        const unsigned op = dec_op(w), f = bits[static_cast<size_t>(d) * nc + src] & 3u;
+        if (!f && op != D_OUTPUT) continue;
+        if (!tan_keyed(tan_raw(w, f, lv.pidx[i], t.const_ops[src], t.const_part[src]), &ents[i]))
+          return false;
+        TeamItem it;
+        if (op == D_OUTPUT) {
+          if (f) it.rd[0] = static_cast<int>(dec_b(w));
+        } else {
+          if (op != D_INPUT && (f & 1u)) it.rd[0] = static_cast<int>(dec_b(w));
+          if (op != D_INPUT && (f & 2u)) it.rd[1] = static_cast<int>(dec_c(w));
+          it.wr[0] = static_cast<int>(dec_a(w));
+          if (op == D_INPUT && !p.identity) it.cost = 3.0f;  // reads a seed
+        }
+        items.push_back(it);
+        at.push_back(i);
+      }
+      begin.push_back(static_cast<int>(items.size()));
+    }
+    lay_out_team(all, where, items, begin, lv.sz_w, 4 << k, ents, at);
+  }
+  if (upload(&p.d_team[k], all) != cudaSuccess || upload(&p.d_team_at[k], where) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  p.team_state[k] = 1;
+  return true;
+}
+
 // The adjoint plan's streams for teams of 4, 8 and 16 warps (once per plan; the reverse level
 // schedule is built). False when they could not be made.
 bool adj_team(Tape& t, AdjPlan& p) {
@@ -1317,24 +1415,10 @@ bool adj_team(Tape& t, AdjPlan& p) {
     }
     begin.push_back(static_cast<int>(items.size()));
   }
-  for (int k = 0; k < kTeamAdjSizes; ++k) {
+  for (int k = 0; k < kTeamDirSizes; ++k) {
     std::vector<uint4> all;
     std::vector<int2> where;
-    for (const std::vector<int>& warp : team_streams(items, begin, lv.sz_w, 4 << k)) {
-      std::vector<KEnt> seq;
-      bool open = false;  // the last entry carries no meeting yet
-      for (int q : warp) {
-        if (q != kTeamBarrier) {
-          seq.push_back(ents[at[q]]);
-          open = true;
-          continue;
-        }
-        if (!open) seq.push_back(KEnt());
-        seq.back().key |= kTeamKeyMeet;
-        open = false;
-      }
-      where.push_back(lay_out(all, seq, kTeamAdjGroup));
-    }
+    lay_out_team(all, where, items, begin, lv.sz_w, 4 << k, ents, at);
     if (upload(&p.d_team[k], all) != cudaSuccess || upload(&p.d_team_at[k], where) != cudaSuccess) {
       cudaGetLastError();
       return false;
@@ -1453,17 +1537,8 @@ bool ensure_levels(Tape& t, bool reverse = false) {
   u64* code = nullptr;
   uint4* team[kTeamSizes] = {};
   int2* team_at[kTeamSizes] = {};
-  int *begin = nullptr, *pidx = nullptr;
-  bool ok = cudaMalloc(&code, lv.code.size() * sizeof(u64)) == cudaSuccess &&
-            cudaMalloc(&begin, lv.begin.size() * sizeof(int)) == cudaSuccess &&
-            cudaMalloc(&pidx, lv.pidx.size() * sizeof(int)) == cudaSuccess;
-  ok = ok &&
-       cudaMemcpy(code, lv.code.data(), lv.code.size() * sizeof(u64), cudaMemcpyHostToDevice) ==
-           cudaSuccess &&
-       cudaMemcpy(begin, lv.begin.data(), lv.begin.size() * sizeof(int),
-                  cudaMemcpyHostToDevice) == cudaSuccess &&
-       cudaMemcpy(pidx, lv.pidx.data(), lv.pidx.size() * sizeof(int), cudaMemcpyHostToDevice) ==
-           cudaSuccess;
+  int* begin = nullptr;
+  bool ok = upload(&code, lv.code) == cudaSuccess && upload(&begin, lv.begin) == cudaSuccess;
   for (int k = 0; k < kTeamSizes && ok && !reverse; ++k) {
     std::vector<uint4> entries;
     std::vector<int2> at;
@@ -1477,17 +1552,16 @@ bool ensure_levels(Tape& t, bool reverse = false) {
       cudaFree(team_at[k]);
     }
     cudaFree(begin);
-    cudaFree(pidx);
     cudaGetLastError();
     return false;
   }
+  const int slots = lv.sz_w;
   if (reverse) {
     t.d_rcode = code;
     t.d_rbegin = begin;
-    cudaFree(pidx);
-    t.h_rlv = std::make_unique<Levels>(std::move(lv));
     t.n_rlevels = nl;
-    t.rlv_sz_w = t.h_rlv->sz_w;
+    t.rlv_sz_w = slots;
+    t.h_rlv = std::make_unique<Levels>(std::move(lv));
   } else {
     t.d_lcode = code;
     for (int k = 0; k < kTeamSizes; ++k) {
@@ -1495,9 +1569,8 @@ bool ensure_levels(Tape& t, bool reverse = false) {
       t.d_team_at[k] = team_at[k];
     }
     t.d_lbegin = begin;
-    t.d_lpidx = pidx;
     t.n_levels = nl;
-    t.lv_sz_w = lv.sz_w;
+    t.lv_sz_w = slots;
   }
   state = 1;
   return true;
@@ -1670,7 +1743,7 @@ cudaError_t launch_tangent_queued(const SweepArgs& a, int grid, bool more_items,
 }
 
 // The keyed streams (every group-size layout) and work order of a tangent plan.
-void set_streams(SweepArgs& a, const TanPlan* tp) {
+void set_streams(SweepArgs& a, TanPlan* tp) {
   for (int gs = 0; gs < kNumGroupSizes; ++gs) {
     a.dstreams[gs] = tp->d_stream[gs];
     a.dchunkss[gs] = tp->d_chunks[gs];
@@ -1747,7 +1820,7 @@ int run_deriv(Tape& t, SweepArgs a, long long m, const DerivReq& rq, cudaStream_
     int ipt = 1, kd = 1;
     tan_variant_shape(v, &ipt, &kd);
     static const std::vector<int> kNoMap;
-    const TanPlan* tp =
+    TanPlan* tp =
         tan_plan(t, ndir, kd, 0, identity, seeded_in, rq.dirmap ? *rq.dirmap : kNoMap,
                  wanted_out, &plan_err);
     if (!tp) return cudaErrorInvalidValue;
@@ -1758,13 +1831,14 @@ int run_deriv(Tape& t, SweepArgs a, long long m, const DerivReq& rq, cudaStream_
   const long long work = tiles * ndir;
   const int cls = size_class(work);
   const bool few = tiles <= 16ll * sms;
-  // the cooperative tangent sweep: a candidate for launches of few tiles whose level schedule
-  // (tangents + activity bytes) fits shared memory
+  const bool kept_forced = !adjoint && t.tuned[kind][cls] == TV_COUNT;  // set_variant
+  // the cooperative sweeps: candidates for launches of few tiles whose level schedule fits shared
+  // memory
   const bool coop_ok =
       few &&
-      (capturing(s) ? (adjoint ? t.rlv_state : t.lv_state) > 0 : ensure_levels(t, adjoint)) &&
-      (adjoint ? smem_coop(t.rlv_sz_w) : smem_tangent_coop(t.lv_sz_w, false)) <=
-          static_cast<size_t>(max_smem_optin()) &&
+      (capturing(s) ? (adjoint ? t.rlv_state : t.tlv_state) > 0
+                    : (adjoint ? ensure_levels(t, true) : ensure_tangent_levels(t))) &&
+      smem_coop(adjoint ? t.rlv_sz_w : t.h_tlv->sz_w) <= static_cast<size_t>(max_smem_optin()) &&
       (!adjoint || (capturing(s) ? ap->team_state > 0 : adj_team(t, *ap)));
   const int kCoop = adjoint ? AV_COUNT : TV_COUNT;
   // adjoint variants kCoop + k: the cooperative sweep by teams of 4 << k warps
@@ -1780,22 +1854,35 @@ int run_deriv(Tape& t, SweepArgs a, long long m, const DerivReq& rq, cudaStream_
         1, std::min<long long>(work, static_cast<long long>(sms) * occ)));
     return launch_adjoint_team(c, grid, s);
   };
-  auto launch_coop_tan = [&]() -> cudaError_t {
+  // the tangent plan of one direction per warp
+  auto tan1 = [&]() -> TanPlan* {
     static const std::vector<int> kNoMap;
-    const TanPlan* tp =
-        tan_plan(t, ndir, 1, 0, identity, seeded_in, rq.dirmap ? *rq.dirmap : kNoMap,
-                 wanted_out, &plan_err);
+    return tan_plan(t, ndir, 1, 0, identity, seeded_in, rq.dirmap ? *rq.dirmap : kNoMap,
+                    wanted_out, &plan_err);
+  };
+  // tangent variants: the cooperative sweep by teams of 4 << k warps is kCoop (k = 0) and, past the
+  // windowed sweep's number, kTeam1 + k - 1. The streams are built for launches of at most 8 items
+  // per SM; larger ones fill the GPU with a warp per item.
+  const int kTeam1 = TV_COUNT + 2;
+  auto team_of = [&](int v) { return v == kCoop ? 0 : v - kTeam1 + 1; };
+  auto tan_team_ok = [&](int k) {
+    if (adjoint || !coop_ok || k < 0 || k >= kTeamDirSizes) return false;
+    TanPlan* tp = tan1();
+    return tp && (capturing(s) ? tp->team_state[k] > 0
+                               : (cls <= size_class(8ll * sms) || kept_forced) &&
+                                     tan_team(t, *tp, k));
+  };
+  auto launch_coop_tan = [&](int k) -> cudaError_t {
+    const TanPlan* tp = tan1();
     if (!tp) return cudaErrorInvalidValue;
     SweepArgs c = a;
     c.t = t.view();
-    c.block = kCoopTanThreads;
+    c.block = 128 << k;
     c.wglob = nullptr;
-    c.dirmap = tp->d_dirmap;
-    const size_t sm = smem_tangent_coop(t.lv_sz_w, false);
-    const int occ = std::max(1, occupancy_tangent_coop(sm, false));
-    const int grid = static_cast<int>(std::max<long long>(
-        1, std::min<long long>(work, static_cast<long long>(sms) * occ)));
-    return launch_tangent_coop(c, grid, s);
+    c.dstream = tp->d_team[k];
+    c.dchunks = tp->d_team_at[k];
+    c.gorder = tp->d_order;
+    return launch_tangent_team(c, grid_for(work, kMaxGrid), smem_coop(t.h_tlv->sz_w), s);
   };
   if (dir_global(t)) {
     // global work vectors: one variant (G=2, 64 registers), one warp per CTA
@@ -1807,7 +1894,7 @@ int run_deriv(Tape& t, SweepArgs a, long long m, const DerivReq& rq, cudaStream_
     cudaError_t e = timed(adjoint ? F_ADJOINT : F_TANGENT, s, [&] {
       if (adjoint) return launch_adjoint(a, grid, 0, s);
       static const std::vector<int> kNoMap;
-      const TanPlan* tp = tan_plan(t, ndir, 1, 0, identity, seeded_in,
+      TanPlan* tp = tan_plan(t, ndir, 1, 0, identity, seeded_in,
                                    rq.dirmap ? *rq.dirmap : kNoMap, wanted_out, &plan_err);
       if (!tp) return cudaErrorInvalidValue;
       set_streams(a, tp);
@@ -1847,13 +1934,14 @@ int run_deriv(Tape& t, SweepArgs a, long long m, const DerivReq& rq, cudaStream_
   const int n_variants = adjoint ? AV_COUNT : TV_COUNT;
   auto usable = [&](int v) {
     if (!adjoint && v == kWin) return win() && win()->usable;
-    if (v >= kCoop && v < kCoop + (adjoint ? kTeamAdjSizes : 1)) return coop_ok;
+    if (!adjoint && v >= kCoop) return tan_team_ok(team_of(v));
+    if (v >= kCoop && v < kCoop + kTeamDirSizes) return coop_ok;
     return v >= 0 && v < n_variants && fits(v);
   };
   auto run_v = [&](int v) {
     if (adjoint) return v >= kCoop ? launch_coop_adj(v - kCoop) : launch(v);
     if (v == kWin) return launch_win();
-    return v == kCoop ? launch_coop_tan() : launch(v);
+    return v >= kCoop ? launch_coop_tan(team_of(v)) : launch(v);
   };
   std::atomic<int>& kept = t.tuned[kind][cls];
   int variant = kept;
@@ -1868,7 +1956,7 @@ int run_deriv(Tape& t, SweepArgs a, long long m, const DerivReq& rq, cudaStream_
       float best = 0;
       // the variants of the kind, then the cooperative sweep (adjoint: by team size), then
       // (tangents) the windowed
-      for (int v = 0; v < n_variants + (adjoint ? kTeamAdjSizes : 2); ++v) {
+      for (int v = 0; v < n_variants + kTeamDirSizes + (adjoint ? 0 : 1); ++v) {
         if (!usable(v)) continue;
         float ms = 0;
         if (int rc = time_runs(s, [&] { return run_v(v); }, &ms)) return plan_err ? plan_err : rc;
@@ -2823,9 +2911,9 @@ int casadi_gb300_tuned_variant(int id, int kind, int* variant) {
   Tape* t = get_tape(id);
   if (!t) return fail(CASADI_GB300_ERR_ID, "no tape with id %d", id);
   if (kind < 0 || kind > 2 || !variant) return fail(CASADI_GB300_ERR_ARG, "bad arguments");
-  // the largest launches' choice (the cooperative adjoint is one variant, whatever its team)
-  *variant = std::min(kept_choice(t->tuned[kind], kSizeClasses - 1),
-                      kind == 2 ? AV_COUNT : TV_COUNT + 1);
+  // the largest launches' choice (the cooperative sweep is one variant, whatever its team)
+  const int kept = kept_choice(t->tuned[kind], kSizeClasses - 1);
+  *variant = kind == 2 ? std::min<int>(kept, AV_COUNT) : kept > TV_COUNT + 1 ? TV_COUNT : kept;
   return 0;
 }
 

@@ -41,10 +41,14 @@ struct BatchHost {
   int n_units = 0;
   int szw = 1, pmax = 0, grid = 1;
   size_t smem = 0;
-  // work-vector residence: 0 shared memory, 1 global memory (grid_gw CTAs), -1 not tuned yet
+  // work-vector residence: 0 shared memory, 1 global memory (grid_gw CTAs), 2 shared by a team of
+  // warps, -1 not tuned yet
   int residence = -1;
   int forced = 0;  // 0 tune, 1 global memory, 2 shared memory
   int grid_gw = 1;
+  bool by_teams = false, adjoints = false;
+  size_t smem_value_team = 0, smem_dir_team = 0;
+  int n_dir_units = 0;     // the last units: directions of split items
   unsigned char* d_gw = nullptr;
   int device = 0;
   cudaStream_t stream = nullptr;  // owned: graph capture needs a non-legacy stream
@@ -97,6 +101,10 @@ int batch_prepare(BatchHost& b) {
   std::vector<std::pair<double, int4>> units, dir_units;
   std::vector<std::pair<size_t, size_t>> flag_off;  // (item, first flag) of split items
   size_t n_flags = 0;
+  // the batch by teams: every item whole, its level schedules there
+  bool team_ok = true;
+  int team_slots = 1, dir_slots = 1;
+  bool adjoints = false;  // of items that are not split
   b.pre.clear();
   b.szw = 1;
   b.pmax = 0;
@@ -114,25 +122,42 @@ int batch_prepare(BatchHost& b) {
       if (static_cast<unsigned>(t->n_partials) >= kMaxPartials)
         return fail(CASADI_GB300_ERR_UNSUPPORTED, "batch item %zu records too many partials", k);
       int err = 0;
-      const TanPlan* tp = tan_plan(*t, it.ndir, 1, 0, true, std::vector<char>(t->n_in, 0),
+      TanPlan* tp = tan_plan(*t, it.ndir, 1, 0, true, std::vector<char>(t->n_in, 0),
                                    it.dirmap, std::vector<char>(t->n_out, 1), &err);
       if (!tp) return err;
       bi.tan_stream = tp->d_stream[group_slot(kBatchTanGroup)];
       bi.tan_chunks = tp->d_chunks[group_slot(kBatchTanGroup)];
+      if (team_ok && ensure_tangent_levels(*t) && tan_team(*t, *tp, 0)) {
+        bi.dir_team = tp->d_team[0];
+        bi.dir_team_at = tp->d_team_at[0];
+        dir_slots = std::max(dir_slots, t->h_tlv->sz_w);
+      }
     } else if (it.ndir > 0) {
       if (static_cast<unsigned>(t->n_partials) >= kMaxPartials)
         return fail(CASADI_GB300_ERR_UNSUPPORTED, "batch item %zu records too many partials", k);
       std::vector<char> seeded(t->n_out);
       for (int j = 0; j < t->n_out; ++j) seeded[j] = it.io[2 * kMaxIo + j].ptr != nullptr;
       int err = 0;
-      const AdjPlan* ap = adj_plan(*t, 1, 0, seeded, &err);
+      AdjPlan* ap = adj_plan(*t, 1, 0, seeded, &err);
       if (!ap) return err;
+      if (team_ok && ensure_levels(*t, true) && adj_team(*t, *ap)) {
+        bi.dir_team = ap->d_team[0];
+        bi.dir_team_at = ap->d_team_at[0];
+        dir_slots = std::max(dir_slots, t->rlv_sz_w);
+      }
       const int2 se = ap->h_chunks[group_slot(kBatchAdjGroup)];
       bi.adj_stream = ap->d_stream[group_slot(kBatchAdjGroup)] + se.x;
       bi.adj_ngr = se.y / kBatchAdjGroup;
       bi.zero_in = ap->d_zero;
       bi.n_zero = ap->n_zero;
     }
+    if (team_ok && ensure_levels(*t)) {
+      bi.t = t->view();
+      bi.team = t->d_team[0];
+      bi.team_at = t->d_team_at[0];
+      team_slots = std::max(team_slots, t->lv_sz_w);
+    }
+    team_ok = team_ok && bi.team && (it.ndir == 0 || bi.dir_team);
     b.szw = std::max(b.szw, t->sz_w);
     const long long tiles = (it.n + 31) / 32;
     if (it.ndir >= 2) {
@@ -175,6 +200,7 @@ int batch_prepare(BatchHost& b) {
       for (long long tile = 0; tile < tiles; ++tile)
         units.push_back({cost, make_int4(static_cast<int>(k), static_cast<int>(tile), -1, 0)});
       if (it.ndir > 0) b.pmax = std::max(b.pmax, t->n_partials);
+      adjoints = adjoints || it.ndir > 0;
     }
     items.push_back(bi);
     io.insert(io.end(), it.io.begin(), it.io.end());
@@ -188,6 +214,7 @@ int batch_prepare(BatchHost& b) {
   ulist.reserve(units.size() + dir_units.size());
   for (const auto& u : units) ulist.push_back(u.second);
   for (const auto& u : dir_units) ulist.push_back(u.second);
+  b.n_dir_units = static_cast<int>(dir_units.size());
   cudaError_t e;
   if (n_flags && (e = cudaMalloc(&b.d_flags, n_flags * sizeof(unsigned))) != cudaSuccess)
     return cuda_fail(e, "cudaMalloc(batch flags)");
@@ -214,12 +241,21 @@ int batch_prepare(BatchHost& b) {
   const size_t gw_bytes = static_cast<size_t>(b.grid_gw) * b.szw * 256;
   if ((e = cudaMalloc(&b.d_gw, std::max<size_t>(gw_bytes, 256))) != cudaSuccess)
     return cuda_fail(e, "cudaMalloc(batch work vectors)");
-  b.residence = b.forced == 1 ? 1 : (b.forced == 2 ? 0 : -1);
+  // Teams where one-warp units would leave an SM fewer than 12 warps: below that the walks are
+  // bound by each warp's own latency (the mixed graphs' 160 slots allow 5 warps; 44.3 ms against
+  // 21.5 by teams), above it the sequential walks need no meetings.
+  b.smem_value_team = smem_team(team_slots, 32 * kBatchTeam, false);
+  b.smem_dir_team = smem_coop(dir_slots);
+  b.by_teams = team_ok && occ < 12 &&
+               std::max(b.smem_value_team, b.smem_dir_team) <= static_cast<size_t>(max_smem_optin());
+  b.adjoints = adjoints;
+  b.residence = b.forced == 1 ? 1 : (b.forced == 2 ? 0 : (b.by_teams ? 2 : -1));
   b.dirty = false;
   return 0;
 }
 
-int batch_enqueue(BatchHost& b, void* scratch, cudaStream_t s, bool gw) {
+int batch_enqueue(BatchHost& b, void* scratch, cudaStream_t s, int residence) {
+  const bool gw = residence == 1;
   cudaError_t e = cudaMemsetAsync(b.d_counter, 0, 2 * sizeof(unsigned), s);
   if (e == cudaSuccess && b.n_flags)
     e = cudaMemsetAsync(b.d_flags, 0, b.n_flags * sizeof(unsigned), s);
@@ -253,6 +289,25 @@ int batch_enqueue(BatchHost& b, void* scratch, cudaStream_t s, bool gw) {
   a.scratch_stride = static_cast<long long>(b.pmax) * 32;
   a.wglob = gw ? b.d_gw : nullptr;
   a.wglob_stride = static_cast<long long>(b.szw) * 256;
+  if (residence == 2) {
+    const int places = std::max(b.grid, b.grid_gw);  // of the scratch
+    const int whole = b.n_units - b.n_dir_units;
+    for (int u0 = 0; u0 < whole; u0 += places) {
+      BatchArgs r = a;
+      r.units = b.d_units + u0;
+      r.n_units = std::min(places, whole - u0);
+      e = launch_batch_team(r, BT_VALUE, b.smem_value_team, s);
+      if (e == cudaSuccess && b.adjoints) e = launch_batch_team(r, BT_ADJOINT, b.smem_dir_team, s);
+      if (e != cudaSuccess) return cuda_fail(e, "batch launch");
+    }
+    if (b.n_dir_units) {
+      a.units = b.d_units + whole;
+      a.n_units = b.n_dir_units;
+      if ((e = launch_batch_team(a, BT_DIRECTION, b.smem_dir_team, s)) != cudaSuccess)
+        return cuda_fail(e, "batch directions launch");
+    }
+    return 0;
+  }
   e = launch_batch(a, gw ? b.grid_gw : b.grid, b.smem, b.n_flags > 0, gw, s);
   if (e != cudaSuccess) return cuda_fail(e, "batch launch");
   return 0;
@@ -348,7 +403,7 @@ int casadi_gb300_batch_set_residence(int batch, int mode) {
   if (!b) return fail(CASADI_GB300_ERR_ID, "no batch %d", batch);
   if (mode < 0 || mode > 2) return fail(CASADI_GB300_ERR_ARG, "residence must be 0, 1 or 2");
   b->forced = mode;
-  b->residence = mode == 1 ? 1 : (mode == 2 ? 0 : -1);
+  b->residence = mode == 1 ? 1 : (mode == 2 ? 0 : (b->by_teams ? 2 : -1));
   if (b->exec) {
     cudaGraphExecDestroy(b->exec);
     b->exec = nullptr;
@@ -406,7 +461,7 @@ int casadi_gb300_batch_run(int batch, void* scratch, size_t scratch_bytes, int u
         }
         int rc = 0;
         if (int trc = time_runs(b->stream, [&] {
-              rc = batch_enqueue(*b, scratch, b->stream, gw == 1);
+              rc = batch_enqueue(*b, scratch, b->stream, gw);
               return cudaSuccess;
             }, &ms[gw], false))
           return trc;
@@ -417,7 +472,6 @@ int casadi_gb300_batch_run(int batch, void* scratch, size_t scratch_bytes, int u
       b->residence = b->smem <= static_cast<size_t>(max_smem_optin()) ? 0 : 1;
     }
   }
-  const bool gw = b->residence == 1;
   if (use_graph) {
     if (b->exec && b->exec_scratch != scratch) {
       cudaGraphExecDestroy(b->exec);
@@ -427,7 +481,7 @@ int casadi_gb300_batch_run(int batch, void* scratch, size_t scratch_bytes, int u
       cudaGraph_t g = nullptr;
       e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
       if (e != cudaSuccess) return cuda_fail(e, "begin capture");
-      int rc = batch_enqueue(*b, scratch, b->stream, gw);
+      int rc = batch_enqueue(*b, scratch, b->stream, b->residence);
       e = cudaStreamEndCapture(b->stream, &g);
       if (rc) {
         if (g) cudaGraphDestroy(g);
@@ -444,7 +498,7 @@ int casadi_gb300_batch_run(int batch, void* scratch, size_t scratch_bytes, int u
   } else {
     int rc = 0;
     e = timed(F_BATCH, b->stream, [&] {
-      rc = batch_enqueue(*b, scratch, b->stream, gw);
+      rc = batch_enqueue(*b, scratch, b->stream, b->residence);
       return cudaSuccess;
     });
     if (rc) return rc;

@@ -446,7 +446,7 @@ constexpr unsigned kTanXMask = (1u << 19) - 1;
 
 // One group of tangent entries (IPT tiles, K directions dir0..): their keys in E, their
 // partials in P/Q.
-template <int G, int IPT, int K, class Units>
+template <int G, int IPT, int K, bool TEAM, class Units>
 __device__ __forceinline__ void tan_group(const Units& u, const uint4 (&E)[G], const double (&P)[G][IPT],
                                           const double (&Q)[G][IPT], unsigned char* wb,
                                           const IoDesc* seed, const IoDesc* sens, bool identity,
@@ -457,7 +457,7 @@ __device__ __forceinline__ void tan_group(const Units& u, const uint4 (&E)[G], c
 #pragma unroll
   for (int i = 0; i < G; ++i) {
     const uint4 cur = E[i];
-    const unsigned key = ent_key(cur.w);
+    const unsigned key = TEAM ? cur.w & (kTeamKeyMeet - 1) : ent_key(cur.w);
     const unsigned xo = K > 1 ? (cur.x & kTanXMask) : cur.x;
     double r[IPT][K];
     switch (key) {
@@ -469,6 +469,7 @@ __device__ __forceinline__ void tan_group(const Units& u, const uint4 (&E)[G], c
             static_cast<double*>(d.ptr)[io_off(d, dir0 + k, cur.z, ig[j])] =
                 key == TK_OUT ? CGB_W(cur.y, j, k) : 0.0;
         }
+        if (TEAM && (cur.w & kTeamKeyMeet)) __syncthreads();
         continue;
       }
       case TK_IN:
@@ -536,10 +537,12 @@ __device__ __forceinline__ void tan_group(const Units& u, const uint4 (&E)[G], c
         }
         continue;
       }
-      default:
-        continue;  // NOP padding
+      default:  // NOP padding
+        if (TEAM && (cur.w & kTeamKeyMeet)) __syncthreads();
+        continue;
     }
     CGB_JK CGB_W(xo, j, k) = r[j][k];
+    if (TEAM && (cur.w & kTeamKeyMeet)) __syncthreads();
   }
 #undef CGB_JK
 #undef CGB_W
@@ -548,7 +551,7 @@ __device__ __forceinline__ void tan_group(const Units& u, const uint4 (&E)[G], c
 // One tangent sweep by one warp over its keyed stream st (body of ngr groups of G, ngr even):
 // IPT tiles (tile j's partials at pt + j*tstride), K directions dir0.. (the union stream of
 // the K directions).
-template <bool kNC, int G, int IPT, int K, class Units>
+template <bool kNC, int G, int IPT, int K, bool TEAM = false, class Units>
 __device__ __forceinline__ void tangent_walk(const Units& u, const uint4* st, int ngr, const double* pt,
                                              const double* pc,
                                              size_t tstride, const bool (&tok)[IPT],
@@ -569,10 +572,10 @@ __device__ __forceinline__ void tangent_walk(const Units& u, const uint4* st, in
   for (int g = 0; g < ngr; g += 2) {
     load_grp<G>(st, g + 2, Eb);
     issue_partials<kNC, G, IPT>(Ea, pt, pc, tstride, tok, Pb, Qb);
-    tan_group<G, IPT, K>(u, Ea, Pa, Qa, wb, seed, sens, identity, active, dir0, ndir, ig);
+    tan_group<G, IPT, K, TEAM>(u, Ea, Pa, Qa, wb, seed, sens, identity, active, dir0, ndir, ig);
     load_grp<G>(st, g + 3, Ea);
     issue_partials<kNC, G, IPT>(Eb, pt, pc, tstride, tok, Pa, Qa);
-    tan_group<G, IPT, K>(u, Eb, Pb, Qb, wb, seed, sens, identity, active, dir0, ndir, ig);
+    tan_group<G, IPT, K, TEAM>(u, Eb, Pb, Qb, wb, seed, sens, identity, active, dir0, ndir, ig);
   }
 }
 
@@ -785,8 +788,8 @@ __global__ void __launch_bounds__(32, MB) k_adjoint(const __grid_constant__ Swee
 // forms, so the sensitivities are the same bits. For launches whose tiles leave the SMs short of
 // warps: the adjoint of the 10000-node random graph at 16384 instances (512 tiles, 3.4 warps per SM
 // in the sequential sweep) 2.69 -> 1.23 ms, of the 20-step rollout at 1001 0.57 -> 0.31 ms.
-constexpr int kTeamAdjThreads = 128 << (kTeamAdjSizes - 1);
-__global__ void __launch_bounds__(kTeamAdjThreads)
+constexpr int kTeamDirThreads = 128 << (kTeamDirSizes - 1);
+__global__ void __launch_bounds__(kTeamDirThreads)
     k_adjoint_team(const __grid_constant__ SweepArgs a) {
   const FmaUnits u = fma_units();
   extern __shared__ __align__(128) unsigned char smem[];
@@ -806,9 +809,34 @@ __global__ void __launch_bounds__(kTeamAdjThreads)
       const IoDesc& d = a.sens[jk.x];
       if (active[0] && d.ptr) static_cast<double*>(d.ptr)[io_off(d, dir, jk.y, ig[0])] = 0.0;
     }
-    adjoint_walk<true, kTeamAdjGroup, 1, true>(u, a.dstream + se.x, se.y / kTeamAdjGroup,
+    adjoint_walk<true, kTeamGroup, 1, true>(u, a.dstream + se.x, se.y / kTeamGroup,
                                                a.partials + tile * tstride + lane, a.t.pconsts,
                                                tstride, tok, wb, a.seed, a.sens, active, dir, ig);
+    __syncthreads();  // the next item's entries write the slots this one reads
+  }
+}
+
+// Cooperative tangent sweep: as the adjoint one, over the level schedule (tan_team).
+__global__ void __launch_bounds__(kTeamDirThreads)
+    k_tangent_team(const __grid_constant__ SweepArgs a) {
+  const FmaUnits u = fma_units();
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  unsigned char* wb = smem + lane * 8;
+  const long long items = (a.n + 31) / 32 * a.ndir;
+  const size_t tstride = static_cast<size_t>(a.t.n_partials) * 32;
+  for (long long item = blockIdx.x; item < items; item += gridDim.x) {
+    const long long tile = item / a.ndir;
+    const int pos = static_cast<int>(item - tile * a.ndir);
+    const int dir = a.gorder ? __ldg(a.gorder + pos) : pos;
+    const long long il = tile * 32 + lane;
+    const bool active[1] = {il < a.n}, tok[1] = {true};
+    const long long ig[1] = {a.i_begin + il};
+    const int2 se = __ldg(a.dchunks + dir * nw + warp);
+    tangent_walk<true, kTeamGroup, 1, 1, true>(u, a.dstream + se.x, se.y / kTeamGroup,
+                                               a.partials + tile * tstride + lane, a.t.pconsts,
+                                               tstride, tok, wb, a.seed, a.sens,
+                                               a.identity_seed != 0, active, dir, a.ndir, ig);
     __syncthreads();  // the next item's entries write the slots this one reads
   }
 }
@@ -1019,21 +1047,9 @@ cudaError_t launch_coop(const SweepArgs& a, bool record, int grid, cudaStream_t 
                 : launch_k(k_coop<false, false>, grid, a.block, smem, a, s);
 }
 
-size_t smem_tangent_coop(int lv_sz_w, bool global) {
-  const size_t slots = static_cast<size_t>(lv_sz_w > 0 ? lv_sz_w : 1);
-  return (global ? 0 : slots * 256) + ((slots + 15) / 16) * 16;
-}
-
-cudaError_t launch_tangent_coop(const SweepArgs& a, int grid, cudaStream_t s) {
-  if (a.block != kCoopTanThreads) return cudaErrorInvalidValue;
-  const size_t smem = smem_tangent_coop(a.t.lv_sz_w, a.wglob != nullptr);
-  return a.wglob ? launch_k(k_tangent_coop<kCoopTanQ, true>, grid, a.block, smem, a, s)
-                 : launch_k(k_tangent_coop<kCoopTanQ, false>, grid, a.block, smem, a, s);
-}
-
-int occupancy_tangent_coop(size_t smem, bool global) {
-  return global ? occ_of_k(k_tangent_coop<kCoopTanQ, true>, kCoopTanThreads, smem)
-                : occ_of_k(k_tangent_coop<kCoopTanQ, false>, kCoopTanThreads, smem);
+cudaError_t launch_tangent_team(const SweepArgs& a, int grid, size_t smem, cudaStream_t s) {
+  if (a.block < 128 || a.block > kTeamDirThreads) return cudaErrorInvalidValue;
+  return launch_k(k_tangent_team, grid, a.block, smem, a, s);
 }
 
 cudaError_t launch_coop_sp(const SweepArgs& a, bool reverse, int grid, cudaStream_t s) {
@@ -1048,7 +1064,7 @@ int occupancy_coop_sp(int threads, size_t smem) {
 }
 
 cudaError_t launch_adjoint_team(const SweepArgs& a, int grid, cudaStream_t s) {
-  if (a.block < 128 || a.block > kTeamAdjThreads) return cudaErrorInvalidValue;
+  if (a.block < 128 || a.block > kTeamDirThreads) return cudaErrorInvalidValue;
   return launch_k(k_adjoint_team, grid, a.block, smem_coop(a.t.rlv_sz_w), a, s);
 }
 
@@ -1236,6 +1252,24 @@ cudaError_t launch_gather(long long n, long long ld, int count, const long long*
   if (bx > 0x7fffffffll) return cudaErrorInvalidValue;
   dim3 grid(static_cast<unsigned>(bx), static_cast<unsigned>(std::min(count, 65535)));
   k_gather<<<grid, 256, 0, s>>>(n, ld, count, src_row, src, dst);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_batch_team(const BatchArgs& b, BatchTeamKind kind, size_t smem, cudaStream_t s) {
+  static const cudaError_t set0 = cudaFuncSetAttribute(
+      k_batch_team, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin());
+  static const cudaError_t set1 = cudaFuncSetAttribute(
+      k_batch_team_dir<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin());
+  static const cudaError_t set2 = cudaFuncSetAttribute(
+      k_batch_team_dir<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin());
+  for (cudaError_t e : {set0, set1, set2})
+    if (e != cudaSuccess) return e;
+  if (kind == BT_VALUE)
+    k_batch_team<<<b.n_units, 32 * kBatchTeam, smem, s>>>(b);
+  else if (kind == BT_ADJOINT)
+    k_batch_team_dir<false><<<b.n_units, 32 * kBatchTeam, smem, s>>>(b);
+  else
+    k_batch_team_dir<true><<<b.n_units, 32 * kBatchTeam, smem, s>>>(b);
   return cudaGetLastError();
 }
 

@@ -96,7 +96,7 @@ enum TanKey : unsigned {
   TK_NOP = 0, TK_OUT0, TK_OUT, TK_IN, TK_MIXED, TK_MIXED_LAST = TK_MIXED + 3,
   CGB_TK_ARITH(CGB_KEY_ENUM) TK_COUNT
 };
-static_assert(TK_COUNT <= 64, "tangent keys fit 6 bits");
+static_assert(TK_COUNT <= 32, "tangent keys fit 5 bits");
 
 // Adjoint contributions of one entry to an operand slot w, from the entry's adjoint s and the
 // operand's partial m: R recorded partial, U unit (ADD, SUB's first operand, ASSIGN and GEN ops
@@ -126,10 +126,10 @@ enum AdjKey : unsigned {
   AK_NOP = 0, AK_OUT_SET, AK_OUT_ADD, AK_IN, CGB_AK_ARITH(CGB_KEY_ENUM) AK_COUNT
 };
 static_assert(AK_COUNT <= 32, "adjoint keys fit 5 bits");
-// Cooperative adjoint: the team meets after the entry (bit 5 of the key).
+// Cooperative tangent and adjoint: the team meets after the entry (bit 5 of the key).
 constexpr unsigned kTeamKeyMeet = 32u;
-constexpr int kTeamAdjGroup = 4;  // entries per pipeline group
-constexpr int kTeamAdjSizes = 3;  // teams of 4, 8 and 16 warps
+constexpr int kTeamGroup = 4;  // entries per pipeline group
+constexpr int kTeamDirSizes = 3;  // teams of 4, 8 and 16 warps
 #undef CGB_KEY_ENUM
 
 // Value entries (k_value, k_batch, k_coop): 16 bytes per instruction.
@@ -194,7 +194,6 @@ struct TapeView {
   // level schedule of the cooperative value/record sweeps (null until first needed)
   const u64* lcode;         // instructions level by level, slots renamed
   const int* lbegin;        // level l is lcode[lbegin[l] .. lbegin[l+1])
-  const int* lpidx;         // first recorded partial of each lcode instruction
   int n_levels;
   int lv_sz_w;              // work-vector length of the renamed slots
   // level schedule of the cooperative reverse sweep (users of each value in order)
@@ -234,7 +233,6 @@ struct SweepArgs {
   // global work vector (null: shared memory): CTA b uses wglob + b*wglob_stride
   unsigned char* wglob;
   long long wglob_stride;
-  const int* dirmap;                // cooperative tangent, identity seeds (see launch_tangent_coop)
   // tangent sweep work queue: items past the grid are claimed from *queue (zeroed before
   // each launch; null: static stride), direction groups of a tile in the order gorder
   // (longest entry stream first; null: natural order)
@@ -264,6 +262,11 @@ struct BatchItem {
   int adj_ngr;              // its groups of kBatchAdjGroup entries
   const int2* zero_in;      // inputs with a structurally zero adjoint
   int n_zero;
+  // cooperative units (k_batch_team): the streams of a kBatchTeam team's warps
+  const uint4* team;
+  const int2* team_at;      // per warp: first entry, blocks
+  const uint4* dir_team;    // keyed adjoint entries, or tangent entries of each direction
+  const int2* dir_team_at;  // per warp (tangent: [direction][warp]): first entry, body entries
   const uint4* tan_stream;  // tangent entry streams (forward)
   const int2* tan_chunks;   // per direction: (first entry, entry count)
   // split items (two or more directions): one record unit per tile writes the tile's partials
@@ -298,6 +301,11 @@ int occupancy_gw_sp();           // ... of the sparsity sweeps
 int occupancy_gw_dir(bool adjoint);  // ... of the derivative sweeps (one warp per CTA)
 cudaError_t launch_gather(long long n, long long ld, int count, const long long* src_row,
                           const double* src, double* dst, cudaStream_t s);
+constexpr int kBatchTeam = 4;  // warps of a cooperative unit: the first team size
+// One launch over b.units, b.n_units: record (or value) walks, the adjoint walks that follow them
+// (both at most as many units as the scratch has places), or single directions of split items
+enum BatchTeamKind { BT_VALUE, BT_ADJOINT, BT_DIRECTION };
+cudaError_t launch_batch_team(const BatchArgs& b, BatchTeamKind kind, size_t smem, cudaStream_t s);
 cudaError_t launch_batch(const BatchArgs& b, int grid, size_t smem, bool split, bool gw,
                          cudaStream_t s);
 int occupancy_batch(size_t smem, bool split, bool gw);
@@ -365,14 +373,10 @@ size_t smem_team(int lv_sz_w, int threads, bool global);
 // schedule's levels, last first); shared memory smem_coop of the schedule's work vector.
 cudaError_t launch_coop_sp(const SweepArgs& a, bool reverse, int grid, cudaStream_t s);
 int occupancy_coop_sp(int threads, size_t smem);
-// Cooperative tangent sweep over recorded partials: one CTA of kCoopTanThreads threads per
-// (tile, direction) item; identity seeds use a.dirmap (flat input nonzero -> direction, null:
-// the nonzero's own index) and a.in_off. Shared memory: smem_tangent_coop.
-constexpr int kCoopTanThreads = 512;
-constexpr int kCoopTanQ = 4;  // instructions per warp and level handled at once
-cudaError_t launch_tangent_coop(const SweepArgs& a, int grid, cudaStream_t s);
-size_t smem_tangent_coop(int lv_sz_w, bool global);
-int occupancy_tangent_coop(size_t smem, bool global);
+// Cooperative tangent sweep over recorded partials: one CTA per (tile, direction) item; a.dchunks
+// holds the keyed streams of the a.block / 32 warps of each direction, a.gorder the directions in
+// work order (null: natural). smem: smem_coop of their level schedule.
+cudaError_t launch_tangent_team(const SweepArgs& a, int grid, size_t smem, cudaStream_t s);
 // Cooperative adjoint sweep over recorded partials: one CTA per (tile, direction) item;
 // a.dstream/a.dchunks are the keyed streams of the a.block / 32 warps, a.zero_in the inputs whose
 // sensitivity is a structural zero. Shared memory: smem_coop of the reverse schedule.

@@ -118,3 +118,86 @@ __global__ void __launch_bounds__(32, 16) k_batch(const __grid_constant__ BatchA
     }
   }
 }
+
+// The batch by teams of kBatchTeam warps, for batches whose longest work vector leaves few warps per
+// SM resident (a team shares one work vector between its warps). The units run in rounds of as many
+// as the scratch has places for: one launch of cooperative value or record walks, a CTA per unit,
+// then one of cooperative adjoint walks over the partials just written; the directions of split
+// items follow, a CTA each. Separate launches, because a persistent CTA that alternates between the
+// walks drifts apart from its neighbours, and then every SM fetches both walks' instructions and
+// streams at different places: 65536 instances of the 5365-node random graph took 9.2 ms in one
+// persistent launch of teams (187940 instances 33.7 ms), 5.4 ms (14.3 ms) in rounds.
+__device__ __forceinline__ double* batch_partials(const BatchArgs& b, const BatchItem& it,
+                                                  const int4& unit, int lane) {
+  return (it.tile_partials
+              ? it.tile_partials + static_cast<size_t>(unit.y) * it.t.n_partials * 32
+              : b.scratch + static_cast<size_t>(blockIdx.x) * b.scratch_stride) + lane;
+}
+
+__global__ void __launch_bounds__(32 * kBatchTeam)
+    k_batch_team(const __grid_constant__ BatchArgs b) {
+  const PlainUnits u;
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int4 unit = __ldg(b.units + blockIdx.x);
+  const BatchItem& it = b.items[unit.x];
+  const long long il = static_cast<long long>(unit.y) * 32 + lane;
+  const bool active = il < it.n;
+  const IoDesc* io = it.io;
+  uint4* ring = reinterpret_cast<uint4*>(smem) + warp * (2 * kEntBlock);
+  unsigned char* wb = smem + kBatchTeam * kEntRingBytes + lane * 8;
+  const int2 vs = __ldg(it.team_at + warp);
+  PairState pair;
+  if (it.ndir == 0) {
+    staged_walk(it.team + vs.x, vs.y, ring, [&](const uint4& e) {
+      double* none = nullptr;
+      value_entry<false>(u, e, wb, none, io, io + kMaxIo, active, il, pair);
+      if (e.w & kTeamMeet) __syncthreads();
+    });
+    return;
+  }
+  double* const pt = batch_partials(b, it, unit, lane);
+  staged_walk(it.team + vs.x, vs.y, ring, [&](const uint4& e) {
+    double* p = pt + static_cast<size_t>((e.w >> kTeamPidxShift) & kTeamPidxMask) * 32;
+    value_entry<true>(u, e, wb, p, io, io + kMaxIo, active, il, pair);
+    if (e.w & kTeamMeet) __syncthreads();
+  });
+}
+
+// SPLIT false: the adjoint of a unit k_batch_team has just recorded (same places); true: direction
+// unit.z, tangent or adjoint, of a split item.
+template <bool SPLIT>
+__global__ void __launch_bounds__(32 * kBatchTeam)
+    k_batch_team_dir(const __grid_constant__ BatchArgs b) {
+  const FmaUnits u = fma_units();
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int4 unit = __ldg(b.units + blockIdx.x);
+  const BatchItem& it = b.items[unit.x];
+  if (!SPLIT && (it.ndir == 0 || it.tile_partials)) return;
+  const long long il = static_cast<long long>(unit.y) * 32 + lane;
+  const int dir = SPLIT ? unit.z : 0;  // an item that is not split has at most one direction
+  const IoDesc* io = it.io;
+  const double* pt = batch_partials(b, it, unit, lane);
+  unsigned char* wb = smem + lane * 8;
+  const bool active[1] = {il < it.n}, tok[1] = {true};
+  const long long ig[1] = {il};
+  if (SPLIT && it.forward) {
+    const int2 se = __ldg(it.dir_team_at + dir * kBatchTeam + warp);
+    tangent_walk<true, kTeamGroup, 1, 1, true>(u, it.dir_team + se.x, se.y / kTeamGroup, pt,
+                                               it.t.pconsts, 0, tok, wb, io + 2 * kMaxIo,
+                                               io + 3 * kMaxIo, true, active, dir, it.ndir, ig);
+    return;
+  }
+  if (active[0]) {
+    for (int k = warp; k < it.n_zero; k += kBatchTeam) {
+      const int2 jk = __ldg(it.zero_in + k);
+      const IoDesc& d = io[3 * kMaxIo + jk.x];
+      if (d.ptr) static_cast<double*>(d.ptr)[io_off(d, dir, jk.y, il)] = 0.0;
+    }
+  }
+  const int2 se = __ldg(it.dir_team_at + warp);
+  adjoint_walk<true, kTeamGroup, 1, true>(u, it.dir_team + se.x, se.y / kTeamGroup, pt,
+                                          it.t.pconsts, 0, tok, wb, io + 2 * kMaxIo,
+                                          io + 3 * kMaxIo, active, dir, ig);
+}

@@ -886,7 +886,9 @@ class CudaMap:
 
 
 class Batch:
-    """Several tapes over their own instance ranges, evaluated in ONE persistent launch.
+    """Several tapes over their own instance ranges, evaluated in ONE launch: a persistent one, or,
+    for tapes whose work vectors leave few warps per SM, a sequence of cooperative ones (one CUDA
+    graph with ``run(graph=True)``).
 
     ``add(tape, args, aseeds=None)`` queues a value sweep (no seeds) or a value + adjoint
     sweep of ``tape`` (a :class:`CudaTape`) on device tensors; it returns ``(res, asens)``
