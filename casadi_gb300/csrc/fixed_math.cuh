@@ -15,9 +15,9 @@
 //   width matched to their weight (errors below 2^-57), one rounding to double at the end. The
 //   largest error is about 0.51 ulp.
 //
-// Arguments outside a routine's range (zeros, subnormals, infinities, NaN, quotients near the
-// ends of the exponent range, huge arguments) make it return false; the caller takes CUDA's
-// function then.
+// Arguments outside a routine's range (subnormals, infinities, NaN, zero numerators, quotients near
+// the ends of the exponent range, huge arguments) make it return false; the caller takes CUDA's
+// function then, the whole warp for one such lane.
 //
 // Plain C++ apart from the seeds and the high products, so the routines can be compiled and
 // checked on the host.
@@ -194,8 +194,8 @@ CGB_FX FxDivisor fx_divisor(double y) {
   d.r = fx_rcp31(static_cast<fx_u32>(d.m >> 21));
   return d;
 }
-// x / y rounded to nearest; false when x, y or the quotient is not a normal number well inside
-// the exponent range.
+// x / y rounded to nearest; false when x, y or the quotient is not a normal number well inside the
+// exponent range.
 CGB_FX bool fx_div(double x, const FxDivisor& y, double* q) {
   const fx_u64 b = fx_bits(x);
   const int ex = fx_expo(b);
@@ -208,9 +208,13 @@ CGB_FX bool fx_div(double x, const FxDivisor& y, double* q) {
          static_cast<unsigned>(e - 1) < 2045u;
 }
 
-// sqrt(x) rounded to nearest, for normal positive x.
+// sqrt(x) rounded to nearest, for normal positive x and zeros.
 CGB_FX bool fx_sqrt(double x, double* s) {
   const fx_u64 b = fx_bits(x);
+  if ((b << 1) == 0) {
+    *s = x;
+    return true;
+  }
   const int ex = static_cast<int>(b >> 52);  // sign included: negative x fails the range check
   const int odd = (ex & 1) ^ 1;              // (ex - 1023) odd
   const fx_u64 a = ((b & kFxMant) | kFxOne) << odd;  // a / 2^52 in [1, 4)
@@ -274,16 +278,16 @@ CGB_FX FxReduced fx_reduce(fx_u64 b, int t, fx_u32 c2, fx_u32 c1, fx_u32 c0) {
 }
 
 // ---- sin and cos --------------------------------------------------------------------------------
-// sin(x) and cos(x) for 2^-1022 <= |x| < 2^15; false outside, and for the few arguments within
+// sin(x) and cos(x) for |x| < 2^15; false outside, and for the few arguments within
 // about 2^-24 of a multiple of pi/2 other than 0, whose reduced argument has too few bits here.
 CGB_FX bool fx_sincos(double x, double* s, double* c) {
   const fx_u64 b = fx_bits(x);
   const int e = fx_expo(b) - 1023;
   const fx_u64 sx = b & kFxSign;
-  if (e < -33) {  // x - x^3/6 rounds to x
+  if (e < -33) {  // x - x^3/6 rounds to x, zeros and subnormals included
     *s = x;
     *c = 1.0;
-    return e > -1023;
+    return true;
   }
   if (e > 14) return false;
   const int t = e + 1;
@@ -347,13 +351,13 @@ CGB_FX fx_u64 fx_exp2(fx_u64 f) {
   p = 0x2c5c85fdf473f455ull + fx_mulhi(f, p);
   return 0x3fffffffffffffedull + fx_mulhi(f, p);
 }
-// exp(x) for 2^-1022 <= |x| < 700
+// exp(x) for |x| < 700
 CGB_FX bool fx_exp(double x, double* y) {
   const fx_u64 b = fx_bits(x);
   const int e = fx_expo(b) - 1023;
-  if (e < -34) {  // 1 + x + x^2/2 rounds to 1 or its neighbour below
-    *y = (b & kFxSign) && e >= -54 ? 1.0 + x : 1.0 + (e >= -54 ? x : 0.0);
-    return e > -1023;
+  if (e < -34) {  // 1 + x + x^2/2 rounds as 1 + x
+    *y = 1.0 + (e >= -54 ? x : 0.0);
+    return true;
   }
   if (e > 9 || (b & ~kFxSign) >= 0x4085e00000000000ull) return false;
   const FxReduced r = fx_reduce(b, e + 2, 0xb8aa3b29u, 0x5c17f0bbu, 0xbe87fed0u);  // log2(e)
@@ -432,6 +436,10 @@ CGB_FX bool fx_tanh(double x, double* y) {
   const fx_u64 b = fx_bits(x);
   const int e = fx_expo(b) - 1023;
   const fx_u64 sx = b & kFxSign;
+  if (e == -1023) {  // zeros and subnormals: x - x^3/3 rounds to x
+    *y = x;
+    return true;
+  }
   if (e < -3) {
     // x (1 - z (t1 - z (t2 - ...))), z = x^2 < 2^-6
     const fx_u64 m = ((b & kFxMant) | kFxOne) << 11;
@@ -446,7 +454,7 @@ CGB_FX bool fx_tanh(double x, double* y) {
     fx_u64 v = m - fx_mulhi(m, fx_mulhi(z, p));
     const int one = static_cast<int>(v >> 63) ^ 1;
     *y = fx_pack(v << one, e + 1023 - one, sx);
-    return e > -1023;
+    return true;
   }
   if (e > 4) {  // |x| >= 32: 1 - 2 exp(-64) rounds to 1; NaN goes to the caller
     *y = fx_dbl(sx | 0x3ff0000000000000ull);

@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(32, 16) k_batch(const __grid_constant__ BatchA
     const BatchItem& it = b.items[unit.x];
     const long long il = static_cast<long long>(unit.y) * 32 + lane;
     const bool active = il < it.n;
+    const long long iv = active ? il : it.n - 1;
     const IoDesc* io = it.io;
     // partials: the item's per-tile buffer (split items) or this CTA's scratch (whole units)
     double* pt = (kSplit && it.tile_partials)
@@ -76,10 +77,10 @@ __global__ void __launch_bounds__(32, 16) k_batch(const __grid_constant__ BatchA
       // record (or value) unit
       if (it.ndir == 0) {
         value_walk<false>(fu, it.t.ventries, it.t.n_vblocks, ring, nullptr, wb, io, io + kMaxIo, active,
-                          il);
+                          iv);
         continue;
       }
-      value_walk<true>(fu, it.t.ventries, it.t.n_vblocks, ring, pt, wb, io, io + kMaxIo, active, il);
+      value_walk<true>(fu, it.t.ventries, it.t.n_vblocks, ring, pt, wb, io, io + kMaxIo, active, iv);
       if (kSplit && it.tile_partials) {
         // split item: publish the tile's partials; its directions are separate units
         __threadfence();
@@ -143,6 +144,7 @@ __global__ void __launch_bounds__(32 * kBatchTeam)
   const BatchItem& it = b.items[unit.x];
   const long long il = static_cast<long long>(unit.y) * 32 + lane;
   const bool active = il < it.n;
+  const long long iv = active ? il : it.n - 1;
   const IoDesc* io = it.io;
   uint4* ring = reinterpret_cast<uint4*>(smem) + warp * (2 * kEntBlock);
   unsigned char* wb = smem + kBatchTeam * kEntRingBytes + lane * 8;
@@ -151,7 +153,7 @@ __global__ void __launch_bounds__(32 * kBatchTeam)
   if (it.ndir == 0) {
     staged_walk(it.team + vs.x, vs.y, ring, [&](const uint4& e) {
       double* none = nullptr;
-      value_entry<false>(u, e, wb, none, io, io + kMaxIo, active, il, pair);
+      value_entry<false>(u, e, wb, none, io, io + kMaxIo, active, iv, pair);
       if (e.w & kTeamMeet) __syncthreads();
     });
     return;
@@ -159,7 +161,7 @@ __global__ void __launch_bounds__(32 * kBatchTeam)
   double* const pt = batch_partials(b, it, unit, lane);
   staged_walk(it.team + vs.x, vs.y, ring, [&](const uint4& e) {
     double* p = pt + static_cast<size_t>((e.w >> kTeamPidxShift) & kTeamPidxMask) * 32;
-    value_entry<true>(u, e, wb, p, io, io + kMaxIo, active, il, pair);
+    value_entry<true>(u, e, wb, p, io, io + kMaxIo, active, iv, pair);
     if (e.w & kTeamMeet) __syncthreads();
   });
 }

@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(kCoopMaxThreads) k_coop(const __grid_constant_
   for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const long long il = tile * 32 + lane;
     const bool active = il < a.n;
-    const long long ig = a.i_begin + il;
+    const long long ig = a.i_begin + (active ? il : a.n - 1);
     double* pt = RECORD ? a.partials + static_cast<size_t>(tile) * a.t.n_partials * 32 + lane
                         : nullptr;
     PairState pair;

@@ -16,7 +16,8 @@ struct PairState {
   double s = 0.0, c = 0.0;
 };
 
-// One entry. pt: where the instruction's first recorded partial of this lane goes (RECORD);
+// One entry. ig: the lane's instance, the range's last one for lanes past its end (which compute
+// like any other, so their values take no special path, and store nothing). pt: where the instruction's first recorded partial of this lane goes (RECORD);
 // advanced past the partials recorded (rows of 32 lanes).
 template <bool RECORD, class Units>
 __device__ __forceinline__ void value_entry(const Units& u, const uint4& e, unsigned char* wb, double*& pt,
@@ -39,7 +40,7 @@ __device__ __forceinline__ void value_entry(const Units& u, const uint4& e, unsi
     case D_INPUT: {
       const IoDesc& d = in[e.y];
       f = 0.0;
-      if (active && d.ptr) f = __ldg(static_cast<const double*>(d.ptr) + io_off(d, 0, e.z, ig));
+      if (d.ptr) f = __ldg(static_cast<const double*>(d.ptr) + io_off(d, 0, e.z, ig));
     } break;
     case D_OUTPUT: {
       const IoDesc& d = out[e.x];
@@ -192,6 +193,6 @@ __global__ void __launch_bounds__(32 * kDirWarps, 28 / kDirWarps) k_value(const 
     double* pt = RECORD ? a.partials + static_cast<size_t>(tile) * a.t.n_partials * 32 + lane
                         : nullptr;
     value_walk<RECORD>(u, a.t.ventries, a.t.n_vblocks, ring, pt, wb, a.in, a.out, il < a.n,
-                       a.i_begin + il);
+                       a.i_begin + (il < a.n ? il : a.n - 1));
   }
 }
