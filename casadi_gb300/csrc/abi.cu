@@ -184,17 +184,15 @@ struct Tape {
   std::atomic<int> primal_tuned[5][kSizeClasses];
   // level schedule of the cooperative value/record sweeps, built on first use
   int lv_state = 0;  // 0 not built, 1 built, -1 unavailable
-  u64* d_lcode = nullptr;
   // the value entries of the level schedule, one stream per warp of a 4 << k warp team
   uint4* d_team[kTeamSizes] = {};
   int2* d_team_at[kTeamSizes] = {};  // per warp: first entry, blocks
-  int* d_lbegin = nullptr;
-  int n_levels = 0, lv_sz_w = 0;
+  int lv_sz_w = 0;
   // the reverse sweep's level schedule (users of each value in order), built on first use
   int rlv_state = 0;
-  u64* d_rcode = nullptr;
-  int* d_rbegin = nullptr;
-  int n_rlevels = 0, rlv_sz_w = 0;
+  uint4* d_rteam[kTeamSizes] = {};  // the reverse sparsity sweep's streams, as d_team
+  int2* d_rteam_at[kTeamSizes] = {};
+  int rlv_sz_w = 0;
   std::unique_ptr<Levels> h_rlv;  // for the adjoint plans' teams
   // level schedule of the cooperative tangent sweep: fewer live slots than the record sweep's (its
   // work vector decides how many teams an SM holds), host only, built on first use
@@ -261,16 +259,14 @@ struct Tape {
     for (int k = 0; k < kTeamSizes; ++k) {
       cudaFree(d_team[k]);
       cudaFree(d_team_at[k]);
+      cudaFree(d_rteam[k]);
+      cudaFree(d_rteam_at[k]);
     }
     cudaFree(d_pofs);
     cudaFree(d_consts);
     cudaFree(d_pconsts);
     cudaFree(d_absent);
     cudaFree(d_err);
-    cudaFree(d_lcode);
-    cudaFree(d_lbegin);
-    cudaFree(d_rcode);
-    cudaFree(d_rbegin);
     if (gw_event) cudaEventSynchronize(gw_event);
     cudaFree(d_gw);
     if (gw_event) cudaEventDestroy(gw_event);
@@ -291,13 +287,7 @@ struct Tape {
     v.sz_w = sz_w;
     v.n_partials = n_partials;
     v.err = d_err;
-    v.lcode = d_lcode;
-    v.lbegin = d_lbegin;
-    v.n_levels = n_levels;
     v.lv_sz_w = lv_sz_w;
-    v.rcode = d_rcode;
-    v.rbegin = d_rbegin;
-    v.n_rlevels = n_rlevels;
     v.rlv_sz_w = rlv_sz_w;
     return v;
   }
@@ -540,9 +530,9 @@ SweepArgs base_args(const Tape& t, long long n, long long i_begin) {
 constexpr int kMaxGrid = 1 << 30;
 
 // Pads an entry stream to whole blocks (at least one); returns their number.
-int pad_block(std::vector<uint4>& v, size_t first = 0) {
+int pad_block(std::vector<uint4>& v, size_t first = 0, unsigned nop = D_NOP) {
   const size_t n = std::max<size_t>(1, (v.size() - first + kEntBlock - 1) / kEntBlock);
-  v.resize(first + n * kEntBlock, make_uint4(0, 0, 0, D_NOP));
+  v.resize(first + n * kEntBlock, make_uint4(0, 0, 0, nop));
   return static_cast<int>(n);
 }
 
@@ -1463,6 +1453,27 @@ enum PrimalKind { PK_EVAL = 0, PK_RECORD, PK_SP_FORWARD, PK_SP_REVERSE, PK_ACTIV
 // whether it is available; never called while the stream is being captured.
 constexpr int kLevelWidth = 64;      // instructions per level
 
+// Lays a team's streams out in whole blocks (nop: the padding's key); at: per warp the first entry
+// and the blocks. Item k of the streams is entry es[k].
+void block_streams(const std::vector<std::vector<int>>& streams, const std::vector<uint4>& es,
+                   unsigned nop, std::vector<uint4>& entries, std::vector<int2>& at) {
+  for (const std::vector<int>& warp : streams) {
+    const size_t first = entries.size();
+    bool open = false;  // the last entry carries no meeting yet
+    for (int k : warp) {
+      if (k == kTeamBarrier) {
+        if (!open) entries.push_back(make_uint4(0, 0, 0, nop));
+        entries.back().w |= kTeamMeet;
+        open = false;
+        continue;
+      }
+      entries.push_back(es[k]);
+      open = true;
+    }
+    at.push_back(make_int2(static_cast<int>(first), pad_block(entries, first, nop)));
+  }
+}
+
 // Entry streams of a `warps`-warp team over the level schedule; at: per warp the first entry and
 // the blocks. The costs (latencies in dependent FP64 operations of about 150 cycles, dispatch
 // and work-vector accesses included) balance the warps: a sincos takes 820 cycles, a recorded
@@ -1490,31 +1501,81 @@ void team_entries(const Tape& t, const Levels& lv, int warps, std::vector<uint4>
       items[k].rd[1] = static_cast<int>(dec_c(w));
     if (op != D_OUTPUT) items[k].wr[0] = static_cast<int>(dec_a(w));
   }
-  for (const std::vector<int>& warp : team_streams(items, lv.begin, lv.sz_w, warps)) {
-    const size_t first = entries.size();
-    bool open = false;  // the last entry carries no meeting yet
-    for (int k : warp) {
-      if (k == kTeamBarrier) {
-        if (!open) entries.push_back(make_uint4(0, 0, 0, D_NOP));
-        entries.back().w |= kTeamMeet;
-        open = false;
-        continue;
-      }
-      uint4 e = value_entry_of(lv.code[k], t.h_consts.data(), t.const_ops[lv.src[k]]);
-      e.w |= (static_cast<unsigned>(lv.pidx[k]) & kTeamPidxMask) << kTeamPidxShift;
-      entries.push_back(e);
-      open = true;
-    }
-    at.push_back(make_int2(static_cast<int>(first), pad_block(entries, first)));
+  std::vector<uint4> es(lv.code.size());
+  for (size_t k = 0; k < es.size(); ++k) {
+    es[k] = value_entry_of(lv.code[k], t.h_consts.data(), t.const_ops[lv.src[k]]);
+    es[k].w |= (static_cast<unsigned>(lv.pidx[k]) & kTeamPidxMask) << kTeamPidxShift;
   }
+  block_streams(team_streams(items, lv.begin, lv.sz_w, warps), es, D_NOP, entries, at);
+}
+
+// Streams of a `warps`-warp team for the reverse sparsity sweep over the reverse level schedule.
+void sp_team_entries(const Tape& t, const Levels& lv, int warps, std::vector<uint4>& entries,
+                     std::vector<int2>& at) {
+  const size_t n = lv.code.size();
+  std::vector<uint4> all(n, make_uint4(0, 0, 0, SP_NOP));
+  std::vector<char> act(std::max(1, lv.sz_w), 0);
+  for (size_t k = n; k-- > 0;) {
+    const u64 w = lv.code[k];
+    const unsigned op = dec_op(w), A = dec_a(w), B = dec_b(w), C = dec_c(w);
+    const unsigned cops = t.const_ops[lv.src[k]];
+    uint4& e = all[k];
+    if (op == D_OUTPUT) {
+      e = make_uint4(A, B * 256u, C, cops ? SP_OUT_CLEAR : act[B] ? SP_OUT_OR : SP_OUT_SET);
+      if (!cops) act[B] = 1;
+    } else if (op == D_INPUT) {
+      if (act[A]) e = make_uint4(A * 256u, B, C, SP_IN);
+      act[A] = 0;
+    } else if (op == D_CONST) {
+      act[A] = 0;
+    } else if (act[A]) {
+      act[A] = 0;
+      unsigned mb = 0, mc = 0;
+      if (!(cops & 1u)) {
+        mb = act[B] ? 2u : 1u;
+        act[B] = 1;
+      }
+      if (C != B && !(cops & 2u)) {
+        mc = act[C] ? 2u : 1u;
+        act[C] = 1;
+      }
+      if (mb || mc) e = make_uint4(A * 256u, B * 256u, C * 256u, SP_ARITH + mb + 4u * mc);
+    }
+  }
+  std::vector<TeamItem> items;
+  std::vector<int> begin{0};
+  std::vector<uint4> es;
+  for (int l = static_cast<int>(lv.begin.size()) - 2; l >= 0; --l) {
+    for (int k = lv.begin[l]; k < lv.begin[l + 1]; ++k) {
+      const uint4& e = all[k];
+      if (e.w == SP_NOP) continue;
+      TeamItem it;
+      if (e.w == SP_IN) {
+        it.rd[0] = static_cast<int>(e.x / 256u);
+      } else if (e.w < SP_IN) {
+        if (e.w != SP_OUT_CLEAR) it.wr[0] = static_cast<int>(e.y / 256u);
+        if (e.w == SP_OUT_OR) it.rd[0] = it.wr[0];
+        it.cost = 4.0f;  // reads global memory
+      } else {
+        const unsigned m = e.w - SP_ARITH;
+        it.rd[0] = static_cast<int>(e.x / 256u);
+        if (m & 3u) it.rd[1] = it.wr[0] = static_cast<int>(e.y / 256u);
+        if (m >> 2) it.rd[2] = it.wr[1] = static_cast<int>(e.z / 256u);
+      }
+      items.push_back(it);
+      es.push_back(e);
+    }
+    begin.push_back(static_cast<int>(items.size()));
+  }
+  block_streams(team_streams(items, begin, lv.sz_w, warps), es, SP_NOP, entries, at);
 }
 
 // The team streams of a.block / 32 warps into a launch's arguments.
-void set_team(SweepArgs& a, const Tape& t) {
+void set_team(SweepArgs& a, const Tape& t, bool sp_reverse = false) {
   int k = 0;
   while (k + 1 < kTeamSizes && (128 << k) < a.block) ++k;
-  a.dstream = t.d_team[k];
-  a.dchunks = t.d_team_at[k];
+  a.dstream = sp_reverse ? t.d_rteam[k] : t.d_team[k];
+  a.dchunks = sp_reverse ? t.d_rteam_at[k] : t.d_team_at[k];
 }
 
 // CTA size of the cooperative value/record/sparsity sweeps: 128, 256, 512 or 1024 threads
@@ -1534,44 +1595,32 @@ bool ensure_levels(Tape& t, bool reverse = false) {
   const int cap = t.sz_w <= 400 ? 400 : t.sz_w + kLevelWidth;
   const int nl = level_schedule(t.h_code, kLevelWidth, cap, lv, err, reverse);
   if (nl <= 0 || lv.code.empty()) return false;
-  u64* code = nullptr;
   uint4* team[kTeamSizes] = {};
   int2* team_at[kTeamSizes] = {};
-  int* begin = nullptr;
-  bool ok = upload(&code, lv.code) == cudaSuccess && upload(&begin, lv.begin) == cudaSuccess;
-  for (int k = 0; k < kTeamSizes && ok && !reverse; ++k) {
+  bool ok = true;
+  for (int k = 0; k < kTeamSizes && ok; ++k) {
     std::vector<uint4> entries;
     std::vector<int2> at;
-    team_entries(t, lv, 4 << k, entries, at);
+    if (reverse)
+      sp_team_entries(t, lv, 4 << k, entries, at);
+    else
+      team_entries(t, lv, 4 << k, entries, at);
     ok = upload(&team[k], entries) == cudaSuccess && upload(&team_at[k], at) == cudaSuccess;
   }
   if (!ok) {
-    cudaFree(code);
     for (int k = 0; k < kTeamSizes; ++k) {
       cudaFree(team[k]);
       cudaFree(team_at[k]);
     }
-    cudaFree(begin);
     cudaGetLastError();
     return false;
   }
-  const int slots = lv.sz_w;
-  if (reverse) {
-    t.d_rcode = code;
-    t.d_rbegin = begin;
-    t.n_rlevels = nl;
-    t.rlv_sz_w = slots;
-    t.h_rlv = std::make_unique<Levels>(std::move(lv));
-  } else {
-    t.d_lcode = code;
-    for (int k = 0; k < kTeamSizes; ++k) {
-      t.d_team[k] = team[k];
-      t.d_team_at[k] = team_at[k];
-    }
-    t.d_lbegin = begin;
-    t.n_levels = nl;
-    t.lv_sz_w = slots;
+  for (int k = 0; k < kTeamSizes; ++k) {
+    (reverse ? t.d_rteam : t.d_team)[k] = team[k];
+    (reverse ? t.d_rteam_at : t.d_team_at)[k] = team_at[k];
   }
+  (reverse ? t.rlv_sz_w : t.lv_sz_w) = lv.sz_w;
+  if (reverse) t.h_rlv = std::make_unique<Levels>(std::move(lv));
   state = 1;
   return true;
 }
@@ -1616,8 +1665,9 @@ int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStrea
       a.block = coop_threads(mode);
       a.t = t.view();
       a.wglob = nullptr;
-      const size_t sm = smem_coop(kind == PK_SP_REVERSE ? t.rlv_sz_w : t.lv_sz_w);
-      grid = grid_for((m + 31) / 32, std::max(1, occupancy_coop_sp(a.block, sm)) * sm_count());
+      set_team(a, t, kind == PK_SP_REVERSE);
+      const size_t sm = smem_team(kind == PK_SP_REVERSE ? t.rlv_sz_w : t.lv_sz_w, a.block, false);
+      grid = grid_for((m + 31) / 32, std::max(1, occupancy_sp_team(a.block, sm)) * sm_count());
     } else if (mode >= M_COOP) {
       a.block = coop_threads(mode);
       a.t = t.view();
@@ -1654,7 +1704,7 @@ int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStrea
     }
     auto launch = [&] {
       if (mode >= M_COOP)
-        return sp_kind ? launch_coop_sp(a, kind == PK_SP_REVERSE, grid, s)
+        return sp_kind ? launch_sp_team(a, kind == PK_SP_REVERSE, grid, s)
                        : launch_coop(a, kind == PK_RECORD, grid, s);
       return go(grid);
     };
@@ -1676,7 +1726,8 @@ int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStrea
   bool can_coop = want_coop && (capturing(s) ? (rev ? t.rlv_state : t.lv_state) > 0
                                              : ensure_levels(t, rev));
   if (can_coop && sp_kind)
-    can_coop = smem_coop(rev ? t.rlv_sz_w : t.lv_sz_w) <= static_cast<size_t>(max_smem_optin());
+    can_coop = smem_team(rev ? t.rlv_sz_w : t.lv_sz_w, kCoopMaxThreads, false) <=
+               static_cast<size_t>(max_smem_optin());
   int coop_default = M_COOP;
   while (coop_threads(coop_default) < coop_threads_for((m + 31) / 32)) ++coop_default;
   if (t.residence == 3 && coop_kind && can_coop) return run(coop_default, true);

@@ -1061,15 +1061,15 @@ cudaError_t launch_tangent_team(const SweepArgs& a, int grid, size_t smem, cudaS
   return launch_k(k_tangent_team, grid, a.block, smem, a, s);
 }
 
-cudaError_t launch_coop_sp(const SweepArgs& a, bool reverse, int grid, cudaStream_t s) {
+cudaError_t launch_sp_team(const SweepArgs& a, bool reverse, int grid, cudaStream_t s) {
   if (a.block < 32 || a.block > kCoopMaxThreads || a.block % 32) return cudaErrorInvalidValue;
-  const size_t smem = smem_coop(reverse ? a.t.rlv_sz_w : a.t.lv_sz_w);
-  return reverse ? launch_k(k_coop_sp<true>, grid, a.block, smem, a, s)
-                 : launch_k(k_coop_sp<false>, grid, a.block, smem, a, s);
+  const size_t smem = smem_team(reverse ? a.t.rlv_sz_w : a.t.lv_sz_w, a.block, false);
+  return reverse ? launch_k(k_sp_team<true>, grid, a.block, smem, a, s)
+                 : launch_k(k_sp_team<false>, grid, a.block, smem, a, s);
 }
 
-int occupancy_coop_sp(int threads, size_t smem) {
-  return occ_of_k(k_coop_sp<false>, threads, smem);
+int occupancy_sp_team(int threads, size_t smem) {
+  return occ_of_k(k_sp_team<true>, threads, smem);
 }
 
 cudaError_t launch_adjoint_team(const SweepArgs& a, int grid, cudaStream_t s) {

@@ -168,6 +168,13 @@ inline uint4 value_entry_of(u64 ins, const double* consts, unsigned const_ops) {
   return e;
 }
 
+// Reverse sparsity entries (k_sp_team<true>), with the fields of the value entries: an operand's
+// first contribution in sweep order is assigned, so no slot is cleared; constants receive none.
+//   SP_OUT_*  x output index, y slot, z nonzero (CLEAR: the output is a constant)
+//   SP_IN     x slot, y input index, z nonzero
+//   SP_ARITH + mb + 4*mc  x result slot, y, z operand slots; m: 0 none, 1 assigned, 2 ORed
+enum SpKey : unsigned { SP_NOP = 0, SP_OUT_SET, SP_OUT_OR, SP_OUT_CLEAR, SP_IN, SP_ARITH };
+
 // One input/output block: element (direction d, nonzero k, instance i) lives at
 // ptr[d*dir_stride + k*nz_stride + i*inst_stride].
 struct IoDesc {
@@ -191,15 +198,8 @@ struct TapeView {
   int sz_w;
   int n_partials;           // partials recorded per instance
   int* err;                 // device error word
-  // level schedule of the cooperative value/record sweeps (null until first needed)
-  const u64* lcode;         // instructions level by level, slots renamed
-  const int* lbegin;        // level l is lcode[lbegin[l] .. lbegin[l+1])
-  int n_levels;
-  int lv_sz_w;              // work-vector length of the renamed slots
-  // level schedule of the cooperative reverse sweep (users of each value in order)
-  const u64* rcode;
-  const int* rbegin;
-  int n_rlevels;
+  // work-vector lengths of the level schedules (0 until first needed)
+  int lv_sz_w;
   int rlv_sz_w;
 };
 
@@ -371,8 +371,8 @@ cudaError_t launch_coop(const SweepArgs& a, bool record, int grid, cudaStream_t 
 size_t smem_team(int lv_sz_w, int threads, bool global);
 // Cooperative sparsity sweeps (forward: the value sweep's levels; reverse: the reverse
 // schedule's levels, last first); shared memory smem_coop of the schedule's work vector.
-cudaError_t launch_coop_sp(const SweepArgs& a, bool reverse, int grid, cudaStream_t s);
-int occupancy_coop_sp(int threads, size_t smem);
+cudaError_t launch_sp_team(const SweepArgs& a, bool reverse, int grid, cudaStream_t s);
+int occupancy_sp_team(int threads, size_t smem);
 // Cooperative tangent sweep over recorded partials: one CTA per (tile, direction) item; a.dchunks
 // holds the keyed streams of the a.block / 32 warps of each direction, a.gorder the directions in
 // work order (null: natural). smem: smem_coop of their level schedule.

@@ -45,74 +45,79 @@ __global__ void __launch_bounds__(kCoopMaxThreads) k_coop(const __grid_constant_
   }
 }
 
-// Cooperative bvec_t sparsity sweeps (SXFunction::sp_forward / sp_reverse): the value
-// sweep's level walk with OR instead of arithmetic; the reverse sweep walks the reverse level
-// schedule last level first (no two users of a value in one level, so no two instructions of
-// a level OR into one slot). OR does not depend on order: the same bits as the sequential
-// sweeps.
+// Cooperative bvec_t sparsity sweeps (SXFunction::sp_forward / sp_reverse) by the same teams: the
+// value sweep's streams with OR instead of arithmetic, and for the reverse sweep streams of their own
+// over the reverse level schedule (sweeps.cuh, "Reverse sparsity entries"). OR does not depend on
+// order: the same bits as the sequential sweeps. The 10000-node random graph at 16384 instances:
+// sp_forward 440 -> 364 us, sp_reverse 508 -> 369 us against a barrier per level.
 template <bool REV>
-__global__ void __launch_bounds__(kCoopMaxThreads) k_coop_sp(const __grid_constant__ SweepArgs a) {
+__global__ void __launch_bounds__(kCoopMaxThreads) k_sp_team(const __grid_constant__ SweepArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
-  u64* w = reinterpret_cast<u64*>(smem);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  uint4* ring = reinterpret_cast<uint4*>(smem) + warp * (2 * kEntBlock);
+  unsigned char* wb = smem + nw * kEntRingBytes + lane * 8;
   const long long ntiles = (a.n + 31) / 32;
-  const int nl = REV ? a.t.n_rlevels : a.t.n_levels;
-  const u64* code = REV ? a.t.rcode : a.t.lcode;
-  const int* lb = REV ? a.t.rbegin : a.t.lbegin;
-  const int lv = REV ? a.t.rlv_sz_w : a.t.lv_sz_w;
+  const int2 se = __ldg(a.dchunks + warp);  // (first entry, blocks) of this warp's stream
+  const uint4* st = a.dstream + se.x;
+#define CGB_U(off) (*reinterpret_cast<u64*>(wb + (off)))
   for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const long long il = tile * 32 + lane;
     const bool active = il < a.n;
     const long long ig = a.i_begin + il;
-    if (REV) {
-      for (int k = warp; k < lv; k += nw) w[k * 32 + lane] = 0;
-      __syncthreads();
-    }
-    for (int step = 0; step < nl; ++step) {
-      const int l = REV ? nl - 1 - step : step;
-      const int beg = __ldg(lb + l), end = __ldg(lb + l + 1);
-      for (int i = beg + warp; i < end; i += nw) {
-        const u64 ins = __ldg(code + i);
-        const unsigned op = dec_op(ins), A = dec_a(ins), B = dec_b(ins), C = dec_c(ins);
-        switch (op) {
+    staged_walk(st, se.y, ring, [&](const uint4& e) {
+      const unsigned key = e.w & 63u;
+      if constexpr (!REV) {
+        if (key - D_CONST > D_OUTPUT - D_CONST && key != D_NOP) {  // most entries: no jump table
+          CGB_U(e.x) = CGB_U(e.y) | CGB_U(e.z);
+        } else switch (key) {
           case D_CONST:
-            w[A * 32 + lane] = 0;
+            CGB_U(e.x) = 0;
             break;
           case D_INPUT: {
-            const IoDesc& d = a.in[B];
-            if (REV) {
-              if (active && d.ptr) static_cast<u64*>(d.ptr)[io_off(d, 0, C, ig)] |= w[A * 32 + lane];
-              w[A * 32 + lane] = 0;
-            } else {
-              u64 v = 0;
-              if (active && d.ptr) v = __ldg(static_cast<const u64*>(d.ptr) + io_off(d, 0, C, ig));
-              w[A * 32 + lane] = v;
-            }
+            const IoDesc& d = a.in[e.y];
+            u64 v = 0;
+            if (active && d.ptr) v = __ldg(static_cast<const u64*>(d.ptr) + io_off(d, 0, e.z, ig));
+            CGB_U(e.x) = v;
           } break;
           case D_OUTPUT: {
-            const IoDesc& d = a.out[A];
-            if (REV) {
-              if (active && d.ptr) {
-                u64* p = static_cast<u64*>(d.ptr) + io_off(d, 0, C, ig);
-                w[B * 32 + lane] |= *p;
-                *p = 0;
-              }
-            } else if (active && d.ptr) {
-              static_cast<u64*>(d.ptr)[io_off(d, 0, C, ig)] = w[B * 32 + lane];
-            }
+            const IoDesc& d = a.out[e.x];
+            if (active && d.ptr) static_cast<u64*>(d.ptr)[io_off(d, 0, e.z, ig)] = CGB_U(e.y);
           } break;
           default:
-            if (REV) {
-              const u64 seed = w[A * 32 + lane];
-              w[A * 32 + lane] = 0;
-              w[B * 32 + lane] |= seed;
-              w[C * 32 + lane] |= seed;
-            } else {
-              w[A * 32 + lane] = w[B * 32 + lane] | w[C * 32 + lane];
+            break;
+        }
+      } else {
+        if (key >= SP_ARITH) {
+          // operand b, then c: nothing, set or OR
+          const unsigned m = key - SP_ARITH, mb = m & 3u, mc = m >> 2;
+          const u64 s = CGB_U(e.x);
+          if (mb) CGB_U(e.y) = mb == 1u ? s : CGB_U(e.y) | s;
+          if (mc) CGB_U(e.z) = mc == 1u ? s : CGB_U(e.z) | s;
+        } else switch (key) {
+          case SP_OUT_SET:
+          case SP_OUT_OR:
+          case SP_OUT_CLEAR: {
+            const IoDesc& d = a.out[e.x];
+            u64 v = 0;
+            if (active && d.ptr) {
+              u64* p = static_cast<u64*>(d.ptr) + io_off(d, 0, e.z, ig);
+              v = *p;
+              *p = 0;
             }
+            if (key == SP_OUT_SET) CGB_U(e.y) = v;
+            if (key == SP_OUT_OR) CGB_U(e.y) |= v;
+          } break;
+          case SP_IN: {
+            const IoDesc& d = a.in[e.y];
+            if (active && d.ptr) static_cast<u64*>(d.ptr)[io_off(d, 0, e.z, ig)] |= CGB_U(e.x);
+          } break;
+          default:
+            break;
         }
       }
-      __syncthreads();
-    }
+      if (e.w & kTeamMeet) __syncthreads();
+    });
+    __syncthreads();  // the next tile's entries write the slots this one reads
   }
+#undef CGB_U
 }
