@@ -127,9 +127,9 @@ int batch_prepare(BatchHost& b) {
       if (!tp) return err;
       bi.tan_stream = tp->d_stream[group_slot(kBatchTanGroup)];
       bi.tan_chunks = tp->d_chunks[group_slot(kBatchTanGroup)];
-      if (team_ok && ensure_tangent_levels(*t) && tan_team(*t, *tp, 0)) {
-        bi.dir_team = tp->d_team[0];
-        bi.dir_team_at = tp->d_team_at[0];
+      if (team_ok && ensure_tangent_levels(*t) && tan_team(*t, *tp, kBatchTeamSize)) {
+        bi.dir_team = tp->d_team[kBatchTeamSize];
+        bi.dir_team_at = tp->d_team_at[kBatchTeamSize];
         dir_slots = std::max(dir_slots, t->h_tlv->sz_w);
       }
     } else if (it.ndir > 0) {
@@ -141,8 +141,8 @@ int batch_prepare(BatchHost& b) {
       AdjPlan* ap = adj_plan(*t, 1, 0, seeded, &err);
       if (!ap) return err;
       if (team_ok && ensure_levels(*t, true) && adj_team(*t, *ap)) {
-        bi.dir_team = ap->d_team[0];
-        bi.dir_team_at = ap->d_team_at[0];
+        bi.dir_team = ap->d_team[kBatchTeamSize];
+        bi.dir_team_at = ap->d_team_at[kBatchTeamSize];
         dir_slots = std::max(dir_slots, t->rlv_sz_w);
       }
       const int2 se = ap->h_chunks[group_slot(kBatchAdjGroup)];
@@ -153,8 +153,8 @@ int batch_prepare(BatchHost& b) {
     }
     if (team_ok && ensure_levels(*t)) {
       bi.t = t->view();
-      bi.team = t->d_team[0];
-      bi.team_at = t->d_team_at[0];
+      bi.team = t->d_team[kBatchTeamSize];
+      bi.team_at = t->d_team_at[kBatchTeamSize];
       team_slots = std::max(team_slots, t->lv_sz_w);
     }
     team_ok = team_ok && bi.team && (it.ndir == 0 || bi.dir_team);
@@ -241,12 +241,14 @@ int batch_prepare(BatchHost& b) {
   const size_t gw_bytes = static_cast<size_t>(b.grid_gw) * b.szw * 256;
   if ((e = cudaMalloc(&b.d_gw, std::max<size_t>(gw_bytes, 256))) != cudaSuccess)
     return cuda_fail(e, "cudaMalloc(batch work vectors)");
-  // Teams where one-warp units would leave an SM fewer than 12 warps: below that the walks are
-  // bound by each warp's own latency (the mixed graphs' 160 slots allow 5 warps; 44.3 ms against
-  // 21.5 by teams), above it the sequential walks need no meetings.
+  // Teams where one-warp units would leave an SM fewer than 20 warps: below that the walks are
+  // bound by each warp's own latency, above it the sequential walks need no meetings. Random graphs
+  // of 4000 nodes, value and adjoint of 65536 instances, one-warp units against teams: 24 slots
+  // (23 warps per SM) 3.74 and 4.84 ms, 45 slots (17 warps) 4.27 and 3.14, 66 slots (12) 6.67 and
+  // 3.08, 142 slots (6) 7.80 and 2.73 ms.
   b.smem_value_team = smem_team(team_slots, 32 * kBatchTeam, false);
   b.smem_dir_team = smem_coop(dir_slots);
-  b.by_teams = team_ok && occ < 12 &&
+  b.by_teams = team_ok && occ < 20 &&
                std::max(b.smem_value_team, b.smem_dir_team) <= static_cast<size_t>(max_smem_optin());
   b.adjoints = adjoints;
   b.residence = b.forced == 1 ? 1 : (b.forced == 2 ? 0 : (b.by_teams ? 2 : -1));

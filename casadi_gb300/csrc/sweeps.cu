@@ -796,9 +796,11 @@ __global__ void __launch_bounds__(32, MB) k_adjoint(const __grid_constant__ Swee
 // is laid out over the warps as keyed streams (adj_team): the same contributions in the same
 // forms, so the sensitivities are the same bits. For launches whose tiles leave the SMs short of
 // warps: the adjoint of the 10000-node random graph at 16384 instances (512 tiles, 3.4 warps per SM
-// in the sequential sweep) 2.69 -> 1.23 ms, of the 20-step rollout at 1001 0.57 -> 0.31 ms.
+// in the sequential sweep) 2.69 -> 0.72 ms. 64 registers a thread keep 32 warps on an SM; without
+// the cap and with groups of four (97 registers) that took 1.23 ms, and Jacobian and adjoint of the
+// 20-step rollout at 1001 instances 851 us in place of 723.
 constexpr int kTeamDirThreads = 128 << (kTeamDirSizes - 1);
-__global__ void __launch_bounds__(kTeamDirThreads)
+__global__ void __launch_bounds__(kTeamDirThreads, 2)
     k_adjoint_team(const __grid_constant__ SweepArgs a) {
   const FmaUnits u = fma_units();
   extern __shared__ __align__(128) unsigned char smem[];
@@ -826,7 +828,7 @@ __global__ void __launch_bounds__(kTeamDirThreads)
 }
 
 // Cooperative tangent sweep: as the adjoint one, over the level schedule (tan_team).
-__global__ void __launch_bounds__(kTeamDirThreads)
+__global__ void __launch_bounds__(kTeamDirThreads, 2)
     k_tangent_team(const __grid_constant__ SweepArgs a) {
   const FmaUnits u = fma_units();
   extern __shared__ __align__(128) unsigned char smem[];

@@ -128,7 +128,7 @@ enum AdjKey : unsigned {
 static_assert(AK_COUNT <= 32, "adjoint keys fit 5 bits");
 // Cooperative tangent and adjoint: the team meets after the entry (bit 5 of the key).
 constexpr unsigned kTeamKeyMeet = 32u;
-constexpr int kTeamGroup = 4;  // entries per pipeline group
+constexpr int kTeamGroup = 2;  // entries per pipeline group: 64 registers a thread (4 take 97)
 constexpr int kTeamDirSizes = 3;  // teams of 4, 8 and 16 warps
 #undef CGB_KEY_ENUM
 
@@ -301,7 +301,7 @@ int occupancy_gw_sp();           // ... of the sparsity sweeps
 int occupancy_gw_dir(bool adjoint);  // ... of the derivative sweeps (one warp per CTA)
 cudaError_t launch_gather(long long n, long long ld, int count, const long long* src_row,
                           const double* src, double* dst, cudaStream_t s);
-constexpr int kBatchTeam = 4;  // warps of a cooperative unit: the first team size
+constexpr int kBatchTeamSize = 1, kBatchTeam = 4 << kBatchTeamSize;  // warps of a cooperative unit
 // One launch over b.units, b.n_units: record (or value) walks, the adjoint walks that follow them
 // (both at most as many units as the scratch has places), or single directions of split items
 enum BatchTeamKind { BT_VALUE, BT_ADJOINT, BT_DIRECTION };

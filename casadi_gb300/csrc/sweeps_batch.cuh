@@ -124,7 +124,10 @@ __global__ void __launch_bounds__(32, 16) k_batch(const __grid_constant__ BatchA
 // SM resident (a team shares one work vector between its warps). The units run in rounds of as many
 // as the scratch has places for: one launch of cooperative value or record walks, a CTA per unit,
 // then one of cooperative adjoint walks over the partials just written; the directions of split
-// items follow, a CTA each. Separate launches, because a persistent CTA that alternates between the
+// items follow, a CTA each. Teams of 8, four to an SM, at 64 registers a thread: the mixed queue
+// (262144 instances) 21.1 -> 16.0 ms against teams of 4 at 90 registers, the MPC directions (14
+// and 10 of 34156 and 76851 instructions, 4096 scenarios) 8.97 -> 6.79 ms; teams of 16, two to an SM,
+// 16.3 and 9.04 ms, five teams of 8 at 48 registers 18.6 and 9.63 ms. Separate launches, because a persistent CTA that alternates between the
 // walks drifts apart from its neighbours, and then every SM fetches both walks' instructions and
 // streams at different places: 65536 instances of the 5365-node random graph took 9.2 ms in one
 // persistent launch of teams (187940 instances 33.7 ms), 5.4 ms (14.3 ms) in rounds.
@@ -135,7 +138,7 @@ __device__ __forceinline__ double* batch_partials(const BatchArgs& b, const Batc
               : b.scratch + static_cast<size_t>(blockIdx.x) * b.scratch_stride) + lane;
 }
 
-__global__ void __launch_bounds__(32 * kBatchTeam)
+__global__ void __launch_bounds__(32 * kBatchTeam, 4)
     k_batch_team(const __grid_constant__ BatchArgs b) {
   const PlainUnits u;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -169,7 +172,7 @@ __global__ void __launch_bounds__(32 * kBatchTeam)
 // SPLIT false: the adjoint of a unit k_batch_team has just recorded (same places); true: direction
 // unit.z, tangent or adjoint, of a split item.
 template <bool SPLIT>
-__global__ void __launch_bounds__(32 * kBatchTeam)
+__global__ void __launch_bounds__(32 * kBatchTeam, 4)
     k_batch_team_dir(const __grid_constant__ BatchArgs b) {
   const FmaUnits u = fma_units();
   extern __shared__ __align__(128) unsigned char smem[];
