@@ -35,9 +35,11 @@ struct BatchHost {
     int item;
     size_t flag0;
     long long tiles;
-    double* partials;
   };
   std::vector<PreRecord> pre;
+  int n_pre_units = 0;  // their (item, tile) units, past the others in d_units
+  int pre_threads = 0;
+  size_t smem_pre = 0;
   int n_units = 0;
   int szw = 1, pmax = 0, grid = 1;
   size_t smem = 0;
@@ -181,7 +183,7 @@ int batch_prepare(BatchHost& b) {
                        smem_team(t->lv_sz_w, coop_threads_for((it.n + 31) / 32), false) <=
                            static_cast<size_t>(max_smem_optin());
       if (pre) {
-        b.pre.push_back({static_cast<int>(k), n_flags, tiles, tp});
+        b.pre.push_back({static_cast<int>(k), n_flags, tiles});
         bi.t = t->view();
       }
       for (long long tile = 0; tile < tiles; ++tile) {
@@ -215,6 +217,31 @@ int batch_prepare(BatchHost& b) {
   for (const auto& u : units) ulist.push_back(u.second);
   for (const auto& u : dir_units) ulist.push_back(u.second);
   b.n_dir_units = static_cast<int>(dir_units.size());
+  b.n_units = static_cast<int>(ulist.size());
+  // The split items' records: one launch of all their tiles, longest tape first, by teams that
+  // together fill the GPU.
+  long long pre_tiles = 0;
+  int pre_slots = 1;
+  std::vector<std::pair<double, int4>> pre_units;
+  for (const auto& pr : b.pre) {
+    const Tape* t = get_tape(b.items[pr.item].tape);
+    pre_tiles += pr.tiles;
+    pre_slots = std::max(pre_slots, t->lv_sz_w);
+    for (long long tile = 0; tile < pr.tiles; ++tile)
+      pre_units.push_back({static_cast<double>(t->n_instr), make_int4(pr.item, static_cast<int>(tile), -1, 0)});
+  }
+  std::stable_sort(pre_units.begin(), pre_units.end(), longest_first);
+  for (const auto& u : pre_units) ulist.push_back(u.second);
+  b.n_pre_units = static_cast<int>(pre_units.size());
+  b.pre_threads = coop_threads_for(pre_tiles);
+  b.smem_pre = smem_team(pre_slots, b.pre_threads, false);
+  for (const auto& pr : b.pre) {
+    const Tape* t = get_tape(b.items[pr.item].tape);
+    int size = 0;
+    while (size + 1 < kTeamSizes && (128 << size) < b.pre_threads) ++size;
+    items[pr.item].team = t->d_team[size];
+    items[pr.item].team_at = t->d_team_at[size];
+  }
   cudaError_t e;
   if (n_flags && (e = cudaMalloc(&b.d_flags, n_flags * sizeof(unsigned))) != cudaSuccess)
     return cuda_fail(e, "cudaMalloc(batch flags)");
@@ -226,7 +253,6 @@ int batch_prepare(BatchHost& b) {
     return cuda_fail(e, "upload batch");
   if (!b.d_counter && (e = cudaMalloc(&b.d_counter, 2 * sizeof(unsigned))) != cudaSuccess)
     return cuda_fail(e, "cudaMalloc(counter)");
-  b.n_units = static_cast<int>(ulist.size());
   b.smem = smem_value(b.szw);
   const int occ = b.smem <= static_cast<size_t>(max_smem_optin())
                       ? std::max(1, occupancy_batch(b.smem, b.n_flags > 0, false))
@@ -262,25 +288,6 @@ int batch_enqueue(BatchHost& b, void* scratch, cudaStream_t s, int residence) {
   if (e == cudaSuccess && b.n_flags)
     e = cudaMemsetAsync(b.d_flags, 0, b.n_flags * sizeof(unsigned), s);
   if (e != cudaSuccess) return cuda_fail(e, "reset batch counter");
-  for (const auto& pr : b.pre) {
-    const auto& it = b.items[pr.item];
-    Tape* t = get_tape(it.tape);
-    if (!t) return fail(CASADI_GB300_ERR_ID, "batch item %d: tape %d is gone", pr.item, it.tape);
-    SweepArgs a = base_args(*t, it.n, 0);
-    for (int j = 0; j < t->n_in; ++j) a.in[j] = it.io[j];
-    for (int j = 0; j < t->n_out; ++j) a.out[j] = it.io[kMaxIo + j];
-    a.partials = pr.partials;
-    a.block = coop_threads_for(pr.tiles);
-    set_team(a, *t);
-    const size_t sm = smem_team(t->lv_sz_w, a.block, false);
-    const int occ = std::max(1, occupancy_coop(a.block, sm, false));
-    const int grid = static_cast<int>(std::min<long long>(pr.tiles, 1ll * occ * sm_count()));
-    if ((e = launch_coop(a, true, grid, s)) != cudaSuccess) return cuda_fail(e, "batch record");
-    // every tile of the item is recorded: its direction units need not wait
-    if ((e = cudaMemsetAsync(b.d_flags + pr.flag0, 0xff, pr.tiles * sizeof(unsigned), s)) !=
-        cudaSuccess)
-      return cuda_fail(e, "batch flags");
-  }
   BatchArgs a;
   a.items = b.d_items;
   a.units = b.d_units;
@@ -291,6 +298,19 @@ int batch_enqueue(BatchHost& b, void* scratch, cudaStream_t s, int residence) {
   a.scratch_stride = static_cast<long long>(b.pmax) * 32;
   a.wglob = gw ? b.d_gw : nullptr;
   a.wglob_stride = static_cast<long long>(b.szw) * 256;
+  if (b.n_pre_units) {
+    a.units = b.d_units + b.n_units;
+    a.n_units = b.n_pre_units;
+    if ((e = launch_batch_team(a, BT_VALUE, b.pre_threads, b.smem_pre, s)) != cudaSuccess)
+      return cuda_fail(e, "batch record");
+    // every tile of the items is recorded: their direction units need not wait
+    for (const auto& pr : b.pre)
+      if ((e = cudaMemsetAsync(b.d_flags + pr.flag0, 0xff, pr.tiles * sizeof(unsigned), s)) !=
+          cudaSuccess)
+        return cuda_fail(e, "batch flags");
+    a.units = b.d_units;
+    a.n_units = b.n_units;
+  }
   if (residence == 2) {
     const int places = std::max(b.grid, b.grid_gw);  // of the scratch
     const int whole = b.n_units - b.n_dir_units;
@@ -298,14 +318,15 @@ int batch_enqueue(BatchHost& b, void* scratch, cudaStream_t s, int residence) {
       BatchArgs r = a;
       r.units = b.d_units + u0;
       r.n_units = std::min(places, whole - u0);
-      e = launch_batch_team(r, BT_VALUE, b.smem_value_team, s);
-      if (e == cudaSuccess && b.adjoints) e = launch_batch_team(r, BT_ADJOINT, b.smem_dir_team, s);
+      e = launch_batch_team(r, BT_VALUE, 32 * kBatchTeam, b.smem_value_team, s);
+      if (e == cudaSuccess && b.adjoints)
+        e = launch_batch_team(r, BT_ADJOINT, 32 * kBatchTeam, b.smem_dir_team, s);
       if (e != cudaSuccess) return cuda_fail(e, "batch launch");
     }
     if (b.n_dir_units) {
       a.units = b.d_units + whole;
       a.n_units = b.n_dir_units;
-      if ((e = launch_batch_team(a, BT_DIRECTION, b.smem_dir_team, s)) != cudaSuccess)
+      if ((e = launch_batch_team(a, BT_DIRECTION, 32 * kBatchTeam, b.smem_dir_team, s)) != cudaSuccess)
         return cuda_fail(e, "batch directions launch");
     }
     return 0;

@@ -1266,7 +1266,8 @@ cudaError_t launch_gather(long long n, long long ld, int count, const long long*
   return cudaGetLastError();
 }
 
-cudaError_t launch_batch_team(const BatchArgs& b, BatchTeamKind kind, size_t smem, cudaStream_t s) {
+cudaError_t launch_batch_team(const BatchArgs& b, BatchTeamKind kind, int threads, size_t smem,
+                              cudaStream_t s) {
   static const cudaError_t set0 = cudaFuncSetAttribute(
       k_batch_team, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin());
   static const cudaError_t set1 = cudaFuncSetAttribute(
@@ -1276,11 +1277,11 @@ cudaError_t launch_batch_team(const BatchArgs& b, BatchTeamKind kind, size_t sme
   for (cudaError_t e : {set0, set1, set2})
     if (e != cudaSuccess) return e;
   if (kind == BT_VALUE)
-    k_batch_team<<<b.n_units, 32 * kBatchTeam, smem, s>>>(b);
+    k_batch_team<<<b.n_units, threads, smem, s>>>(b);
   else if (kind == BT_ADJOINT)
-    k_batch_team_dir<false><<<b.n_units, 32 * kBatchTeam, smem, s>>>(b);
+    k_batch_team_dir<false><<<b.n_units, threads, smem, s>>>(b);
   else
-    k_batch_team_dir<true><<<b.n_units, 32 * kBatchTeam, smem, s>>>(b);
+    k_batch_team_dir<true><<<b.n_units, threads, smem, s>>>(b);
   return cudaGetLastError();
 }
 

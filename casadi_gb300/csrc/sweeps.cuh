@@ -262,7 +262,8 @@ struct BatchItem {
   int adj_ngr;              // its groups of kBatchAdjGroup entries
   const int2* zero_in;      // inputs with a structurally zero adjoint
   int n_zero;
-  // cooperative units (k_batch_team): the streams of a kBatchTeam team's warps
+  // cooperative units (k_batch_team): the streams of a kBatchTeam team's warps (split items
+  // recorded before the directions: of the record team's)
   const uint4* team;
   const int2* team_at;      // per warp: first entry, blocks
   const uint4* dir_team;    // keyed adjoint entries, or tangent entries of each direction
@@ -305,7 +306,9 @@ constexpr int kBatchTeamSize = 1, kBatchTeam = 4 << kBatchTeamSize;  // warps of
 // One launch over b.units, b.n_units: record (or value) walks, the adjoint walks that follow them
 // (both at most as many units as the scratch has places), or single directions of split items
 enum BatchTeamKind { BT_VALUE, BT_ADJOINT, BT_DIRECTION };
-cudaError_t launch_batch_team(const BatchArgs& b, BatchTeamKind kind, size_t smem, cudaStream_t s);
+// threads: 32 * kBatchTeam; record walks of split items may have other teams (a multiple of 32)
+cudaError_t launch_batch_team(const BatchArgs& b, BatchTeamKind kind, int threads, size_t smem,
+                              cudaStream_t s);
 cudaError_t launch_batch(const BatchArgs& b, int grid, size_t smem, bool split, bool gw,
                          cudaStream_t s);
 int occupancy_batch(size_t smem, bool split, bool gw);

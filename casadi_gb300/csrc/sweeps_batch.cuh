@@ -138,7 +138,8 @@ __device__ __forceinline__ double* batch_partials(const BatchArgs& b, const Batc
               : b.scratch + static_cast<size_t>(blockIdx.x) * b.scratch_stride) + lane;
 }
 
-__global__ void __launch_bounds__(32 * kBatchTeam, 4)
+// (blockDim.x: 32 * kBatchTeam, or the warps of the split items' record teams)
+__global__ void __launch_bounds__(kCoopMaxThreads)
     k_batch_team(const __grid_constant__ BatchArgs b) {
   const PlainUnits u;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -150,7 +151,7 @@ __global__ void __launch_bounds__(32 * kBatchTeam, 4)
   const long long iv = active ? il : it.n - 1;
   const IoDesc* io = it.io;
   uint4* ring = reinterpret_cast<uint4*>(smem) + warp * (2 * kEntBlock);
-  unsigned char* wb = smem + kBatchTeam * kEntRingBytes + lane * 8;
+  unsigned char* wb = smem + (blockDim.x >> 5) * kEntRingBytes + lane * 8;
   const int2 vs = __ldg(it.team_at + warp);
   PairState pair;
   if (it.ndir == 0) {
