@@ -1636,7 +1636,17 @@ bool ensure_levels(Tape& t, bool reverse = false) {
   if (static_cast<unsigned>(t.n_partials) > kTeamPidxMask) return false;  // not addressed
   Levels lv;
   std::string err;
-  const int cap = t.sz_w <= 400 ? 400 : t.sz_w + kLevelWidth;
+  // Slots the schedule may keep live: 400, two teams to an SM, for a tape of few live values (looking
+  // ahead finds its parallel work); a tape that keeps more than 128 live is wide by itself, and what
+  // counts is that three or four teams fit (16 slots to spare): the mixed queue of random graphs (160
+  // live) 16.0 -> 14.8 ms, their sparsity sweeps 753 -> 714 us at 190 slots against 400, the MPC
+  // records (50 and 124 live) 2.07 ms at 400 against 2.45 at 190.
+  const int need = t.sz_w + 16;
+  const int cap = t.sz_w <= 128 ? 400
+                  : need <= 190 ? 190
+                  : need <= 266 ? 266
+                  : t.sz_w <= 400 ? 400
+                                  : t.sz_w + kLevelWidth;
   const int nl = level_schedule(t.h_code, kLevelWidth, cap, lv, err, reverse);
   if (nl <= 0 || lv.code.empty()) return false;
   uint4* team[kTeamSizes] = {};
