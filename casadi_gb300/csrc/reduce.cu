@@ -22,16 +22,22 @@ constexpr int kWarpsPerCta = 8;
 // scan, exact as long as every intermediate m stays inside the binade. A CTA takes a chunk of
 // 4096 elements of a row: scan, then every thread replays its eight steps from its own start and
 // looks for the first m outside (2^52, 2^53). Up to there the result is the sequential one; that
-// element is added in FP64, and the scan starts again after it. Where it gets nowhere (sums that
-// stay near zero, infinities and NaN) one thread adds a stretch of elements in order, twice as
-// many each time.
+// element is added in FP64, and the scan goes on after it: by one warp, 128 elements at a time,
+// since failures come in clusters (a sum about a power of two crosses it every third element or
+// so), until four windows have passed without one; a window that ends early is followed by 8, 16,
+// ... 64 elements in FP64 (sums that stay near zero, infinities and NaN: all of them).
 //
-// A dependent FP64 addition takes about 70 cycles. The rollout's cost and 20 shared controls'
-// gradients summed over 131072 instances (21 rows, one launch): 9.0 ms as plain chains, 0.42 ms.
+// A dependent FP64 addition takes about 70 cycles, a warp's window as much as eight of them. The
+// rollout's cost and 20 shared controls' gradients summed over 131072 instances (21 rows, one launch)
+// take 9.0 ms as plain chains and 0.28 to 0.55 ms here, by how long a gradient's sum stays about a
+// power of two; 2.33 ms where one is near zero throughout (5063 crossings). With the CTA's scan after
+// every failure these were 0.32 to 0.72 and 3.39 ms.
 constexpr int kOrdThreads = 512;
 constexpr int kOrdPer = 8;
 constexpr int kOrdChunk = kOrdThreads * kOrdPer;
-constexpr int kOrdMinStretch = 32;  // elements; an attempt costs about as much as 50 additions
+constexpr int kOrdLane = 4, kOrdWindow = 32 * kOrdLane;  // elements of a lane and of a warp's scan
+constexpr int kOrdClean = 4;        // windows without a failure before the CTA scans again
+constexpr int kOrdMinSerial = 8, kOrdMaxSerial = 64;  // a warp's scan costs as much as 8 additions
 constexpr long long kM52 = 1ll << 52, kM53 = 1ll << 53;
 
 // Increments of m over a run of steps that starts at an even (i0) or odd (i1) m.
@@ -65,6 +71,51 @@ __device__ __forceinline__ bool step_of(double x, int es, bool sneg, Inc* out) {
 
 __device__ __forceinline__ int ord_pad(int i) { return i + (i >> 3); }  // conflict-free by eights
 
+// Adds elements [i, i + w) to *s by one warp (w <= kOrdWindow), up to the first that needs a step in
+// FP64; how many were added.
+__device__ __forceinline__ int sum_window(const double* buf, int i, int w, int lane, double* s) {
+  const long long sb = __double_as_longlong(*s);
+  const int es = static_cast<int>((sb >> 52) & 0x7ff);
+  const bool sneg = sb < 0;
+  if (es < 2 || es == 2047) return 0;
+  const long long m0 = (sb & (kM52 - 1)) | kM52;
+  const long long top = (sneg ? kM52 << 11 : 0) | (static_cast<long long>(es) << 52);
+  Inc step[kOrdLane], inc{0, 0};
+  bool out[kOrdLane];
+#pragma unroll
+  for (int j = 0; j < kOrdLane; ++j) {
+    const int k = lane * kOrdLane + j;
+    const bool in = k < w;
+    out[j] = !step_of(in ? buf[ord_pad(i + k)] : 0.0, es, sneg, &step[j]);
+    if (out[j]) step[j] = Inc{0, 0};
+    inc = compose(inc, step[j]);
+  }
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const Inc up = shfl_up(inc, d);
+    if (lane >= d) inc = compose(up, inc);
+  }
+  Inc pre = shfl_up(inc, 1);
+  if (lane == 0) pre = Inc{0, 0};
+  long long m = m0 + ((m0 & 1) ? pre.i1 : pre.i0), m_fail = m;
+  int f = kOrdLane;
+#pragma unroll
+  for (int j = 0; j < kOrdLane; ++j) {
+    const long long mj = m + ((m & 1) ? step[j].i1 : step[j].i0);
+    if (f == kOrdLane && lane * kOrdLane + j < w && (out[j] || mj <= kM52 || mj >= kM53)) {
+      f = j;
+      m_fail = m;
+    }
+    m = mj;
+  }
+  const unsigned failed = __ballot_sync(kFull, f < kOrdLane);
+  const int at = failed ? __ffs(failed) - 1 : 31;
+  const long long end = __shfl_sync(kFull, failed ? m_fail : m, at);
+  const int got = failed ? at * kOrdLane + __shfl_sync(kFull, f, at) : w;
+  *s = __longlong_as_double(top | (end & (kM52 - 1)));
+  return got;
+}
+
 struct SumRowsArgs {
   SumRows g[kMaxSumGroups];
   int count;
@@ -91,7 +142,7 @@ __global__ void __launch_bounds__(kOrdThreads)
       }
     };
     fetch(0);
-    int stretch = kOrdMinStretch;
+    int serial = kOrdMinSerial;
     for (long long pos = 0; pos < n; pos += kOrdChunk) {
       __syncthreads();
 #pragma unroll
@@ -164,39 +215,45 @@ __global__ void __launch_bounds__(kOrdThreads)
           const long long top = (sneg ? kM52 << 11 : 0) | (static_cast<long long>(es) << 52);
           if (fail >= cnt) {
             s = __longlong_as_double(top | ((m0 + ((m0 & 1) ? tot1 : tot0)) & (kM52 - 1)));
-            stretch = kOrdMinStretch;
             break;
           }
           if (mine == fail) sum_at = __longlong_as_double(top | (m_fail & (kM52 - 1)));
         } else if (t == 0) {
           sum_at = s;
         }
-        // elements fail, fail + 1, ... in FP64: one where the scan got somewhere, else a stretch
-        int len = 1;
-        if (fail - off < 2 * kOrdMinStretch) {
-          len = stretch;
-          stretch = min(2 * stretch, kOrdChunk);
-        } else {
-          stretch = kOrdMinStretch;
-        }
-        len = min(len, cnt - fail);
         __syncthreads();
-        if (t == 0) {
+        if (warp == 0) {
           double acc = sum_at;
           int i = fail;
-          for (; i + 8 <= fail + len; i += 8) {
-            double v[8];
+          for (int clean = 0; i < cnt && clean < kOrdClean;) {
+            // the failing element in FP64 (in a stretch of failures: some more)
+            const int end = min(i + serial, cnt);
+            for (; i + 8 <= end; i += 8) {
+              double v[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = buf[ord_pad(i + k)];
+              for (int k = 0; k < 8; ++k) v[k] = buf[ord_pad(i + k)];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) acc = __dadd_rn(acc, v[k]);
+              for (int k = 0; k < 8; ++k) acc = __dadd_rn(acc, v[k]);
+            }
+            for (; i < end; ++i) acc = __dadd_rn(acc, buf[ord_pad(i)]);
+            for (clean = 0; i < cnt && clean < kOrdClean; ++clean) {
+              const int w = min(kOrdWindow, cnt - i), got = sum_window(buf, i, w, lane, &acc);
+              i += got;
+              if (got < w) {
+                serial = got < 2 * kOrdMinSerial ? min(2 * serial, kOrdMaxSerial) : kOrdMinSerial;
+                break;
+              }
+            }
           }
-          for (; i < fail + len; ++i) acc = __dadd_rn(acc, buf[ord_pad(i)]);
-          sum_at = acc;
+          if (lane == 0) {
+            sum_at = acc;
+            fail_at = i;
+          }
         }
         __syncthreads();
         s = sum_at;
-        off = fail + len;
+        off = fail_at;
+        __syncthreads();
       }
     }
     if (t == 0) a.g[g].dst[r] = s;

@@ -269,3 +269,21 @@ def test_instance_order_sum_is_the_sequential_sum(gpu_lib, kind, n):
         want = np.cumsum(np.concatenate([np.zeros((3, 1)), rows * [[1], [1], [-1]]], 1), 1)[:, -1]
     both_nan = np.isnan(got) & np.isnan(want)
     assert (both_nan | (got.view(np.uint64) == want.view(np.uint64))).all(), (got, want)
+
+
+@pytest.mark.parametrize("level", [0.0, 256.0, -1.0, 2.0 ** -1021])
+@pytest.mark.parametrize("n", [127, 128, 129, 130, 641, 4224, 20003])
+def test_instance_order_sum_near_a_binade_edge(gpu_lib, level, n):
+    """Sums that stay about a power of two (or zero), so that the scan meets failures every few
+    elements and every window of a warp's scan ends somewhere: the sequential sum's bits."""
+    rng = np.random.default_rng(n)
+    x = S.sym("x", 3)
+    f = S.Function("I", [x], [[x[0], x[1], x[2]]])
+    scale = abs(level) / 256 if level else 1.0
+    rows = rng.standard_normal((3, n)) * scale * np.array([[1.0], [0.05], [1e-3]])
+    rows[:, 0] = level
+    sign = np.sign(rows[:, 1:]) * np.sign(np.cumsum(rows, 1)[:, :-1] - level)
+    rows[:, 1:] *= np.where((sign > 0) & (rng.random((3, n - 1)) < 0.1), -1.0, 1.0)  # drawn back
+    got = host(CudaMapSum(f, n, reduce_out=[True]).eval(dev([rows])))[0]
+    want = np.cumsum(np.concatenate([np.zeros((3, 1)), rows], 1), 1)[:, -1]
+    assert (got.view(np.uint64) == want.view(np.uint64)).all(), (got, want)
