@@ -58,10 +58,12 @@ def make_workload(name, instances=None):
 
 
 # ---- algorithmic work per instance --------------------------------------------------------------
-# Counted in FP64-pipe instructions (DADD, DMUL and DFMA each count one; a libm call counts its
-# measured DFMA-instruction equivalents from op_weights.json), split by kind: on GB300 the pipe
-# issues a DFMA chain at a higher rate than DADD or DMUL (casadi_gb300_fp64_rate, measured in the
-# same run), so each kernel's ceiling is the rate of its own instruction mix.
+# Counted in FP64-pipe instructions (DADD, DMUL and DFMA each count one), split by kind: on GB300
+# the pipe issues a DFMA chain at a higher rate than DADD or DMUL (casadi_gb300_fp64_rate, measured
+# in the same run), so each kernel's ceiling is the rate of its own instruction mix. Division, the
+# square root, sin, cos, exp, log, tanh, comparisons, minima and maxima are computed in integer
+# arithmetic and count nothing; the rarer functions count the DFMA-instruction equivalents of
+# op_weights.json. The derivative sweeps issue their products and sums as DFMA.
 def _carries(op):
     from casadi_gb300 import calculus as C
     zero_d0 = {C.OP_LT, C.OP_LE, C.OP_EQ, C.OP_NE, C.OP_NOT, C.OP_AND, C.OP_OR, C.OP_FLOOR,
@@ -149,15 +151,21 @@ def structural_adjoint_ops(tape, seeded_out):
     """FP64 instructions of one adjoint direction by kind (the adjoint kernel's cases): a
     seeded output or an ADD/SUB/ASSIGN/NEG/TWICE/IF_ELSE_ZERO contribution that is not the
     slot's first one DADD; a general op's contribution DMUL when first, else one DFMA into the
-    running adjoint."""
+    running adjoint. Nothing is contributed to a constant."""
     from casadi_gb300 import calculus as C
     ops, i0, i1, i2 = (tape.op.tolist(), tape.i0.tolist(), tape.i1.tolist(), tape.i2.tolist())
+    is_const, const_ops = [False] * max(1, tape.sz_w), []
+    for k, op in enumerate(ops):
+        const_ops.append((op not in (C.OP_CONST, C.OP_INPUT) and is_const[i1[k]],
+                          op in C.BINARY_OPS and is_const[i2[k]]))
+        if op != C.OP_OUTPUT:
+            is_const[i0[k]] = op == C.OP_CONST
     act = [False] * max(1, tape.sz_w)
     mix = _mix()
     for k in range(len(ops) - 1, -1, -1):
         op = ops[k]
         if op == C.OP_OUTPUT:
-            if seeded_out[i0[k]]:
+            if seeded_out[i0[k]] and not const_ops[k][0]:
                 mix["dadd"] += 1 if act[i1[k]] else 0
                 act[i1[k]] = True
             continue
@@ -168,8 +176,8 @@ def structural_adjoint_ops(tape, seeded_out):
             continue
         act[i0[k]] = False
         c0, c1 = _carries(op)
-        for slot, carries in ((i1[k], c0), (i2[k], c1 and op in C.BINARY_OPS)):
-            if not carries:
+        for j, (slot, carries) in enumerate(((i1[k], c0), (i2[k], c1 and op in C.BINARY_OPS))):
+            if not carries or const_ops[k][j]:
                 continue
             first = not act[slot]
             if op in (C.OP_ADD, C.OP_SUB, C.OP_ASSIGN, C.OP_NEG, C.OP_IF_ELSE_ZERO, C.OP_TWICE):
@@ -180,7 +188,7 @@ def structural_adjoint_ops(tape, seeded_out):
     return mix
 
 
-SIMPLE_OPS = ("ADD", "SUB", "MUL", "SQ", "IF_ELSE_ZERO", "LT", "LE", "EQ", "NE", "FMIN", "FMAX")
+SIMPLE_OPS = ("ADD", "SUB", "MUL", "SQ")
 
 
 def sincos_pairs(tape):
@@ -217,36 +225,29 @@ def sincos_reuse(tape):
 def algorithmic_flops(tape, weights, rates, seeded_out=None, unit_dirs=True, wanted_out=None):
     """Per instance and kernel family: FP64-pipe instructions ("instr") and their time at the
     measured rates expressed in DFMA-chain instructions ("dfma_time"); the family's ceiling
-    is rate_dfma * instr / dfma_time. Value and record sweeps: simple ops (one DADD or DMUL
-    each, weight 1) at the DADD/DMUL rate, libm calls at their measured DFMA equivalents
-    (op_weights.json); TWICE, the sign-bit ops and selections cost no FP64 instruction. A SIN or
-    COS that takes the previous one's sin/cos pair costs none; a record of SIN or COS is one
-    sincos (the value and the partial), and so is the value of the first of a pair
-    (sincos_pairs)."""
+    is rate_dfma * instr / dfma_time. Value and record sweeps: ADD, SUB, MUL and SQ one DADD or
+    DMUL each, the functions without an integer routine at their DFMA equivalents
+    (op_weights.json, "fp64_weights"), everything else none. Derivative sweeps: DFMA."""
     from casadi_gb300 import calculus as C
     slow = rates["dfma"] / min(rates["dadd"], rates["dmul"])
     out = {"eval": {"instr": 0.0, "dfma_time": 0.0}, "record": {"instr": 0.0, "dfma_time": 0.0}}
-    pairs = sincos_pairs(tape)
-    reuse, first = pairs["reuse"], pairs["first"]
     for op, cnt in zip(*np.unique(tape.op, return_counts=True)):
         op = int(op)
         if op in (C.OP_CONST, C.OP_INPUT, C.OP_OUTPUT):
             continue
         name = C.OP_NAMES[op]
-        w = 0.0 if name == "TWICE" else float(weights.get(name, 1.0))
+        w = float(weights.get(name, 0.0))
         t = w * (slow if name in SIMPLE_OPS else 1.0)
         wp = float(weights.get(name + "_partial", 0.0))
-        ec, fc = cnt - reuse.get(op, 0) - first.get(op, 0), first.get(op, 0)
-        out["eval"]["instr"] += ec * w + fc * (w + wp)
-        out["eval"]["dfma_time"] += ec * t + fc * (t + wp)
-        rc = cnt - reuse.get(op, 0)
-        out["record"]["instr"] += rc * (w + wp)
-        out["record"]["dfma_time"] += rc * (t + wp)
+        out["eval"]["instr"] += cnt * w
+        out["eval"]["dfma_time"] += cnt * t
+        out["record"]["instr"] += cnt * (w + wp)
+        out["record"]["dfma_time"] += cnt * (t + wp * slow)
     seeded_out = seeded_out or [True] * len(tape.nnz_out)
     for fam, mix in (("tangent", structural_tangent_ops(tape, unit_dirs, wanted_out=wanted_out)),
                      ("adjoint", structural_adjoint_ops(tape, seeded_out))):
         out[fam] = {"instr": float(sum(mix.values())), "mix": mix,
-                    "dfma_time": mix["dfma"] + (mix["dadd"] + mix["dmul"]) * slow}
+                    "dfma_time": float(sum(mix.values()))}
     for v in out.values():
         v["peak"] = rates["dfma"] * v["instr"] / v["dfma_time"] if v["dfma_time"] else None
     return out
@@ -256,7 +257,7 @@ def load_weights():
     p = os.path.join(ROOT, "casadi_gb300", "op_weights.json")
     if os.path.exists(p):
         with open(p) as f:
-            return json.load(f)["weights"]
+            return json.load(f)["fp64_weights"]
     return {}
 
 
@@ -1133,10 +1134,11 @@ def run_native(a):
                      "unit": "T FP64 instr/s", "frac": achieved / peak if peak else None,
                      "traffic": traffic,
                      "traffic_unit": "bytes per launch (ncu, scaled from the committed capture)",
-                     "flop": "one FP64-pipe instruction (DADD, DMUL, DFMA); libm calls weighted by "
-                             "casadi_gb300/op_weights.json; derivative sweeps count structural work "
-                             "(a two-operand tangent: DMUL + DFMA; a later adjoint contribution: "
-                             "one DFMA)",
+                     "flop": "one FP64-pipe instruction (DADD, DMUL, DFMA); division, sqrt, sin, cos, "
+                             "exp, log and tanh run in integer arithmetic and count none (the value "
+                             "and record sweeps are bound by the integer pipes: their frac is the "
+                             "FP64 pipe's share); derivative sweeps count structural work (a "
+                             "two-operand tangent: two; a later adjoint contribution: one)",
                      "peak_source": "FP64 chain probes of this run (casadi_gb300_fp64_rate: "
                                     "every thread of a full grid runs 8 independent chains; "
                                     "thread-level instructions per second), weighted by the "
