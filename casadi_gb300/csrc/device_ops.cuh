@@ -219,15 +219,56 @@ __device__ __forceinline__ double d_fmax(double x, double y) {
   return d_key(y) > d_key(x) ? y : x;
 }
 
-// CUDA's functions for the arguments the integer routines leave out, out of line: rarely
-// reached, and one copy serves every use in a kernel.
-static __device__ __noinline__ double slow_div(double x, double y) { return __ddiv_rn(x, y); }
-static __device__ __noinline__ double slow_sqrt(double x) { return __dsqrt_rn(x); }
-static __device__ __noinline__ double slow_sin(double x) { return sin(x); }
-static __device__ __noinline__ double slow_cos(double x) { return cos(x); }
-static __device__ __noinline__ double slow_exp(double x) { return exp(x); }
-static __device__ __noinline__ double slow_log(double x) { return log(x); }
-static __device__ __noinline__ double slow_tanh(double x) { return tanh(x); }
+// The arguments the integer routines leave out, out of line: rarely reached, and one copy serves
+// every use in a kernel. Zeros, infinities, NaN and results that overflow or underflow are settled
+// here; CUDA's functions for the rest. A graph whose values run off keeps whole tiles on them: record
+// and adjoint of the unbounded 10000-node graph at 16384 instances 2.97 -> 1.94 ms.
+constexpr unsigned long long kInfBits2 = 0xffe0000000000000ull;  // magnitude of infinity, doubled
+__device__ __forceinline__ unsigned long long mag2(double x) {  // 0: zero, > kInfBits2: NaN
+  return static_cast<unsigned long long>(__double_as_longlong(x)) << 1;
+}
+__device__ __forceinline__ double signed_of(unsigned long long sign_src, unsigned long long bits) {
+  return __longlong_as_double(static_cast<long long>((sign_src & 0x8000000000000000ull) | bits));
+}
+static __device__ __noinline__ double slow_div(double x, double y) {
+  const unsigned long long ax = mag2(x), ay = mag2(y);
+  if (ax > kInfBits2 || ay > kInfBits2) return __dadd_rn(x, y);  // NaN
+  const bool zero = ax == 0 || ay == kInfBits2, inf = ay == 0 || ax == kInfBits2;
+  if (zero && inf) return CUDART_NAN;  // 0/0, inf/inf
+  if (zero || inf)
+    return signed_of(static_cast<unsigned long long>(__double_as_longlong(x) ^ __double_as_longlong(y)),
+                     inf ? kInfBits2 >> 1 : 0);
+  return __ddiv_rn(x, y);
+}
+static __device__ __noinline__ double slow_sqrt(double x) {
+  const unsigned long long ax = mag2(x);
+  if (ax > kInfBits2 || (ax == kInfBits2 && __double_as_longlong(x) > 0)) return __dadd_rn(x, x);
+  if (ax != 0 && __double_as_longlong(x) < 0) return CUDART_NAN;
+  return __dsqrt_rn(x);
+}
+static __device__ __noinline__ double slow_sin(double x) {
+  return mag2(x) >= kInfBits2 ? __dsub_rn(x, x) : sin(x);
+}
+static __device__ __noinline__ double slow_cos(double x) {
+  return mag2(x) >= kInfBits2 ? __dsub_rn(x, x) : cos(x);
+}
+static __device__ __noinline__ double slow_exp(double x) {
+  if (mag2(x) > kInfBits2) return __dadd_rn(x, x);
+  const long long b = __double_as_longlong(x);
+  if ((b & 0x7fffffffffffffffll) >= 0x4087500000000000ll)  // |x| >= 746
+    return b < 0 ? 0.0 : CUDART_INF;
+  return exp(x);
+}
+static __device__ __noinline__ double slow_log(double x) {
+  const unsigned long long ax = mag2(x);
+  if (ax == 0) return -CUDART_INF;
+  if (ax > kInfBits2) return __dadd_rn(x, x);
+  if (__double_as_longlong(x) < 0) return CUDART_NAN;
+  return ax == kInfBits2 ? x : log(x);
+}
+static __device__ __noinline__ double slow_tanh(double x) {
+  return mag2(x) > kInfBits2 ? __dadd_rn(x, x) : tanh(x);
+}
 
 // x / y for a divisor prepared once (y: the same value)
 __device__ __forceinline__ double d_div(double x, double y, const FxDivisor& d) {
