@@ -2123,7 +2123,6 @@ int run_ad_multi(Tape& t, long long n, const IoDesc* in, const IoDesc* out,
       a.queue = reinterpret_cast<unsigned long long*>(static_cast<char*>(scratch) + used);
     a.pofs = t.d_pofs;
     a.n_code = t.n_chunks * kChunk;
-    for (int j = 0, off = 0; j < t.n_in; off += t.nnz_in[j], ++j) a.in_off[j] = off;
     std::memcpy(a.in, in, sizeof(IoDesc) * t.n_in);
     std::memcpy(a.out, out, sizeof(IoDesc) * t.n_out);
     if (!recorded)

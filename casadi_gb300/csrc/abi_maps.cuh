@@ -466,7 +466,6 @@ int accum_forward_values(Tape& t, int N, int n_accum, long long n, long long ld,
       a.partials = reinterpret_cast<double*>(partials + k * accum_call_partials(t, n));
       a.pofs = t.d_pofs;
       a.n_code = t.n_chunks * kChunk;
-      for (int j = 0, off = 0; j < t.n_in; off += t.nnz_in[j], ++j) a.in_off[j] = off;
     }
     for (int j = 0; j < t.n_in; ++j) {
       const int nz = t.nnz_in[j];

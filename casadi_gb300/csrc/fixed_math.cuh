@@ -12,8 +12,10 @@
 //   doubles, so one more bit than the result and no sticky bit decides the rounding.
 // * fx_sincos, fx_exp, fx_log, fx_tanh evaluate in 64-bit fixed point: argument reduction by a
 //   96-bit constant, Chebyshev interpolants of the functions with the coefficients' and products'
-//   width matched to their weight (errors below 2^-57), one rounding to double at the end. The
-//   largest error is about 0.51 ulp.
+//   width matched to their weight (errors below 2^-57), one rounding to double at the end. Largest
+//   error against 113-bit references over 2^21 arguments a range, CUDA's function beside it: sin and
+//   cos 0.504 ulp up to 3.2 (1.39) and 0.69 up to 100 (1.47), exp 0.532 (0.864), log 0.532
+//   (0.547), tanh 0.597 (1.42).
 //
 // Arguments outside a routine's range (subnormals, infinities, NaN, zero numerators, quotients near
 // the ends of the exponent range, huge arguments) make it return false; the caller takes CUDA's

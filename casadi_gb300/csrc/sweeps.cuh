@@ -220,7 +220,6 @@ struct SweepArgs {
   IoDesc out[kMaxIo];       // values out
   IoDesc seed[kMaxIo];      // forward: input seeds / adjoint: output seeds
   IoDesc sens[kMaxIo];      // forward: output sensitivities / adjoint: input sensitivities
-  int in_off[kMaxIo];       // flat offset of each input's first nonzero (identity seeds)
   const int2* zero_in;              // adjoint: (input, nonzero) pairs with a zero sensitivity
   int n_zero;
   // keyed entry streams (host-compiled, one layout per group size; the launchers pick the

@@ -465,7 +465,8 @@ CASADI_GB300_API int casadi_gb300_star_coloring(int n, const int* colind, const 
  * sweep, nadj > 0 the value sweep plus nadj adjoint directions (aseed/asens as in
  * casadi_gb300_reverse). casadi_gb300_batch_run evaluates every item in ONE persistent launch
  * whose warps drain a longest-first list of (item, 32-instance tile) units, so tapes of
- * uneven length and instance count keep the GPU full. With use_graph the launch is captured
+ * uneven length and instance count keep the GPU full; where work vectors leave an SM few warps, a
+ * sequence of launches in which teams of warps take the units. With use_graph the launch is captured
  * once into a CUDA graph (on a stream the batch owns, ordered after and before the caller's
  * stream) and replayed; adding items or changing the scratch buffer re-captures it.
  * casadi_gb300_batch_add returns the item index. An item with two or more directions is
