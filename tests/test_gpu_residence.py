@@ -149,3 +149,25 @@ def test_every_team_size_gives_the_sequential_bits(gpu_lib, tiles):
             t.sync()
         for a, b in zip(*got):
             assert_bitexact(a, b, "team, %d tiles" % tiles)
+
+
+@pytest.mark.parametrize("nodes,window", [(300, 200), (700, 256)])
+def test_cooperative_adjoint_of_a_large_launch(gpu_lib, nodes, window):
+    """A tape with many live values takes the cooperative adjoint in launches of any size: more
+    than 16 tiles per SM, a ragged last tile, the sequential sweep's bits."""
+    n = 77824 + 3 * 32 + 5
+    g = W.random_dag(n_in=40, n_nodes=nodes, n_out=4, seed=nodes, window=window, bounded=True)
+    rng = np.random.default_rng(nodes)
+    args = _dev(W.dag_inputs(n, n_in=40, seed=3))
+    seeds = _dev([rng.standard_normal((1, 4, n))])
+    ct = R.CudaTape(g)
+    ct.set_variant(2, 0)
+    want = ct.reverse(args, seeds)[1]
+    ct.set_variant(2, 6)
+    got = ct.reverse(args, seeds)[1]
+    for x, y in zip(got, want):
+        assert bool((x.view(torch.int64) == y.view(torch.int64)).all())
+    ct.set_variant(2, -1)
+    for x, y in zip(ct.reverse(args, seeds)[1], want):  # tuned
+        assert bool((x.view(torch.int64) == y.view(torch.int64)).all())
+    ct.sync()
