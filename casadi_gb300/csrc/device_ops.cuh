@@ -163,11 +163,12 @@ __device__ __forceinline__ double d_neg(double x) {
 // is incremented with an integer add, which is exactly 2*x; zeros, subnormals, the largest
 // binade, inf and NaN go through the FP64 add. Identical to __dadd_rn(x, x) in every case;
 // keeps the FP64 pipe free for the common case.
+static __device__ __noinline__ double slow_twice(double x) { return __dadd_rn(x, x); }
 __device__ __forceinline__ double d_twice(double x) {
   const long long b = __double_as_longlong(x);
   const unsigned e = static_cast<unsigned>((b >> 52) & 0x7ff);
   if (e - 1u < 2045u) return __longlong_as_double(b + (1ll << 52));
-  return __dadd_rn(x, x);
+  return slow_twice(x);  // out of line: a predicated addition would occupy the pipe all the same
 }
 __device__ __forceinline__ double d_fabs(double x) {
   return __longlong_as_double(__double_as_longlong(x) & (long long)~kSignBit);
@@ -268,6 +269,18 @@ static __device__ __noinline__ double slow_log(double x) {
 }
 static __device__ __noinline__ double slow_tanh(double x) {
   return mag2(x) > kInfBits2 ? __dadd_rn(x, x) : tanh(x);
+}
+
+// a * 2^k, dz = k << 20: an addition to the exponent; a product where a or the result is not a normal
+// number.
+static __device__ __noinline__ double slow_scale(double a, int dz) {
+  return __dmul_rn(a, __hiloint2double(0x3ff00000 + dz, 0));
+}
+__device__ __forceinline__ double d_scale(double a, int dz) {
+  const int hi = __double2hiint(a), e = hi & 0x7ff00000;
+  const bool ok = static_cast<unsigned>(e - 0x100000) < 0x7fe00000u &&
+                  static_cast<unsigned>(e) + dz - 0x100000u < 0x7fe00000u;
+  return ok ? __hiloint2double(hi + dz, __double2loint(a)) : slow_scale(a, dz);
 }
 
 // x / y for a divisor prepared once (y: the same value)

@@ -417,6 +417,7 @@ __device__ __forceinline__ double tf_eval(const Units& u, double p, double q, do
   else if constexpr (F == TF_YMZ) return u_sub(u, a, b);
   else if constexpr (F == TF_NY) return d_neg(a);
   else if constexpr (F == TF_2Y) return d_twice(a);
+  else if constexpr (F == TF_SY) return d_scale(a, __double2hiint(b));
   else return d_iszero(q) ? 0.0 : b;  // TF_IFZ
 }
 
@@ -486,7 +487,9 @@ __device__ __forceinline__ void tan_group(const Units& u, const uint4 (&E)[G], c
   case KEY:                                                              \
     CGB_JK {                                                             \
       const double av = tf_uses_y(F) ? CGB_W(cur.y, j, k) : 0.0;         \
-      const double bv = tf_uses_z(F) ? CGB_W(cur.z, j, k) : 0.0;         \
+      const double bv = tf_uses_z(F)  ? CGB_W(cur.z, j, k)               \
+                        : F == TF_SY ? __hiloint2double(cur.z, 0)        \
+                                     : 0.0;                              \
       r[j][k] = tf_eval<F>(u, P[i][j], Q[i][j], av, bv);                    \
     }                                                                    \
     break;

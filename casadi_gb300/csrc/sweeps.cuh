@@ -66,11 +66,12 @@ enum TanForm : int {
   TF_YMZ,   // a - b                   (SUB)
   TF_NY,    // -a                      (NEG)
   TF_2Y,    // 2a                      (TWICE)
-  TF_IFZ    // q == 0 ? 0 : b          (IF_ELSE_ZERO)
+  TF_IFZ,   // q == 0 ? 0 : b          (IF_ELSE_ZERO)
+  TF_SY     // a times a power of two  (a constant partial; z: what it adds to a's high word)
 };
 __host__ __device__ constexpr bool tf_uses_y(int f) {
   return f == TF_PY || f == TF_PYQZ || f == TF_Y || f == TF_YQZ || f == TF_YZ || f == TF_YMZ ||
-         f == TF_NY || f == TF_2Y;
+         f == TF_NY || f == TF_2Y || f == TF_SY;
 }
 __host__ __device__ constexpr bool tf_uses_z(int f) {
   return f == TF_QZ || f == TF_PYQZ || f == TF_Z || f == TF_YQZ || f == TF_YZ || f == TF_NZ ||
@@ -86,7 +87,7 @@ __host__ __device__ constexpr bool tf_uses_q(int f) {
 #define CGB_TK_ARITH(X)                                                                      \
   X(TK_PY, TF_PY) X(TK_QZ, TF_QZ) X(TK_Y, TF_Y) X(TK_Z, TF_Z) X(TK_NZ, TF_NZ)                 \
   X(TK_NY, TF_NY) X(TK_2Y, TF_2Y) X(TK_IFZ, TF_IFZ) X(TK_PYQZ, TF_PYQZ) X(TK_YQZ, TF_YQZ)    \
-  X(TK_YZ, TF_YZ) X(TK_YMZ, TF_YMZ)
+  X(TK_YZ, TF_YZ) X(TK_YMZ, TF_YMZ) X(TK_SY, TF_SY)
 #define CGB_KEY_ENUM(K, ...) K,
 // TK_OUT0/TK_OUT: an output's sensitivity (x output, y slot, z nonzero) is 0 or the slot's
 // tangent; TK_IN: an input's seed (x slot, y input, z nonzero); TK_MIXED + pm: a union-stream

@@ -63,3 +63,30 @@ def test_constant_operands_in_every_variant(gpu_lib, n):
     for g, w in zip(_host(asens), wa):
         assert_bitexact(g, w, "batch")
     ct.sync()
+
+
+@pytest.mark.parametrize("factor", [0.5, 4.0, 2.0 ** -1000, 2.0 ** 1000, 2.0 ** -1022, -0.5])
+def test_tangents_of_products_with_powers_of_two(gpu_lib, factor):
+    """A product's tangent with a power of two as the partial is an exponent addition: seeds that
+    are zero, subnormal, huge, infinite or NaN, and results that leave the normal range, in every
+    variant, against the oracle's product."""
+    x = S.sym("x", 2)
+    t = S.Function("P", [x], [[factor * x[0], x[1] * factor + 0.25 * x[0]]]).tape
+    v = np.array([0.0, -0.0, 1.0, -3.7, 1e-300, -1e300, 5e-324, 2.2250738585072014e-308, np.inf, -np.inf,
+                  np.nan, 1.7976931348623157e308, 3e-310, 2.0 ** -50, 1e154])
+    seeds = np.stack([v, v[::-1]])[None]
+    seeds = np.concatenate([np.tile(seeds, (1, 1, 9)), np.ones((1, 2, 135))])
+    n = seeds.shape[2]
+    args = [np.random.default_rng(1).standard_normal((2, n))]
+    with np.errstate(all="ignore"):
+        _, want = O.forward(t, args, [seeds], n)
+        _, wj = O.jacobian(t, args, n)
+    ct = R.CudaTape(t)
+    for k in range(R.TAN_WINDOWED + 1):
+        ct.set_variant(0, k)
+        ct.set_variant(1, k)
+        for g, w in zip(_host(ct.forward(_dev(args), _dev([seeds]))[1]), want):
+            assert_bitexact(g, w, "forward, variant %d" % k)
+        for g, w in zip(_host(ct.jacobian(_dev(args))[1]), wj):
+            assert_bitexact(g, w, "jacobian, variant %d" % k)
+    ct.sync()
