@@ -110,7 +110,8 @@ def structural_tangent_ops(tape, unit_dirs=True, ndir=None, wanted_out=None):
     split by kind, following the structural rules the sweeps apply (the tangent kernel's
     cases): ADD/SUB of two carried operands one DADD; a general op one DMUL per carried
     operand, two carried: DMUL + DFMA; TWICE, NEG, ASSIGN, IF_ELSE_ZERO none (integer
-    exponent/sign operations, selections). Instructions that reach no output of
+    exponent/sign operations, selections), nor a product with a constant power of two (an exponent
+    addition). Instructions that reach no output of
     ``wanted_out`` (the outputs whose sensitivities are requested) count nothing."""
     from casadi_gb300 import calculus as C
     nz = sum(tape.nnz_in)
@@ -119,6 +120,14 @@ def structural_tangent_ops(tape, unit_dirs=True, ndir=None, wanted_out=None):
     carry = {op: _carries(op) for op in set(ops)}
     need = _needed(tape, wanted_out)
     mix = _mix()
+    const, scaled = {}, set()
+    for k, op in enumerate(ops):
+        if op == C.OP_MUL:
+            v = [const[s] for s in (i1[k], i2[k]) if const.get(s) is not None]
+            if len(v) == 1 and v[0] != 1.0 and np.frexp(v[0])[0] == 0.5:
+                scaled.add(k)
+        if op != C.OP_OUTPUT:
+            const[i0[k]] = float(tape.d[k]) if op == C.OP_CONST else None
     for d in range(nz if unit_dirs else 1):
         act = [False] * max(1, tape.sz_w)
         for k, op in enumerate(ops):
@@ -138,7 +147,7 @@ def structural_tangent_ops(tape, unit_dirs=True, ndir=None, wanted_out=None):
                 continue
             if op in (C.OP_ADD, C.OP_SUB):
                 mix["dadd"] += 1 if (cb and cc) else 0
-            elif op in (C.OP_TWICE, C.OP_NEG, C.OP_ASSIGN, C.OP_IF_ELSE_ZERO):
+            elif op in (C.OP_TWICE, C.OP_NEG, C.OP_ASSIGN, C.OP_IF_ELSE_ZERO) or k in scaled:
                 pass
             else:
                 mix["dmul"] += 1
