@@ -48,7 +48,7 @@ struct BatchHost {
   int residence = -1;
   int forced = 0;  // 0 tune, 1 global memory, 2 shared memory
   int grid_gw = 1;
-  bool by_teams = false, adjoints = false;
+  bool by_teams = false, whole_dirs = false;  // whole_dirs: items of one direction
   size_t smem_value_team = 0, smem_dir_team = 0;
   int n_dir_units = 0;     // the last units: directions of split items
   unsigned char* d_gw = nullptr;
@@ -106,7 +106,7 @@ int batch_prepare(BatchHost& b) {
   // the batch by teams: every item whole, its level schedules there
   bool team_ok = true;
   int team_slots = 1, dir_slots = 1;
-  bool adjoints = false;  // of items that are not split
+  bool whole_dirs = false;  // items of one direction, which are not split
   b.pre.clear();
   b.szw = 1;
   b.pmax = 0;
@@ -202,7 +202,7 @@ int batch_prepare(BatchHost& b) {
       for (long long tile = 0; tile < tiles; ++tile)
         units.push_back({cost, make_int4(static_cast<int>(k), static_cast<int>(tile), -1, 0)});
       if (it.ndir > 0) b.pmax = std::max(b.pmax, t->n_partials);
-      adjoints = adjoints || it.ndir > 0;
+      whole_dirs = whole_dirs || it.ndir > 0;
     }
     items.push_back(bi);
     io.insert(io.end(), it.io.begin(), it.io.end());
@@ -276,7 +276,7 @@ int batch_prepare(BatchHost& b) {
   b.smem_dir_team = smem_coop(dir_slots);
   b.by_teams = team_ok && occ < 20 &&
                std::max(b.smem_value_team, b.smem_dir_team) <= static_cast<size_t>(max_smem_optin());
-  b.adjoints = adjoints;
+  b.whole_dirs = whole_dirs;
   b.residence = b.forced == 1 ? 1 : (b.forced == 2 ? 0 : (b.by_teams ? 2 : -1));
   b.dirty = false;
   return 0;
@@ -319,8 +319,8 @@ int batch_enqueue(BatchHost& b, void* scratch, cudaStream_t s, int residence) {
       r.units = b.d_units + u0;
       r.n_units = std::min(places, whole - u0);
       e = launch_batch_team(r, BT_VALUE, 32 * kBatchTeam, b.smem_value_team, s);
-      if (e == cudaSuccess && b.adjoints)
-        e = launch_batch_team(r, BT_ADJOINT, 32 * kBatchTeam, b.smem_dir_team, s);
+      if (e == cudaSuccess && b.whole_dirs)
+        e = launch_batch_team(r, BT_WHOLE, 32 * kBatchTeam, b.smem_dir_team, s);
       if (e != cudaSuccess) return cuda_fail(e, "batch launch");
     }
     if (b.n_dir_units) {

@@ -1281,7 +1281,7 @@ cudaError_t launch_batch_team(const BatchArgs& b, BatchTeamKind kind, int thread
     if (e != cudaSuccess) return e;
   if (kind == BT_VALUE)
     k_batch_team<<<b.n_units, threads, smem, s>>>(b);
-  else if (kind == BT_ADJOINT)
+  else if (kind == BT_WHOLE)
     k_batch_team_dir<false><<<b.n_units, threads, smem, s>>>(b);
   else
     k_batch_team_dir<true><<<b.n_units, threads, smem, s>>>(b);

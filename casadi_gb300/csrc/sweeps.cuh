@@ -303,9 +303,10 @@ int occupancy_gw_dir(bool adjoint);  // ... of the derivative sweeps (one warp p
 cudaError_t launch_gather(long long n, long long ld, int count, const long long* src_row,
                           const double* src, double* dst, cudaStream_t s);
 constexpr int kBatchTeamSize = 1, kBatchTeam = 4 << kBatchTeamSize;  // warps of a cooperative unit
-// One launch over b.units, b.n_units: record (or value) walks, the adjoint walks that follow them
-// (both at most as many units as the scratch has places), or single directions of split items
-enum BatchTeamKind { BT_VALUE, BT_ADJOINT, BT_DIRECTION };
+// One launch over b.units, b.n_units: record (or value) walks, the one direction of items that are
+// not split after them (both at most as many units as the scratch has places), or single directions
+// of split items
+enum BatchTeamKind { BT_VALUE, BT_WHOLE, BT_DIRECTION };
 // threads: 32 * kBatchTeam; record walks of split items may have other teams (a multiple of 32)
 cudaError_t launch_batch_team(const BatchArgs& b, BatchTeamKind kind, int threads, size_t smem,
                               cudaStream_t s);

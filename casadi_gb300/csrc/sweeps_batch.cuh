@@ -170,8 +170,8 @@ __global__ void __launch_bounds__(kCoopMaxThreads)
   });
 }
 
-// SPLIT false: the adjoint of a unit k_batch_team has just recorded (same places); true: direction
-// unit.z, tangent or adjoint, of a split item.
+// SPLIT false: the one direction, tangent or adjoint, of a unit k_batch_team has just recorded (same
+// places); true: direction unit.z of a split item.
 template <bool SPLIT>
 __global__ void __launch_bounds__(32 * kBatchTeam, 4)
     k_batch_team_dir(const __grid_constant__ BatchArgs b) {
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(32 * kBatchTeam, 4)
   unsigned char* wb = smem + lane * 8;
   const bool active[1] = {il < it.n}, tok[1] = {true};
   const long long ig[1] = {il};
-  if (SPLIT && it.forward) {
+  if (it.forward) {
     const int2 se = __ldg(it.dir_team_at + dir * kBatchTeam + warp);
     tangent_walk<true, kTeamGroup, 1, 1, true>(u, it.dir_team + se.x, se.y / kTeamGroup, pt,
                                                it.t.pconsts, 0, tok, wb, io + 2 * kMaxIo,

@@ -162,3 +162,45 @@ def test_batch_residence_gives_the_same_bits(gpu_lib, mode):
             want_r, want_s = t.reverse(dargs, dseeds)
             for g, w in zip(res + asens, want_r + want_s):
                 assert same_bits(g.cpu().numpy(), w.cpu().numpy()).all()
+
+
+@pytest.mark.parametrize("others", [0, 1, 2])
+@pytest.mark.parametrize("n", [1, 33, 1000, 40000])
+def test_one_colour_jacobians_in_a_batch_of_teams(gpu_lib, n, others):
+    """A coloured Jacobian of one colour has one direction and is not split, unlike one of more
+    colours: alone and beside value, adjoint and two-colour items, on a tape whose work vector leaves
+    few warps per SM (the batch by teams) and on a narrow one, the general forward sweep's bits."""
+    wide = W.random_dag(n_in=20, n_nodes=900, n_out=5, seed=4, window=256, bounded=True)
+    narrow = W.random_dag(n_in=20, n_nodes=200, n_out=3, seed=5, window=16, bounded=True)
+    tapes = [R.CudaTape(f) for f in (wide, narrow)]
+    assert tapes[0].sz_w >= 60  # fewer than 20 one-warp CTAs of the record sweep fit an SM
+    args = [_cuda(a) for a in W.dag_inputs(n, n_in=20, seed=6)]
+    b = R.Batch()
+    queued, checks = [], []
+    for t, f in zip(tapes, (wide, narrow)):
+        color = np.full(20, -1, np.int32)
+        color[::3] = 0
+        seeds = torch.zeros((1, 20, n), dtype=torch.float64, device="cuda")
+        seeds[0, ::3] = 1.0
+        queued.append((b.add_jacobian_colored(t, args, 1, color), t, seeds))
+        if others:
+            aseeds = [_cuda(s) for s in _seeds(f, n, 1, 7)]
+            checks.append((b.add(t, args, aseeds), t, aseeds))
+        if others > 1:
+            two = np.arange(20, dtype=np.int32) % 2
+            seeds = torch.stack([_cuda(np.repeat((two == d)[:, None] * 1.0, n, 1)) for d in (0, 1)])
+            queued.append((b.add_jacobian_colored(t, args, 2, two), t, seeds))
+    for graph in (False, True, True):
+        for comp, _, _ in queued:
+            for c in comp:
+                c.fill_(float("nan"))
+        b.run(graph=graph)
+        b.status()
+        for comp, t, seeds in queued:
+            _, want = t.forward(args, [seeds])
+            for g, w in zip(comp, want):
+                assert same_bits(g.cpu().numpy(), w.cpu().numpy()).all()
+        for (res, asens), t, aseeds in checks:
+            want_r, want_s = t.reverse(args, aseeds)
+            for g, w in zip(res + asens, want_r + want_s):
+                assert same_bits(g.cpu().numpy(), w.cpu().numpy()).all()
