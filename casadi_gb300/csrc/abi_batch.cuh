@@ -80,9 +80,19 @@ BatchHost* get_batch(int id) {
   return g_batches[id].get();
 }
 
+// The items' tapes are still registered: a prepared batch (and its captured graph) points into
+// their device buffers, so a run without one of them is refused.
+int batch_tapes(const BatchHost& b) {
+  for (size_t k = 0; k < b.items.size(); ++k)
+    if (!get_tape(b.items[k].tape))
+      return fail(CASADI_GB300_ERR_ID, "batch item %zu: tape %d is gone", k, b.items[k].tape);
+  return 0;
+}
+
 // Build items, the longest-first unit list and the launch shape.
 int batch_prepare(BatchHost& b) {
   if (!b.dirty) return 0;
+  if (int rc = batch_tapes(b)) return rc;
   if (b.exec) {
     cudaGraphExecDestroy(b.exec);
     b.exec = nullptr;
@@ -113,7 +123,6 @@ int batch_prepare(BatchHost& b) {
   for (size_t k = 0; k < b.items.size(); ++k) {
     const auto& it = b.items[k];
     Tape* t = get_tape(it.tape);
-    if (!t) return fail(CASADI_GB300_ERR_ID, "batch item %zu: tape %d is gone", k, it.tape);
     BatchItem bi;
     std::memset(&bi, 0, sizeof(bi));
     bi.t = t->view();
@@ -463,6 +472,7 @@ int casadi_gb300_batch_run(int batch, void* scratch, size_t scratch_bytes, int u
   int cur = -1;
   cudaGetDevice(&cur);
   if (cur != b->device) return fail(CASADI_GB300_ERR_ARG, "batch lives on device %d", b->device);
+  if (int rc = batch_tapes(*b)) return rc;
   if (int rc = batch_prepare(*b)) return rc;
   const size_t need = static_cast<size_t>(std::max(b->grid, b->grid_gw)) * b->pmax * 32 * 8;
   if (need > 0 && (!scratch || scratch_bytes < need))

@@ -204,3 +204,30 @@ def test_one_colour_jacobians_in_a_batch_of_teams(gpu_lib, n, others):
             want_r, want_s = t.reverse(args, aseeds)
             for g, w in zip(res + asens, want_r + want_s):
                 assert same_bits(g.cpu().numpy(), w.cpu().numpy()).all()
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("nadj", [0, 1, 3])
+def test_batch_whose_tape_was_freed_is_refused(gpu_lib, nadj, graph):
+    """Whole items and split ones (three directions: recorded by a launch of their own): after the
+    tape is freed a run is refused before anything is launched, prepared or captured before or not,
+    and the batch's other results stay as they were."""
+    lib = R.load()
+    f = W.cartpole_rollout(4)
+    args = [_cuda(a) for a in W.cartpole_inputs(200, steps=4, seed=3)]
+    for prepared in (False, True):
+        t = R.CudaTape(f)
+        b = R.Batch()
+        res, _ = b.add(t, args, [_cuda(s) for s in _seeds(f, 200, nadj, 3)] if nadj else None)
+        if prepared:
+            b.run(graph=graph)
+            b.status()
+        before = [r.clone() for r in res]
+        assert lib.casadi_gb300_tape_free(t.id) == 0
+        with pytest.raises(R.CasadiGpuError, match="is gone"):
+            b.run(graph=graph)
+        torch.cuda.synchronize()
+        if prepared:
+            for g, w in zip(res, before):
+                assert same_bits(g.cpu().numpy(), w.cpu().numpy()).all()
+        t.id = None
