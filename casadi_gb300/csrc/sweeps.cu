@@ -29,6 +29,7 @@
 // flight and returns. No kernel traps.
 #include <algorithm>
 
+#include "smem_limit.cuh"
 #include "sweeps.cuh"
 
 namespace cgb {
@@ -986,6 +987,24 @@ int max_smem_optin() {
   return v;
 }
 
+// Raises a kernel's dynamic shared memory limit on the current device to the most it allows beside
+// the kernel's static shared memory (smem_limit.cuh).
+static cudaError_t raise_smem(const void* kernel) {
+  static SmemLimits limits;
+  int dev = 0;
+  if (cudaError_t e = cudaGetDevice(&dev)) return e;
+  return static_cast<cudaError_t>(limits.once(kernel, dev, [&]() -> int {
+    cudaFuncAttributes fa;
+    if (cudaError_t e = cudaFuncGetAttributes(&fa, kernel)) return e;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                max_smem_optin() - static_cast<int>(fa.sharedSizeBytes));
+  }));
+}
+template <class K>
+static cudaError_t raise_smem(K* kernel) {
+  return raise_smem(reinterpret_cast<const void*>(kernel));
+}
+
 template <class K>
 static int occ_of_k(K kernel, int block, size_t smem) {
   int n = 0;
@@ -1271,14 +1290,10 @@ cudaError_t launch_gather(long long n, long long ld, int count, const long long*
 
 cudaError_t launch_batch_team(const BatchArgs& b, BatchTeamKind kind, int threads, size_t smem,
                               cudaStream_t s) {
-  static const cudaError_t set0 = cudaFuncSetAttribute(
-      k_batch_team, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin());
-  static const cudaError_t set1 = cudaFuncSetAttribute(
-      k_batch_team_dir<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin());
-  static const cudaError_t set2 = cudaFuncSetAttribute(
-      k_batch_team_dir<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin());
-  for (cudaError_t e : {set0, set1, set2})
-    if (e != cudaSuccess) return e;
+  const cudaError_t e = kind == BT_VALUE   ? raise_smem(k_batch_team)
+                        : kind == BT_WHOLE ? raise_smem(k_batch_team_dir<false>)
+                                           : raise_smem(k_batch_team_dir<true>);
+  if (e != cudaSuccess) return e;
   if (kind == BT_VALUE)
     k_batch_team<<<b.n_units, threads, smem, s>>>(b);
   else if (kind == BT_WHOLE)
@@ -1290,14 +1305,9 @@ cudaError_t launch_batch_team(const BatchArgs& b, BatchTeamKind kind, int thread
 
 cudaError_t launch_batch(const BatchArgs& b, int grid, size_t smem, bool split, bool gw,
                          cudaStream_t s) {
-  // the attribute is raised once to the device maximum, so a captured graph never depends on
-  // a later call lowering it
-  static const cudaError_t set0 = cudaFuncSetAttribute(
-      k_batch<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin());
-  static const cudaError_t set1 = cudaFuncSetAttribute(
-      k_batch<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin());
-  if (set0 != cudaSuccess) return set0;
-  if (set1 != cudaSuccess) return set1;
+  if (!gw)
+    if (cudaError_t e = split ? raise_smem(k_batch<true, false>) : raise_smem(k_batch<false, false>))
+      return e;
   if (smem > static_cast<size_t>(max_smem_optin())) return cudaErrorInvalidValue;
   if (gw) {
     if (split)
