@@ -1008,20 +1008,18 @@ static cudaError_t raise_smem(K* kernel) {
 template <class K>
 static int occ_of_k(K kernel, int block, size_t smem) {
   int n = 0;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
+  if (raise_smem(kernel) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, block, smem) != cudaSuccess) {
+    cudaGetLastError();
     return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, block, smem) != cudaSuccess)
-    return 0;
+  }
   return n;
 }
 
 template <class K>
 static cudaError_t launch_k(K kernel, dim3 grid, int block, size_t smem, const SweepArgs& a,
                             cudaStream_t s) {
-  cudaError_t e =
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
+  if (cudaError_t e = raise_smem(kernel)) return e;
   kernel<<<grid, block, smem, s>>>(a);
   return cudaGetLastError();
 }
@@ -1332,58 +1330,33 @@ int occupancy_sp(int block, size_t smem) {
   }
 }
 
-template <class K>
-static int occ_of(K kernel, int block, size_t smem) {
-  int n = 0;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
-    return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, block, smem) != cudaSuccess)
-    return 0;
-  return n;
-}
-
 int occupancy_batch(size_t smem, bool split, bool gw) {
   if (gw)
-    return split ? occ_of(k_batch<true, true>, 32, kEntRingBytes)
-                 : occ_of(k_batch<false, true>, 32, kEntRingBytes);
-  int n = 0;
-  if (split) {
-    if (cudaFuncSetAttribute(k_batch<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             max_smem_optin()) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batch<true, false>, 32, smem) !=
-            cudaSuccess)
-      return 0;
-  } else {
-    if (cudaFuncSetAttribute(k_batch<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             max_smem_optin()) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batch<false, false>, 32, smem) !=
-            cudaSuccess)
-      return 0;
-  }
-  return n;
+    return split ? occ_of_k(k_batch<true, true>, 32, kEntRingBytes)
+                 : occ_of_k(k_batch<false, true>, 32, kEntRingBytes);
+  return split ? occ_of_k(k_batch<true, false>, 32, smem) : occ_of_k(k_batch<false, false>, 32, smem);
 }
 
 int occupancy_dense(int dir_warps, size_t smem) {
   switch (dir_warps) {
-    case 1: return occ_of(k_adjoint_tape<1>, 32, smem);
-    case 2: return occ_of(k_adjoint_tape<2>, 64, smem);
-    case 4: return occ_of(k_adjoint_tape<4>, 128, smem);
-    case 6: return occ_of(k_adjoint_tape<6>, 192, smem);
-    case 8: return occ_of(k_adjoint_tape<8>, 256, smem);
+    case 1: return occ_of_k(k_adjoint_tape<1>, 32, smem);
+    case 2: return occ_of_k(k_adjoint_tape<2>, 64, smem);
+    case 4: return occ_of_k(k_adjoint_tape<4>, 128, smem);
+    case 6: return occ_of_k(k_adjoint_tape<6>, 192, smem);
+    case 8: return occ_of_k(k_adjoint_tape<8>, 256, smem);
     default: return 0;
   }
 }
 
 int occupancy_gw_dir(bool adjoint) {
-  return adjoint ? occ_of(k_adjoint<2, 32, 1, true>, 32, 0) : occ_of(k_tangent<2, 32, 1, 1, true>, 32, 0);
+  return adjoint ? occ_of_k(k_adjoint<2, 32, 1, true>, 32, 0) : occ_of_k(k_tangent<2, 32, 1, 1, true>, 32, 0);
 }
 
 int occupancy_dir(int variant, bool adjoint, size_t smem) {
   if (adjoint) {
     switch (variant) {
 #define CGB_OCC(V, G, MB, IPT) \
-  case V: return occ_of(k_adjoint<G, MB, IPT>, 32, smem);
+  case V: return occ_of_k(k_adjoint<G, MB, IPT>, 32, smem);
       CGB_ADJ_VARIANTS(CGB_OCC)
 #undef CGB_OCC
       default: return 0;
@@ -1391,7 +1364,7 @@ int occupancy_dir(int variant, bool adjoint, size_t smem) {
   }
   switch (variant) {
 #define CGB_OCC(V, G, MB, IPT, K) \
-  case V: return occ_of(k_tangent<G, MB, IPT, K>, 32, smem);
+  case V: return occ_of_k(k_tangent<G, MB, IPT, K>, 32, smem);
     CGB_TAN_VARIANTS(CGB_OCC)
 #undef CGB_OCC
     default: return 0;
