@@ -217,6 +217,10 @@ struct Tape {
   int* d_err = nullptr;
   // launch shapes
   int primal_block = 128, primal_grid_cap = 1;
+  // occupancies that decide launches' shapes and routes, asked for once (asked for in every call, an
+  // eval of 100 instances with shared work vectors took 6.65 us of host time, not 5.83)
+  WarpOcc value_occ[2][2];  // [record][global work vector]
+  int adjoint_occ = 0;      // one-warp CTAs of the adjoint sweep per SM
   std::mutex shape_mtx;
   // derivative-sweep variant per kind (seeded/identity tangent, adjoint) and launch size class
   // (size_class of tiles x directions); tangent kinds may keep the cooperative sweep (TV_COUNT)
@@ -410,7 +414,7 @@ int sm_count() {
 }
 
 // Pick the CTA shape of the sparsity sweeps that keeps the most threads resident given the
-// shared-memory footprint.
+// shared-memory footprint; the occupancies the other sweeps' shapes follow from.
 void choose_shapes(Tape& t) {
   const int max_smem = max_smem_optin();
   const int sms = sm_count();
@@ -425,6 +429,10 @@ void choose_shapes(Tape& t) {
       t.primal_grid_cap = occ * sms;
     }
   }
+  for (bool record : {false, true})
+    for (bool global : {false, true})
+      t.value_occ[record][global] = occupancy_value(record, t.sz_w, global);
+  t.adjoint_occ = occupancy_dir(0, true, smem_lean(t.dir_sz_w, 1, 0));
 }
 
 // Shape of a derivative-sweep launch: DW warps (one direction each) per CTA on one 32-instance
@@ -1751,8 +1759,8 @@ int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStrea
     } else if (global) {
       // a work-vector block per thread: several warps per CTA in every kind
       const bool value = kind == PK_EVAL || kind == PK_RECORD;
-      const WarpShape sh = value ? shape_value(kind == PK_RECORD, t.sz_w, true,
-                                             (m + 31) / 32, sm_count())
+      const WarpShape sh = value ? shape_value(t.value_occ[kind == PK_RECORD][1], (m + 31) / 32,
+                                             sm_count())
                                  : WarpShape{std::max(1, occupancy_gw_sp()), kGwBlock};
       a.block = sh.block;
       grid = grid_for((m + a.block - 1) / a.block, sh.ctas * sm_count());
@@ -1763,7 +1771,7 @@ int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStrea
       if (value) a.wglob_stride = static_cast<long long>(std::max(1, t.sz_w)) * 256;  // per warp
     } else if (kind == PK_EVAL || kind == PK_RECORD) {
       a.block =
-          shape_value(kind == PK_RECORD, t.sz_w, false, (m + 31) / 32, sm_count()).block;
+          shape_value(t.value_occ[kind == PK_RECORD][0], (m + 31) / 32, sm_count()).block;
       a.wglob = nullptr;
       grid = grid_for((m + a.block - 1) / a.block, kMaxGrid);  // a warp per tile
     } else {
@@ -1957,8 +1965,7 @@ int run_deriv(Tape& t, SweepArgs a, long long m, const DerivReq& rq, cudaStream_
   // memory; the adjoint also for any launch of a tape whose work vector leaves an SM fewer than 20
   // one-warp CTAs (the batch's rule, batch_prepare): record and adjoint of 131072 instances of a
   // 4000-node graph with 142 live values 8.68 -> 5.49 ms
-  const bool wide = adjoint && !dir_global(t) &&
-                    occupancy_dir(0, true, smem_lean(t.dir_sz_w, 1, 0)) < 20;
+  const bool wide = adjoint && !dir_global(t) && t.adjoint_occ < 20;
   const bool coop_ok =
       (few || wide) &&
       (capturing(s) ? (adjoint ? t.rlv_state : t.tlv_state) > 0

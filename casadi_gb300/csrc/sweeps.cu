@@ -1114,33 +1114,37 @@ cudaError_t launch_sp_reverse(const SweepArgs& a, int grid, cudaStream_t s) {
   CGB_DISPATCH_BS(k_sp_reverse)
 }
 
-// The CTA shape (1, 2 or 4 independent warps of smem bytes each) that keeps the most warps
-// resident, the fewest warps per CTA on a tie. A launch whose warps are all resident with one warp
-// per CTA takes that: single warps spread over the SMs evenly (record of the rollout at 65536
-// instances 0.71 ms against 0.75 ms with two per CTA).
+// Resident CTAs per SM of 1, 2 and 4 independent warps of smem bytes each (0: does not fit).
 template <class K>
-static WarpShape warp_shape(K kernel, size_t smem, long long warps, int sms) {
+static WarpOcc warp_occ(K kernel, size_t smem) {
+  WarpOcc o;
+  for (int k = 0; k < kWarpShapes; ++k)
+    o.ctas[k] = (smem << k) <= static_cast<size_t>(max_smem_optin())
+                    ? occ_of_k(kernel, 32 << k, smem << k) : 0;
+  return o;
+}
+
+WarpOcc occupancy_value(bool record, int sz_w, bool global) {
+  const size_t smem = global ? kEntRingBytes : smem_value(sz_w);
+  if (global)
+    return record ? warp_occ(k_value<true, true>, smem) : warp_occ(k_value<false, true>, smem);
+  return record ? warp_occ(k_value<true, false>, smem) : warp_occ(k_value<false, false>, smem);
+}
+
+// The CTA shape that keeps the most warps resident, the fewest warps per CTA on a tie. A launch
+// whose warps are all resident with one warp per CTA takes that: single warps spread over the SMs
+// evenly (record of the rollout at 65536 instances 0.71 ms against 0.75 ms with two per CTA).
+WarpShape shape_value(const WarpOcc& o, long long warps, int sms) {
   WarpShape best{1, 32};
   int most = 0;
-  for (int nw = 1; nw <= kDirWarps; nw *= 2) {
-    if (nw * smem > static_cast<size_t>(max_smem_optin())) break;
-    const int occ = occ_of_k(kernel, 32 * nw, nw * smem);
-    if (occ * nw > most) {
-      most = occ * nw;
-      best = WarpShape{occ, 32 * nw};
+  for (int k = 0; k < kWarpShapes && o.ctas[k] > 0; ++k) {
+    if (o.ctas[k] << k > most) {
+      most = o.ctas[k] << k;
+      best = WarpShape{o.ctas[k], 32 << k};
     }
     if (warps <= static_cast<long long>(most) * sms) break;
   }
   return best;
-}
-
-WarpShape shape_value(bool record, int sz_w, bool global, long long warps, int sms) {
-  const size_t smem = global ? kEntRingBytes : smem_value(sz_w);
-  if (global)
-    return record ? warp_shape(k_value<true, true>, smem, warps, sms)
-                  : warp_shape(k_value<false, true>, smem, warps, sms);
-  return record ? warp_shape(k_value<true, false>, smem, warps, sms)
-                : warp_shape(k_value<false, false>, smem, warps, sms);
 }
 int occupancy_gw_sp() { return occ_of_k(k_sp_reverse<kGwBlock, true>, kGwBlock, kHeaderBytes); }
 

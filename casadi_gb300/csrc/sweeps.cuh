@@ -291,13 +291,18 @@ struct BatchArgs {
 };
 
 constexpr int kGwBlock = 128;   // threads per CTA of the global-work-vector value sweeps
-constexpr int kDirWarps = 4;     // most warps per CTA of the sweeps of independent warps
+constexpr int kWarpShapes = 3;   // CTAs of 1, 2 and 4 independent warps
+constexpr int kDirWarps = 1 << (kWarpShapes - 1);
 struct WarpShape {
   int ctas;    // resident CTAs per SM
   int block;   // threads per CTA
 };
+struct WarpOcc {
+  int ctas[kWarpShapes] = {};  // resident CTAs per SM by shape
+};
+WarpOcc occupancy_value(bool record, int sz_w, bool global);
 // Shape of a value/record launch of `warps` tiles
-WarpShape shape_value(bool record, int sz_w, bool global, long long warps, int sms);
+WarpShape shape_value(const WarpOcc& o, long long warps, int sms);
 int occupancy_gw_sp();           // ... of the sparsity sweeps
 int occupancy_gw_dir(bool adjoint);  // ... of the derivative sweeps (one warp per CTA)
 cudaError_t launch_gather(long long n, long long ld, int count, const long long* src_row,
