@@ -1397,7 +1397,10 @@ bool tan_team(Tape& t, TanPlan& p, int k) {
   std::vector<KEnt> ents(n);
   for (int d = 0; d < p.ndir; ++d) {
     if (!p.identity && d > 0) {  // general seeds: one set of streams serves every direction
-      where.insert(where.end(), where.begin(), where.begin() + (4 << k));
+      for (int w = 0; w < (4 << k); ++w) {
+        const int2 at0 = where[w];
+        where.push_back(at0);
+      }
       continue;
     }
     std::vector<TeamItem> items;

@@ -14,7 +14,7 @@ import oracle as O
 from casadi_gb300 import calculus as C
 from casadi_gb300 import sx as S
 from casadi_gb300 import workloads as W
-from casadi_gb300.runtime import CudaMap, CudaTape, CasadiGpuError
+from casadi_gb300.runtime import N_TAN_VARIANTS, CudaMap, CudaTape, CasadiGpuError
 
 from helpers import (EXACT_OPS, RTOL, assert_bitexact, assert_close, golden_list, golden_tape,
                      load_npz, magnitudes, value_bounds)
@@ -769,3 +769,22 @@ def test_windowed_tangent_gives_the_warp_sweep_bits(gpu_lib, case):
     for x, y in zip(got, want):
         assert_bitexact(x, y, "windowed tangent, " + case)
     ct.sync()
+
+
+@pytest.mark.parametrize("nfwd", [1, 2, 3, 9, 33])
+def test_general_seeds_by_teams_in_any_number_of_directions(gpu_lib, nfwd):
+    """General forward seeds by the cooperative sweep: one set of streams serves every direction, each
+    with its seeds and the sequential sweep's bits."""
+    f = W.cartpole_rollout(6)
+    n = 65
+    rng = np.random.default_rng(nfwd)
+    args = dev(W.cartpole_inputs(n, steps=6, seed=nfwd))
+    seeds = dev([rng.standard_normal((nfwd, k, n)) for k in f.tape.nnz_in])
+    got = []
+    for v in (0, N_TAN_VARIANTS - 1):
+        t = CudaTape(f)
+        t.set_variant(0, v)
+        got.append(host(t.forward(args, seeds)[1]))
+        t.sync()
+    for a, b in zip(*got):
+        assert_bitexact(a, b, "%d directions" % nfwd)
