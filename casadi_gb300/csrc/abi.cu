@@ -83,6 +83,14 @@ int reference_opcode(unsigned dop) {
   }
 }
 
+// What a tape or plan builds on first use, under its tape's lock: 0 not built, 1 built, -1
+// unavailable. Atomic: a call under capture only looks whether it is there, without the lock, and
+// what was written before the 1 has to be visible to it.
+struct BuildState : std::atomic<int> {
+  BuildState() : std::atomic<int>(0) {}
+  using std::atomic<int>::operator=;
+};
+
 // Activity plan of the tangent sweep for one seed pattern and launch shape.
 struct TanPlan {
   int ndir = 0, dw = 0, ch = 0;
@@ -99,7 +107,7 @@ struct TanPlan {
   int* d_order = nullptr;     // groups in work order, longest stream first (null: natural)
   // the cooperative sweep (dw 1): per direction, one keyed stream per warp of a 4 << k warp team
   // over the level schedule, laid out for groups of kTeamGroup
-  int team_state[kTeamDirSizes] = {};  // 0 not built, 1 built, -1 unavailable
+  BuildState team_state[kTeamDirSizes];
   uint4* d_team[kTeamDirSizes] = {};
   int2* d_team_at[kTeamDirSizes] = {};  // [direction][warp]
   ~TanPlan() {
@@ -146,7 +154,7 @@ struct AdjPlan {
   int n_zero = 0;
   // the cooperative sweep: one keyed stream per warp of a 4 << k warp team over the reverse level
   // schedule, laid out for groups of kTeamGroup
-  int team_state = 0;  // 0 not built, 1 built, -1 unavailable
+  BuildState team_state;
   uint4* d_team[kTeamDirSizes] = {};
   int2* d_team_at[kTeamDirSizes] = {};
   ~AdjPlan() {
@@ -183,20 +191,20 @@ struct Tape {
   // 2 and up cooperative level sweep (autotuned)
   std::atomic<int> primal_tuned[5][kSizeClasses];
   // level schedule of the cooperative value/record sweeps, built on first use
-  int lv_state = 0;  // 0 not built, 1 built, -1 unavailable
+  BuildState lv_state;
   // the value entries of the level schedule, one stream per warp of a 4 << k warp team
   uint4* d_team[kTeamSizes] = {};
   int2* d_team_at[kTeamSizes] = {};  // per warp: first entry, blocks
   int lv_sz_w = 0;
   // the reverse sweep's level schedule (users of each value in order), built on first use
-  int rlv_state = 0;
+  BuildState rlv_state;
   uint4* d_rteam[kTeamSizes] = {};  // the reverse sparsity sweep's streams, as d_team
   int2* d_rteam_at[kTeamSizes] = {};
   int rlv_sz_w = 0;
   std::unique_ptr<Levels> h_rlv;  // for the adjoint plans' teams
   // level schedule of the cooperative tangent sweep: fewer live slots than the record sweep's (its
   // work vector decides how many teams an SM holds), host only, built on first use
-  int tlv_state = 0;
+  BuildState tlv_state;
   std::unique_ptr<Levels> h_tlv;
   // global work vector: per-CTA blocks, grown on demand; uses on different streams are
   // ordered by gw_event
@@ -1656,7 +1664,7 @@ int coop_threads_for(long long tiles) {
 }
 bool ensure_levels(Tape& t, bool reverse = false) {
   std::lock_guard<std::mutex> lk(t.shape_mtx);
-  int& state = reverse ? t.rlv_state : t.lv_state;
+  BuildState& state = reverse ? t.rlv_state : t.lv_state;
   if (state != 0) return state > 0;
   state = -1;
   if (static_cast<unsigned>(t.n_partials) > kTeamPidxMask) return false;  // not addressed
