@@ -1,8 +1,8 @@
 // Reductions over instances (MapSum). See reduce.cuh for the two summation orders.
 //
-// The instance-order kernel gives each row to a CTA; the tree kernel runs one warp per work item
-// with coalesced loads along the instance axis (rows are instance-minor) and is bound by HBM (one
-// read of the block).
+// The instance-order sums give each row to a CTA, or, where rows are many or short, to a thread
+// (in_chains); the tree kernel runs one warp per work item with coalesced loads along the instance
+// axis (rows are instance-minor) and is bound by HBM (one read of the block).
 #include <algorithm>
 
 #include "reduce.cuh"
@@ -12,6 +12,7 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kWarpsPerCta = 8;
+constexpr int kChainThreads = 128;
 
 // ---- instance-order sums ------------------------------------------------------------------------
 // ((0 + x0) + x1) + ... rounds at every step, so the order of the additions cannot change; but
@@ -260,6 +261,29 @@ __global__ void __launch_bounds__(kOrdThreads)
   }
 }
 
+// The same sums with one thread per row running its chain of additions: 43 ns an element whatever
+// else runs (a dependent FP64 addition), a row beside the others as long as the pipe has room. For
+// many rows or few instances (in_chains).
+__global__ void __launch_bounds__(kChainThreads)
+    k_sum_instance_chain(const __grid_constant__ SumRowsArgs a, long long n) {
+  long long r = static_cast<long long>(blockIdx.x) * kChainThreads + threadIdx.x;
+  int g = 0;
+  while (g < a.count && r >= a.g[g].rows) r -= a.g[g++].rows;
+  if (g >= a.count) return;
+  const double* row = a.g[g].src + r * a.g[g].ld;
+  double acc = 0.0;
+  long long i = 0;
+  for (; i + 8 <= n; i += 8) {
+    double v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = __ldg(row + i + j);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc = __dadd_rn(acc, v[j]);
+  }
+  for (; i < n; ++i) acc = __dadd_rn(acc, __ldg(row + i));
+  a.g[g].dst[r] = acc;
+}
+
 // One level of the blocked tree: item (r, b) sums x[r][b*256 .. b*256+255] into y[r][b].
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
     k_sum_tree_level(long long rows, long long m, const double* __restrict__ src, long long ld,
@@ -371,6 +395,24 @@ cudaError_t reduce_sum(long long rows, long long n, const double* src, long long
   }
 }
 
+// Whether `rows` sums over n instances run as chains of additions, a thread per row, or as scans, a
+// CTA per row. A scan costs more the more CTAs share an SM and the longer a sum stays near zero or
+// about a power of two, a chain costs its length; with q rows per SM the scan starts where what it
+// saves on terms of one sign makes up for what it loses on terms that cancel: from 512 instances at q
+// = 1, 1024 q up to q = 16, nowhere past that. In us, chain and scan of terms of one sign (terms that
+// cancel): 21 rows, 256 instances 16, 20 (25), 1024: 50, 27 (65), 8192: 360, 56 (410); 304 rows, 2048:
+// 143, 46 (123); 608 rows, 4096: 282, 103 (405); 1000 rows, 1024: 76, 83 (205), 8192: 570, 220 (1040);
+// 2000 rows, 4096: 285, 303 (1070), 16384: 1730, 570 (3170); 4000 rows, 1024: 76, 269 (690), 16384:
+// 1630, 1090 (5980); 64000 rows, 64: 23, 1720 (1890).
+bool in_chains(long long rows, long long n) {
+  int dev = 0, sms = 1;
+  cudaGetDevice(&dev);
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
+    sms = 1;
+  const long long q = (rows + sms - 1) / sms;
+  return q > 16 || n < (q == 1 ? 512 : 1024 * q);
+}
+
 cudaError_t reduce_sum_instance_multi(const SumRows* groups, int count, long long n,
                                       cudaStream_t s) {
   // at most kMaxSumGroups groups per launch (the launch's parameter block holds them); more
@@ -385,8 +427,13 @@ cudaError_t reduce_sum_instance_multi(const SumRows* groups, int count, long lon
     }
     a.count = c;
     if (total == 0) continue;
-    const unsigned grid = static_cast<unsigned>(std::min<long long>(total, 1 << 20));
-    k_sum_instance_order<<<grid, kOrdThreads, 0, s>>>(a, total, n);
+    if (in_chains(total, n)) {
+      const long long grid = (total + kChainThreads - 1) / kChainThreads;
+      k_sum_instance_chain<<<static_cast<unsigned>(grid), kChainThreads, 0, s>>>(a, n);
+    } else {
+      const unsigned grid = static_cast<unsigned>(std::min<long long>(total, 1 << 20));
+      k_sum_instance_order<<<grid, kOrdThreads, 0, s>>>(a, total, n);
+    }
     if (cudaError_t e = cudaGetLastError()) return e;
   }
   return cudaSuccess;

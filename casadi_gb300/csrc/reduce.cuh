@@ -28,8 +28,8 @@ size_t reduce_scratch_bytes(long long rows, long long n, int order);
 // dst[r] (= or +=, see `accumulate`) the sum of row r. `scratch` as reduce_scratch_bytes.
 cudaError_t reduce_sum(long long rows, long long n, const double* src, long long ld, double* dst,
                        int order, double* scratch, cudaStream_t s);
-// Several blocks of rows summed in instance order (kOrderInstance) by one launch, one CTA per
-// row. Same bits as reduce_sum.
+// Several blocks of rows summed in instance order (kOrderInstance) by one launch, one CTA or one
+// thread per row. Same bits as reduce_sum.
 struct SumRows {
   const double* src;  // rows of n values, row r at src + r*ld
   long long ld;

@@ -287,3 +287,39 @@ def test_instance_order_sum_near_a_binade_edge(gpu_lib, level, n):
     got = host(CudaMapSum(f, n, reduce_out=[True]).eval(dev([rows])))[0]
     want = np.cumsum(np.concatenate([np.zeros((3, 1)), rows], 1), 1)[:, -1]
     assert (got.view(np.uint64) == want.view(np.uint64)).all(), (got, want)
+
+
+@pytest.mark.parametrize("per_sm", [1, 2, 16])
+@pytest.mark.parametrize("more_rows", [0, 1])
+@pytest.mark.parametrize("more", [-1, 0])
+def test_instance_order_sums_on_both_sides_of_the_chains_rule(gpu_lib, per_sm, more_rows, more):
+    """Sums run as a chain per thread below 1024 q instances for q rows per SM (512 for one) and past 16
+    rows per SM, else as a CTA's scan: at edges of the rule, in rows and in instances, the sequential
+    sum's bits (terms of one sign, cancelling ones and infinities)."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rows = per_sm * sms + more_rows
+    q = per_sm + more_rows
+    n = (512 if q == 1 else 1024 * q) + more
+    rng = np.random.default_rng(rows)
+    x = S.sym("x", rows)
+    f = S.Function("R", [x], [[x[k] for k in range(rows)]])
+    v = rng.standard_normal((rows, n))
+    v[::2] = np.abs(v[::2])
+    v[7, n // 2] = np.inf
+    got = host(CudaMapSum(f, n, reduce_out=[True]).eval(dev([v])))[0]
+    want = np.cumsum(np.concatenate([np.zeros((rows, 1)), v], 1), 1)[:, -1]
+    assert (got.view(np.uint64) == want.view(np.uint64)).all()
+
+
+def test_instance_order_sums_of_many_short_rows(gpu_lib):
+    """20000 summed outputs over a few instances: the sequential sum's bits."""
+    rng = np.random.default_rng(1)
+    x = S.sym("x", 4)
+    c = rng.uniform(0.5, 2.0, 20000)
+    f = S.Function("R", [x], [[x[k % 4] + float(c[k]) for k in range(20000)]])
+    for n in (1, 7, 8, 33):
+        v = rng.standard_normal((4, n))
+        got = host(CudaMapSum(f, n, reduce_out=[True]).eval(dev([v])))[0]
+        terms = v[np.arange(20000) % 4] + c[:, None]
+        want = np.cumsum(np.concatenate([np.zeros((20000, 1)), terms], 1), 1)[:, -1]
+        assert (got.view(np.uint64) == want.view(np.uint64)).all()
