@@ -76,11 +76,11 @@ __global__ void __launch_bounds__(32, 16) k_batch(const __grid_constant__ BatchA
     if (!kSplit || unit.z < 0) {
       // record (or value) unit
       if (it.ndir == 0) {
-        value_walk<false>(fu, it.t.ventries, it.t.n_vblocks, ring, nullptr, wb, io, io + kMaxIo, active,
+        value_walk<false, true>(fu, it.t.ventries, it.t.n_vblocks, ring, nullptr, wb, io, io + kMaxIo, active,
                           iv);
         continue;
       }
-      value_walk<true>(fu, it.t.ventries, it.t.n_vblocks, ring, pt, wb, io, io + kMaxIo, active, iv);
+      value_walk<true, true>(fu, it.t.ventries, it.t.n_vblocks, ring, pt, wb, io, io + kMaxIo, active, iv);
       if (kSplit && it.tile_partials) {
         // split item: publish the tile's partials; its directions are separate units
         __threadfence();
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kCoopMaxThreads)
   if (it.ndir == 0) {
     staged_walk(it.team + vs.x, vs.y, ring, [&](const uint4& e) {
       double* none = nullptr;
-      value_entry<false>(u, e, wb, none, io, io + kMaxIo, active, iv, pair);
+      value_entry<false, false>(u, e, wb, none, io, io + kMaxIo, active, iv, pair);
       if (e.w & kTeamMeet) __syncthreads();
     });
     return;
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(kCoopMaxThreads)
   double* const pt = batch_partials(b, it, unit, lane);
   staged_walk(it.team + vs.x, vs.y, ring, [&](const uint4& e) {
     double* p = pt + static_cast<size_t>((e.w >> kTeamPidxShift) & kTeamPidxMask) * 32;
-    value_entry<true>(u, e, wb, p, io, io + kMaxIo, active, iv, pair);
+    value_entry<true, false>(u, e, wb, p, io, io + kMaxIo, active, iv, pair);
     if (e.w & kTeamMeet) __syncthreads();
   });
 }

@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(kCoopMaxThreads) k_coop(const __grid_constant_
     staged_walk(st, se.y, ring, [&](const uint4& e) {
       double* p = RECORD ? pt + static_cast<size_t>((e.w >> kTeamPidxShift) & kTeamPidxMask) * 32
                          : nullptr;
-      value_entry<RECORD>(u, e, wb, p, a.in, a.out, active, ig, pair);
+      value_entry<RECORD, false>(u, e, wb, p, a.in, a.out, active, ig, pair);
       if (e.w & kTeamMeet) __syncthreads();
     });
     __syncthreads();  // the next tile's entries write the slots this one reads

@@ -18,8 +18,13 @@ struct PairState {
 
 // One entry. ig: the lane's instance, the range's last one for lanes past its end (which compute
 // like any other, so their values take no special path, and store nothing). pt: where the instruction's first recorded partial of this lane goes (RECORD);
-// advanced past the partials recorded (rows of 32 lanes).
-template <bool RECORD, class Units>
+// advanced past the partials recorded (rows of 32 lanes). SMALL: the operations of a few integer
+// instructions (comparisons, FMIN, FMAX, selections, SIGN, FLOOR, ...) have cases of their own instead
+// of a call. k_batch's walks, which the calls made slower than CUDA's functions inline had been (value
+// and adjoint of 262144 instances in us, inline functions, calls, cases: a graph of LT, LE and
+// IF_ELSE_ZERO 3018, 3793, 2850; of SIGN, COPYSIGN and FLOOR 2763, 3187, 2664; the 20-step rollout 6830,
+// 4980, 4958); in the sweeps of one tape the cases make the rollout 1 to 4 % slower (1591 -> 1631 us).
+template <bool RECORD, bool SMALL, class Units>
 __device__ __forceinline__ void value_entry(const Units& u, const uint4& e, unsigned char* wb, double*& pt,
                                             const IoDesc* in, const IoDesc* out, bool active,
                                             long long ig, PairState& pair) {
@@ -33,6 +38,18 @@ __device__ __forceinline__ void value_entry(const Units& u, const uint4& e, unsi
     }                                       \
     pt += 32;                               \
   }
+#define CGB_SMALL(OP)                                         \
+  case SMALL ? OP : 64u + OP: {                               \
+    const double x = CGB_X, y = is_binary(OP) ? CGB_Y : 0.0;  \
+    if constexpr (RECORD) {                                   \
+      double d0 = 0.0, d1 = 0.0;                              \
+      f = dev_fun_der(OP, x, y, d0, d1);                      \
+      if (partial_mask(OP) & 1u) CGB_REC(64u, d0)             \
+      if (partial_mask(OP) & 2u) CGB_REC(128u, d1)            \
+    } else {                                                  \
+      f = dev_fun(OP, x, y);                                  \
+    }                                                         \
+  } break;
   double f;
   switch (e.w & 63u) {
     case D_NOP: return;
@@ -94,6 +111,20 @@ __device__ __forceinline__ void value_entry(const Units& u, const uint4& e, unsi
       f = d_fabs(x);
       CGB_REC(64u, d_sign(x))
     } break;
+    CGB_SMALL(D_LT)
+    CGB_SMALL(D_LE)
+    CGB_SMALL(D_EQ)
+    CGB_SMALL(D_NE)
+    CGB_SMALL(D_NOT)
+    CGB_SMALL(D_AND)
+    CGB_SMALL(D_OR)
+    CGB_SMALL(D_FLOOR)
+    CGB_SMALL(D_CEIL)
+    CGB_SMALL(D_SIGN)
+    CGB_SMALL(D_COPYSIGN)
+    CGB_SMALL(D_IF_ELSE_ZERO)
+    CGB_SMALL(D_FMIN)
+    CGB_SMALL(D_FMAX)
     default: {
       // the other operations, out of line: one copy serves every kernel
       const double x = CGB_X, y = CGB_Y;
@@ -109,6 +140,7 @@ __device__ __forceinline__ void value_entry(const Units& u, const uint4& e, unsi
     }
   }
   wreg(wb, e.x) = f;
+#undef CGB_SMALL
 #undef CGB_REC
 #undef CGB_X
 #undef CGB_Y
@@ -155,13 +187,13 @@ __device__ __forceinline__ void staged_walk(const uint4* st, int nblocks, uint4*
 }
 
 // The nblocks entry blocks of one tile by one warp.
-template <bool RECORD>
+template <bool RECORD, bool SMALL = false>
 __device__ __forceinline__ void value_walk(const PlainUnits& u, const uint4* st, int nblocks, uint4* ring, double* pt,
                                            unsigned char* wb, const IoDesc* in,
                                            const IoDesc* out, bool active, long long ig) {
   PairState pair;
   staged_walk(st, nblocks, ring, [&](const uint4& e) {
-    value_entry<RECORD>(u, e, wb, pt, in, out, active, ig, pair);
+    value_entry<RECORD, SMALL>(u, e, wb, pt, in, out, active, ig, pair);
   });
 }
 

@@ -231,3 +231,34 @@ def test_batch_whose_tape_was_freed_is_refused(gpu_lib, nadj, graph):
             for g, w in zip(res, before):
                 assert same_bits(g.cpu().numpy(), w.cpu().numpy()).all()
         t.id = None
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_small_operations_in_a_persistent_batch(gpu_lib, mode):
+    """Comparisons, logic, minima, selections, signs and rounding have cases of their own in the
+    persistent batch: values and adjoints on zeros, infinities, NaN and ordinary arguments, the bits of
+    the sweeps of one tape (which call them)."""
+    from casadi_gb300 import calculus as C
+    from casadi_gb300 import sx as S
+    rng = np.random.default_rng(2)
+    v = np.concatenate([[0.0, -0.0, np.inf, -np.inf, np.nan, 1.0, -1.0, 0.5, -2.5, 5e-324, -1e300],
+                        rng.standard_normal(6)])
+    args = [_cuda(w.ravel()[None]) for w in np.meshgrid(v, v)]
+    n = v.size ** 2
+    seed = _cuda(rng.standard_normal((1, 1, n)))
+    b = R.Batch()
+    b.set_residence(mode)
+    queued = []
+    for op in (C.OP_LT, C.OP_LE, C.OP_EQ, C.OP_NE, C.OP_NOT, C.OP_AND, C.OP_OR, C.OP_FLOOR, C.OP_CEIL,
+               C.OP_SIGN, C.OP_COPYSIGN, C.OP_IF_ELSE_ZERO, C.OP_FMIN, C.OP_FMAX):
+        two = op in C.BINARY_OPS
+        t = R.CudaTape(S.Tape([C.OP_INPUT, C.OP_INPUT, op, C.OP_OUTPUT], [0, 1, 2, 0], [0, 1, 0, 2],
+                              [0, 0, 1 if two else 0, 0], [0.0] * 4, [1, 1], [1], 3))
+        queued.append((op, t, b.add(t, args)[0], []))
+        queued.append((op, t) + tuple(b.add(t, args, [seed])))
+    b.run()
+    b.status()
+    for op, t, res, asens in queued:
+        want_r, want_s = t.reverse(args, [seed])
+        for g, w in zip(list(res) + list(asens), list(want_r) + list(want_s if asens else [])):
+            assert same_bits(g.cpu().numpy(), w.cpu().numpy()).all(), C.OP_NAMES[op]
