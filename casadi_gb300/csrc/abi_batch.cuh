@@ -113,12 +113,26 @@ int batch_prepare(BatchHost& b) {
   std::vector<std::pair<double, int4>> units, dir_units;
   std::vector<std::pair<size_t, size_t>> flag_off;  // (item, first flag) of split items
   size_t n_flags = 0;
-  // the batch by teams: every item whole, its level schedules there
-  bool team_ok = true;
+  b.szw = 1;
+  bool split = false;  // items of two or more directions
+  for (const auto& it : b.items) {
+    b.szw = std::max(b.szw, get_tape(it.tape)->sz_w);
+    split = split || it.ndir >= 2;
+  }
+  b.smem = smem_value(b.szw);
+  const int occ = b.smem <= static_cast<size_t>(max_smem_optin())
+                      ? std::max(1, occupancy_batch(b.smem, split, false))
+                      : 1;
+  // Teams where one-warp units would leave an SM fewer than 20 warps: below that the walks are
+  // bound by each warp's own latency, above it the sequential walks need no meetings. Random graphs
+  // of 4000 nodes, value and adjoint of 65536 instances, one-warp units against teams: 24 slots
+  // (23 warps per SM) 3.74 and 4.84 ms, 45 slots (17 warps) 4.27 and 3.14, 66 slots (12) 6.67 and
+  // 3.08, 142 slots (6) 7.80 and 2.73 ms. They need every item's streams: a batch that runs without
+  // them builds none (values and adjoint of the 20-step rollout: 0.40 ms to prepare, not 4.3).
+  bool team_ok = occ < 20;
   int team_slots = 1, dir_slots = 1;
   bool whole_dirs = false;  // items of one direction, which are not split
   b.pre.clear();
-  b.szw = 1;
   b.pmax = 0;
   for (size_t k = 0; k < b.items.size(); ++k) {
     const auto& it = b.items[k];
@@ -169,7 +183,6 @@ int batch_prepare(BatchHost& b) {
       team_slots = std::max(team_slots, t->lv_sz_w);
     }
     team_ok = team_ok && bi.team && (it.ndir == 0 || bi.dir_team);
-    b.szw = std::max(b.szw, t->sz_w);
     const long long tiles = (it.n + 31) / 32;
     if (it.ndir >= 2) {
       // split: one record unit per tile into the item's own partial buffer, then one unit
@@ -262,10 +275,6 @@ int batch_prepare(BatchHost& b) {
     return cuda_fail(e, "upload batch");
   if (!b.d_counter && (e = cudaMalloc(&b.d_counter, 2 * sizeof(unsigned))) != cudaSuccess)
     return cuda_fail(e, "cudaMalloc(counter)");
-  b.smem = smem_value(b.szw);
-  const int occ = b.smem <= static_cast<size_t>(max_smem_optin())
-                      ? std::max(1, occupancy_batch(b.smem, b.n_flags > 0, false))
-                      : 1;
   b.grid = std::max(1, std::min(sm_count() * occ, std::max(1, b.n_units)));
   // global-memory work vectors: residency capped by registers (and at 8 CTAs per SM, which
   // bounds the per-CTA partial scratch the caller provides)
@@ -276,14 +285,9 @@ int batch_prepare(BatchHost& b) {
   const size_t gw_bytes = static_cast<size_t>(b.grid_gw) * b.szw * 256;
   if ((e = cudaMalloc(&b.d_gw, std::max<size_t>(gw_bytes, 256))) != cudaSuccess)
     return cuda_fail(e, "cudaMalloc(batch work vectors)");
-  // Teams where one-warp units would leave an SM fewer than 20 warps: below that the walks are
-  // bound by each warp's own latency, above it the sequential walks need no meetings. Random graphs
-  // of 4000 nodes, value and adjoint of 65536 instances, one-warp units against teams: 24 slots
-  // (23 warps per SM) 3.74 and 4.84 ms, 45 slots (17 warps) 4.27 and 3.14, 66 slots (12) 6.67 and
-  // 3.08, 142 slots (6) 7.80 and 2.73 ms.
   b.smem_value_team = smem_team(team_slots, 32 * kBatchTeam, false);
   b.smem_dir_team = smem_coop(dir_slots);
-  b.by_teams = team_ok && occ < 20 &&
+  b.by_teams = team_ok &&
                std::max(b.smem_value_team, b.smem_dir_team) <= static_cast<size_t>(max_smem_optin());
   b.whole_dirs = whole_dirs;
   b.residence = b.forced == 1 ? 1 : (b.forced == 2 ? 0 : (b.by_teams ? 2 : -1));
