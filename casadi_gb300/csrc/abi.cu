@@ -1809,15 +1809,22 @@ int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStrea
   const int cls = size_class((m + 31) / 32);
   const bool few = (m + 31) / 32 <= 16ll * sm_count();
   // the cooperative sweep is a candidate for launches of few tiles (or when forced); the
-  // sparsity sweeps' version needs its schedule's work vector in shared memory
+  // sparsity sweeps' version needs its schedule's work vector in shared memory, beside the team's
+  // entry rings
   const bool want_coop = coop_kind && (few || t.residence == 3);
   bool can_coop = want_coop && (capturing(s) ? (rev ? t.rlv_state : t.lv_state) > 0
                                              : ensure_levels(t, rev));
-  if (can_coop && sp_kind)
-    can_coop = smem_team(rev ? t.rlv_sz_w : t.lv_sz_w, kCoopMaxThreads, false) <=
-               static_cast<size_t>(max_smem_optin());
+  auto coop_fits = [&](int mode) {
+    return !sp_kind || smem_team(rev ? t.rlv_sz_w : t.lv_sz_w, coop_threads(mode), false) <=
+                           static_cast<size_t>(max_smem_optin());
+  };
+  can_coop = can_coop && coop_fits(M_COOP);
+  int coop_last = M_COOP_LAST;
+  while (coop_last > M_COOP && !coop_fits(coop_last)) --coop_last;
   int coop_default = M_COOP;
-  while (coop_threads(coop_default) < coop_threads_for((m + 31) / 32)) ++coop_default;
+  while (coop_default < coop_last &&
+         coop_threads(coop_default) < coop_threads_for((m + 31) / 32))
+    ++coop_default;
   if (t.residence == 3 && coop_kind && can_coop) return run(coop_default, true);
   if (t.residence == 1 || !fits_smem(t.sz_w)) {
     if (!(coop_kind && can_coop && few && t.residence != 1)) return run(M_GLOBAL, true);
@@ -1828,7 +1835,7 @@ int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStrea
   if (fits_smem(t.sz_w)) cand[nc++] = M_SHARED;
   cand[nc++] = M_GLOBAL;
   if (coop_kind && can_coop && (few || t.residence == 3))
-    for (int c = M_COOP; c <= M_COOP_LAST; ++c) cand[nc++] = c;
+    for (int c = M_COOP; c <= coop_last; ++c) cand[nc++] = c;
   std::atomic<int>& choice = t.primal_tuned[kind][cls];
   // sp_reverse consumes its seeds and cannot be timed twice: it follows sp_forward's choice
   if (rev && choice < 0 && t.primal_tuned[PK_SP_FORWARD][cls] >= 0)
@@ -1853,7 +1860,8 @@ int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStrea
     return 0;  // every run produced the same (complete) results
   }
   const int chosen = kept_choice(t.primal_tuned[kind], cls);
-  if (chosen >= 0 && (chosen < M_COOP || can_coop) && (chosen != M_SHARED || fits_smem(t.sz_w)))
+  if (chosen >= 0 && (chosen < M_COOP || (can_coop && chosen <= coop_last)) &&
+      (chosen != M_SHARED || fits_smem(t.sz_w)))
     return run(chosen, true);
   return run(cand[0], true);
 }

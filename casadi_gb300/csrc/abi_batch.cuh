@@ -202,8 +202,7 @@ int batch_prepare(BatchHost& b) {
       // few tiles: the record sweep runs cooperatively (several warps per tile) before the
       // persistent launch instead of as one-warp record units
       const bool pre = tiles <= 4ll * sm_count() && ensure_levels(*t) &&
-                       smem_team(t->lv_sz_w, coop_threads_for((it.n + 31) / 32), false) <=
-                           static_cast<size_t>(max_smem_optin());
+                       smem_team(t->lv_sz_w, 128, false) <= static_cast<size_t>(max_smem_optin());
       if (pre) {
         b.pre.push_back({static_cast<int>(k), n_flags, tiles});
         bi.t = t->view();
@@ -256,6 +255,9 @@ int batch_prepare(BatchHost& b) {
   for (const auto& u : pre_units) ulist.push_back(u.second);
   b.n_pre_units = static_cast<int>(pre_units.size());
   b.pre_threads = coop_threads_for(pre_tiles);
+  while (b.pre_threads > 128 && smem_team(pre_slots, b.pre_threads, false) >
+                                    static_cast<size_t>(max_smem_optin()))
+    b.pre_threads /= 2;  // the team's entry rings beside the longest work vector
   b.smem_pre = smem_team(pre_slots, b.pre_threads, false);
   for (const auto& pr : b.pre) {
     const Tape* t = get_tape(b.items[pr.item].tape);

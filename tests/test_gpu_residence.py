@@ -9,6 +9,7 @@ import pytest
 
 import oracle as O
 from casadi_gb300 import runtime as R
+from casadi_gb300 import sx as S
 from casadi_gb300 import workloads as W
 
 from helpers import assert_adjoint_close, assert_bitexact, assert_close, magnitudes, value_bounds
@@ -171,3 +172,43 @@ def test_cooperative_adjoint_of_a_large_launch(gpu_lib, nodes, window):
     for x, y in zip(ct.reverse(args, seeds)[1], want):  # tuned
         assert bool((x.view(torch.int64) == y.view(torch.int64)).all())
     ct.sync()
+
+
+@pytest.mark.parametrize("slots", [838, 845, 861, 877, 893, 902])
+@pytest.mark.parametrize("n", [33, 8000])
+def test_teams_at_the_shared_memory_limit(gpu_lib, slots, n):
+    """Work vectors of the level schedules from where a team of 32 warps still fits beside its entry
+    rings (16 KB) to where one of 4 warps (2 KB) no longer does: the sparsity sweeps and a batch's
+    recorded items take the largest team that fits, with the sequential sweeps' bits."""
+    k = 2 * (slots - 69)  # the schedule may keep 64 slots more than the k/2 + 5 live ones
+    x = S.sym("x", k)
+    p = [x[i] * x[(i + 1) % k] for i in range(k)]
+    q = [p[i] + p[k - 1 - i] for i in range(k // 2)]
+    prod = q[0]
+    for v in q[1:]:
+        prod = prod * v
+    f = S.Function("w", [x], [[prod, sum(p[1:], p[0])]])
+    g = torch.Generator(device="cuda").manual_seed(slots)
+    bits = torch.randint(0, 1 << 62, (k, n), dtype=torch.int64, device="cuda", generator=g)
+    sp = []
+    for mode in (2, 3, 0):
+        t = R.CudaTape(f)
+        t.set_residence(mode)
+        out = t.sp_forward([bits])[0]
+        seeds = [out.clone()]
+        sens = [torch.zeros((k, n), dtype=torch.int64, device="cuda")]
+        t.sp_reverse(sens, seeds)
+        sp.append((out, sens[0], seeds[0]))
+        t.sync()
+    for other in sp[1:]:
+        for a, b in zip(sp[0], other):
+            assert bool((a == b).all())
+    args = [torch.rand((k, n), dtype=torch.float64, device="cuda", generator=g) * 1e-3 + 1.0]
+    aseeds = [torch.rand((2, 2, n), dtype=torch.float64, device="cuda", generator=g)]
+    b = R.Batch()
+    res, asens = b.add(t, args, aseeds)
+    b.run()
+    b.status()
+    want_r, want_s = t.reverse(args, aseeds)
+    for a, w in zip(list(res) + list(asens), list(want_r) + list(want_s)):
+        assert_bitexact(a.cpu().numpy(), w.cpu().numpy(), "batch, %d slots" % slots)
