@@ -23,6 +23,7 @@
 #include "schedule.cuh"
 #include "reduce.cuh"
 #include "serial.cuh"
+#include "size_class.cuh"
 #include "sweeps.cuh"
 
 using namespace cgb;
@@ -170,24 +171,13 @@ struct AdjPlan {
   }
 };
 
-// Launch size class of the tuner: the power of two below the number of work items (32-instance
-// tiles, times directions in the derivative sweeps). One class for everything up to 16 tiles per
-// SM kept the variant that a first call of 4 tiles chose for launches of 2000: the cart-pole step
-// at 65536 instances ran the cooperative sweep a 100-instance call had picked, 129 us against 69.
-constexpr int kSizeClasses = 32;
-int size_class(long long items) {
-  int c = 0;
-  while (c + 1 < kSizeClasses && (items >> (c + 1)) > 0) ++c;
-  return c;
-}
-
 struct Tape {
   int device = 0;
   int n_instr = 0, n_in = 0, n_out = 0, sz_w = 0, n_partials = 0, n_chunks = 0;
   int ref_sz_w = 0;  // the work-vector length the tape came with (sz_w: after scheduling)
   int residence = 0;  // work vector: 0 auto (shared memory when it fits, value sweeps tuned),
                       // 1 global memory, 2 shared memory whenever it fits
-  // per PrimalKind and launch size class (size_class of the tiles): 0 shared, 1 global,
+  // per PrimalKind and launch size class (size_class.cuh, items: tiles): 0 shared, 1 global,
   // 2 and up cooperative level sweep (autotuned)
   std::atomic<int> primal_tuned[5][kSizeClasses];
   // level schedule of the cooperative value/record sweeps, built on first use
@@ -231,7 +221,7 @@ struct Tape {
   int adjoint_occ = 0;      // one-warp CTAs of the adjoint sweep per SM
   std::mutex shape_mtx;
   // derivative-sweep variant per kind (seeded/identity tangent, adjoint) and launch size class
-  // (size_class of tiles x directions); tangent kinds may keep the cooperative sweep (TV_COUNT)
+  // (items: tiles x directions); tangent kinds may keep the cooperative sweep (TV_COUNT)
   std::atomic<int> tuned[3][kSizeClasses];
   // one thread tunes a tape at a time; others meanwhile run the untuned defaults
   std::mutex tune_mtx;
@@ -1499,22 +1489,22 @@ bool adj_team(Tape& t, AdjPlan& p) {
 // Device time of `fn` (launches on stream s): one run to load the kernel and warm the caches,
 // then the fastest of three timed ones (of one when it takes over half a millisecond; a run
 // that takes 50 us when warm takes several times that when its kernel is loaded first). With
-// `warm` false, one timed run only.
+// `warm` false, one timed run only. `best` (0: none) is the fastest candidate so far: one whose first
+// run takes a quarter longer and 3 ms more, for loading, is not run again.
 template <class F>
-int time_runs(cudaStream_t s, F fn, float* ms, bool warm = true) {
+int time_runs(cudaStream_t s, F fn, float* ms, bool warm = true, float best = 0) {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   cudaError_t e = cudaEventCreate(&e0);
   if (e == cudaSuccess) e = cudaEventCreate(&e1);
-  if (warm && e == cudaSuccess) e = fn();
-  for (int r = 0; r < (warm ? 3 : 1) && e == cudaSuccess; ++r) {
+  for (int r = warm ? -1 : 0; r < (warm ? 3 : 1) && e == cudaSuccess; ++r) {
     float t = 0;
     e = cudaEventRecord(e0, s);
     if (e == cudaSuccess) e = fn();
     if (e == cudaSuccess) e = cudaEventRecord(e1, s);
     if (e == cudaSuccess) e = cudaEventSynchronize(e1);
     if (e == cudaSuccess) e = cudaEventElapsedTime(&t, e0, e1);
-    *ms = r == 0 ? t : std::min(*ms, t);
-    if (*ms > 0.5f) break;
+    *ms = r <= 0 ? t : std::min(*ms, t);
+    if (r < 0 ? best > 0 && t > 1.25f * best + 3.0f : *ms > 0.5f) break;
   }
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
@@ -1718,16 +1708,6 @@ void reset_primal_tuning(Tape& t) {
     for (auto& c : k) c = -1;
 }
 
-// The kept choice of class c, or of the nearest tuned class (calls that cannot tune: under
-// capture, or while another thread tunes the tape); -1: none.
-int kept_choice(const std::atomic<int> (&row)[kSizeClasses], int c) {
-  for (int d = 0; d < kSizeClasses; ++d) {
-    if (c - d >= 0 && row[c - d] >= 0) return row[c - d];
-    if (c + d < kSizeClasses && row[c + d] >= 0) return row[c + d];
-  }
-  return -1;
-}
-
 int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStream_t s) {
   static const int fam[] = {F_EVAL, F_RECORD, F_SP_FORWARD, F_SP_REVERSE, F_ACTIVITY};
   static const char* what[] = {"eval launch", "record sweep launch", "sp_forward launch",
@@ -1806,8 +1786,8 @@ int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStrea
   };
   const bool coop_kind = kind == PK_EVAL || kind == PK_RECORD || sp_kind;
   const bool rev = kind == PK_SP_REVERSE;
-  const int cls = size_class((m + 31) / 32);
   const bool few = (m + 31) / 32 <= 16ll * sm_count();
+  const int cls = size_class((m + 31) / 32, few, sm_count());
   // the cooperative sweep is a candidate for launches of few tiles (or when forced); the
   // sparsity sweeps' version needs its schedule's work vector in shared memory, beside the team's
   // entry rings
@@ -1836,10 +1816,9 @@ int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStrea
   cand[nc++] = M_GLOBAL;
   if (coop_kind && can_coop && (few || t.residence == 3))
     for (int c = M_COOP; c <= coop_last; ++c) cand[nc++] = c;
-  std::atomic<int>& choice = t.primal_tuned[kind][cls];
-  // sp_reverse consumes its seeds and cannot be timed twice: it follows sp_forward's choice
-  if (rev && choice < 0 && t.primal_tuned[PK_SP_FORWARD][cls] >= 0)
-    choice = t.primal_tuned[PK_SP_FORWARD][cls].load();
+  // sp_reverse consumes its seeds and cannot be timed twice: it follows sp_forward's choices
+  auto& choices = t.primal_tuned[rev ? PK_SP_FORWARD : kind];
+  std::atomic<int>& choice = choices[cls];
   // residence is tuned like the derivative variants: every candidate timed on the first
   // call of each kind and size class (every sweep here but sp_reverse, which consumes its
   // seeds, can run twice with the same results)
@@ -1847,23 +1826,24 @@ int primal_launch(Tape& t, SweepArgs& a, long long m, PrimalKind kind, cudaStrea
   if (choice < 0 && nc > 1 && g_autotune && kind != PK_SP_REVERSE && !capturing(s) &&
       tune_lock.try_lock()) {
     float ms[2 + kTeamSizes] = {};
+    int best = 0;
     for (int c = 0; c < nc; ++c) {
       int rc = 0;
-      if (int trc = time_runs(s, [&] { rc = run(cand[c], false); return cudaSuccess; }, &ms[c]))
+      if (int trc = time_runs(s, [&] { rc = run(cand[c], false); return cudaSuccess; }, &ms[c],
+                              true, c ? ms[best] : 0))
         return trc;
       if (rc) return rc;
-    }
-    int best = 0;
-    for (int c = 1; c < nc; ++c)
       if (ms[c] < ms[best]) best = c;
+    }
     choice = cand[best];
     return 0;  // every run produced the same (complete) results
   }
-  const int chosen = kept_choice(t.primal_tuned[kind], cls);
-  if (chosen >= 0 && (chosen < M_COOP || (can_coop && chosen <= coop_last)) &&
-      (chosen != M_SHARED || fits_smem(t.sz_w)))
-    return run(chosen, true);
-  return run(cand[0], true);
+  // the class's choice, or the nearest one's (calls that cannot tune: under capture, or while
+  // another thread tunes the tape)
+  const int chosen = kept_choice(choices, cls, [&](int mode) {
+    return mode >= M_COOP ? can_coop && mode <= coop_last : mode != M_SHARED || fits_smem(t.sz_w);
+  });
+  return run(chosen >= 0 ? chosen : cand[0], true);
 }
 
 // One derivative sweep after the record sweep: ndir directions, forward (seeded or identity)
@@ -1977,8 +1957,8 @@ int run_deriv(Tape& t, SweepArgs a, long long m, const DerivReq& rq, cudaStream_
     return launch_tangent_queued(a, grid, grid < work_of(v), v, s);
   };
   const long long work = tiles * ndir;
-  const int cls = size_class(work);
   const bool few = tiles <= 16ll * sms;
+  const int cls = size_class(work, few, sms);
   const bool kept_forced = !adjoint && t.tuned[kind][cls] == TV_COUNT;  // set_variant
   // the cooperative sweeps: candidates for launches of few tiles whose level schedule fits shared
   // memory; the adjoint also for any launch of a tape whose work vector leaves an SM fewer than 20
@@ -2012,15 +1992,19 @@ int run_deriv(Tape& t, SweepArgs a, long long m, const DerivReq& rq, cudaStream_
                     wanted_out, &plan_err);
   };
   // tangent variants: the cooperative sweep by teams of 4 << k warps is kCoop (k = 0) and, past the
-  // windowed sweep's number, kTeam1 + k - 1. The streams are built for launches of at most 8 items
-  // per SM; larger ones fill the GPU with a warp per item.
+  // windowed sweep's number, kTeam1 + k - 1. The streams are built for launches of at most 16 items
+  // per SM, whose time is mostly latency. Jacobians in ms with and without them: the 20-step rollout
+  // 0.59, 0.85 at 10 items per SM, 0.76, 0.80 at 20, 1.09, 1.09 at 40; a 3000-node graph of short
+  // reach 1.04, 1.26 at 20; a 2000-node graph of long reach 0.32, 0.77 at 13, 0.47, 1.10 at 20, 0.85,
+  // 2.04 at 40, so wide tapes would gain past the line as well, at the price of scheduling every
+  // direction's streams for three team sizes on first use.
   const int kTeam1 = TV_COUNT + 2;
   auto team_of = [&](int v) { return v == kCoop ? 0 : v - kTeam1 + 1; };
   auto tan_team_ok = [&](int k) {
     if (adjoint || !coop_ok || k < 0 || k >= kTeamDirSizes) return false;
     TanPlan* tp = tan1();
     return tp && (capturing(s) ? tp->team_state[k] > 0
-                               : (cls <= size_class(8ll * sms) || kept_forced) &&
+                               : (work <= 16ll * sms || kept_forced) &&
                                      tan_team(t, *tp, k));
   };
   auto launch_coop_tan = [&](int k) -> cudaError_t {
@@ -2110,7 +2094,8 @@ int run_deriv(Tape& t, SweepArgs a, long long m, const DerivReq& rq, cudaStream_
       for (int v = 0; v < n_variants + kTeamDirSizes + (adjoint ? 0 : 1); ++v) {
         if (!usable(v)) continue;
         float ms = 0;
-        if (int rc = time_runs(s, [&] { return run_v(v); }, &ms)) return plan_err ? plan_err : rc;
+        if (int rc = time_runs(s, [&] { return run_v(v); }, &ms, true, best))
+          return plan_err ? plan_err : rc;
         if (variant < 0 || ms < best) {
           best = ms;
           variant = v;
@@ -2121,8 +2106,8 @@ int run_deriv(Tape& t, SweepArgs a, long long m, const DerivReq& rq, cudaStream_
     }
     // the nearest class's choice, else the first variant of each list: fastest on the tapes
     // measured
-    variant = kept_choice(t.tuned[kind], cls);
-    if (variant < 0 || !usable(variant)) {
+    variant = kept_choice(t.tuned[kind], cls, usable);
+    if (variant < 0) {
       variant = 0;
       while (variant < n_variants && !fits(variant)) ++variant;
     }
@@ -3063,7 +3048,7 @@ int casadi_gb300_tuned_variant(int id, int kind, int* variant) {
   if (!t) return fail(CASADI_GB300_ERR_ID, "no tape with id %d", id);
   if (kind < 0 || kind > 2 || !variant) return fail(CASADI_GB300_ERR_ARG, "bad arguments");
   // the largest launches' choice (the cooperative sweep is one variant, whatever its team)
-  const int kept = kept_choice(t->tuned[kind], kSizeClasses - 1);
+  const int kept = kept_choice(t->tuned[kind], kSizeClasses - 1, [](int) { return true; });
   *variant = kind == 2 ? std::min<int>(kept, AV_COUNT) : kept > TV_COUNT + 1 ? TV_COUNT : kept;
   return 0;
 }

@@ -394,12 +394,13 @@ CASADI_GB300_API int casadi_gb300_map_jacobian_reverse(int id, int mem, int64_t 
                            int nadj, const double* const* aseed, double* const* asens);
 
 /* Autotuning of the derivative sweeps (on by default): the first call of each kind
- * (0 seeded forward, 1 Jacobian, 2 adjoint) and launch size (powers of two of the work items:
- * 32-instance tiles times directions) on a tape times each kernel variant warm on that wave
- * (large launches: those that fill the GPU several times; small launches also try the
- * cooperative level sweep), keeps the fastest for the tape and synchronizes the stream; it is
- * skipped while the stream is being captured into a CUDA graph, where the choice of the nearest
- * tuned size runs.
+ * (0 seeded forward, 1 Jacobian, 2 adjoint) and launch size on a tape times each kernel variant
+ * warm on that wave (large launches: those that fill the GPU several times; small launches also
+ * try the cooperative level sweep), keeps the fastest for the tape and synchronizes the stream;
+ * it is skipped while the stream is being captured into a CUDA graph, where the choice of the
+ * nearest tuned size runs. Launch sizes are ten classes by work items (32-instance tiles times
+ * directions) per SM: up to 1, 2, 4, ... 64 and more with at most 16 tiles per SM, up to 64 and
+ * more with more tiles.
  * Variants differ only in speed: every variant does the same arithmetic in the same order.
  * casadi_gb300_tuned_variant reports the kept variant of the largest tuned size (-1: not tuned
  * yet). No counterpart in
