@@ -200,35 +200,23 @@ def structural_adjoint_ops(tape, seeded_out):
 SIMPLE_OPS = ("ADD", "SUB", "MUL", "SQ")
 
 
-def sincos_pairs(tape):
-    """SIN/COS pairs of one operand value (the library's rule, on the scheduled tape): per op,
-    the instructions that take the previous SIN/COS's sin/cos again ("reuse") and those whose
-    sincos a later one takes ("first")."""
+def sincos_reuse(tape):
+    """SIN/COS instructions that take the sin/cos pair the previous SIN/COS of the same operand value
+    computed (the library's rule, on the scheduled tape): op -> count."""
     from casadi_gb300 import calculus as C
     from casadi_gb300 import runtime as R
     t = R.schedule(tape)
-    ver, cache, owner = {}, None, None
-    reuse, first = {C.OP_SIN: 0, C.OP_COS: 0}, set()
+    ver, cache = {}, None
+    reuse = {C.OP_SIN: 0, C.OP_COS: 0}
     for k in range(t.n_instr):
         o = int(t.op[k])
-        if o in (C.OP_SIN, C.OP_COS):
+        if o in reuse:
             key = (int(t.i1[k]), ver.get(int(t.i1[k])))
-            if key == cache:
-                reuse[o] += 1
-                first.add(owner)
-            else:
-                cache, owner = key, k
+            reuse[o] += key == cache
+            cache = key
         if o != C.OP_OUTPUT:
             ver[int(t.i0[k])] = k
-    firsts = {C.OP_SIN: 0, C.OP_COS: 0}
-    for k in first:
-        firsts[int(t.op[k])] += 1
-    return {"reuse": reuse, "first": firsts}
-
-
-def sincos_reuse(tape):
-    """SIN/COS instructions that take the previous SIN/COS's sin/cos pair: op -> count."""
-    return sincos_pairs(tape)["reuse"]
+    return reuse
 
 
 def algorithmic_flops(tape, weights, rates, seeded_out=None, unit_dirs=True, wanted_out=None):

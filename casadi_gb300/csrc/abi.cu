@@ -1664,7 +1664,9 @@ bool ensure_levels(Tape& t, bool reverse = false) {
   // ahead finds its parallel work); a tape that keeps more than 128 live is wide by itself, and what
   // counts is that three or four teams fit (16 slots to spare): the mixed queue of random graphs (160
   // live) 16.0 -> 14.8 ms, their sparsity sweeps 753 -> 714 us at 190 slots against 400, the MPC
-  // records (50 and 124 live) 2.07 ms at 400 against 2.45 at 190.
+  // records (50 and 124 live) 2.07 ms at 400 against 2.45 at 190; nothing between 124 and 160 live has
+  // been measured. 190 and 266 are, two slots less, what an SM's 228 KB leave four and three teams of 16
+  // warps beside 8 KB of entry rings and the 1 KB kept back for a CTA: 57 and 76 KB less 9, at 256 bytes.
   const int need = t.sz_w + 16;
   const int cap = t.sz_w <= 128 ? 400
                   : need <= 190 ? 190

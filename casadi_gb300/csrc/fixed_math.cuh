@@ -14,9 +14,9 @@
 //   96-bit constant, Chebyshev interpolants of the functions with the coefficients' and products'
 //   width matched to their weight (errors below 2^-57), one rounding to double at the end. Largest
 //   error against 113-bit references over 8 million arguments a range (CUDA's function beside it, over
-//   2 million): sin and cos 0.505 ulp up to 3.2 (1.39), up to 100 (1.47) and up to 2^15, exp 0.540
-//   (0.864), log 0.533 (0.547), tanh 0.612 (1.42), just above 1/8, where the quotient takes over from
-//   the series with its smallest result; 0.57 from 0.13 on.
+//   2 million): sin and cos 0.505 ulp up to 3.2 (1.39), up to 100 (1.47) and up to 2^15, 0.544 next to
+//   multiples of pi/2, exp 0.540 (0.864), log 0.533 (0.547), tanh 0.612 (1.42), just above 1/8, where
+//   the quotient takes over from the series with its smallest result; 0.57 from 0.13 on.
 //
 // Arguments outside a routine's range (subnormals, infinities, NaN, zero numerators, quotients near
 // the ends of the exponent range, huge arguments) make it return false: what it left in the result is

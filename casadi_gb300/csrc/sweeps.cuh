@@ -7,7 +7,7 @@
 
 namespace cgb {
 
-constexpr int kChunk = 256;      // instructions per staged chunk (2 KiB), value sweeps
+constexpr int kChunk = 256;      // instructions per staged chunk (2 KiB), sparsity and activity sweeps
 constexpr int kPofsGran = 16;    // granularity of the per-chunk partial offsets
 constexpr int kLeanPB = 63;      // partials per staged chunk block (plan-free adjoint)
 // entries per software-pipelined group of the batch kernel's tangent and adjoint walks: small
@@ -325,15 +325,15 @@ constexpr int kErrBadOpcode = 2;     // an instruction with an unknown opcode wa
 
 // Shared memory a launch needs (bytes).
 size_t smem_primal(int sz_w, int block);  // sparsity and activity sweeps: ring + work vectors
-size_t smem_value(int sz_w);              // value and record sweeps: one tile's work vector
+size_t smem_value(int sz_w);              // value and record sweeps: entry ring + one tile's work vector
 size_t smem_dir(int sz_w, int dir_warps, int chunk);   // plan-free adjoint (8-byte stream)
 size_t smem_lean(int sz_w, int dir_warps, int chunk);  // lean tangent / adjoint
 int max_smem_optin();
 
 cudaError_t launch_eval(const SweepArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_record(const SweepArgs& a, int grid, cudaStream_t s);
-// Derivative sweeps: 1-D grid whose size is a multiple of the direction-group count
-// ceil(ndir / (block/32)); CTA b works on direction group b % groups.
+// Derivative sweeps: one-warp CTAs that stride over the (tile, direction group) items, or claim them
+// from a.queue, one CTA per place on the GPU.
 // Variants of the warp-independent derivative sweeps: entries per software-pipeline group,
 // a register cap that lets more one-warp CTAs reside per SM, 32-instance tiles per warp (IPT)
 // and, for the tangent sweep, directions per warp (K, walking the union stream of K
@@ -363,7 +363,7 @@ __host__ __device__ inline int win_header_words(int dirs) { return (dirs + 3 + 3
 size_t smem_tangent_win(int sz_w, int dirs, int stages, int rows, int ents);
 cudaError_t launch_tangent_win(const SweepArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_adjoint(const SweepArgs& a, int grid, int variant, cudaStream_t s);
-// The adjoint sweep without an activity plan (see k_adjoint<DW, true>).
+// The adjoint sweep without an activity plan (k_adjoint_tape<DW>).
 cudaError_t launch_adjoint_dense(const SweepArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_sp_forward(const SweepArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_sp_reverse(const SweepArgs& a, int grid, cudaStream_t s);
@@ -379,7 +379,7 @@ constexpr int kCoopMaxThreads = 1024;
 cudaError_t launch_coop(const SweepArgs& a, bool record, int grid, cudaStream_t s);
 size_t smem_team(int lv_sz_w, int threads, bool global);
 // Cooperative sparsity sweeps (forward: the value sweep's levels; reverse: the reverse
-// schedule's levels, last first); shared memory smem_coop of the schedule's work vector.
+// schedule's levels, last first); shared memory smem_team of the schedule's work vector.
 cudaError_t launch_sp_team(const SweepArgs& a, bool reverse, int grid, cudaStream_t s);
 int occupancy_sp_team(int threads, size_t smem);
 // Cooperative tangent sweep over recorded partials: one CTA per (tile, direction) item; a.dchunks

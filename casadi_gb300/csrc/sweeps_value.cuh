@@ -8,8 +8,8 @@
 // One entry per instruction (sweeps.cuh, "Value entries"): the slots as byte offsets into the
 // work vector w[slot][lane], a constant's bits in place of its operands, and the key of a
 // jump-table case that holds the operation's own loads, arithmetic and stores. A warp owns a
-// 32-instance tile and reads the entries straight from global memory (the same line for every
-// lane, cached), the next one in flight while the current one computes.
+// 32-instance tile and walks the entries from a ring in shared memory that it stages itself, a block
+// of 16 in flight while the last one is walked (stage_block).
 // ---------------------------------------------------------------------------------------------
 // The last sin/cos pair of a sweep (VK_SIN_REUSE, VK_COS_REUSE take it again).
 struct PairState {
