@@ -43,6 +43,7 @@ struct BatchHost {
   int n_units = 0;
   int szw = 1, pmax = 0, grid = 1;
   size_t smem = 0;
+  BatchForm form = BF_SHARED;  // of the shared-memory launch
   // work-vector residence: 0 shared memory, 1 global memory (grid_gw CTAs), 2 shared by a team of
   // warps, -1 not tuned yet
   int residence = -1;
@@ -120,16 +121,17 @@ int batch_prepare(BatchHost& b) {
     split = split || it.ndir >= 2;
   }
   b.smem = smem_value(b.szw);
-  const int occ = b.smem <= static_cast<size_t>(max_smem_optin())
-                      ? std::max(1, occupancy_batch(b.smem, split, false))
-                      : 1;
+  auto occ_of = [&](BatchForm form) {
+    return b.smem <= static_cast<size_t>(max_smem_optin())
+               ? std::max(1, occupancy_batch(b.smem, split, form)) : 1;
+  };
   // Teams where one-warp units would leave an SM fewer than 20 warps: below that the walks are
   // bound by each warp's own latency, above it the sequential walks need no meetings. Random graphs
   // of 4000 nodes, value and adjoint of 65536 instances, one-warp units against teams: 24 slots
-  // (23 warps per SM) 3.74 and 4.84 ms, 45 slots (17 warps) 4.27 and 3.14, 66 slots (12) 6.67 and
+  // (20 warps per SM) 3.74 and 4.84 ms, 45 slots (17 warps) 4.27 and 3.14, 66 slots (12) 6.67 and
   // 3.08, 142 slots (6) 7.80 and 2.73 ms. They need every item's streams: a batch that runs without
   // them builds none (values and adjoint of the 20-step rollout: 0.40 ms to prepare, not 4.3).
-  bool team_ok = occ < 20;
+  bool team_ok = occ_of(BF_SHARED) < 20;
   int team_slots = 1, dir_slots = 1;
   bool whole_dirs = false;  // items of one direction, which are not split
   b.pre.clear();
@@ -277,10 +279,16 @@ int batch_prepare(BatchHost& b) {
     return cuda_fail(e, "upload batch");
   if (!b.d_counter && (e = cudaMalloc(&b.d_counter, 2 * sizeof(unsigned))) != cudaSuccess)
     return cuda_fail(e, "cudaMalloc(counter)");
-  b.grid = std::max(1, std::min(sm_count() * occ, std::max(1, b.n_units)));
+  // more units at a time than one-warp CTAs of the uncapped form are resident (the directions of split
+  // items start as their records end: two directions of 40000 instances of the rollout, 8 record and 16
+  // direction units per SM, take 1.71 ms uncapped and 1.84 capped)
+  const int at_once = std::max(b.n_dir_units, b.n_units - b.n_dir_units);
+  b.form = at_once > sm_count() * occ_of(BF_SHARED) && occ_of(BF_DENSE) > occ_of(BF_SHARED)
+               ? BF_DENSE : BF_SHARED;
+  b.grid = std::max(1, std::min(sm_count() * occ_of(b.form), std::max(1, b.n_units)));
   // global-memory work vectors: residency capped by registers (and at 8 CTAs per SM, which
   // bounds the per-CTA partial scratch the caller provides)
-  const int occ_gw = std::max(1, std::min(8, occupancy_batch(kEntRingBytes, b.n_flags > 0, true)));
+  const int occ_gw = std::max(1, std::min(8, occupancy_batch(kEntRingBytes, b.n_flags > 0, BF_GLOBAL)));
   b.grid_gw = std::max(1, std::min(sm_count() * occ_gw, std::max(1, b.n_units)));
   cudaFree(b.d_gw);
   b.d_gw = nullptr;
@@ -346,7 +354,7 @@ int batch_enqueue(BatchHost& b, void* scratch, cudaStream_t s, int residence) {
     }
     return 0;
   }
-  e = launch_batch(a, gw ? b.grid_gw : b.grid, b.smem, b.n_flags > 0, gw, s);
+  e = launch_batch(a, gw ? b.grid_gw : b.grid, b.smem, b.n_flags > 0, gw ? BF_GLOBAL : b.form, s);
   if (e != cudaSuccess) return cuda_fail(e, "batch launch");
   return 0;
 }

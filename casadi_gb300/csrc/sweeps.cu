@@ -1305,23 +1305,22 @@ cudaError_t launch_batch_team(const BatchArgs& b, BatchTeamKind kind, int thread
   return cudaGetLastError();
 }
 
-cudaError_t launch_batch(const BatchArgs& b, int grid, size_t smem, bool split, bool gw,
+cudaError_t launch_batch(const BatchArgs& b, int grid, size_t smem, bool split, BatchForm form,
                          cudaStream_t s) {
-  if (!gw)
-    if (cudaError_t e = split ? raise_smem(k_batch<true, false>) : raise_smem(k_batch<false, false>))
-      return e;
   if (smem > static_cast<size_t>(max_smem_optin())) return cudaErrorInvalidValue;
-  if (gw) {
-    if (split)
-      k_batch<true, true><<<grid, 32, kEntRingBytes, s>>>(b);
-    else
-      k_batch<false, true><<<grid, 32, kEntRingBytes, s>>>(b);
-  } else if (split) {
-    k_batch<true, false><<<grid, 32, smem, s>>>(b);
-  } else {
-    k_batch<false, false><<<grid, 32, smem, s>>>(b);
+  auto go = [&](auto* kernel, size_t bytes) {
+    if (cudaError_t e = raise_smem(kernel)) return e;
+    kernel<<<grid, 32, bytes, s>>>(b);
+    return cudaGetLastError();
+  };
+  switch (form) {
+    case BF_GLOBAL:
+      return split ? go(k_batch<true, true, 16>, kEntRingBytes) : go(k_batch<false, true, 16>, kEntRingBytes);
+    case BF_DENSE:
+      return split ? go(k_batch<true, false, 28>, smem) : go(k_batch<false, false, 28>, smem);
+    default:
+      return split ? go(k_batch<true, false, 16>, smem) : go(k_batch<false, false, 16>, smem);
   }
-  return cudaGetLastError();
 }
 
 int occupancy_sp(int block, size_t smem) {
@@ -1334,11 +1333,16 @@ int occupancy_sp(int block, size_t smem) {
   }
 }
 
-int occupancy_batch(size_t smem, bool split, bool gw) {
-  if (gw)
-    return split ? occ_of_k(k_batch<true, true>, 32, kEntRingBytes)
-                 : occ_of_k(k_batch<false, true>, 32, kEntRingBytes);
-  return split ? occ_of_k(k_batch<true, false>, 32, smem) : occ_of_k(k_batch<false, false>, 32, smem);
+int occupancy_batch(size_t smem, bool split, BatchForm form) {
+  switch (form) {
+    case BF_GLOBAL:
+      return split ? occ_of_k(k_batch<true, true, 16>, 32, kEntRingBytes)
+                   : occ_of_k(k_batch<false, true, 16>, 32, kEntRingBytes);
+    case BF_DENSE:
+      return split ? occ_of_k(k_batch<true, false, 28>, 32, smem) : occ_of_k(k_batch<false, false, 28>, 32, smem);
+    default:
+      return split ? occ_of_k(k_batch<true, false, 16>, 32, smem) : occ_of_k(k_batch<false, false, 16>, 32, smem);
+  }
 }
 
 int occupancy_dense(int dir_warps, size_t smem) {

@@ -315,9 +315,12 @@ enum BatchTeamKind { BT_VALUE, BT_WHOLE, BT_DIRECTION };
 // threads: 32 * kBatchTeam; record walks of split items may have other teams (a multiple of 32)
 cudaError_t launch_batch_team(const BatchArgs& b, BatchTeamKind kind, int threads, size_t smem,
                               cudaStream_t s);
-cudaError_t launch_batch(const BatchArgs& b, int grid, size_t smem, bool split, bool gw,
+// The persistent batch: work vectors in shared memory, for few units per SM or (dense) more, or in
+// global memory (b.wglob)
+enum BatchForm { BF_SHARED, BF_DENSE, BF_GLOBAL };
+cudaError_t launch_batch(const BatchArgs& b, int grid, size_t smem, bool split, BatchForm form,
                          cudaStream_t s);
-int occupancy_batch(size_t smem, bool split, bool gw);
+int occupancy_batch(size_t smem, bool split, BatchForm form);
 
 // Error bits written to TapeView::err.
 constexpr int kErrWaitTimeout = 1;   // a bounded wait on a staged chunk ran out

@@ -48,8 +48,13 @@ cudaError_t launch_wait_probe(const unsigned* flag, unsigned* err, cudaStream_t 
 // without any run the instance that holds only the whole-unit path. GW: the work vector lives
 // in global memory (per-CTA blocks) instead of shared memory, so residency is not capped by
 // the longest tape's work vector.
-template <bool kSplit, bool GW>
-__global__ void __launch_bounds__(32, 16) k_batch(const __grid_constant__ BatchArgs b) {
+// MB 28: 72 registers, 28 CTAs to an SM, for batches of more units than the 20 per SM that are resident
+// with the 86 to 90 registers of MB 16 (5 warps to a sub-partition's 16384): those would take a second
+// wave (100000 instances of the 20-step rollout, 20.6 units per SM: values 1174 and adjoint 2832 us
+// against 742 and 1842; of a graph of sums and products 660 and 1562 against 399 and 981). Smaller
+// batches run MB 16, 1 to 4 % faster for the moves the cap costs.
+template <bool kSplit, bool GW, int MB>
+__global__ void __launch_bounds__(32, MB) k_batch(const __grid_constant__ BatchArgs b) {
   extern __shared__ __align__(128) unsigned char smem[];
   const PlainUnits fu;
   const int lane = threadIdx.x;

@@ -262,3 +262,24 @@ def test_small_operations_in_a_persistent_batch(gpu_lib, mode):
         want_r, want_s = t.reverse(args, [seed])
         for g, w in zip(list(res) + list(asens), list(want_r) + list(want_s if asens else [])):
             assert same_bits(g.cpu().numpy(), w.cpu().numpy()).all(), C.OP_NAMES[op]
+
+
+@pytest.mark.parametrize("units", [0, 1, 7 * 152 + 3])
+@pytest.mark.parametrize("nadj", [0, 1, 2])
+def test_batches_on_both_sides_of_a_full_gpu(gpu_lib, nadj, units):
+    """Batches of as many units as are resident at 20 one-warp CTAs per SM, one more and some more (the
+    form of fewer registers): the bits of the sweeps of one tape."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    f = W.cartpole_rollout(1)
+    t = R.CudaTape(f)
+    assert t.sz_w <= 30  # registers, not shared memory, decide how many CTAs are resident
+    n = 32 * ((20 * sms + units) // max(1, nadj)) - 3  # a unit per tile, or per tile and direction
+    args = [_cuda(a) for a in W.cartpole_inputs(n, steps=1, seed=units)]
+    seeds = [_cuda(s) for s in _seeds(f, n, nadj, 9)] if nadj else None
+    b = R.Batch()
+    res, asens = b.add(t, args, seeds)
+    b.run()
+    b.status()
+    want_r, want_s = t.reverse(args, seeds) if nadj else (t.eval(args), [])
+    for g, w in zip(list(res) + list(asens), list(want_r) + list(want_s)):
+        assert same_bits(g.cpu().numpy(), w.cpu().numpy()).all()
