@@ -90,6 +90,14 @@ int batch_tapes(const BatchHost& b) {
   return 0;
 }
 
+// The residence before tuning: a forced one (shared memory where the entry ring fits beside the longest
+// work vector, which the last two slots before the limit leave no room for), teams, or to be tuned.
+int batch_residence(const BatchHost& b) {
+  if (b.forced == 1) return 1;
+  if (b.forced == 2) return b.smem <= static_cast<size_t>(max_smem_optin()) ? 0 : 1;
+  return b.by_teams ? 2 : -1;
+}
+
 // Build items, the longest-first unit list and the launch shape.
 int batch_prepare(BatchHost& b) {
   if (!b.dirty) return 0;
@@ -300,7 +308,7 @@ int batch_prepare(BatchHost& b) {
   b.by_teams = team_ok &&
                std::max(b.smem_value_team, b.smem_dir_team) <= static_cast<size_t>(max_smem_optin());
   b.whole_dirs = whole_dirs;
-  b.residence = b.forced == 1 ? 1 : (b.forced == 2 ? 0 : (b.by_teams ? 2 : -1));
+  b.residence = batch_residence(b);
   b.dirty = false;
   return 0;
 }
@@ -449,7 +457,7 @@ int casadi_gb300_batch_set_residence(int batch, int mode) {
   if (!b) return fail(CASADI_GB300_ERR_ID, "no batch %d", batch);
   if (mode < 0 || mode > 2) return fail(CASADI_GB300_ERR_ARG, "residence must be 0, 1 or 2");
   b->forced = mode;
-  b->residence = mode == 1 ? 1 : (mode == 2 ? 0 : (b->by_teams ? 2 : -1));
+  b->residence = batch_residence(*b);
   if (b->exec) {
     cudaGraphExecDestroy(b->exec);
     b->exec = nullptr;

@@ -1307,7 +1307,9 @@ cudaError_t launch_batch_team(const BatchArgs& b, BatchTeamKind kind, int thread
 
 cudaError_t launch_batch(const BatchArgs& b, int grid, size_t smem, bool split, BatchForm form,
                          cudaStream_t s) {
-  if (smem > static_cast<size_t>(max_smem_optin())) return cudaErrorInvalidValue;
+  // smem: entry ring and work vector; in global memory the ring alone is the CTA's
+  if (smem - (form == BF_GLOBAL ? kEntRingBytes : 0) > static_cast<size_t>(max_smem_optin()))
+    return cudaErrorInvalidValue;
   auto go = [&](auto* kernel, size_t bytes) {
     if (cudaError_t e = raise_smem(kernel)) return e;
     kernel<<<grid, 32, bytes, s>>>(b);

@@ -283,3 +283,32 @@ def test_batches_on_both_sides_of_a_full_gpu(gpu_lib, nadj, units):
     want_r, want_s = t.reverse(args, seeds) if nadj else (t.eval(args), [])
     for g, w in zip(list(res) + list(asens), list(want_r) + list(want_s)):
         assert same_bits(g.cpu().numpy(), w.cpu().numpy()).all()
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("slots", [905, 906, 907, 908])
+def test_batch_at_the_shared_memory_limit(gpu_lib, slots, mode):
+    """Work vectors of up to 908 slots (227 KB) run in a batch whether or not the entry ring has room
+    beside them, with the bits of the sweeps of one tape."""
+    from casadi_gb300 import sx as S
+    k, n = 2 * (slots - 5), 65
+    x = S.sym("x", k)
+    p = [x[i] * x[(i + 1) % k] for i in range(k)]
+    q = [p[i] + p[k - 1 - i] for i in range(k // 2)]
+    prod = q[0]
+    for v in q[1:]:
+        prod = prod * v
+    t = R.CudaTape(S.Function("w", [x], [[prod, sum(p[1:], p[0])]]))
+    assert t.sz_w == slots
+    g = torch.Generator(device="cuda").manual_seed(slots)
+    args = [torch.rand((k, n), dtype=torch.float64, device="cuda", generator=g) * 1e-3 + 0.7]
+    seeds = [torch.rand((1, 2, n), dtype=torch.float64, device="cuda", generator=g)]
+    b = R.Batch()
+    b.set_residence(mode)
+    res, asens = b.add(t, args, seeds)
+    values, _ = b.add(t, args)
+    b.run()
+    b.status()
+    want_r, want_s = t.reverse(args, seeds)
+    for got, w in zip(list(res) + list(asens) + list(values), list(want_r) + list(want_s) + list(want_r)):
+        assert same_bits(got.cpu().numpy(), w.cpu().numpy()).all()

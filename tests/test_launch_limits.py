@@ -1,5 +1,5 @@
 """Kernels' shared memory limits: raised once per kernel and device (csrc/smem_limit.cuh, compiled
-for the host with a counting stand-in for the driver call)."""
+for the host with a counting stand-in for the CUDA call)."""
 import os
 import subprocess
 
